@@ -450,7 +450,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         }
         for (int h = 0; h < 2; ++h) {
             mbar_init(smem_u32(&sm.bar_q_full[h]), 1);
-            mbar_init(smem_u32(&sm.bar_q_empty[h]), 1);              // one arrival per item and head slot
+            mbar_init(smem_u32(&sm.bar_q_empty[h]), 1);              // one arrival per item that uses the head slot
             mbar_init(smem_u32(&sm.bar_s_full[h]), 1);
             mbar_init(smem_u32(&sm.bar_p_full[h][0]), 4);          // one arrival per softmax warp
             mbar_init(smem_u32(&sm.bar_p_full[h][1]), 4);
@@ -534,9 +534,12 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 if (!ok) break;
-                if (ic > 0) ok = warp_wait<kRelaxNs>(smem_u32(&sm.bar_q_empty[h]), (ic - 1) & 1, abort_flag, p.status, kErrQ);
-                if (!ok) break;
+                // only a slot that held a query head before is waited for, and an empty one never arrives: the issuer of an
+                // empty slot may run a whole item ahead of the other one, so that an arrival per item would complete the
+                // barrier twice before this warp looks at it, and the wait for the older phase would not end
                 if (h < hd.nslots) {
+                    if (q_loads[h] > 0) ok = warp_wait<kRelaxNs>(smem_u32(&sm.bar_q_empty[h]), (q_loads[h] - 1) & 1, abort_flag, p.status, kErrQ);
+                    if (!ok) break;
                     if (lane == 0) {
                         mbar_expect_tx(smem_u32(&sm.bar_q_full[h]), TILE_BYTES);
                         for (int x = 0; x < NBOX; ++x)
@@ -676,7 +679,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                     // an empty head slot only keeps the counts going; for a used one the head's softmax warps release the
                     // ring slots and the Q tile when they see the scores (a commit costs the issuer ~50 cycles each)
                     mbar_arrive(smem_u32(&sm.bar_empty[g % NS]));
-                    if (n == 1) mbar_arrive(smem_u32(&sm.bar_q_empty[h]));
                 }
             }
             if (active) pipe_release(&sm.pipe_lock, lane);
@@ -729,7 +731,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                             tc_commit(smem_u32(&sm.bar_s_full[h]));
                         } else {
                             mbar_arrive(smem_u32(&sm.bar_empty[gk % NS]));
-                            if (j + 2 == n) mbar_arrive(smem_u32(&sm.bar_q_empty[h]));   // the last Q.K^T of the item
                         }
                     }
                 }
