@@ -413,18 +413,10 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 const int k0 = walk.next(partial) * kTile;
                 uint32_t bits[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
                 if (partial) {
-                    const int nvis = max(0, min(min(qpos - k0 + 1, p.Nkv - k0), kTile));
 #pragma unroll
-                    for (int w = 0; w < 4; ++w) bits[w] = range_mask(0, nvis, w);
-                    const int c_first = k0 / p.C, c_last = min((k0 + kTile - 1) / p.C, p.Nc - 1);
-#pragma unroll 1
-                    for (int cc = c_first; cc <= c_last; ++cc) {
-                        if (qpos > lim[cc]) {
-                            const int lo = max(cc * p.C - k0, 0), hi = min((cc + 1) * p.C - k0, kTile);
-#pragma unroll
-                            for (int w = 0; w < 4; ++w) bits[w] &= ~range_mask(lo, hi, w);
-                        }
-                    }
+                    for (int w = 0; w < 4; ++w)
+                        bits[w] = p.c_shift >= 5 ? visible_bits_coarse(lim, k0 + 32 * w, qpos, p.Nkv, p.c_shift)
+                                                 : visible_bits(lim, k0 + 32 * w + lane, qpos - lane, p.Nkv, p.C, p.c_shift, lane);
                 }
                 TR(0);
                 ok = warp_wait(smem_u32(&sm.bar_s_full[h]), gt & 1, abort_flag, p.status, kErrSFull);

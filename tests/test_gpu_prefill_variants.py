@@ -23,3 +23,14 @@ def test_items_with_an_empty_head_slot(B, Hq, Hkv, N, D, C, SW):
     roles = orc.make_roles(B, Hkv, -(-N // C), 0.1, 0.3, seed=N)
     q, k, v = inputs(B, Hq, Hkv, N, D, seed=N + D, sigma=0.5)
     assert_close_attn(run_prefill(q, k, v, roles, C, SW), orc.prefill_attention(q, k, v, roles, C, SW))
+
+
+@pytest.mark.parametrize('C', [1, 3, 8, 24, 32, 40, 64, 96])
+def test_mask_bits_of_every_chunk_granularity(C):
+    """Row masks from transposed column bits (chunks finer than 32 keys or no power of two) and from one compare per 32 columns
+    (the others): tiles cut by the causal edge, by window and local limits and by the end of the sequence."""
+    B, Hq, Hkv, N, D = 1, 4, 2, 777, 64
+    SW = C * max(1, 150 // C)
+    roles = orc.make_roles(B, Hkv, -(-N // C), 0.1, 0.4, seed=C)
+    q, k, v = inputs(B, Hq, Hkv, N, D, seed=C, sigma=0.5)
+    assert_close_attn(run_prefill(q, k, v, roles, C, SW), orc.prefill_attention(q, k, v, roles, C, SW))
