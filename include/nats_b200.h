@@ -290,6 +290,13 @@ int nats_b200_decode_step_place(const uint8_t* d_roles, void* d_cache_k, void* d
                                 int64_t* d_size_global, int64_t* d_size_local, int32_t* d_state,
                                 int B, int Hkv, int D, int C, int SW, void* stream);
 
+/* Both in one launch: the last block of every (b,kv-head) places the chunk.  Same results as the two calls. */
+int nats_b200_decode_step(const void* d_q, const void* d_k_new, const void* d_v_new, void* d_o, const uint8_t* d_roles,
+                          void* d_cache_k, void* d_cache_v, uint8_t* d_valid, int Lcap,
+                          int64_t* d_size_global, int64_t* d_size_local, int32_t* d_state,
+                          int max_len_bound, int B, int Hq, int Hkv, int D, int C, int SW, float sm_scale,
+                          void* d_workspace, size_t workspace_bytes, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

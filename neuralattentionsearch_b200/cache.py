@@ -237,18 +237,16 @@ class NAtSChunkLayerCache:
 
     def decode_step_static(self, xq: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor, roles: torch.Tensor,
                            out: torch.Tensor, sm_scale: float | None = None, recording: bool = False) -> torch.Tensor:
-        """One decode step -- append, attention, placement if the token completes a chunk -- as launches whose parameters
+        """One decode step -- append, attention, placement if the token completes a chunk -- as one launch whose parameters
         do not change from step to step.  All tensors bf16 and contiguous: xq / out [B,Hq,1,D], k_new / v_new [B,Hkv,1,D];
         roles uint8 [B,Hkv] = role of the chunk this token completes (read on the device only if it does).  The host
         counters advance by one step.  While a graph is being recorded pass ``recording=True`` (the launches are captured, not
         run, so the host counters stay); after replaying the recorded step n times call ``note_static_steps(n)``."""
         D = xq.shape[-1]
         scale = (1.0 / math.sqrt(D)) if sm_scale is None else sm_scale
-        F_.decode_step_fwd(xq, k_new, v_new, out, self._buf_k, self._buf_v, self._buf_valid, self.size_global_kv,
-                           self.size_local_kv, self._state, self._static_bound, self.chunk_size, self.sliding_window_size,
-                           scale, self._dec_ws)
-        F_.decode_step_place(roles, self._buf_k, self._buf_v, self._buf_valid, self.size_global_kv, self.size_local_kv,
-                             self._state, self.chunk_size, self.sliding_window_size)
+        F_.decode_step(xq, k_new, v_new, out, roles, self._buf_k, self._buf_v, self._buf_valid, self.size_global_kv,
+                       self.size_local_kv, self._state, self._static_bound, self.chunk_size, self.sliding_window_size,
+                       scale, self._dec_ws)
         if not recording:
             self.note_static_steps(1)
         return out

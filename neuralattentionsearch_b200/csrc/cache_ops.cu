@@ -3,7 +3,7 @@
 // for the scans, 16-byte vectorised row copies for the data movement.
 #include <stdarg.h>
 
-#include "common.cuh"
+#include "place.cuh"
 
 namespace nats {
 
@@ -422,79 +422,13 @@ __global__ void __launch_bounds__(kCopyThreads) cache_append_kernel(const Append
 // =================================================================================================
 // decode_place: a chunk completed by decode steps goes to the ring and, unless sliding, behind the kept chunks
 // =================================================================================================
-struct PlaceParams {
-    const uint8_t* roles;                         // [BH]
-    uint8_t* ck; uint8_t* cv; uint8_t* valid;
-    long long* size_global; long long* size_local; int32_t* state;
-    int C, SW, Lcap, rowB, tail;
-    int from_state;                               // 1: static launch -- act only if state[4] + 1 == C, ring position = state[5]
-};
-
 __global__ void __launch_bounds__(kCopyThreads) decode_place_kernel(const PlaceParams p) {
-    const int bh = blockIdx.x, tid = threadIdx.x;
-    const int vpt = p.rowB >> 4, tpp = kCopyThreads / vpt;
-    const int trow = tid / vpt, tvec = (tid % vpt) << 4;
-    uint8_t* ck = p.ck + (size_t)bh * p.Lcap * p.rowB;
-    uint8_t* cv = p.cv + (size_t)bh * p.Lcap * p.rowB;
-    uint8_t* valid = p.valid + (size_t)bh * p.Lcap;
     int tail = p.tail;
     if (p.from_state) {
         if (p.state[4] + 1 != p.C) return;        // the step did not complete a chunk (uniform for the grid)
         tail = p.state[5];
     }
-    const int role = p.roles[bh];
-    const int T0 = p.state[0];
-    const long long sg = p.size_global[bh], sl = p.size_local[bh];
-    const int len = (int)(sg + sl);
-    const uint4 zero = make_uint4(0, 0, 0, 0);
-    int dst, new_len;
-    long long nsg = sg, nsl = sl;
-    if (role == NATS_ROLE_GLOBAL) { dst = (int)sg; nsg = sg + p.C; nsl = 0; }
-    else if (role == NATS_ROLE_LOCAL) { dst = len; nsl = sl + p.C; }
-    else { dst = -1; }
-    new_len = (int)(nsg + nsl);
-    if (trow < tpp) {
-        for (int i = trow; i < p.C; i += tpp) {
-            const size_t src = (size_t)(T0 + i) * p.rowB + tvec;
-            const uint4 kk = ld16(ck + src), vv = ld16(cv + src);
-            const int slot = (tail + i) % p.SW;
-            const size_t rdst = (size_t)slot * p.rowB + tvec;
-            const bool sw = role == NATS_ROLE_SLIDING;
-            st16(ck + rdst, sw ? kk : zero);
-            st16(cv + rdst, sw ? vv : zero);
-            if (tvec == 0) valid[slot] = sw ? 1 : 0;
-            if (dst >= 0 && dst != T0) {
-                const size_t mdst = (size_t)(dst + i) * p.rowB + tvec;
-                st16(ck + mdst, kk);
-                st16(cv + mdst, vv);
-            }
-        }
-    }
-    __syncthreads();   // every read of the pending chunk is done before the region behind the new length is cleared
-    if (trow < tpp) {
-        // cleared: the locals a global chunk has just dropped, [new_len, len), and the slot of the pending chunk unless the
-        // chunk stayed there; everything else behind a head's length is zero already
-        for (int d = new_len + trow; d < len; d += tpp) {
-            const size_t o = (size_t)d * p.rowB + tvec;
-            st16(ck + o, zero);
-            st16(cv + o, zero);
-            if (tvec == 0) valid[d] = 0;
-        }
-        const int end = min(T0 + p.C, p.Lcap);
-        for (int d = max(T0, new_len) + trow; d < end; d += tpp) {
-            const size_t o = (size_t)d * p.rowB + tvec;
-            st16(ck + o, zero);
-            st16(cv + o, zero);
-            if (tvec == 0) valid[d] = 0;
-        }
-        if (dst >= 0)
-            for (int i = trow; i < p.C; i += tpp)
-                if (tvec == 0) valid[dst + i] = 1;
-    }
-    if (tid == 0) {
-        p.size_global[bh] = nsg;
-        p.size_local[bh] = nsl;
-    }
+    const int new_len = place_chunk<kCopyThreads>(p, blockIdx.x, p.state[0], tail);
     publish_max_len(p.state, new_len, gridDim.x);
 }
 

@@ -10,7 +10,7 @@
 // is then small enough that the kernel is limited by HBM, not by issue slots.
 // Blocks of a (batch, kv-head) leave partial (max, sum, acc) in the workspace; the block that arrives last combines
 // them (an atomic ticket, nobody waits).  The block owning the last logical token also appends it to the cache.
-#include "common.cuh"
+#include "place.cuh"
 
 namespace nats {
 
@@ -39,11 +39,54 @@ struct DecodeParams {
     const long long* size_local;
     const int32_t* state;          // [0] = T0
     int32_t* counters;             // [B*Hkv]   (workspace)
-    float* partials;               // [B*Hkv, max_splits, nrep, D+2]   (workspace)
+    float* partials;               // [B*Hkv, max_splits (x strands), nrep, D+2]   (workspace)
     int Hq, Hkv, nrep, Lcap, SW, fill, max_splits;
     int fill_from_state;           // 1: the number of tokens in the unfinished chunk is read from state[4] (static launches)
     float scale_log2;              // sm_scale * log2(e)
+    PlaceParams place;             // STEP kernels only
 };
+
+// Ticket of a block that has left its results: true for the last of n blocks of the (batch, kv-head).
+__device__ __forceinline__ bool last_arrival(int32_t* counter, int n) {
+    __shared__ int s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const int ticket = atomicAdd(counter, 1);
+        s_last = (ticket == n - 1);
+        if (s_last) *counter = 0;
+    }
+    __syncthreads();
+    if (s_last) __threadfence();
+    return s_last;
+}
+
+// The end of a whole decode step, run by the last block of every (batch, kv-head): nobody reads that head's cache any more.
+// If the token has completed a chunk, the chunk is placed; the last head to come here advances the step counters (every
+// block of the launch has read them by then: each of them, those without a segment included, took a ticket first).
+__device__ __forceinline__ void finish_step(const DecodeParams& p, int bh, int n_heads, int T0, int fill) {
+    const PlaceParams& pl = p.place;
+    const bool complete = fill + 1 == pl.C;
+    const int tail = pl.state[5];
+    int new_len = 0;
+    if (complete) new_len = place_chunk<kDecThreads>(pl, bh, T0, tail);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (complete) atomicMax(&pl.state[1], new_len);
+        __threadfence();
+        if (atomicAdd(&pl.state[2], 1) == n_heads - 1) {
+            __threadfence();
+            pl.state[2] = 0;
+            if (complete) {
+                pl.state[0] = atomicExch(&pl.state[1], 0);
+                pl.state[4] = 0;
+                pl.state[5] = (tail + pl.C) % pl.SW;
+            } else {
+                pl.state[4] = fill + 1;
+            }
+        }
+    }
+}
 
 __device__ __forceinline__ float fast_exp2(float x) {
     float y;
@@ -78,7 +121,8 @@ __device__ __forceinline__ uint32_t pack2_bf16(float lo, float hi) {
     return r;
 }
 
-template <int D>
+// STEP: the placement of a completed chunk and the step counters in the same launch (see finish_step)
+template <int D, bool STEP>
 __global__ void __launch_bounds__(kDecThreads) decode_kernel(const DecodeParams p) {
     constexpr int ROWB = D * 2;                      // bytes of a K or V row
     constexpr int CHUNKS = ROWB / 16;                // 16-byte chunks per row: 16 (D = 128) or 8 (D = 64)
@@ -86,6 +130,7 @@ __global__ void __launch_bounds__(kDecThreads) decode_kernel(const DecodeParams 
     constexpr int STAGE_BYTES = 2 * TILE_BYTES;
     constexpr int CP_PER_LANE = kTileTok * CHUNKS / 32;   // cp.async per lane for one of K / V
     constexpr int ROWS_PER_CP = 32 / CHUNKS;         // rows one warp-wide cp.async covers
+    constexpr int PSTRIDE = D + 2;                   // floats of a partial result per query head
     constexpr unsigned FULL = 0xffffffffu;
     const float NEG_INF = -INFINITY;
 
@@ -98,12 +143,12 @@ __global__ void __launch_bounds__(kDecThreads) decode_kernel(const DecodeParams 
     const int fill = p.fill_from_state ? p.state[4] : p.fill;
     const int Ltot = len + fill + 1;
     const int nsplit = (Ltot + kSeg - 1) / kSeg;
-    if (seg >= nsplit) return;
+    if (!STEP && seg >= nsplit) return;
+    if (seg < nsplit) {
     const int r0 = seg * kSeg, r1 = min(Ltot, r0 + kSeg);
 
     extern __shared__ __align__(128) uint8_t dsm[];
     __shared__ __align__(16) uint8_t s_ring_ok[kSeg];
-    __shared__ int s_last;
     // after the main loop the ring memory holds the per-warp partial results
     float (*s_acc)[kMaxRep][D] = reinterpret_cast<float (*)[kMaxRep][D]>(dsm);
     float (*s_m)[kMaxRep] = reinterpret_cast<float (*)[kMaxRep]>(dsm + kDecWarps * kMaxRep * D * 4);
@@ -272,7 +317,6 @@ __global__ void __launch_bounds__(kDecThreads) decode_kernel(const DecodeParams 
             *reinterpret_cast<float2*>(&s_acc[warp][hrow][n * 8 + quad * 2]) = make_float2(oacc[n][0], oacc[n][1]);
     }
     __syncthreads();
-    constexpr int PSTRIDE = D + 2;
     float* part_out = p.partials + ((size_t)bh * p.max_splits + seg) * nrep * PSTRIDE;
     for (int idx = tid; idx < nrep * D; idx += kDecThreads) {
         const int h = idx / D, d = idx % D;
@@ -295,18 +339,12 @@ __global__ void __launch_bounds__(kDecThreads) decode_kernel(const DecodeParams 
             if (d == 0) { part_out[h * PSTRIDE + D] = mf; part_out[h * PSTRIDE + D + 1] = l; }
         }
     }
-    if (nsplit == 1) return;
-    // ---- the last block of this (batch, kv-head) combines the splits ----
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) {
-        const int ticket = atomicAdd(&p.counters[bh], 1);
-        s_last = (ticket == nsplit - 1);
     }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
+    if (!STEP && nsplit == 1) return;
+    // ---- the last block of this (batch, kv-head) combines the splits ----
+    if (!last_arrival(&p.counters[bh], STEP ? (int)gridDim.x : nsplit)) return;
     const float* parts = p.partials + (size_t)bh * p.max_splits * nrep * PSTRIDE;
+    if (nsplit > 1)
     for (int idx = tid; idx < nrep * D; idx += kDecThreads) {
         const int h = idx / D, d = idx % D;
         float mf = NEG_INF;
@@ -322,29 +360,296 @@ __global__ void __launch_bounds__(kDecThreads) decode_kernel(const DecodeParams 
         const float inv = l > 0.f ? 1.f / l : 0.f;
         p.o[((size_t)b * p.Hq + (size_t)hkv * nrep + h) * D + d] = __float2bfloat16_rn(a * inv);
     }
-    if (tid == 0) p.counters[bh] = 0;
+    if (STEP) finish_step(p, bh, gridDim.y * gridDim.z, T0, fill);
 }
 
+// =================================================================================================
+// The same step for launches that would leave most of the chip idle (few sequences, short caches)
+// =================================================================================================
+// decode_kernel gives a segment's 64 tiles to the four warps of one block, two tiles of each in flight: with fewer blocks
+// than SMs a step then lasts as long as 16 tiles one after the other.  Here every one of those warps gets a block of its own
+// (a "strand": tiles s, s + 4, ... of the segment), which issues the copies of all its (at most 16) tiles at once.  The four
+// warps of the block compute the scores of four tiles each; after one block barrier each of them walks over all tiles for
+// a quarter of the columns of O.  The arithmetic on every value is the one of decode_kernel in the same order -- the running
+// maximum, the row sum and each accumulator see the strand's tiles in sequence, strands and segments are combined in the same
+// two steps -- so that a head's output does not depend on which of the two kernels the size of the batch selects.
+// With the placement in the same launch, 192 replayed steps of 2 sequences x 8 kv-heads over ~2.9k rows and their prompt of
+// 6000 tokens take 3.95 instead of 5.43 ms.
+constexpr int kStrandTiles = kSeg / kTileTok / kDecWarps;
+constexpr int kStrandTilesPerWarp = kStrandTiles / kDecWarps;
+static_assert(kStrandTiles % kDecWarps == 0, "tiles of a strand are dealt to the warps in equal numbers");
+
 template <int D>
-static cudaError_t launch_decode(const DecodeParams& p, dim3 grid, cudaStream_t st) {
-    constexpr int smem = kDecWarps * kDecStages * 2 * kTileTok * D * 2;
-    // the opt-in to more than 48 KB of dynamic shared memory is a per-device attribute of the kernel
-    constexpr int kMaxDev = 64;
-    static bool attr_set[kMaxDev] = {};
+constexpr int strand_smem() { return kStrandTiles * (2 * kTileTok * D * 2 + 32 * 16 + kMaxRep * 4); }
+
+template <int D, bool STEP>
+__global__ void __launch_bounds__(kDecThreads) decode_strand_kernel(const DecodeParams p) {
+    constexpr int ROWB = D * 2, CHUNKS = ROWB / 16, TILE_BYTES = kTileTok * ROWB, STAGE_BYTES = 2 * TILE_BYTES;
+    constexpr int CP_PER_LANE = kTileTok * CHUNKS / 32, ROWS_PER_CP = 32 / CHUNKS;
+    constexpr int TPW = kStrandTilesPerWarp, PSTRIDE = D + 2;
+    constexpr int NP = D / 16 / kDecWarps;           // 16-column blocks of O per warp
+    constexpr unsigned FULL = 0xffffffffu;
+    const float NEG_INF = -INFINITY;
+
+    const int seg = blockIdx.x / kDecWarps, strand = blockIdx.x % kDecWarps, hkv = blockIdx.y, b = blockIdx.z;
+    const int bh = b * p.Hkv + hkv;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nrep = p.nrep;
+    const int len = (int)(p.size_global[bh] + p.size_local[bh]);
+    const int T0 = p.state[0];
+    const int fill = p.fill_from_state ? p.state[4] : p.fill;
+    const int Ltot = len + fill + 1;
+    const int nsplit = (Ltot + kSeg - 1) / kSeg;
+    if (!STEP && seg >= nsplit) return;
+    extern __shared__ __align__(128) uint8_t dsm[];
+    float* parts = p.partials + (size_t)bh * p.max_splits * kDecWarps * nrep * PSTRIDE;
+    if (seg < nsplit) {
+    const int r0 = seg * kSeg, r1 = min(Ltot, r0 + kSeg);
+
+    float4* s_score = reinterpret_cast<float4*>(dsm + kStrandTiles * STAGE_BYTES);             // [tile][lane]
+    float (*s_tmax)[kMaxRep] = reinterpret_cast<float (*)[kMaxRep]>(dsm + kStrandTiles * (STAGE_BYTES + 32 * 16));
+    __shared__ unsigned s_vmask[kStrandTiles];
+
+    const __nv_bfloat16* ck = p.ck + (size_t)bh * p.Lcap * D;
+    const __nv_bfloat16* cv = p.cv + (size_t)bh * p.Lcap * D;
+    const uint8_t* valid = p.valid + (size_t)bh * p.Lcap;
+    const __nv_bfloat16* kn = p.k_new + (size_t)bh * D;
+    const __nv_bfloat16* vn = p.v_new + (size_t)bh * D;
+
+    // the block that owns the last logical token appends it (nobody reads that cache row in this launch)
+    if (strand == 0 && r1 == Ltot && warp == 0 && lane < CHUNKS) {
+        const size_t dst = ((size_t)bh * p.Lcap + T0 + fill) * D + lane * 8;
+        st16(p.ck + dst, ld16(kn + lane * 8));
+        st16(p.cv + dst, ld16(vn + lane * 8));
+        if (lane == 0) p.valid[(size_t)bh * p.Lcap + T0 + fill] = 1;
+    }
+
+    // ---- which tokens of this warp's tiles exist and are valid, then all of their copies (one group per tile) ----
+    const uint32_t tiles = (uint32_t)__cvta_generic_to_shared(dsm);
+    unsigned vmask[TPW];
+    {
+        bool ok[TPW];
+#pragma unroll
+        for (int x = 0; x < TPW; ++x) {
+            const int i = r0 + ((x * kDecWarps + warp) * kDecWarps + strand) * kTileTok + lane;
+            ok[x] = lane < kTileTok && i < r1;
+            if (ok[x] && i < p.SW) ok[x] = valid[i] != 0;
+        }
+#pragma unroll
+        for (int x = 0; x < TPW; ++x) vmask[x] = __ballot_sync(FULL, ok[x]) & 0xffffu;
+    }
+#pragma unroll
+    for (int x = 0; x < TPW; ++x) {
+        const int t = x * kDecWarps + warp;                                   // tile of the strand
+        const int i0 = r0 + (t * kDecWarps + strand) * kTileTok;
+        if (vmask[x] != 0u) {
+            const uint32_t dst = tiles + t * STAGE_BYTES;
+            const int c = lane % CHUNKS, rsub = lane / CHUNKS;
+            // whole tile inside ring + kept tokens: logical == physical
+            const bool plain = i0 + kTileTok <= len;
+#pragma unroll
+            for (int y = 0; y < CP_PER_LANE; ++y) {
+                const int r = y * ROWS_PER_CP + rsub;
+                const int i = i0 + r;
+                const bool ok = plain || i < r1;
+                const __nv_bfloat16 *kp = ck, *vp = cv;
+                if (plain || i < len) { kp = ck + (size_t)i * D; vp = cv + (size_t)i * D; }
+                else if (i < len + fill) { const size_t ph = (size_t)(T0 + (i - len)); kp = ck + ph * D; vp = cv + ph * D; }
+                else if (ok) { kp = kn; vp = vn; }
+                const uint32_t off = r * ROWB + ((c ^ (r & 7)) << 4);
+                cp_async16(dst + off, kp + c * 8, ok);
+                cp_async16(dst + TILE_BYTES + off, vp + c * 8, ok);
+            }
+        }
+        cp_async_commit();
+    }
+    const int hrow = lane >> 2, quad = lane & 3;
+    uint32_t qa[D / 16][2];
+    {
+        const __nv_bfloat16* qrow = p.q + ((size_t)b * p.Hq + (size_t)hkv * nrep + hrow) * D;
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks) {
+            qa[ks][0] = hrow < nrep ? *reinterpret_cast<const uint32_t*>(qrow + ks * 16 + quad * 2) : 0u;
+            qa[ks][1] = hrow < nrep ? *reinterpret_cast<const uint32_t*>(qrow + ks * 16 + 8 + quad * 2) : 0u;
+        }
+    }
+    // ---- scores of this warp's tiles ----
+#pragma unroll
+    for (int x = 0; x < TPW; ++x) {
+        const int t = x * kDecWarps + warp;
+        if (x == 0) cp_async_wait<TPW - 1>();
+        else if (x == 1) cp_async_wait<TPW - 2>();
+        else if (x == 2) cp_async_wait<(TPW > 2 ? TPW - 3 : 0)>();
+        else cp_async_wait<0>();
+        __syncwarp();                                // every lane's copies of the tile are there
+        if (lane == 0) s_vmask[t] = vmask[x];
+        if (vmask[x] == 0u) continue;
+        const uint32_t sk = tiles + t * STAGE_BYTES;
+        float sc[2][4];
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+            sc[nt][0] = sc[nt][1] = sc[nt][2] = sc[nt][3] = 0.f;
+            const int r = nt * 8 + (lane & 7);
+#pragma unroll
+            for (int kp = 0; kp < D / 32; ++kp) {
+                uint32_t kb[4];
+                const int chunk = kp * 4 + (lane >> 3);
+                ldmatrix_x4(sk + r * ROWB + ((chunk ^ (r & 7)) << 4), kb);
+                mma_bf16(sc[nt], qa[2 * kp][0], 0u, qa[2 * kp][1], 0u, kb[0], kb[1]);
+                mma_bf16(sc[nt], qa[2 * kp + 1][0], 0u, qa[2 * kp + 1][1], 0u, kb[2], kb[3]);
+            }
+        }
+        float s[4];
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+                s[nt * 2 + e] = ((vmask[x] >> (nt * 8 + quad * 2 + e)) & 1u) ? sc[nt][e] * p.scale_log2 : NEG_INF;
+        float mt = fmaxf(fmaxf(s[0], s[1]), fmaxf(s[2], s[3]));
+        mt = fmaxf(mt, __shfl_xor_sync(FULL, mt, 1));
+        mt = fmaxf(mt, __shfl_xor_sync(FULL, mt, 2));
+        s_score[t * 32 + lane] = make_float4(s[0], s[1], s[2], s[3]);
+        if (quad == 0) s_tmax[t][hrow] = mt;
+    }
+    static_assert(TPW >= 2 && TPW <= 4, "wait counts above");
+    __syncthreads();
+    // ---- online softmax over the strand's tiles; this warp's columns of O += P . V ----
+    float oacc[2 * NP][4];
+#pragma unroll
+    for (int n = 0; n < 2 * NP; ++n) { oacc[n][0] = oacc[n][1] = oacc[n][2] = oacc[n][3] = 0.f; }
+    float m_run = NEG_INF, l_run = 0.f;
+    const int n_tiles = (r1 - r0 + kTileTok - 1) / kTileTok;
+    const int my_tiles = (n_tiles - strand + kDecWarps - 1) / kDecWarps;
+#pragma unroll 4
+    for (int t = 0; t < my_tiles; ++t) {
+        if (s_vmask[t] == 0u) continue;              // nothing visible in this tile (nothing was copied either)
+        const float4 s = s_score[t * 32 + lane];
+        const float m_new = fmaxf(m_run, s_tmax[t][hrow]);
+        const float mu = (m_new == NEG_INF) ? 0.f : m_new;
+        const float alpha = fast_exp2(m_run - mu);
+        const float p0 = fast_exp2(s.x - mu), p1 = fast_exp2(s.y - mu), p2 = fast_exp2(s.z - mu), p3 = fast_exp2(s.w - mu);
+        l_run = l_run * alpha + (p0 + p1) + (p2 + p3);
+        m_run = m_new;
+#pragma unroll
+        for (int n = 0; n < 2 * NP; ++n) { oacc[n][0] *= alpha; oacc[n][1] *= alpha; }
+        const uint32_t pa0 = pack2_bf16(p0, p1), pa2 = pack2_bf16(p2, p3);
+        const uint32_t sv = tiles + t * STAGE_BYTES + TILE_BYTES;
+#pragma unroll
+        for (int np = 0; np < NP; ++np) {
+            uint32_t vb[4];
+            const int r = ((lane >> 3) & 1) * 8 + (lane & 7);
+            const int chunk = (warp * NP + np) * 2 + (lane >> 4);
+            ldmatrix_x4_trans(sv + r * ROWB + ((chunk ^ (r & 7)) << 4), vb);
+            mma_bf16(oacc[2 * np], pa0, 0u, pa2, 0u, vb[0], vb[1]);
+            mma_bf16(oacc[2 * np + 1], pa0, 0u, pa2, 0u, vb[2], vb[3]);
+        }
+    }
+    l_run += __shfl_xor_sync(FULL, l_run, 1);
+    l_run += __shfl_xor_sync(FULL, l_run, 2);
+    // ---- partial result of the strand ----
+    if (hrow < nrep) {
+        float* out = parts + ((size_t)blockIdx.x * nrep + hrow) * PSTRIDE;
+#pragma unroll
+        for (int n = 0; n < 2 * NP; ++n)
+            *reinterpret_cast<float2*>(out + warp * (D / kDecWarps) + n * 8 + quad * 2) = make_float2(oacc[n][0], oacc[n][1]);
+        if (warp == 0 && quad == 0) { out[D] = m_run; out[D + 1] = l_run; }
+    }
+    }
+    const int n_strands = nsplit * kDecWarps;
+    if (!last_arrival(&p.counters[bh], STEP ? (int)gridDim.x : n_strands)) return;
+    // ---- the last block of this (batch, kv-head): strands of a segment, then segments ----
+    // weights first (they do not depend on the column): strand within its segment, segment within the head
+    float* s_wgt = reinterpret_cast<float*>(dsm);                              // [n_strands][nrep]
+    float* s_seg_m = s_wgt + n_strands * nrep;                                 // [nsplit][nrep] segment maximum, then its weight
+    float* s_seg_l = s_seg_m + nsplit * nrep;                                  // [nsplit][nrep] segment row sum
+    for (int idx = tid; idx < nsplit * nrep; idx += kDecThreads) {
+        const int sgm = idx / nrep, h = idx % nrep;
+        float mw[kDecWarps], lw[kDecWarps];
+        float mf = NEG_INF;
+#pragma unroll
+        for (int w = 0; w < kDecWarps; ++w) {
+            const float* ps = parts + ((size_t)(sgm * kDecWarps + w) * nrep + h) * PSTRIDE + D;
+            mw[w] = __ldcg(ps);
+            lw[w] = __ldcg(ps + 1);
+            mf = fmaxf(mf, mw[w]);
+        }
+        const float mu = (mf == NEG_INF) ? 0.f : mf;
+        float l = 0.f;
+#pragma unroll
+        for (int w = 0; w < kDecWarps; ++w) {
+            const float wgt = fast_exp2(mw[w] - mu);
+            s_wgt[(sgm * kDecWarps + w) * nrep + h] = wgt;
+            l = fmaf(lw[w], wgt, l);
+        }
+        s_seg_m[idx] = mf;
+        s_seg_l[idx] = l;
+    }
+    __syncthreads();
+    for (int idx = tid; idx < nrep * D; idx += kDecThreads) {
+        const int h = idx / D, d = idx % D;
+        float mf = NEG_INF;
+        for (int sgm = 0; sgm < nsplit; ++sgm) mf = fmaxf(mf, s_seg_m[sgm * nrep + h]);
+        const float mu = (mf == NEG_INF) ? 0.f : mf;
+        float a = 0.f, l = 0.f;
+#pragma unroll 2
+        for (int sgm = 0; sgm < nsplit; ++sgm) {
+            float as = 0.f;
+#pragma unroll
+            for (int w = 0; w < kDecWarps; ++w) {
+                const int st = sgm * kDecWarps + w;
+                as = fmaf(__ldcg(parts + ((size_t)st * nrep + h) * PSTRIDE + d), s_wgt[st * nrep + h], as);
+            }
+            const float wgt = fast_exp2(s_seg_m[sgm * nrep + h] - mu);
+            a = fmaf(as, wgt, a);
+            l = fmaf(s_seg_l[sgm * nrep + h], wgt, l);
+        }
+        const float inv = l > 0.f ? 1.f / l : 0.f;
+        p.o[((size_t)b * p.Hq + (size_t)hkv * nrep + h) * D + d] = __float2bfloat16_rn(a * inv);
+    }
+    if (STEP) finish_step(p, bh, gridDim.y * gridDim.z, T0, fill);
+}
+
+// Segments of a launch up to which every strand gets its own block: 4 x 74 strands are two per SM.
+#ifndef NATS_STRAND_SEGMENTS
+#define NATS_STRAND_SEGMENTS 74
+#endif
+constexpr int kStrandSegments = NATS_STRAND_SEGMENTS;
+
+// the opt-in to more than 48 KB of dynamic shared memory is a per-device attribute of a kernel
+template <class Kernel>
+static cudaError_t allow_smem(Kernel kernel, int smem, bool (&done)[64]) {
     int dev = -1;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= kMaxDev || !attr_set[dev]) {
-        e = cudaFuncSetAttribute(decode_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return e;
-        if (dev >= 0 && dev < kMaxDev) attr_set[dev] = true;
+    if (dev < 0 || dev >= 64 || !done[dev]) {
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
     }
-    decode_kernel<D><<<grid, kDecThreads, smem, st>>>(p);
+    return e;
+}
+
+template <int D, bool STEP>
+static cudaError_t launch_decode(const DecodeParams& p, dim3 grid, cudaStream_t st) {
+    cudaError_t e;
+    if ((long long)grid.x * grid.y * grid.z <= kStrandSegments) {
+        static bool done[64] = {};
+        if ((e = allow_smem(decode_strand_kernel<D, STEP>, strand_smem<D>(), done)) != cudaSuccess) return e;
+        grid.x *= kDecWarps;
+        decode_strand_kernel<D, STEP><<<grid, kDecThreads, strand_smem<D>(), st>>>(p);
+        return cudaGetLastError();
+    }
+    constexpr int smem = kDecWarps * kDecStages * 2 * kTileTok * D * 2;
+    static bool done[64] = {};
+    if ((e = allow_smem(decode_kernel<D, STEP>, smem, done)) != cudaSuccess) return e;
+    decode_kernel<D, STEP><<<grid, kDecThreads, smem, st>>>(p);
     return cudaGetLastError();
 }
 
 static size_t decode_counter_bytes(int B, int Hkv) { return align_up((size_t)B * Hkv * sizeof(int32_t), 256); }
 static int decode_max_splits(int max_len) { return cdiv(max_len + 1, kSeg); }
+// partial results kept per (batch, kv-head) and split: one, or one per strand where a launch may be of that kind (a launch has
+// at least one segment per (batch, kv-head))
+static int decode_parts_per_split(int B, int Hkv) { return (long long)B * Hkv <= kStrandSegments ? kDecWarps : 1; }
 
 }  // namespace nats
 
@@ -354,13 +659,13 @@ extern "C" __attribute__((visibility("default"))) size_t nats_b200_decode_worksp
     if (B <= 0 || Hq <= 0 || Hkv <= 0 || D <= 0 || max_len < 0 || Hq % Hkv) return 0;
     const int nrep = Hq / Hkv;
     return decode_counter_bytes(B, Hkv) +
-           (size_t)B * Hkv * decode_max_splits(max_len) * nrep * (D + 2) * sizeof(float);
+           (size_t)B * Hkv * decode_max_splits(max_len) * decode_parts_per_split(B, Hkv) * nrep * (D + 2) * sizeof(float);
 }
 
 static int decode_impl(const void* d_q, const void* d_k_new, const void* d_v_new, void* d_o,
                        void* d_cache_k, void* d_cache_v, uint8_t* d_valid, int Lcap,
                        const int64_t* d_size_global, const int64_t* d_size_local, const int32_t* d_state,
-                       int fill, int max_len_bound, int fill_from_state,
+                       int fill, int max_len_bound, int fill_from_state, const uint8_t* d_roles,
                        int B, int Hq, int Hkv, int D, int C, int SW, float sm_scale,
                        void* d_workspace, size_t workspace_bytes, void* stream) {
     NATS_CHECK_ARG(B > 0 && Hq > 0 && Hkv > 0 && Hq % Hkv == 0, "bad head counts B=%d Hq=%d Hkv=%d", B, Hq, Hkv);
@@ -390,7 +695,17 @@ static int decode_impl(const void* d_q, const void* d_k_new, const void* d_v_new
     p.max_splits = decode_max_splits(max_len);
     p.scale_log2 = sm_scale * 1.4426950408889634f;
     dim3 grid(cdiv(max_len_bound + fill + 1, kSeg), Hkv, B);
-    cudaError_t e = (D == 64) ? launch_decode<64>(p, grid, (cudaStream_t)stream) : launch_decode<128>(p, grid, (cudaStream_t)stream);
+    const bool step = d_roles != nullptr;
+    p.place = PlaceParams{};
+    if (step) {
+        p.place.roles = d_roles; p.place.ck = (uint8_t*)d_cache_k; p.place.cv = (uint8_t*)d_cache_v; p.place.valid = d_valid;
+        p.place.size_global = (long long*)d_size_global; p.place.size_local = (long long*)d_size_local;
+        p.place.state = const_cast<int32_t*>(d_state);
+        p.place.C = C; p.place.SW = SW; p.place.Lcap = Lcap; p.place.rowB = D * 2;
+    }
+    const cudaStream_t st = (cudaStream_t)stream;
+    cudaError_t e = (D == 64) ? (step ? launch_decode<64, true>(p, grid, st) : launch_decode<64, false>(p, grid, st))
+                              : (step ? launch_decode<128, true>(p, grid, st) : launch_decode<128, false>(p, grid, st));
     NATS_CHECK_CUDA(e);
     return NATS_OK;
 }
@@ -402,7 +717,7 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_decode_fwd(const
                                     int B, int Hq, int Hkv, int D, int C, int SW, float sm_scale,
                                     void* d_workspace, size_t workspace_bytes, void* stream) {
     return decode_impl(d_q, d_k_new, d_v_new, d_o, d_cache_k, d_cache_v, d_valid, Lcap, d_size_global, d_size_local, d_state,
-                       fill, max_len_bound, 0, B, Hq, Hkv, D, C, SW, sm_scale, d_workspace, workspace_bytes, stream);
+                       fill, max_len_bound, 0, nullptr, B, Hq, Hkv, D, C, SW, sm_scale, d_workspace, workspace_bytes, stream);
 }
 
 extern "C" __attribute__((visibility("default"))) int nats_b200_decode_step_fwd(const void* d_q, const void* d_k_new, const void* d_v_new, void* d_o,
@@ -412,5 +727,15 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_decode_step_fwd(
                                          void* d_workspace, size_t workspace_bytes, void* stream) {
     // the fill is read on the device: size everything for the largest one
     return decode_impl(d_q, d_k_new, d_v_new, d_o, d_cache_k, d_cache_v, d_valid, Lcap, d_size_global, d_size_local, d_state,
-                       C - 1, max_len_bound, 1, B, Hq, Hkv, D, C, SW, sm_scale, d_workspace, workspace_bytes, stream);
+                       C - 1, max_len_bound, 1, nullptr, B, Hq, Hkv, D, C, SW, sm_scale, d_workspace, workspace_bytes, stream);
+}
+
+extern "C" __attribute__((visibility("default"))) int nats_b200_decode_step(const void* d_q, const void* d_k_new, const void* d_v_new, void* d_o,
+                                         const uint8_t* d_roles, void* d_cache_k, void* d_cache_v, uint8_t* d_valid, int Lcap,
+                                         int64_t* d_size_global, int64_t* d_size_local, int32_t* d_state,
+                                         int max_len_bound, int B, int Hq, int Hkv, int D, int C, int SW, float sm_scale,
+                                         void* d_workspace, size_t workspace_bytes, void* stream) {
+    NATS_CHECK_ARG(d_roles != nullptr, "null pointer");
+    return decode_impl(d_q, d_k_new, d_v_new, d_o, d_cache_k, d_cache_v, d_valid, Lcap, d_size_global, d_size_local, d_state,
+                       C - 1, max_len_bound, 1, d_roles, B, Hq, Hkv, D, C, SW, sm_scale, d_workspace, workspace_bytes, stream);
 }

@@ -545,6 +545,18 @@ def decode_step_fwd(q: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor, o
               sliding_window, float(sm_scale), _p(workspace), workspace.numel(), _stream(q.device))
 
 
+def decode_step(q: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor, o: torch.Tensor, roles: torch.Tensor, cache_k: torch.Tensor,
+                cache_v: torch.Tensor, valid: torch.Tensor, size_global: torch.Tensor, size_local: torch.Tensor,
+                state: torch.Tensor, max_len_bound: int, chunk_size: int, sliding_window: int, sm_scale: float,
+                workspace: torch.Tensor) -> None:
+    """``decode_step_fwd`` and ``decode_step_place`` in one launch."""
+    B, Hq, _, D = q.shape
+    Hkv = k_new.shape[1]
+    _call(q.device, 'nats_b200_decode_step', _p(q), _p(k_new), _p(v_new), _p(o), _p(roles), _p(cache_k), _p(cache_v), _p(valid),
+              cache_k.shape[2], _p(size_global), _p(size_local), _p(state), max_len_bound, B, Hq, Hkv, D, chunk_size,
+              sliding_window, float(sm_scale), _p(workspace), workspace.numel(), _stream(q.device))
+
+
 def decode_step_place(roles: torch.Tensor, cache_k: torch.Tensor, cache_v: torch.Tensor, valid: torch.Tensor,
                       size_global: torch.Tensor, size_local: torch.Tensor, state: torch.Tensor, chunk_size: int,
                       sliding_window: int) -> None:
