@@ -58,13 +58,15 @@ const char* nats_b200_build_info(void);
  *   d_lim        int32 [B,Hkv,Nc]            (out)
  *   d_tile_max   int32 [B,Hkv,Nt], Nt = ceil(N/128)   (out)
  *   d_tile_min   int32 [B,Hkv,Nt]            (out)
- *   d_kept_tiles int64 [B,Hkv] or NULL       (out) number of 128x128 (q tile, kv tile) pairs the prefill computes
+ *   d_kept_tiles int64 [B,Hkv] or NULL       (out) number of 128x128 (q tile, kv tile) pairs with a visible entry (what the
+ *                prefill computes; with chunks below 128 it may gather the visible chunks of several into one)
  */
 int nats_b200_role_prep(const uint8_t* d_roles, int B, int Hkv, int N, int C, int SW,
                         int32_t* d_lim, int32_t* d_tile_max, int32_t* d_tile_min, int64_t* d_kept_tiles,
                         void* stream);
 
-/* Bytes of workspace nats_b200_prefill_fwd needs (lim + tile_max + tile_min, 256-byte aligned parts). */
+/* Bytes of workspace nats_b200_prefill_fwd wants (lim + tile_max + tile_min, 256-byte aligned parts; for chunk sizes that
+ * divide 128 also the lists of the chunks that stay visible, without which the call works but visits more tiles). */
 size_t nats_b200_prefill_workspace_bytes(int B, int Hkv, int N, int C);
 
 /* Role-masked causal flash attention of the first prefill call.

@@ -23,27 +23,30 @@ constexpr int kScanThreads = 256;
 // =================================================================================================
 // role_prep: per-chunk row limit, per-tile max/min limit, kept-tile count
 // =================================================================================================
+constexpr int kPrepThreads = 1024, kPrepWarps = kPrepThreads / 32;
+
 // Row limits of Nc chunks whose first token sits at position pos0: lim[c] = last query position that may see chunk c.
-// Next-global index by a reversed inclusive min-scan, 256 chunks at a time from the end of the sequence; the last chunk
-// counts as global.  *first_gf receives the index of the first global (or last) chunk.  All threads of the block call.
+// The index of the next global chunk (the last chunk counts as global) is a reversed inclusive min-scan, kPrepThreads chunks
+// at a time from the end of the sequence: a ballot per warp, the warps' results side by side in shared memory, one block
+// barrier per step (the buffer alternates).  *first_gf receives the index of the first global (or last) chunk.  All threads
+// of the block call; the limits are visible to the block on return.
 __device__ void scan_role_limits(const uint8_t* __restrict__ roles, int Nc, int C, int SW, int pos0,
-                                 int32_t* __restrict__ lim, int* s, int* carry, int* first_gf) {
-    const int tid = threadIdx.x;
-    if (tid == 0) *carry = Nc - 1;
-    __syncthreads();
-    for (int hi = Nc; hi > 0; hi -= kScanThreads) {
+                                 int32_t* __restrict__ lim, int (*s)[kPrepWarps], int* first_gf) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int carry = Nc - 1, buf = 0;
+    for (int hi = Nc; hi > 0; hi -= kPrepThreads, buf ^= 1) {
         const int c = hi - 1 - tid;
         const int role = (c >= 0) ? roles[c] : NATS_ROLE_LOCAL;
         const bool gf = c >= 0 && (role == NATS_ROLE_GLOBAL || c == Nc - 1);
-        s[tid] = gf ? c : kNoLimit;
+        const unsigned m = __ballot_sync(0xffffffffu, gf);
+        const int w_first = hi - 1 - warp * 32;                            // chunk of lane 0; chunks descend with the lane
+        if (lane == 0) s[buf][warp] = m ? w_first - (31 - __clz(m)) : kNoLimit;       // the warp's smallest such chunk
         __syncthreads();
-        for (int o = 1; o < kScanThreads; o <<= 1) {
-            const int v = (tid >= o) ? s[tid - o] : kNoLimit;
-            __syncthreads();
-            s[tid] = min(s[tid], v);
-            __syncthreads();
-        }
-        const int fill = min(s[tid], *carry);
+        const int all = s[buf][lane];
+        const int before = __reduce_min_sync(0xffffffffu, lane < warp ? all : kNoLimit);
+        const unsigned mine = m & (0xffffffffu >> (31 - lane));
+        int fill = min(before, carry);
+        if (mine) fill = min(fill, w_first - (31 - __clz(mine)));
         if (c >= 0) {
             long long l;
             if (role == NATS_ROLE_SLIDING) l = (long long)pos0 + (long long)c * C + SW + C - 1;
@@ -52,28 +55,41 @@ __device__ void scan_role_limits(const uint8_t* __restrict__ roles, int Nc, int 
             lim[c] = (int)min(l, (long long)kNoLimit);
             if (c == 0) *first_gf = fill;
         }
-        __syncthreads();
-        if (tid == kScanThreads - 1) *carry = fill;
-        __syncthreads();
+        carry = min(carry, __reduce_min_sync(0xffffffffu, all));
     }
+    __syncthreads();
 }
+static_assert(kPrepWarps == 32, "a warp holds one value per warp of the block");
 
 // Per 128-row KV tile: max / min of the limits of the chunks it overlaps, and how many query tiles keep it.  Query row i
-// sits at position q_off + i; there are Nt query tiles of 128 rows.  Returns this thread's share of the kept count.
+// sits at position q_off + i; there are Nt query tiles of 128 rows.  Fine chunks: a warp per tile (coalesced loads); others:
+// a thread per tile.  open_max (may be null): max over the chunks that are not visible for good.  Returns this thread's share
+// of the kept count.
 __device__ unsigned long long tile_limits(const int32_t* __restrict__ lim, int Nkv, int C, int Ntk, int q_off, int Nt,
-                                          int32_t* __restrict__ tmax, int32_t* __restrict__ tmin) {
+                                          int32_t* __restrict__ tmax, int32_t* __restrict__ tmin, int32_t* __restrict__ open_max) {
     unsigned long long mine = 0;
-    for (int kt = threadIdx.x; kt < Ntk; kt += kScanThreads) {
+    const bool wide = C < 16;
+    const int lane = threadIdx.x & 31;
+    const int first_tile = wide ? threadIdx.x >> 5 : threadIdx.x, step = wide ? kPrepWarps : kPrepThreads;
+    for (int kt = first_tile; kt < Ntk; kt += step) {
         const int c0 = (int)(((long long)kt * kTile) / C);
         const int c1 = (int)(min((long long)kt * kTile + kTile - 1, (long long)Nkv - 1) / C);
-        int mx = -1, mn = kNoLimit;
-        for (int c = c0; c <= c1; ++c) {
+        int mx = -1, mn = kNoLimit, om = -1;
+        for (int c = wide ? c0 + lane : c0; c <= c1; c += wide ? 32 : 1) {
             const int l = lim[c];
             mx = max(mx, l);
             mn = min(mn, l);
+            if (l != kNoLimit) om = max(om, l);
+        }
+        if (wide) {
+            mx = __reduce_max_sync(0xffffffffu, mx);
+            mn = __reduce_min_sync(0xffffffffu, mn);
+            om = __reduce_max_sync(0xffffffffu, om);
+            if (lane != 0) continue;
         }
         tmax[kt] = mx;
         tmin[kt] = mn;
+        if (open_max != nullptr) open_max[kt] = om;
         // query tiles t that keep the tile: last row position >= first tile row, first row position <= mx
         const long long first = (long long)kt * kTile - q_off - (kTile - 1);
         const int t_min = first <= 0 ? 0 : (int)((first + kTile - 1) / kTile);
@@ -85,23 +101,45 @@ __device__ unsigned long long tile_limits(const int32_t* __restrict__ lim, int N
     return mine;
 }
 
-__global__ void __launch_bounds__(kScanThreads)
+// The chunks that stay visible for good, in order, and how many of them lie in front of every 128-row tile (chunks divide a
+// tile: cpt per tile).  All threads of the block call, after scan_role_limits.
+__device__ void list_far_chunks(const int32_t* __restrict__ lim, int Nc, int cpt, int32_t* __restrict__ list,
+                                int32_t* __restrict__ before_tile, int (*s)[kPrepWarps]) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int base = 0, buf = 0;
+    for (int c0 = 0; c0 < Nc; c0 += kPrepThreads, buf ^= 1) {
+        const int c = c0 + tid;
+        const bool keep = c < Nc && lim[c] == kNoLimit;
+        const unsigned m = __ballot_sync(0xffffffffu, keep);
+        if (lane == 0) s[buf][warp] = __popc(m);
+        __syncthreads();
+        const int all = s[buf][lane];
+        const int rank = base + __reduce_add_sync(0xffffffffu, lane < warp ? all : 0) + __popc(m & ((1u << lane) - 1u));
+        if (keep) list[rank] = c;
+        if (c < Nc && c % cpt == 0) before_tile[c / cpt] = rank;
+        base += __reduce_add_sync(0xffffffffu, all);
+    }
+}
+
+__global__ void __launch_bounds__(kPrepThreads)
 role_prep_kernel(const uint8_t* __restrict__ roles, int Nc, int N, int C, int SW, int Nt,
                  int32_t* __restrict__ lim, int32_t* __restrict__ tmax, int32_t* __restrict__ tmin,
-                 long long* __restrict__ kept) {
+                 long long* __restrict__ kept, FarLists far) {
     const int bh = blockIdx.x, tid = threadIdx.x;
     roles += (size_t)bh * Nc;
     lim += (size_t)bh * Nc;
     tmax += (size_t)bh * Nt;
     tmin += (size_t)bh * Nt;
-    __shared__ int s[kScanThreads];
-    __shared__ int carry, first_gf;
+    __shared__ int s[2][kPrepWarps];
+    __shared__ int first_gf;
     __shared__ unsigned long long kept_sm;
     if (tid == 0) kept_sm = 0;
-    scan_role_limits(roles, Nc, C, SW, 0, lim, s, &carry, &first_gf);
-    const unsigned long long mine = tile_limits(lim, N, C, Nt, 0, Nt, tmax, tmin);
+    scan_role_limits(roles, Nc, C, SW, 0, lim, s, &first_gf);
+    const unsigned long long mine = tile_limits(lim, N, C, Nt, 0, Nt, tmax, tmin, far.list ? far.open_max + (size_t)bh * Nt : nullptr);
+    if (far.list != nullptr)
+        list_far_chunks(lim, Nc, kTile / C, far.list + (size_t)bh * Nc, far.before_tile + (size_t)bh * Nt, s);
     if (kept != nullptr) {
-        atomicAdd(&kept_sm, mine);
+        if (mine) atomicAdd(&kept_sm, mine);
         __syncthreads();
         if (tid == 0) kept[bh] = (long long)kept_sm;
     }
@@ -115,24 +153,25 @@ struct PastPrepParams {
     const long long* size_global; const long long* size_local;
     int32_t* lim; int32_t* tmax; int32_t* tmin; long long* kept;
     int Ncn, Lcap, T0, C, SW, tail, Nq, q_off, Nkv, Nc, Ntk, Nt;
+    FarLists far;
 };
 
-__global__ void __launch_bounds__(kScanThreads) role_prep_past_kernel(const PastPrepParams p) {
+__global__ void __launch_bounds__(kPrepThreads) role_prep_past_kernel(const PastPrepParams p) {
     const int bh = blockIdx.x, tid = threadIdx.x;
     const uint8_t* roles = p.roles + (size_t)bh * p.Ncn;
     const uint8_t* valid = p.valid + (size_t)bh * p.Lcap;
     int32_t* lim = p.lim + (size_t)bh * p.Nc;
-    __shared__ int s[kScanThreads];
-    __shared__ int carry, first_gf;
+    __shared__ int s[2][kPrepWarps];
+    __shared__ int first_gf;
     __shared__ unsigned long long kept_sm;
     if (tid == 0) kept_sm = 0;
     const int n_old = p.T0 / p.C, W = p.SW / p.C;
     // new chunks: the rule of a first call, positions counted from T0
-    scan_role_limits(roles, p.Ncn, p.C, p.SW, p.T0, lim + n_old, s, &carry, &first_gf);
+    scan_role_limits(roles, p.Ncn, p.C, p.SW, p.T0, lim + n_old, s, &first_gf);
     // cached chunks
     const int sg = (int)(p.size_global[bh] / p.C), sl = (int)(p.size_local[bh] / p.C);
     const long long lim_local = (long long)p.T0 + ((long long)first_gf + 1) * p.C - 1;   // until the first new global chunk ends
-    for (int j = tid; j < n_old; j += kScanThreads) {
+    for (int j = tid; j < n_old; j += kPrepThreads) {
         int l;
         if (j < W) {
             // ring slot j was written `age` chunks before the newest one; a sliding chunk is seen by the SW/C chunks after it
@@ -148,10 +187,12 @@ __global__ void __launch_bounds__(kScanThreads) role_prep_past_kernel(const Past
         lim[j] = l;
     }
     __syncthreads();
-    const unsigned long long mine = tile_limits(lim, p.Nkv, p.C, p.Ntk, p.q_off, p.Nt,
-                                                p.tmax + (size_t)bh * p.Ntk, p.tmin + (size_t)bh * p.Ntk);
+    const unsigned long long mine = tile_limits(lim, p.Nkv, p.C, p.Ntk, p.q_off, p.Nt, p.tmax + (size_t)bh * p.Ntk, p.tmin + (size_t)bh * p.Ntk,
+                                                p.far.list ? p.far.open_max + (size_t)bh * p.Ntk : nullptr);
+    if (p.far.list != nullptr)
+        list_far_chunks(lim, p.Nc, kTile / p.C, p.far.list + (size_t)bh * p.Nc, p.far.before_tile + (size_t)bh * p.Ntk, s);
     if (p.kept != nullptr) {
-        atomicAdd(&kept_sm, mine);
+        if (mine) atomicAdd(&kept_sm, mine);
         __syncthreads();
         if (tid == 0) p.kept[bh] = (long long)kept_sm;
     }
@@ -453,16 +494,21 @@ static int check_common(int B, int Hkv, int N, int C, int SW) {
     return NATS_OK;
 }
 
-extern "C" __attribute__((visibility("default"))) int nats_b200_role_prep(const uint8_t* d_roles, int B, int Hkv, int N, int C, int SW,
-                                   int32_t* d_lim, int32_t* d_tile_max, int32_t* d_tile_min, int64_t* d_kept_tiles,
-                                   void* stream) {
+int nats::role_prep(const uint8_t* d_roles, int B, int Hkv, int N, int C, int SW, int32_t* d_lim, int32_t* d_tile_max,
+                    int32_t* d_tile_min, int64_t* d_kept_tiles, const FarLists& far, void* stream) {
     if (int rc = check_common(B, Hkv, N, C, SW)) return rc;
     NATS_CHECK_ARG(d_roles && d_lim && d_tile_max && d_tile_min, "null pointer");
     const int Nc = cdiv(N, C), Nt = cdiv(N, kTile);
-    role_prep_kernel<<<B * Hkv, kScanThreads, 0, (cudaStream_t)stream>>>(
-        d_roles, Nc, N, C, SW, Nt, d_lim, d_tile_max, d_tile_min, (long long*)d_kept_tiles);
+    role_prep_kernel<<<B * Hkv, kPrepThreads, 0, (cudaStream_t)stream>>>(
+        d_roles, Nc, N, C, SW, Nt, d_lim, d_tile_max, d_tile_min, (long long*)d_kept_tiles, far);
     NATS_CHECK_CUDA(cudaGetLastError());
     return NATS_OK;
+}
+
+extern "C" __attribute__((visibility("default"))) int nats_b200_role_prep(const uint8_t* d_roles, int B, int Hkv, int N, int C, int SW,
+                                   int32_t* d_lim, int32_t* d_tile_max, int32_t* d_tile_min, int64_t* d_kept_tiles,
+                                   void* stream) {
+    return role_prep(d_roles, B, Hkv, N, C, SW, d_lim, d_tile_max, d_tile_min, d_kept_tiles, FarLists{}, stream);
 }
 
 extern "C" __attribute__((visibility("default"))) int nats_b200_visible_counts(const int32_t* d_lim, int B, int Hq, int Hkv, int N, int C,
@@ -488,10 +534,10 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_evict_plan(const
     return NATS_OK;
 }
 
-extern "C" __attribute__((visibility("default"))) int nats_b200_role_prep_past(
+int nats::role_prep_past(
     const uint8_t* d_roles_new, const uint8_t* d_valid, const int64_t* d_size_global, const int64_t* d_size_local,
     int B, int Hkv, int x_len, int C, int SW, int valid_stride, int t0, int fill, int tail,
-    int32_t* d_lim, int32_t* d_tile_max, int32_t* d_tile_min, int64_t* d_kept_tiles, void* stream) {
+    int32_t* d_lim, int32_t* d_tile_max, int32_t* d_tile_min, int64_t* d_kept_tiles, const FarLists& far, void* stream) {
     if (int rc = check_common(B, Hkv, x_len, C, SW)) return rc;
     NATS_CHECK_ARG(d_roles_new && d_valid && d_size_global && d_size_local && d_lim && d_tile_max && d_tile_min, "null pointer");
     NATS_CHECK_ARG(t0 >= SW && t0 % C == 0 && fill >= 0 && fill < C, "tail offset %d must be a chunk multiple >= the window, fill %d in [0, chunk)", t0, fill);
@@ -505,9 +551,18 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_role_prep_past(
     p.Ncn = cdiv(fill + x_len, C); p.Lcap = valid_stride; p.T0 = t0; p.C = C; p.SW = SW; p.tail = tail;
     p.Nq = x_len; p.q_off = t0 + fill; p.Nkv = t0 + fill + x_len;
     p.Nc = cdiv(p.Nkv, C); p.Ntk = cdiv(p.Nkv, kTile); p.Nt = cdiv(x_len, kTile);
-    role_prep_past_kernel<<<B * Hkv, kScanThreads, 0, (cudaStream_t)stream>>>(p);
+    p.far = far;
+    role_prep_past_kernel<<<B * Hkv, kPrepThreads, 0, (cudaStream_t)stream>>>(p);
     NATS_CHECK_CUDA(cudaGetLastError());
     return NATS_OK;
+}
+
+extern "C" __attribute__((visibility("default"))) int nats_b200_role_prep_past(
+    const uint8_t* d_roles_new, const uint8_t* d_valid, const int64_t* d_size_global, const int64_t* d_size_local,
+    int B, int Hkv, int x_len, int C, int SW, int valid_stride, int t0, int fill, int tail,
+    int32_t* d_lim, int32_t* d_tile_max, int32_t* d_tile_min, int64_t* d_kept_tiles, void* stream) {
+    return role_prep_past(d_roles_new, d_valid, d_size_global, d_size_local, B, Hkv, x_len, C, SW, valid_stride, t0, fill, tail,
+                          d_lim, d_tile_max, d_tile_min, d_kept_tiles, FarLists{}, stream);
 }
 
 extern "C" __attribute__((visibility("default"))) int nats_b200_evict_plan_past(

@@ -30,6 +30,22 @@ int fail(int code, const char* fmt, ...);
             return ::nats::fail(NATS_ERR_CUDA, "%s failed: %s", #expr, cudaGetErrorString(e_));   \
     } while (0)
 
+// Chunks that stay visible for good, per (batch, kv-head): list [Nc] = their indices in order, before_tile [Ntk] = how many of
+// them lie in front of a 128-row KV tile, open_max [Ntk] = largest row limit of the tile's other chunks (-1: it has none).
+// list == nullptr: not wanted.  Only for chunk sizes that divide a tile.
+struct FarLists {
+    int32_t* list = nullptr;
+    int32_t* before_tile = nullptr;
+    int32_t* open_max = nullptr;
+};
+
+// the C entry points nats_b200_role_prep / _past with the lists beside the limits
+int role_prep(const uint8_t* d_roles, int B, int Hkv, int N, int C, int SW, int32_t* d_lim, int32_t* d_tile_max,
+              int32_t* d_tile_min, int64_t* d_kept_tiles, const FarLists& far, void* stream);
+int role_prep_past(const uint8_t* d_roles_new, const uint8_t* d_valid, const int64_t* d_size_global, const int64_t* d_size_local,
+                   int B, int Hkv, int x_len, int C, int SW, int valid_stride, int t0, int fill, int tail,
+                   int32_t* d_lim, int32_t* d_tile_max, int32_t* d_tile_min, int64_t* d_kept_tiles, const FarLists& far, void* stream);
+
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 inline int cdiv(int a, int b) { return (a + b - 1) / b; }
 

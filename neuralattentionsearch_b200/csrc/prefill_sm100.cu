@@ -11,6 +11,12 @@
 //   warps 4-7   softmax of head slot 0: one thread per query row, the 128-entry score row read with tcgen05.ld, online
 //   warps 8-11  softmax of head slot 1  softmax in registers, P written back over S as packed bf16
 //
+// Chunks finer than a tile: far behind the queries only the global chunks are still visible, a few in every tile.  Those
+// are not computed in place but gathered: the keys of 128 / C listed chunks (FarLists) make a full tile, copied chunk by
+// chunk (boxes of C rows) or, below 8 rows, with tile::gather4.  The bitmap then only holds the tiles from the first one on
+// in which some other chunk is still visible.  The work of a query tile falls from the tiles that hold a visible key towards
+// the keys that are visible: prompt of 8192 tokens with one role per token, 10 % global, 0.91 -> 0.29 ms; forward of
+// 8 x 4096 tokens with chunks of 16, 0.51 -> 0.26 ms.
 // Which KV tiles are visited comes from the role bitmap: a bitmap of kept tiles is built in shared memory from the
 // per-tile max / min row limits (nats_b200_role_prep); tiles without a visible entry are never loaded.  Only tiles
 // whose min limit does not cover the whole query tile (and the diagonal) pay for per-element masking.
@@ -57,6 +63,11 @@ struct PrefillParams {
     const int32_t* lim;               // [B,Hkv,Nc]: last query POSITION that may see KV chunk c
     const int32_t* tile_max;          // [B,Hkv,Ntk]: max / min of lim over the chunks of a 128-row KV tile
     const int32_t* tile_min;
+    // chunks visible for good (see FarLists), or all nullptr: the tiles in front of the first tile with another visible chunk
+    // are not walked, their listed chunks are gathered into full tiles instead
+    const int32_t* far_list;
+    const int32_t* far_before;
+    const int32_t* far_open;
     int32_t* status;
     int32_t* work_counter;            // next work item; zero at launch
     int total_items;                  // B * Hkv * n_groups * Nt
@@ -65,6 +76,8 @@ struct PrefillParams {
     // Nc / Ntk: chunks / 128-row tiles of the KV sequence, Nt: query tiles.
     int Hq, Hkv, N, Nkv, q_off, C, Nc, Nt, Ntk, nrep, n_groups;   // n_groups = ceil(nrep / heads per item)
     int c_shift;                      // log2(C), -1 if C is no power of two
+    int head_rows;                    // rows from one kv-head to the next
+
     float scale_log2;
 };
 
@@ -134,6 +147,12 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
     asm volatile(
         "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5}], [%2], %6;"
         ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "l"(policy) : "memory");
+}
+// four rows (r0 .. r3 of a 2-D map whose box is one row high), 64 columns from c0
+__device__ __forceinline__ void tma_gather4(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int r0, int r1, int r2, int r3, uint64_t policy) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5, %6, %7}], [%2], %8;"
+        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(r0), "r"(r1), "r"(r2), "r"(r3), "l"(policy) : "memory");
 }
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
@@ -330,8 +349,8 @@ struct ItemHeader {
     int b, bh;      // batch index, b * Hkv + kv-head
     int head0;      // query head of slot 0
     int nslots;     // 1 or 2 query heads in this item
-    int n_kept;     // kept 128-column KV tiles
-    int pad;
+    int n_kept;     // 128-column KV tiles: gathered ones first, then the kept tiles of the bitmap
+    int far_keys;   // keys of the gathered tiles (the last one may be part empty)
 };
 
 constexpr int kBitWords = kMaxTiles / 32;
@@ -435,10 +454,14 @@ __device__ __forceinline__ void pipe_release(int* lock, int lane) {
 // ->  O += P.V_j  ->  S = Q.K_{j+1}^T.  The two heads
 // run this chain half a period apart, so that one head's softmax (MUFU and issue slots of the four SM sub-partitions)
 // overlaps the other head's MMAs on the tensor pipe.
-template <int D>
+//
+// FINE: chunks that are not a multiple of 32 keys, or gathered tiles.  Without it the loops carry neither the transposed masks
+// nor the gathered tiles: 32k tokens with chunks of 128 take 1.7 % longer with both in the code.
+template <int D, bool FINE>
 __global__ void __launch_bounds__(kPrefillThreads, 1)
 prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-               const __grid_constant__ CUtensorMap map_v, const PrefillParams p) {
+               const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_k_far,
+               const __grid_constant__ CUtensorMap map_v_far, const PrefillParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     using Smem = PrefillSmem<D>;
     Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
@@ -524,23 +547,40 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 const int kt_last = q_hi / kTile;
                 const int32_t* tmax = p.tile_max + (size_t)bh * p.Ntk;
                 const int32_t* tmin = p.tile_min + (size_t)bh * p.Ntk;
+                // The tiles in front of near_first hold no visible chunk but listed ones: they are left out of the bitmap.
+                // near_first <= the tile of the first query row, so every listed key in front of it is in that row's past.
+                const int32_t* open = FINE && p.far_open != nullptr ? p.far_open + (size_t)bh * p.Ntk : nullptr;
+                const int near_cap = q_lo / kTile;
+                int near_first = open != nullptr ? -1 : 0;
                 for (int s0 = 0; s0 <= kt_last; s0 += 32) {        // tiles 0..kt_last with a visible entry
                     const int kt = s0 + lane;
                     const bool keep = kt <= kt_last && tmax[kt] >= q_lo;
                     // element masking is needed where the causal edge or a chunk's row limit cuts through the tile
                     const bool partial = keep && (kt * kTile + kTile - 1 > q_lo || tmin[kt] < q_hi);
-                    const unsigned m = __ballot_sync(0xffffffffu, keep);
-                    const unsigned pm = __ballot_sync(0xffffffffu, partial);
+                    unsigned m = __ballot_sync(0xffffffffu, keep);
+                    unsigned pm = __ballot_sync(0xffffffffu, partial);
+                    if (near_first < 0) {
+                        const unsigned om = __ballot_sync(0xffffffffu, kt <= near_cap && (kt == near_cap || open[kt] >= q_lo));
+                        if (om != 0u) near_first = s0 + __ffs(om) - 1;
+                        const unsigned from = om != 0u ? 0xffffffffu << (near_first - s0) : 0u;
+                        m &= from;
+                        pm &= from;
+                    }
                     if (lane == 0) {
                         sm.keep[slot][s0 >> 5] = m;
                         sm.part[slot][s0 >> 5] = pm;
                     }
                     n_kept += __popc(m);
                 }
+                int far_keys = 0;
+                if (open != nullptr) {
+                    far_keys = p.far_before[(size_t)bh * p.Ntk + near_first] * p.C;
+                    n_kept += (far_keys + kTile - 1) / kTile;
+                }
                 if (lane == 0) {
                     ItemHeader hd;
                     hd.valid = 1; hd.t = t; hd.b = z; hd.bh = bh; hd.head0 = hkv * p.nrep + grp * Smem::kHeads;
-                    hd.nslots = min(Smem::kHeads, p.nrep - grp * Smem::kHeads); hd.n_kept = n_kept; hd.pad = 0;
+                    hd.nslots = min(Smem::kHeads, p.nrep - grp * Smem::kHeads); hd.n_kept = n_kept; hd.far_keys = far_keys;
                     sm.item[slot] = hd;
                 }
             } else if (lane == 0) {
@@ -595,9 +635,29 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             if (!hd.valid) break;
             TileWalk walk;
             walk.init(sm.keep[slot], sm.part[slot]);
+            const int n_far = (hd.far_keys + kTile - 1) / kTile;
+            const int32_t* far_list = p.far_list + (size_t)hd.bh * p.Nc;       // read only while n_far > 0
             for (int j = 0; j < hd.n_kept && ok; ++j) {
                 bool partial;
-                const int row0 = walk.next(partial) * kTile;
+                const bool far = FINE && j < n_far;
+                const int row0 = far ? 0 : walk.next(partial) * kTile;
+                // rows of a gathered tile.  Chunks of 8 rows and more: lane i copies whole chunks, i-th of the tile, 32 rows
+                // further on, ...; a slot behind the last listed chunk takes rows behind the sequence, which read as zero.
+                // Finer chunks: lane i copies the four rows 4 i .. 4 i + 3; a key behind the last one repeats the last one.
+                // Both kinds of filler are masked.
+                int4 rows = make_int4(0, 0, 0, 0);
+                const int cpt = far ? kTile >> p.c_shift : 1;
+                if (far && p.C < 8) {
+                    int* r = &rows.x;
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) {
+                        const int key = min(j * kTile + lane * 4 + x, hd.far_keys - 1);
+                        r[x] = hd.bh * p.head_rows + far_list[key / p.C] * p.C + key % p.C;
+                    }
+                } else if (far) {
+                    const int i = j * cpt + (lane & (cpt - 1));
+                    rows.x = i * p.C < hd.far_keys ? far_list[i] * p.C : p.Nkv;
+                }
 #pragma unroll 1
                 for (int kv = 0; kv < 2 && ok; ++kv, ++g) {
                     const int s = g % NS;
@@ -618,11 +678,26 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 #endif
                     if (lane == 0 && !withhold) {
                         mbar_expect_tx(smem_u32(&sm.bar_full[s]), TILE_BYTES);
-                        const CUtensorMap* map = kv == 0 ? &map_k : &map_v;
-                        for (int x = 0; x < NBOX; ++x)
-                            tma_load_3d(smem_u32(&sm.ring[s][x * kBoxBytes]), map, smem_u32(&sm.bar_full[s]), x * 64, row0, hd.bh, pol_kv);
+                        if (!far) {
+                            const CUtensorMap* map = kv == 0 ? &map_k : &map_v;
+                            for (int x = 0; x < NBOX; ++x)
+                                tma_load_3d(smem_u32(&sm.ring[s][x * kBoxBytes]), map, smem_u32(&sm.bar_full[s]), x * 64, row0, hd.bh, pol_kv);
+                        }
                     }
                     __syncwarp();
+                    if (far && !withhold) {
+                        const CUtensorMap* map = kv == 0 ? &map_k_far : &map_v_far;
+                        const uint32_t dst = smem_u32(&sm.ring[s][0]), bar = smem_u32(&sm.bar_full[s]);
+                        if (p.C < 8) {
+                            for (int x = 0; x < NBOX; ++x)
+                                tma_gather4(dst + x * kBoxBytes + lane * 512, map, bar, x * 64, rows.x, rows.y, rows.z, rows.w, pol_kv);
+                        } else {
+                            // cpt <= 16 divides 32: the lanes of a chunk share its boxes
+                            for (int x = lane / cpt; x < NBOX; x += 32 / cpt)
+                                tma_load_3d(dst + x * kBoxBytes + (lane & (cpt - 1)) * p.C * 128, map, bar, x * 64, rows.x, hd.bh, pol_kv);
+                        }
+                        __syncwarp();
+                    }
                 }
             }
             if (ok && lane == 0) mbar_arrive(smem_u32(&sm.bar_list_empty[slot]));
@@ -803,13 +878,20 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 walk.init(sm.keep[slot], sm.part[slot]);
                 for (int j = 0; j < n; ++j, ++gt) {
                     bool partial;
-                    const int k0 = walk.next(partial) * kTile;    // first key column of this tile
                     // visibility bits of this row for the 128 columns of a tile that is not fully visible
                     uint32_t bits[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
-                    if (partial) {
+                    const int far_left = FINE ? hd.far_keys - j * kTile : 0;             // keys of the gathered tiles from this tile on
+                    if (far_left > 0) {
+                        // a gathered tile: all its keys are visible to every row; the last one may be part empty
+                        partial = far_left < kTile;
+                        if (partial) {
+#pragma unroll
+                            for (int w = 0; w < 4; ++w) bits[w] = far_left >= 32 * w + 32 ? 0xffffffffu : far_left <= 32 * w ? 0u : (1u << (far_left - 32 * w)) - 1u;
+                        }
+                    } else if (const int k0 = walk.next(partial) * kTile; partial) {    // k0: first key column of the tile
 #pragma unroll
                         for (int w = 0; w < 4; ++w)
-                            bits[w] = p.c_shift >= 5 ? visible_bits_coarse(lim, k0 + 32 * w, qpos, p.Nkv, p.c_shift)
+                            bits[w] = !FINE || p.c_shift >= 5 ? visible_bits_coarse(lim, k0 + 32 * w, qpos, p.Nkv, p.c_shift)
                                                      : visible_bits(lim, k0 + 32 * w + lane, qpos - lane, p.Nkv, p.C, p.c_shift, lane);
                     }
                     // S of tile j is complete; so is O += P.V of tile j - 1, which the same thread issued in front of it
@@ -1002,8 +1084,8 @@ static EncodeTiledFn get_encode_fn() {
 
 // [heads, N, D] bf16 viewed as a 3-D tensor (D innermost); box = 64 x box_rows x 1 with 128-byte swizzle; rows past N read zero
 // 3-D map over [heads, rows, D] bf16; consecutive heads are head_stride_rows rows apart (>= rows: a cache buffer is
-// longer than the part of it that is valid; rows behind `rows` read as zero).
-static int make_map(CUtensorMap* map, const void* base, int heads, int N, int D, int box_rows, long long head_stride_rows = 0) {
+// longer than the part of it that is valid; rows behind `rows` read as zero).  flat: a 2-D map over `rows` rows.
+static int make_map(CUtensorMap* map, const void* base, long long heads, long long N, int D, int box_rows, long long head_stride_rows = 0, bool flat = false) {
     EncodeTiledFn fn = get_encode_fn();
     if (!fn) return fail(NATS_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     if (head_stride_rows <= 0) head_stride_rows = N;
@@ -1011,44 +1093,59 @@ static int make_map(CUtensorMap* map, const void* base, int heads, int N, int D,
     cuuint64_t strides[2] = {(cuuint64_t)D * 2, (cuuint64_t)head_stride_rows * D * 2};
     cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
     cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, flat ? 2 : 3, const_cast<void*>(base), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(NATS_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
     return NATS_OK;
 }
 
-struct PrefillWs { size_t lim, tmax, tmin, counter, total; };
-// N = rows of the KV sequence
+struct PrefillWs { size_t lim, tmax, tmin, counter, total, list, before, open, total_far; };
+// N = rows of the KV sequence.  `total` bytes are enough for any call; with `total_far` bytes the lists of the chunks that
+// stay visible have room behind them (0: this chunk size has no such lists).
 static PrefillWs prefill_ws(int B, int Hkv, int N, int C) {
-    PrefillWs w;
+    PrefillWs w = {};
     const size_t Nc = cdiv(N, C), Nt = cdiv(N, kTile);
+    const size_t per_tile = align_up((size_t)B * Hkv * Nt * 4, 256), per_chunk = align_up((size_t)B * Hkv * Nc * 4, 256);
     w.lim = 0;
-    w.tmax = align_up((size_t)B * Hkv * Nc * 4, 256);
-    w.tmin = w.tmax + align_up((size_t)B * Hkv * Nt * 4, 256);
-    w.counter = w.tmin + align_up((size_t)B * Hkv * Nt * 4, 256);
+    w.tmax = per_chunk;
+    w.tmin = w.tmax + per_tile;
+    w.counter = w.tmin + per_tile;
     w.total = w.counter + 256;
+    if (C < kTile && kTile % C == 0) {
+        w.list = w.total;
+        w.before = w.list + per_chunk;
+        w.open = w.before + per_tile;
+        w.total_far = w.open + per_tile;
+    }
     return w;
+}
+
+// Whether a call gathers the far chunks.  Below kFarMinRows positions there are at most 15 tiles in front of a query tile
+// and little to gather.  The rows of all heads must be addressable by the 32-bit row index of a gather.
+constexpr int kFarMinRows = 2048;
+static bool use_far_lists(const PrefillWs& w, size_t workspace_bytes, int B, int Hkv, int N, int q_off, long long head_rows, bool pair) {
+    return w.total_far != 0 && workspace_bytes >= w.total_far && q_off + N >= kFarMinRows && !pair && (long long)B * Hkv * head_rows <= 0x7fffffffLL;
 }
 
 constexpr int kMaxDevices = 64;
 
-template <int D>
-static int launch_prefill(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const PrefillParams& p,
-                          cudaStream_t st) {
+template <int D, bool FINE>
+static int launch_prefill(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mkf,
+                          const CUtensorMap& mvf, const PrefillParams& p, cudaStream_t st) {
     const size_t smem = sizeof(PrefillSmem<D>);
     int dev = 0, sms = 0;
     NATS_CHECK_CUDA(cudaGetDevice(&dev));
     // the opt-in to more than 48 KB of dynamic shared memory is a per-device attribute of the kernel
     static bool attr_set[kMaxDevices] = {};
     if (dev < 0 || dev >= kMaxDevices || !attr_set[dev]) {
-        NATS_CHECK_CUDA(cudaFuncSetAttribute(prefill_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        NATS_CHECK_CUDA(cudaFuncSetAttribute(prefill_kernel<D, FINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         if (dev >= 0 && dev < kMaxDevices) attr_set[dev] = true;
     }
     NATS_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     NATS_CHECK_CUDA(cudaMemsetAsync(p.work_counter, 0, sizeof(int32_t), st));
     const int grid = p.total_items < sms ? p.total_items : sms;      // one persistent CTA per SM
-    prefill_kernel<D><<<grid, kPrefillThreads, smem, st>>>(mq, mk, mv, p);
+    prefill_kernel<D, FINE><<<grid, kPrefillThreads, smem, st>>>(mq, mk, mv, mkf, mvf, p);
     NATS_CHECK_CUDA(cudaGetLastError());
     return NATS_OK;
 }
@@ -1085,13 +1182,24 @@ static bool use_pair_kernel(int D, int nrep) {
 static int run_prefill(const void* d_q, const void* d_k, const void* d_v, void* d_o, int B, int Hq, int Hkv, int N, int Nkv,
                        int q_off, long long kv_head_stride, int D, int C, float sm_scale, const int32_t* lim,
                        const int32_t* tmax, const int32_t* tmin, int32_t* counter, int32_t* d_status, cudaStream_t st,
-                       float* d_lse = nullptr) {
+                       const FarLists& far, float* d_lse = nullptr) {
     const bool pair = use_pair_kernel(D, Hq / Hkv);
-    CUtensorMap mq, mk, mv;
+    CUtensorMap mq, mk, mv, mkf, mvf;
     if (int rc = make_map(&mq, d_q, B * Hq, N, D, 128)) return rc;
     if (int rc = make_map(&mk, d_k, B * Hkv, Nkv, D, pair ? 64 : 128, kv_head_stride)) return rc;     // a pair's CTA loads half the rows of a K tile
     if (int rc = make_map(&mv, d_v, B * Hkv, Nkv, D, 128, kv_head_stride)) return rc;
+    const long long head_rows = kv_head_stride > 0 ? kv_head_stride : Nkv;
+    mkf = mk;
+    mvf = mv;
+    if (far.list != nullptr) {
+        // boxes of one chunk, or of single rows of all heads for the gather of four rows
+        const bool rows = C < 8;
+        const long long heads = rows ? 1 : (long long)B * Hkv, n = rows ? (long long)B * Hkv * head_rows : Nkv;
+        if (int rc = make_map(&mkf, d_k, heads, n, D, rows ? 1 : C, head_rows, rows)) return rc;
+        if (int rc = make_map(&mvf, d_v, heads, n, D, rows ? 1 : C, head_rows, rows)) return rc;
+    }
     PrefillParams p;
+    p.far_list = far.list; p.far_before = far.before_tile; p.far_open = far.open_max; p.head_rows = (int)head_rows;
     p.o = (__nv_bfloat16*)d_o; p.lse = d_lse; p.lim = lim; p.tile_max = tmax; p.tile_min = tmin; p.status = d_status;
     p.Hq = Hq; p.Hkv = Hkv; p.N = N; p.Nkv = Nkv; p.q_off = q_off; p.C = C;
     p.c_shift = (C & (C - 1)) ? -1 : __builtin_ctz((unsigned)C);
@@ -1108,9 +1216,14 @@ static int run_prefill(const void* d_q, const void* d_k, const void* d_v, void* 
         p.total_items = B * Hkv * p.n_groups * p.Nt;
         return launch_prefill_pair(mq, mk, mv, p, st);
     }
-    if (D == 64) return launch_prefill<64>(mq, mk, mv, p, st);
-    if (D == 256) return launch_prefill<256>(mq, mk, mv, p, st);
-    return launch_prefill<128>(mq, mk, mv, p, st);
+    if (p.c_shift >= 5 && far.list == nullptr) {
+        if (D == 64) return launch_prefill<64, false>(mq, mk, mv, mkf, mvf, p, st);
+        if (D == 256) return launch_prefill<256, false>(mq, mk, mv, mkf, mvf, p, st);
+        return launch_prefill<128, false>(mq, mk, mv, mkf, mvf, p, st);
+    }
+    if (D == 64) return launch_prefill<64, true>(mq, mk, mv, mkf, mvf, p, st);
+    if (D == 256) return launch_prefill<256, true>(mq, mk, mv, mkf, mvf, p, st);
+    return launch_prefill<128, true>(mq, mk, mv, mkf, mvf, p, st);
 }
 
 }  // namespace nats
@@ -1119,7 +1232,8 @@ using namespace nats;
 
 extern "C" __attribute__((visibility("default"))) size_t nats_b200_prefill_workspace_bytes(int B, int Hkv, int N, int C) {
     if (B <= 0 || Hkv <= 0 || N <= 0 || C <= 0) return 0;
-    return prefill_ws(B, Hkv, N, C).total;
+    const PrefillWs w = prefill_ws(B, Hkv, N, C);
+    return w.total_far ? w.total_far : w.total;
 }
 
 static int prefill_first_call(const void* d_q, const void* d_k, const void* d_v, void* d_o, const uint8_t* d_roles,
@@ -1142,11 +1256,14 @@ static int prefill_first_call(const void* d_q, const void* d_k, const void* d_v,
     int32_t* lim = (int32_t*)(ws + w.lim);
     int32_t* tmax = (int32_t*)(ws + w.tmax);
     int32_t* tmin = (int32_t*)(ws + w.tmin);
-    if (int rc = nats_b200_role_prep(d_roles, B, Hkv, N, C, SW, lim, tmax, tmin, d_kept_tiles, stream)) return rc;
+    FarLists far;
+    if (use_far_lists(w, workspace_bytes, B, Hkv, N, 0, N, use_pair_kernel(D, Hq / Hkv)))
+        far = {(int32_t*)(ws + w.list), (int32_t*)(ws + w.before), (int32_t*)(ws + w.open)};
+    if (int rc = role_prep(d_roles, B, Hkv, N, C, SW, lim, tmax, tmin, d_kept_tiles, far, stream)) return rc;
     if (d_n_visible != nullptr)
         if (int rc = nats_b200_visible_counts(lim, B, Hq, Hkv, N, C, d_n_visible, stream)) return rc;
     return run_prefill(d_q, d_k, d_v, d_o, B, Hq, Hkv, N, N, 0, 0, D, C, sm_scale, lim, tmax, tmin,
-                       (int32_t*)(ws + w.counter), d_status, (cudaStream_t)stream, d_lse);
+                       (int32_t*)(ws + w.counter), d_status, (cudaStream_t)stream, far, d_lse);
 }
 
 extern "C" __attribute__((visibility("default"))) int nats_b200_prefill_fwd(const void* d_q, const void* d_k, const void* d_v, void* d_o, const uint8_t* d_roles,
@@ -1169,7 +1286,7 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_prefill_fwd_stat
 
 extern "C" __attribute__((visibility("default"))) size_t nats_b200_prefill_past_workspace_bytes(int B, int Hkv, int n_kv, int C) {
     if (B <= 0 || Hkv <= 0 || n_kv <= 0 || C <= 0) return 0;
-    return prefill_ws(B, Hkv, n_kv, C).total;
+    return nats_b200_prefill_workspace_bytes(B, Hkv, n_kv, C);
 }
 
 extern "C" __attribute__((visibility("default"))) int nats_b200_prefill_past_fwd(
@@ -1197,10 +1314,13 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_prefill_past_fwd
     int32_t* lim = (int32_t*)(ws + w.lim);
     int32_t* tmax = (int32_t*)(ws + w.tmax);
     int32_t* tmin = (int32_t*)(ws + w.tmin);
-    if (int rc = nats_b200_role_prep_past(d_roles_new, d_valid, d_size_global, d_size_local, B, Hkv, x_len, C, SW,
-                                          valid_stride, t0, fill, tail, lim, tmax, tmin, d_kept_tiles, stream)) return rc;
+    FarLists far;
+    if (use_far_lists(w, workspace_bytes, B, Hkv, x_len, t0 + fill, cache_capacity, use_pair_kernel(D, Hq / Hkv)))
+        far = {(int32_t*)(ws + w.list), (int32_t*)(ws + w.before), (int32_t*)(ws + w.open)};
+    if (int rc = role_prep_past(d_roles_new, d_valid, d_size_global, d_size_local, B, Hkv, x_len, C, SW,
+                                          valid_stride, t0, fill, tail, lim, tmax, tmin, d_kept_tiles, far, stream)) return rc;
     return run_prefill(d_q, d_cache_k, d_cache_v, d_o, B, Hq, Hkv, x_len, (int)n_kv, t0 + fill, cache_capacity, D, C, sm_scale,
-                       lim, tmax, tmin, (int32_t*)(ws + w.counter), d_status, (cudaStream_t)stream);
+                       lim, tmax, tmin, (int32_t*)(ws + w.counter), d_status, (cudaStream_t)stream, far);
 }
 
 // =================================================================================================
@@ -1242,7 +1362,7 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_prefill_fwd_stat
     int B, int Hq, int Hkv, int N, int D, int C, int SW, float sm_scale,
     int64_t* d_kept_tiles, int32_t* d_status, void* stream) {
     if (B <= 0 || Hkv <= 0 || N <= 0 || C <= 0) return fail(NATS_ERR_INVALID_ARG, "bad shape B=%d Hkv=%d N=%d C=%d", B, Hkv, N, C);
-    const size_t need = nats_b200_prefill_workspace_bytes(B, Hkv, N, C);
+    const size_t need = nats::prefill_ws(B, Hkv, N, C).total;
     if (need > nats::kStaticScratchBytes)
         return fail(NATS_ERR_WORKSPACE,
                     "this shape needs %zu bytes of role metadata, the built-in scratch holds %zu: use nats_b200_prefill_fwd "

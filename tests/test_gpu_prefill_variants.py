@@ -34,3 +34,44 @@ def test_mask_bits_of_every_chunk_granularity(C):
     roles = orc.make_roles(B, Hkv, -(-N // C), 0.1, 0.4, seed=C)
     q, k, v = inputs(B, Hq, Hkv, N, D, seed=C, sigma=0.5)
     assert_close_attn(run_prefill(q, k, v, roles, C, SW), orc.prefill_attention(q, k, v, roles, C, SW))
+
+
+@pytest.mark.parametrize('C,N,p_global,p_local', [(1, 2048, 0.1, 0.3), (2, 2500, 0.05, 0.3), (4, 2177, 0.2, 0.1), (8, 2300, 0.1, 0.3),
+                                                  (16, 3001, 0.03, 0.1), (32, 2600, 0.3, 0.0), (64, 4000, 0.1, 0.6), (16, 2304, 1.0, 0.0),
+                                                  (1, 2304, 0.0, 1.0), (32, 2304, 0.0, 0.0)])
+@pytest.mark.parametrize('D', [64, 128, 256])
+def test_far_chunks_are_gathered(C, N, p_global, p_local, D):
+    """Prompts long enough for the gathered tiles: every way of gathering (single rows, boxes of 8 to 64 rows), a last gathered
+    tile that is full, part empty or missing (no global chunk but the first), all chunks global, all local."""
+    B, Hq, Hkv = (2, 4, 2) if D == 64 else (1, 3, 1)
+    SW = C * max(1, 200 // C)
+    roles = orc.make_roles(B, Hkv, -(-N // C), p_global, p_local, seed=N + C)
+    q, k, v = inputs(B, Hq, Hkv, N, D, seed=N, sigma=0.5)
+    assert_close_attn(run_prefill(q, k, v, roles, C, SW), orc.prefill_attention(q, k, v, roles, C, SW))
+
+
+@pytest.mark.parametrize('C', [1, 16, 64])
+def test_far_chunks_of_a_call_over_a_cache(C):
+    """Segments over the compacted cache (ragged, the second one starting inside a chunk) equal one call over the sequence."""
+    from neuralattentionsearch_b200 import NAtSChunkLayerCache, check_status, prefill_attention
+    B, Hq, Hkv, D, SW = 2, 4, 2, 128, 256
+    lens = [1500, 1301, 900]
+    N = sum(lens)
+    roles = torch.from_numpy(orc.make_roles(B, Hkv, -(-N // C), 0.08, 0.25, seed=C)).to(dev())
+    q, k, v = (t.to(dev()).bfloat16() for t in inputs(B, Hq, Hkv, N, D, seed=C, sigma=0.5))
+    whole = orc.prefill_attention(q.float().cpu(), k.float().cpu(), v.float().cpu(), roles.cpu().numpy(), C, SW)
+    cache = NAtSChunkLayerCache(B, Hkv, SW, chunk_size=C, device=dev())
+    pos = 0
+    for n in lens:
+        s = slice(pos, pos + n)
+        r = roles[..., pos // C:-(-(pos + n) // C)].clone()
+        last = (pos + n) // C if (pos + n) % C else -1           # an unfinished last chunk counts as global
+        if last >= 0:
+            r[..., -1] = 0
+        cache.update(k[:, :, s], v[:, :, s], r.contiguous())
+        o = prefill_attention(q[:, :, s].contiguous(), k[:, :, s].contiguous(), v[:, :, s].contiguous(), r.contiguous(), C, SW) if pos == 0 \
+            else cache.prefill_attention(q[:, :, s].contiguous())
+        cache.post_update(n)
+        check_status(dev())
+        assert_close_attn(o, whole[:, :, s])
+        pos += n
