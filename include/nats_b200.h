@@ -85,6 +85,18 @@ int nats_b200_prefill_fwd(const void* d_q, const void* d_k, const void* d_v, voi
                           void* d_workspace, size_t workspace_bytes, int64_t* d_kept_tiles, int32_t* d_status,
                           void* stream);
 
+/* The same with a choice of output: o_tokens != 0 writes d_o token by token, [B,N,Hq,D], the layout an output projection
+ * reads; o_f32 != 0 writes fp32 (not rounded to bf16). */
+int nats_b200_prefill_fwd_out(const void* d_q, const void* d_k, const void* d_v, void* d_o, int o_tokens, int o_f32,
+                              const uint8_t* d_roles, int B, int Hq, int Hkv, int N, int D, int C, int SW, float sm_scale,
+                              void* d_workspace, size_t workspace_bytes, int64_t* d_kept_tiles, int32_t* d_status,
+                              void* stream);
+
+/* bf16 copies (round to nearest even) of up to three fp32 arrays of n0, n1, n2 elements in one launch; all pointers 16-byte
+ * aligned, counts multiples of 8, a count of 0 skips its array. */
+int nats_b200_to_bf16(const float* d_x0, void* d_y0, long long n0, const float* d_x1, void* d_y1, long long n1,
+                      const float* d_x2, void* d_y2, long long n2, void* stream);
+
 /* The forward with the two per-row statistics the reference's training forward hands to its backward
  * (src/nats/models/transformer/triton/nats_chunk_attention.py:319-330): M = m_i + log2(l_i), the base-2 log of the row's
  * sum of exp2(score * sm_scale * log2 e) over its visible keys, and N_VALID_BLOCKS, the number of keys the row sees
@@ -150,6 +162,11 @@ int nats_b200_evict_compact(const void* d_k, const void* d_v, const uint8_t* d_r
                             const int64_t* d_size_global, const int64_t* d_size_local, const int32_t* d_state,
                             int B, int Hkv, int N, int D, int C, int SW,
                             void* d_cache_k, void* d_cache_v, uint8_t* d_valid, int Lcap, void* stream);
+/* The same for K and V in fp32 (rounded to bf16 as they are moved: only the kept rows are read). */
+int nats_b200_evict_compact_f32(const float* d_k, const float* d_v, const uint8_t* d_roles, const int32_t* d_rank,
+                                const int64_t* d_size_global, const int64_t* d_size_local, const int32_t* d_state,
+                                int B, int Hkv, int N, int D, int C, int SW,
+                                void* d_cache_k, void* d_cache_v, uint8_t* d_valid, int Lcap, void* stream);
 
 /* ------------------------------------------------------------------------------------------------
  * Multi-token call over an existing compacted cache (segmented prefill, a further turn of a conversation).

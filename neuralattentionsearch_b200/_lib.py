@@ -19,12 +19,15 @@ SIGNATURES = {
     'nats_b200_role_prep': (_I, [_P, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P]),
     'nats_b200_prefill_workspace_bytes': (_SZ, [_I, _I, _I, _I]),
     'nats_b200_prefill_fwd': (_I, [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _P, _SZ, _P, _P, _P]),
+    'nats_b200_prefill_fwd_out': (_I, [_P, _P, _P, _P, _I, _I, _P, _I, _I, _I, _I, _I, _I, _I, _F, _P, _SZ, _P, _P, _P]),
+    'nats_b200_to_bf16': (_I, [_P, _P, _c.c_longlong, _P, _P, _c.c_longlong, _P, _P, _c.c_longlong, _P]),
     'nats_b200_prefill_fwd_stats': (_I, [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _P, _SZ, _P, _P, _P, _P, _P]),
     'nats_b200_visible_counts': (_I, [_P, _I, _I, _I, _I, _I, _P, _P]),
     'nats_b200_prefill_static_scratch_bytes': (_SZ, []),
     'nats_b200_prefill_fwd_static': (_I, [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _P, _P, _P]),
     'nats_b200_evict_plan': (_I, [_P, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P]),
     'nats_b200_evict_compact': (_I, [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P, _P, _I, _P]),
+    'nats_b200_evict_compact_f32': (_I, [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P, _P, _I, _P]),
     'nats_b200_cache_append': (_I, [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P]),
     'nats_b200_role_prep_past': (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P]),
     'nats_b200_prefill_past_workspace_bytes': (_SZ, [_I, _I, _I, _I]),

@@ -146,7 +146,8 @@ class BaseNAtSChunkAttentionLayer(nn.Module):
         x_len = xq.shape[-2]
         if layer_cache.get_seq_length() == 0:
             roles = F_.roles_from_token_states_info(kwargs['token_states_info'])
-            output = F_.prefill_attention(xq, keys, values, roles, self.chunk_size, self.local_seq_max_length, self.sm_scale)
+            output = F_.prefill_attention(xq, keys, values, roles, self.chunk_size, self.local_seq_max_length, self.sm_scale,
+                                          token_major=True)
         elif x_len == 1:
             output = layer_cache.decode_attention(xq, self.sm_scale)
         else:

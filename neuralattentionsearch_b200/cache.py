@@ -369,8 +369,11 @@ class NAtSChunkLayerCache:
         C, SW = self.chunk_size, self.sliding_window_size
         k, v = self._pending
         self._pending = None
-        kb = k.to(torch.bfloat16).contiguous()
-        vb = v.to(torch.bfloat16).contiguous()
+        if x_len >= C and F_.is_plain_fp32(k) and F_.is_plain_fp32(v):
+            kb, vb = k, v                                         # the compaction rounds the rows it keeps
+        else:
+            kb = k.to(torch.bfloat16).contiguous()
+            vb = v.to(torch.bfloat16).contiguous()
         B, H, N, D = kb.shape
         rem = N % C
         n_full = N // C

@@ -124,7 +124,8 @@ __device__ void list_far_chunks(const int32_t* __restrict__ lim, int Nc, int cpt
 __global__ void __launch_bounds__(kPrepThreads)
 role_prep_kernel(const uint8_t* __restrict__ roles, int Nc, int N, int C, int SW, int Nt,
                  int32_t* __restrict__ lim, int32_t* __restrict__ tmax, int32_t* __restrict__ tmin,
-                 long long* __restrict__ kept, FarLists far) {
+                 long long* __restrict__ kept, FarLists far, int32_t* __restrict__ counter) {
+    if (counter != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *counter = 0;
     const int bh = blockIdx.x, tid = threadIdx.x;
     roles += (size_t)bh * Nc;
     lim += (size_t)bh * Nc;
@@ -154,9 +155,11 @@ struct PastPrepParams {
     int32_t* lim; int32_t* tmax; int32_t* tmin; long long* kept;
     int Ncn, Lcap, T0, C, SW, tail, Nq, q_off, Nkv, Nc, Ntk, Nt;
     FarLists far;
+    int32_t* counter;
 };
 
 __global__ void __launch_bounds__(kPrepThreads) role_prep_past_kernel(const PastPrepParams p) {
+    if (p.counter != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *p.counter = 0;
     const int bh = blockIdx.x, tid = threadIdx.x;
     const uint8_t* roles = p.roles + (size_t)bh * p.Ncn;
     const uint8_t* valid = p.valid + (size_t)bh * p.Lcap;
@@ -198,20 +201,48 @@ __global__ void __launch_bounds__(kPrepThreads) role_prep_past_kernel(const Past
     }
 }
 
-// Number of keys every query row may see (first call): sum over the chunks in front of the row.  One thread per row of a
-// kv-head; the count is written for each query head of the group.
+// Number of keys every query row may see (first call).  A chunk c ends being visible in front of chunk (lim[c] + 1) / C: limits
+// are one short of a chunk boundary.  A row of chunk x sees the rows up to its own, less C for every chunk that has ended by
+// x.  A block takes span chunks of a kv-head: one pass over the limits counts the chunks that have ended in front of its first
+// chunk and, in a histogram, at each of its chunks; a scan turns it into the number per chunk, and the rows are written for
+// each query head of the group.  (A loop over the chunks in front of every row is quadratic in the length.)
+constexpr int kCountRows = 4096;                 // rows per block, about
+
 __global__ void __launch_bounds__(kScanThreads)
-visible_count_kernel(const int32_t* __restrict__ lim, int Hq, int Hkv, int N, int C, int Nc, int32_t* __restrict__ out) {
-    const int bh = blockIdx.y;
-    const int q = blockIdx.x * kScanThreads + threadIdx.x;
-    if (q >= N) return;
+visible_count_kernel(const int32_t* __restrict__ lim, int Hq, int Hkv, int N, int C, int Nc, int span, int32_t* __restrict__ out) {
+    const int bh = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     lim += (size_t)bh * Nc;
-    const int c_last = q / C;
-    int n = 0;
-    for (int c = 0; c <= c_last; ++c)
-        if (q <= lim[c]) n += min(q - c * C + 1, C);
+    const int x0 = blockIdx.x * span, x1 = min(x0 + span, Nc);
+    __shared__ int ended[kScanThreads];          // [i]: chunks that end in front of chunk x0 + i, then the running total
+    __shared__ int s_warp[kScanThreads / 32];
+    __shared__ int s_before;
+    ended[tid] = 0;
+    if (tid == 0) s_before = 0;
+    __syncthreads();
+    int before = 0;
+    for (int c = tid; c < x1; c += kScanThreads) {
+        const int l = lim[c];
+        if (l == kNoLimit) continue;
+        const int e = (l + 1) / C;
+        if (e < x0) ++before;
+        else if (e < x1) atomicAdd(&ended[e - x0], 1);
+    }
+    before = __reduce_add_sync(0xffffffffu, before);
+    if (lane == 0 && before) atomicAdd(&s_before, before);
+    __syncthreads();
+    const int incl = warp_incl_scan(ended[tid], lane);
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    int total = s_before + incl;
+    for (int w = 0; w < warp; ++w) total += s_warp[w];
+    ended[tid] = total;
+    __syncthreads();
     const int nrep = Hq / Hkv, b = bh / Hkv, hkv = bh % Hkv;
-    for (int r = 0; r < nrep; ++r) out[((size_t)b * Hq + hkv * nrep + r) * N + q] = n;
+    const long long q1 = min((long long)x1 * C, (long long)N);
+    for (long long q = (long long)x0 * C + tid; q < q1; q += kScanThreads) {
+        const int n = (int)q + 1 - C * ended[(int)(q / C) - x0];
+        for (int r = 0; r < nrep; ++r) out[((size_t)b * Hq + hkv * nrep + r) * N + q] = n;
+    }
 }
 
 // =================================================================================================
@@ -238,56 +269,49 @@ __device__ __forceinline__ void publish_max_len(int32_t* state, int len, int nbl
 // base == nullptr: first call (the cache is empty: sizes are outputs).  Otherwise the sizes are read and updated, and
 // base[bh] receives the chunk slot (counted from position 0) the first kept chunk of this call goes to: behind the
 // kept locals if the call brings no global chunk, else behind the kept globals (the locals in front of it are dropped).
-__global__ void __launch_bounds__(kScanThreads)
+__global__ void __launch_bounds__(kPrepThreads)
 evict_plan_kernel(const uint8_t* __restrict__ roles, int Nc, int n_full, int C, int SW,
                   int32_t* __restrict__ rank, long long* __restrict__ size_global,
                   long long* __restrict__ size_local, int32_t* __restrict__ state, int32_t* __restrict__ base) {
     const int bh = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     roles += (size_t)bh * Nc;
     rank += (size_t)bh * Nc;
-    __shared__ int s_last_g;
-    __shared__ int s_warp[kScanThreads / 32];
-    __shared__ int s_base, s_ng;
-    if (tid == 0) { s_last_g = -1; s_base = 0; s_ng = 0; }
-    __syncthreads();
+    __shared__ int s_last[kPrepWarps];
+    __shared__ int s_count[2][kPrepWarps];
     // pass 1: last global chunk among the complete chunks
     int lg = -1;
-    for (int c = tid; c < n_full; c += kScanThreads)
+    for (int c = tid; c < n_full; c += kPrepThreads)
         if (roles[c] == NATS_ROLE_GLOBAL) lg = c;
-    for (int o = 16; o > 0; o >>= 1) lg = max(lg, __shfl_xor_sync(0xffffffffu, lg, o));
-    if (lane == 0 && lg >= 0) atomicMax(&s_last_g, lg);
+    lg = __reduce_max_sync(0xffffffffu, lg);
+    if (lane == 0) s_last[warp] = lg;
     __syncthreads();
-    const int last_g = s_last_g;
-    // pass 2: ordered ranks of the kept chunks
-    for (int c0 = 0; c0 < Nc; c0 += kScanThreads) {
+    const int last_g = __reduce_max_sync(0xffffffffu, s_last[lane]);
+    // pass 2: ordered ranks of the kept chunks, kPrepThreads at a time: ballots, the warps' counts side by side in shared
+    // memory (kept in the low half, global in the high half), one block barrier per step (the buffer alternates)
+    int n_kept = 0, n_g = 0, buf = 0;
+    for (int c0 = 0; c0 < Nc; c0 += kPrepThreads, buf ^= 1) {
         const int c = c0 + tid;
         const int role = (c < n_full) ? roles[c] : -1;
         const bool is_g = role == NATS_ROLE_GLOBAL;
         const bool keep = is_g || (role == NATS_ROLE_LOCAL && c > last_g);
         const unsigned m = __ballot_sync(0xffffffffu, keep);
         const unsigned mg = __ballot_sync(0xffffffffu, is_g);
-        if (lane == 0) s_warp[warp] = __popc(m);
-        if (lane == 0 && mg) atomicAdd(&s_ng, __popc(mg));
+        if (lane == 0) s_count[buf][warp] = __popc(m) | (__popc(mg) << 16);
         __syncthreads();
-        int before = s_base;
-        for (int w = 0; w < warp; ++w) before += s_warp[w];
+        const int all = s_count[buf][lane];
+        const int before = n_kept + __reduce_add_sync(0xffffffffu, lane < warp ? all & 0xffff : 0);
         // kept chunk: its rank; other chunks: -1 - (kept chunks in front of it), so that the number of kept chunks up to any
         // index can be read off without a scan (the compaction finds the chunk of a given rank by bisection)
         const int kept_before = before + __popc(m & ((1u << lane) - 1u));
         if (c < Nc) rank[c] = keep ? kept_before : -1 - kept_before;
-        __syncthreads();
-        if (tid == 0) {
-            int tot = 0;
-            for (int w = 0; w < kScanThreads / 32; ++w) tot += s_warp[w];
-            s_base += tot;
-        }
-        __syncthreads();
+        n_kept += __reduce_add_sync(0xffffffffu, all & 0xffff);
+        n_g += __reduce_add_sync(0xffffffffu, all >> 16);
     }
-    const int n_kept = s_base, n_g = s_ng;
     long long sg0 = SW, sl0 = 0;
     if (base != nullptr) { sg0 = size_global[bh]; sl0 = size_local[bh]; }
     const long long sg = sg0 + (long long)C * n_g;
     const long long sl = (last_g >= 0 ? 0 : sl0) + (long long)C * (n_kept - n_g);
+    __syncthreads();                                      // every thread has read the sizes
     if (tid == 0) {
         size_global[bh] = sg;
         size_local[bh] = sl;
@@ -316,13 +340,21 @@ struct CompactParams {
     int nB;                                      // blocks of the ring section
 };
 
+// eight bf16 of a source row: from bf16, or from fp32 rounded on the way (the source row is twice as long)
+template <bool F32>
+__device__ __forceinline__ uint4 load_row_vec(const uint8_t* base, size_t off) {
+    if (!F32) return ld16_stream(base + off);
+    return round8(ld16_stream(base + 2 * off), ld16_stream(base + 2 * off + 16));
+}
+
+template <bool F32>
 __global__ void __launch_bounds__(kCopyThreads) evict_compact_kernel(const CompactParams p) {
     const int bh = blockIdx.y, tid = threadIdx.x;
     const int vpt = p.rowB >> 4;                          // 16-byte vectors per token row
     const int tpp = kCopyThreads / vpt;                   // tokens per pass
     const int trow = tid / vpt, tvec = (tid % vpt) << 4;
-    const uint8_t* k = p.k + (size_t)bh * p.src_stride * p.rowB;
-    const uint8_t* v = p.v + (size_t)bh * p.src_stride * p.rowB;
+    const uint8_t* k = p.k + (size_t)bh * p.src_stride * p.rowB * (F32 ? 2 : 1);
+    const uint8_t* v = p.v + (size_t)bh * p.src_stride * p.rowB * (F32 ? 2 : 1);
     uint8_t* ck = p.ck + (size_t)bh * p.Lcap * p.rowB;
     uint8_t* cv = p.cv + (size_t)bh * p.Lcap * p.rowB;
     uint8_t* valid = p.valid + (size_t)bh * p.Lcap;
@@ -348,8 +380,8 @@ __global__ void __launch_bounds__(kCopyThreads) evict_compact_kernel(const Compa
             if (j < n_fills) {
                 const bool sw = roles[(src0 + j) / p.C] == NATS_ROLE_SLIDING;
                 const size_t src = (size_t)(p.src_off + src0 + j) * p.rowB + tvec;
-                st16(ck + dst, sw ? ld16_stream(k + src) : zero);
-                st16(cv + dst, sw ? ld16_stream(v + src) : zero);
+                st16(ck + dst, sw ? load_row_vec<F32>(k, src) : zero);
+                st16(cv + dst, sw ? load_row_vec<F32>(v, src) : zero);
                 if (tvec == 0) valid[slot] = sw ? 1 : 0;
             } else if (past) {
                 st16(ck + dst, ld16_stream(k + dst));
@@ -418,8 +450,8 @@ __global__ void __launch_bounds__(kCopyThreads) evict_compact_kernel(const Compa
             a[u] = b[u] = zero;
             if (sr[u] >= 0) {
                 const size_t src = (size_t)sr[u] * p.rowB + tvec;
-                a[u] = ld16_stream(k + src);
-                b[u] = ld16_stream(v + src);
+                a[u] = load_row_vec<F32>(k, src);
+                b[u] = load_row_vec<F32>(v, src);
             }
         }
 #pragma unroll
@@ -430,6 +462,21 @@ __global__ void __launch_bounds__(kCopyThreads) evict_compact_kernel(const Compa
             st16(cv + dst, b[u]);
         }
     }
+}
+
+// bf16 copies of up to three fp32 arrays: a caller's q, k and v in one launch.  Bound by HBM at sizes that matter and by the
+// launch at small ones.
+struct Bf16Params {
+    const uint8_t* x[3]; uint8_t* y[3];
+    long long n8[3];                             // groups of eight elements
+};
+
+__global__ void __launch_bounds__(kCopyThreads) to_bf16_kernel(const Bf16Params p) {
+    const long long step = (long long)gridDim.x * kCopyThreads;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+        for (long long i = (long long)blockIdx.x * kCopyThreads + threadIdx.x; i < p.n8[a]; i += step)
+            st16(p.y[a] + i * 16, round8(ld16_stream(p.x[a] + i * 32), ld16_stream(p.x[a] + i * 32 + 16)));
 }
 
 // Appends the K/V of new tokens to a cache buffer at row `pos` of every (b,h) and marks them valid.
@@ -495,12 +542,12 @@ static int check_common(int B, int Hkv, int N, int C, int SW) {
 }
 
 int nats::role_prep(const uint8_t* d_roles, int B, int Hkv, int N, int C, int SW, int32_t* d_lim, int32_t* d_tile_max,
-                    int32_t* d_tile_min, int64_t* d_kept_tiles, const FarLists& far, void* stream) {
+                    int32_t* d_tile_min, int64_t* d_kept_tiles, const FarLists& far, int32_t* d_counter, void* stream) {
     if (int rc = check_common(B, Hkv, N, C, SW)) return rc;
     NATS_CHECK_ARG(d_roles && d_lim && d_tile_max && d_tile_min, "null pointer");
     const int Nc = cdiv(N, C), Nt = cdiv(N, kTile);
     role_prep_kernel<<<B * Hkv, kPrepThreads, 0, (cudaStream_t)stream>>>(
-        d_roles, Nc, N, C, SW, Nt, d_lim, d_tile_max, d_tile_min, (long long*)d_kept_tiles, far);
+        d_roles, Nc, N, C, SW, Nt, d_lim, d_tile_max, d_tile_min, (long long*)d_kept_tiles, far, d_counter);
     NATS_CHECK_CUDA(cudaGetLastError());
     return NATS_OK;
 }
@@ -508,7 +555,7 @@ int nats::role_prep(const uint8_t* d_roles, int B, int Hkv, int N, int C, int SW
 extern "C" __attribute__((visibility("default"))) int nats_b200_role_prep(const uint8_t* d_roles, int B, int Hkv, int N, int C, int SW,
                                    int32_t* d_lim, int32_t* d_tile_max, int32_t* d_tile_min, int64_t* d_kept_tiles,
                                    void* stream) {
-    return role_prep(d_roles, B, Hkv, N, C, SW, d_lim, d_tile_max, d_tile_min, d_kept_tiles, FarLists{}, stream);
+    return role_prep(d_roles, B, Hkv, N, C, SW, d_lim, d_tile_max, d_tile_min, d_kept_tiles, FarLists{}, nullptr, stream);
 }
 
 extern "C" __attribute__((visibility("default"))) int nats_b200_visible_counts(const int32_t* d_lim, int B, int Hq, int Hkv, int N, int C,
@@ -516,8 +563,11 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_visible_counts(c
     NATS_CHECK_ARG(B > 0 && Hq > 0 && Hkv > 0 && N > 0 && C > 0 && Hq % Hkv == 0 && (long long)B * Hkv <= 65535,
                    "bad shape B=%d Hq=%d Hkv=%d N=%d C=%d", B, Hq, Hkv, N, C);
     NATS_CHECK_ARG(d_lim && d_n_visible, "null pointer");
-    dim3 grid(cdiv(N, kScanThreads), B * Hkv);
-    visible_count_kernel<<<grid, kScanThreads, 0, (cudaStream_t)stream>>>(d_lim, Hq, Hkv, N, C, cdiv(N, C), d_n_visible);
+    const int Nc = cdiv(N, C);
+    int span = kCountRows / C;
+    span = span < 1 ? 1 : span > kScanThreads ? kScanThreads : span;
+    dim3 grid(cdiv(Nc, span), B * Hkv);
+    visible_count_kernel<<<grid, kScanThreads, 0, (cudaStream_t)stream>>>(d_lim, Hq, Hkv, N, C, Nc, span, d_n_visible);
     NATS_CHECK_CUDA(cudaGetLastError());
     return NATS_OK;
 }
@@ -528,7 +578,7 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_evict_plan(const
     if (int rc = check_common(B, Hkv, N, C, SW)) return rc;
     NATS_CHECK_ARG(d_roles && d_rank && d_size_global && d_size_local && d_state, "null pointer");
     const int Nc = cdiv(N, C);
-    evict_plan_kernel<<<B * Hkv, kScanThreads, 0, (cudaStream_t)stream>>>(
+    evict_plan_kernel<<<B * Hkv, kPrepThreads, 0, (cudaStream_t)stream>>>(
         d_roles, Nc, N / C, C, SW, d_rank, (long long*)d_size_global, (long long*)d_size_local, d_state, nullptr);
     NATS_CHECK_CUDA(cudaGetLastError());
     return NATS_OK;
@@ -537,7 +587,7 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_evict_plan(const
 int nats::role_prep_past(
     const uint8_t* d_roles_new, const uint8_t* d_valid, const int64_t* d_size_global, const int64_t* d_size_local,
     int B, int Hkv, int x_len, int C, int SW, int valid_stride, int t0, int fill, int tail,
-    int32_t* d_lim, int32_t* d_tile_max, int32_t* d_tile_min, int64_t* d_kept_tiles, const FarLists& far, void* stream) {
+    int32_t* d_lim, int32_t* d_tile_max, int32_t* d_tile_min, int64_t* d_kept_tiles, const FarLists& far, int32_t* d_counter, void* stream) {
     if (int rc = check_common(B, Hkv, x_len, C, SW)) return rc;
     NATS_CHECK_ARG(d_roles_new && d_valid && d_size_global && d_size_local && d_lim && d_tile_max && d_tile_min, "null pointer");
     NATS_CHECK_ARG(t0 >= SW && t0 % C == 0 && fill >= 0 && fill < C, "tail offset %d must be a chunk multiple >= the window, fill %d in [0, chunk)", t0, fill);
@@ -552,6 +602,7 @@ int nats::role_prep_past(
     p.Nq = x_len; p.q_off = t0 + fill; p.Nkv = t0 + fill + x_len;
     p.Nc = cdiv(p.Nkv, C); p.Ntk = cdiv(p.Nkv, kTile); p.Nt = cdiv(x_len, kTile);
     p.far = far;
+    p.counter = d_counter;
     role_prep_past_kernel<<<B * Hkv, kPrepThreads, 0, (cudaStream_t)stream>>>(p);
     NATS_CHECK_CUDA(cudaGetLastError());
     return NATS_OK;
@@ -562,7 +613,7 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_role_prep_past(
     int B, int Hkv, int x_len, int C, int SW, int valid_stride, int t0, int fill, int tail,
     int32_t* d_lim, int32_t* d_tile_max, int32_t* d_tile_min, int64_t* d_kept_tiles, void* stream) {
     return role_prep_past(d_roles_new, d_valid, d_size_global, d_size_local, B, Hkv, x_len, C, SW, valid_stride, t0, fill, tail,
-                          d_lim, d_tile_max, d_tile_min, d_kept_tiles, FarLists{}, stream);
+                          d_lim, d_tile_max, d_tile_min, d_kept_tiles, FarLists{}, nullptr, stream);
 }
 
 extern "C" __attribute__((visibility("default"))) int nats_b200_evict_plan_past(
@@ -570,7 +621,7 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_evict_plan_past(
     int64_t* d_size_global, int64_t* d_size_local, int32_t* d_state, void* stream) {
     if (int rc = check_common(B, Hkv, n_tokens, C, SW)) return rc;
     NATS_CHECK_ARG(d_roles_new && d_rank && d_base && d_size_global && d_size_local && d_state, "null pointer");
-    evict_plan_kernel<<<B * Hkv, kScanThreads, 0, (cudaStream_t)stream>>>(
+    evict_plan_kernel<<<B * Hkv, kPrepThreads, 0, (cudaStream_t)stream>>>(
         d_roles_new, cdiv(n_tokens, C), n_tokens / C, C, SW, d_rank, (long long*)d_size_global, (long long*)d_size_local,
         d_state, d_base);
     NATS_CHECK_CUDA(cudaGetLastError());
@@ -583,7 +634,8 @@ static int check_row(int D) {
     return NATS_OK;
 }
 
-extern "C" __attribute__((visibility("default"))) int nats_b200_evict_compact(const void* d_k, const void* d_v, const uint8_t* d_roles, const int32_t* d_rank,
+template <bool F32>
+static int evict_compact_first(const void* d_k, const void* d_v, const uint8_t* d_roles, const int32_t* d_rank,
                                        const int64_t* d_size_global, const int64_t* d_size_local, const int32_t* d_state,
                                        int B, int Hkv, int N, int D, int C, int SW,
                                        void* d_cache_k, void* d_cache_v, uint8_t* d_valid, int Lcap, void* stream) {
@@ -603,9 +655,25 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_evict_compact(co
     p.nB = cdiv(SW, kTokPerBlock);
     const int nC = cdiv(Lcap - SW, kTokPerBlock);
     dim3 grid(p.nB + nC, B * Hkv);
-    evict_compact_kernel<<<grid, kCopyThreads, 0, (cudaStream_t)stream>>>(p);
+    evict_compact_kernel<F32><<<grid, kCopyThreads, 0, (cudaStream_t)stream>>>(p);
     NATS_CHECK_CUDA(cudaGetLastError());
     return NATS_OK;
+}
+
+extern "C" __attribute__((visibility("default"))) int nats_b200_evict_compact(const void* d_k, const void* d_v, const uint8_t* d_roles, const int32_t* d_rank,
+                                       const int64_t* d_size_global, const int64_t* d_size_local, const int32_t* d_state,
+                                       int B, int Hkv, int N, int D, int C, int SW,
+                                       void* d_cache_k, void* d_cache_v, uint8_t* d_valid, int Lcap, void* stream) {
+    return evict_compact_first<false>(d_k, d_v, d_roles, d_rank, d_size_global, d_size_local, d_state, B, Hkv, N, D, C, SW, d_cache_k, d_cache_v,
+                                      d_valid, Lcap, stream);
+}
+
+extern "C" __attribute__((visibility("default"))) int nats_b200_evict_compact_f32(const float* d_k, const float* d_v, const uint8_t* d_roles, const int32_t* d_rank,
+                                       const int64_t* d_size_global, const int64_t* d_size_local, const int32_t* d_state,
+                                       int B, int Hkv, int N, int D, int C, int SW,
+                                       void* d_cache_k, void* d_cache_v, uint8_t* d_valid, int Lcap, void* stream) {
+    return evict_compact_first<true>(d_k, d_v, d_roles, d_rank, d_size_global, d_size_local, d_state, B, Hkv, N, D, C, SW, d_cache_k, d_cache_v,
+                                      d_valid, Lcap, stream);
 }
 
 extern "C" __attribute__((visibility("default"))) int nats_b200_evict_compact_past(
@@ -634,7 +702,29 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_evict_compact_pa
     p.nB = cdiv(SW, kTokPerBlock);
     const int nC = cdiv(Lcap - SW, kTokPerBlock);
     dim3 grid(p.nB + nC, B * Hkv);
-    evict_compact_kernel<<<grid, kCopyThreads, 0, (cudaStream_t)stream>>>(p);
+    evict_compact_kernel<false><<<grid, kCopyThreads, 0, (cudaStream_t)stream>>>(p);
+    NATS_CHECK_CUDA(cudaGetLastError());
+    return NATS_OK;
+}
+
+extern "C" __attribute__((visibility("default"))) int nats_b200_to_bf16(
+    const float* d_x0, void* d_y0, long long n0, const float* d_x1, void* d_y1, long long n1,
+    const float* d_x2, void* d_y2, long long n2, void* stream) {
+    const float* x[3] = {d_x0, d_x1, d_x2};
+    void* y[3] = {d_y0, d_y1, d_y2};
+    const long long n[3] = {n0, n1, n2};
+    Bf16Params p;
+    long long most = 0;
+    for (int a = 0; a < 3; ++a) {
+        NATS_CHECK_ARG(n[a] >= 0 && n[a] % 8 == 0, "element counts must be multiples of 8, got %lld", n[a]);
+        NATS_CHECK_ARG(n[a] == 0 || (x[a] && y[a]), "null pointer");
+        NATS_CHECK_ARG(((uintptr_t)x[a] | (uintptr_t)y[a]) % 16 == 0, "pointers must be 16-byte aligned");
+        p.x[a] = (const uint8_t*)x[a]; p.y[a] = (uint8_t*)y[a]; p.n8[a] = n[a] / 8;
+        most = p.n8[a] > most ? p.n8[a] : most;
+    }
+    if (most == 0) return NATS_OK;
+    const long long blocks = (most + kCopyThreads - 1) / kCopyThreads;
+    to_bf16_kernel<<<(int)(blocks < 148 * 8 ? blocks : 148 * 8), kCopyThreads, 0, (cudaStream_t)stream>>>(p);
     NATS_CHECK_CUDA(cudaGetLastError());
     return NATS_OK;
 }

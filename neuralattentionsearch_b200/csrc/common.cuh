@@ -39,12 +39,12 @@ struct FarLists {
     int32_t* open_max = nullptr;
 };
 
-// the C entry points nats_b200_role_prep / _past with the lists beside the limits
+// the C entry points nats_b200_role_prep / _past with the lists beside the limits; *d_counter (may be null) is set to zero
 int role_prep(const uint8_t* d_roles, int B, int Hkv, int N, int C, int SW, int32_t* d_lim, int32_t* d_tile_max,
-              int32_t* d_tile_min, int64_t* d_kept_tiles, const FarLists& far, void* stream);
+              int32_t* d_tile_min, int64_t* d_kept_tiles, const FarLists& far, int32_t* d_counter, void* stream);
 int role_prep_past(const uint8_t* d_roles_new, const uint8_t* d_valid, const int64_t* d_size_global, const int64_t* d_size_local,
                    int B, int Hkv, int x_len, int C, int SW, int valid_stride, int t0, int fill, int tail,
-                   int32_t* d_lim, int32_t* d_tile_max, int32_t* d_tile_min, int64_t* d_kept_tiles, const FarLists& far, void* stream);
+                   int32_t* d_lim, int32_t* d_tile_max, int32_t* d_tile_min, int64_t* d_kept_tiles, const FarLists& far, int32_t* d_counter, void* stream);
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 inline int cdiv(int a, int b) { return (a + b - 1) / b; }
@@ -68,6 +68,18 @@ __device__ __forceinline__ uint4 ld16_stream(const void* p) {
     asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
+}
+
+// eight fp32 values (two vectors) rounded to bf16
+__device__ __forceinline__ uint4 round8(uint4 lo, uint4 hi) {
+    const uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+    uint32_t r[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const __nv_bfloat162 b = __floats2bfloat162_rn(__uint_as_float(w[2 * i]), __uint_as_float(w[2 * i + 1]));
+        r[i] = *reinterpret_cast<const uint32_t*>(&b);
+    }
+    return make_uint4(r[0], r[1], r[2], r[3]);
 }
 
 }  // namespace nats

@@ -512,7 +512,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 tc_fence_after();
                 const float inv = l_sum > 0.f ? 1.f / l_sum : 0.f;
                 const int qi = hd.t * kTile + row;
-                __nv_bfloat16* orow = p.o + (((size_t)hd.b * p.Hq + hd.head0 + h) * p.N + qi) * D;
+                __nv_bfloat16* orow = (__nv_bfloat16*)p.o + hd.b * p.o_batch + (hd.head0 + h) * p.o_head + qi * p.o_row;
                 if (p.lse != nullptr && qi < p.N)
                     p.lse[((size_t)hd.b * p.Hq + hd.head0 + h) * p.N + qi] = l_sum > 0.f ? m_ref + log2f(l_sum) : -INFINITY;
                 uint32_t oreg[D];

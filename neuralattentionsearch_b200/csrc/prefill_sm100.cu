@@ -58,7 +58,9 @@ constexpr unsigned long long kWaitLimitNs = NATS_WAIT_LIMIT_NS;
 enum : int { kErrQ = 1, kErrKvFull, kErrKvEmpty, kErrSFull, kErrPFull, kErrOFull, kErrList, kErrOEmpty, kErrSmemAlign, kErrPipeLock };
 
 struct PrefillParams {
-    __nv_bfloat16* o;                 // [B,Hq,N,D]
+    void* o;                          // [B,Hq,N,D], or with the heads inside the tokens [B,N,Hq,D]: strides in elements
+    long long o_batch, o_head, o_row;
+    int o_f32;                        // 0: bf16, 1: fp32
     float* lse;                       // [B,Hq,N] or nullptr: log2 of the row's sum of exp2(score * scale * log2 e)
     const int32_t* lim;               // [B,Hkv,Nc]: last query POSITION that may see KV chunk c
     const int32_t* tile_max;          // [B,Hkv,Ntk]: max / min of lim over the chunks of a 128-row KV tile
@@ -69,7 +71,7 @@ struct PrefillParams {
     const int32_t* far_before;
     const int32_t* far_open;
     int32_t* status;
-    int32_t* work_counter;            // next work item; zero at launch
+    int32_t* work_counter;            // next work item; zero at launch (the role metadata kernel in front clears it)
     int total_items;                  // B * Hkv * n_groups * Nt
     // N query rows; query row i sits at position q_off + i of the KV sequence of Nkv rows (a first call has q_off = 0 and
     // Nkv = N; a call over an existing cache attends to the cache rows in front of its own tokens).
@@ -995,7 +997,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                     tc_fence_after();
                     const float inv = l_sum > 0.f ? 1.f / l_sum : 0.f;
                     const int qi = hd.t * kTile + row;           // query row
-                    __nv_bfloat16* orow = p.o + (((size_t)hd.b * p.Hq + hd.head0 + h) * p.N + qi) * D;
+                    const long long o_at = hd.b * p.o_batch + (hd.head0 + h) * p.o_head + qi * p.o_row;
+                    __nv_bfloat16* orow = (__nv_bfloat16*)p.o + o_at;
                     constexpr int OW = D < 128 ? D : 128;          // columns of O held in registers at a time
                     if (p.lse != nullptr && qi < p.N)
                         p.lse[((size_t)hd.b * p.Hq + hd.head0 + h) * p.N + qi] = l_sum > 0.f ? m_ref + log2f(l_sum) : -INFINITY;
@@ -1013,7 +1016,23 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 #ifdef NATS_TRACE
                         { const unsigned long long t_ = clock64(); tr_epi_ld += t_ - tr_t; tr_t = t_; }
 #endif
-                        if (qi < p.N) {
+                        if (p.o_f32) {
+                            if (qi < p.N) {
+                                float* frow = (float*)p.o + o_at + c0;
+#pragma unroll
+                                for (int i = 0; i < OW; i += 8) {
+                                    uint32_t w[8];
+#pragma unroll
+                                    for (int x = 0; x < 8; ++x) w[x] = __float_as_uint(__uint_as_float(oreg[i + x]) * inv);
+                                    if (o_wide) {
+                                        st32(frow + i, w);
+                                    } else {
+                                        st16(frow + i, make_uint4(w[0], w[1], w[2], w[3]));
+                                        st16(frow + i + 4, make_uint4(w[4], w[5], w[6], w[7]));
+                                    }
+                                }
+                            }
+                        } else if (qi < p.N) {
                             // a thread owns a whole output row (D * 2 bytes): 32-byte stores, one full sector each
 #pragma unroll
                             for (int i = 0; i < OW; i += 16) {
@@ -1143,7 +1162,6 @@ static int launch_prefill(const CUtensorMap& mq, const CUtensorMap& mk, const CU
         if (dev >= 0 && dev < kMaxDevices) attr_set[dev] = true;
     }
     NATS_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    NATS_CHECK_CUDA(cudaMemsetAsync(p.work_counter, 0, sizeof(int32_t), st));
     const int grid = p.total_items < sms ? p.total_items : sms;      // one persistent CTA per SM
     prefill_kernel<D, FINE><<<grid, kPrefillThreads, smem, st>>>(mq, mk, mv, mkf, mvf, p);
     NATS_CHECK_CUDA(cudaGetLastError());
@@ -1182,8 +1200,8 @@ static bool use_pair_kernel(int D, int nrep) {
 static int run_prefill(const void* d_q, const void* d_k, const void* d_v, void* d_o, int B, int Hq, int Hkv, int N, int Nkv,
                        int q_off, long long kv_head_stride, int D, int C, float sm_scale, const int32_t* lim,
                        const int32_t* tmax, const int32_t* tmin, int32_t* counter, int32_t* d_status, cudaStream_t st,
-                       const FarLists& far, float* d_lse = nullptr) {
-    const bool pair = use_pair_kernel(D, Hq / Hkv);
+                       const FarLists& far, float* d_lse = nullptr, bool o_tokens = false, bool o_f32 = false) {
+    const bool pair = use_pair_kernel(D, Hq / Hkv) && !o_f32;
     CUtensorMap mq, mk, mv, mkf, mvf;
     if (int rc = make_map(&mq, d_q, B * Hq, N, D, 128)) return rc;
     if (int rc = make_map(&mk, d_k, B * Hkv, Nkv, D, pair ? 64 : 128, kv_head_stride)) return rc;     // a pair's CTA loads half the rows of a K tile
@@ -1200,7 +1218,11 @@ static int run_prefill(const void* d_q, const void* d_k, const void* d_v, void* 
     }
     PrefillParams p;
     p.far_list = far.list; p.far_before = far.before_tile; p.far_open = far.open_max; p.head_rows = (int)head_rows;
-    p.o = (__nv_bfloat16*)d_o; p.lse = d_lse; p.lim = lim; p.tile_max = tmax; p.tile_min = tmin; p.status = d_status;
+    p.o_batch = (long long)N * Hq * D;
+    p.o_head = o_tokens ? D : (long long)N * D;
+    p.o_row = o_tokens ? (long long)Hq * D : D;
+    p.o_f32 = o_f32;
+    p.o = d_o; p.lse = d_lse; p.lim = lim; p.tile_max = tmax; p.tile_min = tmin; p.status = d_status;
     p.Hq = Hq; p.Hkv = Hkv; p.N = N; p.Nkv = Nkv; p.q_off = q_off; p.C = C;
     p.c_shift = (C & (C - 1)) ? -1 : __builtin_ctz((unsigned)C);
     p.Nc = cdiv(Nkv, C); p.Nt = cdiv(N, kTile); p.Ntk = cdiv(Nkv, kTile);
@@ -1239,7 +1261,8 @@ extern "C" __attribute__((visibility("default"))) size_t nats_b200_prefill_works
 static int prefill_first_call(const void* d_q, const void* d_k, const void* d_v, void* d_o, const uint8_t* d_roles,
                               int B, int Hq, int Hkv, int N, int D, int C, int SW, float sm_scale,
                               void* d_workspace, size_t workspace_bytes, int64_t* d_kept_tiles, int32_t* d_status,
-                              void* stream, float* d_lse, int32_t* d_n_visible) {
+                              void* stream, float* d_lse, int32_t* d_n_visible, bool o_tokens = false,
+                              bool o_f32 = false) {
     NATS_CHECK_ARG(B > 0 && Hq > 0 && Hkv > 0 && N > 0 && Hq % Hkv == 0, "bad shape B=%d Hq=%d Hkv=%d N=%d", B, Hq, Hkv, N);
     NATS_CHECK_ARG(C > 0 && SW > 0 && SW % C == 0, "sliding window %d must be a positive multiple of the chunk size %d", SW, C);
     NATS_CHECK_ARG(d_q && d_k && d_v && d_o && d_roles && d_workspace && d_status, "null pointer");
@@ -1257,13 +1280,13 @@ static int prefill_first_call(const void* d_q, const void* d_k, const void* d_v,
     int32_t* tmax = (int32_t*)(ws + w.tmax);
     int32_t* tmin = (int32_t*)(ws + w.tmin);
     FarLists far;
-    if (use_far_lists(w, workspace_bytes, B, Hkv, N, 0, N, use_pair_kernel(D, Hq / Hkv)))
+    if (use_far_lists(w, workspace_bytes, B, Hkv, N, 0, N, use_pair_kernel(D, Hq / Hkv) && !o_f32))
         far = {(int32_t*)(ws + w.list), (int32_t*)(ws + w.before), (int32_t*)(ws + w.open)};
-    if (int rc = role_prep(d_roles, B, Hkv, N, C, SW, lim, tmax, tmin, d_kept_tiles, far, stream)) return rc;
+    if (int rc = role_prep(d_roles, B, Hkv, N, C, SW, lim, tmax, tmin, d_kept_tiles, far, (int32_t*)(ws + w.counter), stream)) return rc;
     if (d_n_visible != nullptr)
         if (int rc = nats_b200_visible_counts(lim, B, Hq, Hkv, N, C, d_n_visible, stream)) return rc;
     return run_prefill(d_q, d_k, d_v, d_o, B, Hq, Hkv, N, N, 0, 0, D, C, sm_scale, lim, tmax, tmin,
-                       (int32_t*)(ws + w.counter), d_status, (cudaStream_t)stream, far, d_lse);
+                       (int32_t*)(ws + w.counter), d_status, (cudaStream_t)stream, far, d_lse, o_tokens, o_f32);
 }
 
 extern "C" __attribute__((visibility("default"))) int nats_b200_prefill_fwd(const void* d_q, const void* d_k, const void* d_v, void* d_o, const uint8_t* d_roles,
@@ -1272,6 +1295,14 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_prefill_fwd(cons
                                      void* stream) {
     return prefill_first_call(d_q, d_k, d_v, d_o, d_roles, B, Hq, Hkv, N, D, C, SW, sm_scale, d_workspace, workspace_bytes,
                               d_kept_tiles, d_status, stream, nullptr, nullptr);
+}
+
+extern "C" __attribute__((visibility("default"))) int nats_b200_prefill_fwd_out(
+    const void* d_q, const void* d_k, const void* d_v, void* d_o, int o_tokens, int o_f32, const uint8_t* d_roles,
+    int B, int Hq, int Hkv, int N, int D, int C, int SW, float sm_scale, void* d_workspace, size_t workspace_bytes,
+    int64_t* d_kept_tiles, int32_t* d_status, void* stream) {
+    return prefill_first_call(d_q, d_k, d_v, d_o, d_roles, B, Hq, Hkv, N, D, C, SW, sm_scale, d_workspace, workspace_bytes,
+                              d_kept_tiles, d_status, stream, nullptr, nullptr, o_tokens != 0, o_f32 != 0);
 }
 
 extern "C" __attribute__((visibility("default"))) int nats_b200_prefill_fwd_stats(
@@ -1318,7 +1349,7 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_prefill_past_fwd
     if (use_far_lists(w, workspace_bytes, B, Hkv, x_len, t0 + fill, cache_capacity, use_pair_kernel(D, Hq / Hkv)))
         far = {(int32_t*)(ws + w.list), (int32_t*)(ws + w.before), (int32_t*)(ws + w.open)};
     if (int rc = role_prep_past(d_roles_new, d_valid, d_size_global, d_size_local, B, Hkv, x_len, C, SW,
-                                          valid_stride, t0, fill, tail, lim, tmax, tmin, d_kept_tiles, far, stream)) return rc;
+                                          valid_stride, t0, fill, tail, lim, tmax, tmin, d_kept_tiles, far, (int32_t*)(ws + w.counter), stream)) return rc;
     return run_prefill(d_q, d_cache_k, d_cache_v, d_o, B, Hq, Hkv, x_len, (int)n_kv, t0 + fill, cache_capacity, D, C, sm_scale,
                        lim, tmax, tmin, (int32_t*)(ws + w.counter), d_status, (cudaStream_t)stream, far);
 }

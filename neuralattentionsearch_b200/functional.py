@@ -197,11 +197,28 @@ def _as_bf16(t: torch.Tensor) -> torch.Tensor:
     return t.to(torch.bfloat16).contiguous()
 
 
+def is_plain_fp32(t: torch.Tensor) -> bool:
+    """What the kernels that round fp32 on the way can read: contiguous, 16-byte aligned, whole groups of eight."""
+    return t.dtype == torch.float32 and t.is_contiguous() and t.data_ptr() % 16 == 0 and t.numel() % 8 == 0
+
+
+def _qkv_as_bf16(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor):
+    """bf16 copies of q, k, v; fp32 inputs are rounded in one launch."""
+    if not (is_plain_fp32(q) and is_plain_fp32(k) and is_plain_fp32(v)):
+        return _as_bf16(q), _as_bf16(k), _as_bf16(v)
+    outs = [torch.empty_like(t, dtype=torch.bfloat16) for t in (q, k, v)]
+    _call(q.device, 'nats_b200_to_bf16', _p(q), _p(outs[0]), q.numel(), _p(k), _p(outs[1]), k.numel(), _p(v), _p(outs[2]), v.numel(),
+          _stream(q.device))
+    return outs
+
+
 def prefill_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, roles: torch.Tensor, chunk_size: int,
                       sliding_window: int, sm_scale: float | None = None,
-                      kept_tiles: torch.Tensor | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
+                      kept_tiles: torch.Tensor | None = None, out: torch.Tensor | None = None,
+                      token_major: bool = False) -> torch.Tensor:
     """Role-masked causal attention of a first prefill call.  q [B,Hq,N,D], k/v [B,Hkv,N,D] (cast to bf16 if
-    needed), roles uint8 [B,Hkv,ceil(N/C)].  Returns o [B,Hq,N,D] in q's dtype."""
+    needed), roles uint8 [B,Hkv,ceil(N/C)].  Returns o [B,Hq,N,D] in q's dtype.  ``token_major=True``: o is a view of a
+    [B,N,Hq,D] tensor, so that ``o.transpose(1, 2)`` is contiguous (what an output projection reads)."""
     dev = _need_cuda(q, k, v, roles)
     B, Hq, N, D = q.shape
     Hkv = k.shape[1]
@@ -212,7 +229,7 @@ def prefill_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, roles: 
         raise ValueError(f'roles must be uint8 [{B},{Hkv},{nc}], got {roles.dtype} {tuple(roles.shape)}')
     _check_head_dim(D)
     scale = (1.0 / math.sqrt(D)) if sm_scale is None else float(sm_scale)
-    qb, kb, vb = _as_bf16(q), _as_bf16(k), _as_bf16(v)
+    qb, kb, vb = _qkv_as_bf16(q, k, v)
     if D in PADDED_HEAD_DIMS:
         # narrow heads run in the 64-wide kernel on zero-padded copies: the scores are unchanged by zero columns of q and
         # k, the extra output columns are zero and dropped (the scale still comes from the real head_dim)
@@ -222,15 +239,22 @@ def prefill_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, roles: 
         qb, kb, vb = (torch.nn.functional.pad(t, pad) for t in (qb, kb, vb))
     if out is not None and (out.shape != qb.shape or out.dtype != torch.bfloat16 or not out.is_contiguous()):
         raise ValueError('out must be a contiguous bf16 tensor shaped like q')
-    o = torch.empty_like(qb) if out is None else out
+    padded = D in PADDED_HEAD_DIMS
+    o_f32 = q.dtype == torch.float32 and out is None and not padded       # the kernel writes fp32 itself
+    token_major = token_major and out is None and not padded
+    if out is not None or padded:
+        o = torch.empty_like(qb) if out is None else out
+    else:
+        dtype = torch.float32 if o_f32 else torch.bfloat16
+        o = torch.empty(B, N, Hq, D, dtype=dtype, device=dev).transpose(1, 2) if token_major else torch.empty(B, Hq, N, D, dtype=dtype, device=dev)
     lib = _lib.lib()
     nbytes = lib.nats_b200_prefill_workspace_bytes(B, Hkv, N, chunk_size)
     ws = _workspace('prefill', dev, nbytes)
-    _call(dev, 'nats_b200_prefill_fwd', _p(qb), _p(kb), _p(vb), _p(o), _p(roles.contiguous()), B, Hq, Hkv, N, qb.shape[-1],
-              chunk_size, sliding_window, scale, _p(ws), ws.numel(), _p(kept_tiles), _p(status_word(dev)), _stream(dev))
-    if D in PADDED_HEAD_DIMS:
+    _call(dev, 'nats_b200_prefill_fwd_out', _p(qb), _p(kb), _p(vb), _p(o), int(token_major), int(o_f32), _p(roles.contiguous()), B, Hq, Hkv, N,
+              qb.shape[-1], chunk_size, sliding_window, scale, _p(ws), ws.numel(), _p(kept_tiles), _p(status_word(dev)), _stream(dev))
+    if padded:
         o = o[..., :D].contiguous()
-    return o if q.dtype == torch.bfloat16 else o.to(q.dtype)
+    return o if o.dtype == q.dtype else o.to(q.dtype)
 
 
 class HostPrefillPipeline:
@@ -438,8 +462,9 @@ def evict_plan(roles: torch.Tensor, n: int, chunk_size: int, sliding_window: int
 def evict_compact(k: torch.Tensor, v: torch.Tensor, roles: torch.Tensor, rank: torch.Tensor, size_global: torch.Tensor,
                   size_local: torch.Tensor, state: torch.Tensor, chunk_size: int, sliding_window: int,
                   cache_k: torch.Tensor, cache_v: torch.Tensor, valid: torch.Tensor) -> None:
+    """K / V bf16, or fp32 (see ``is_plain_fp32``), which is rounded as it is moved."""
     B, H, N, D = k.shape
-    _call(k.device, 'nats_b200_evict_compact', _p(k), _p(v), _p(roles), _p(rank), _p(size_global), _p(size_local), _p(state),
+    _call(k.device, 'nats_b200_evict_compact_f32' if k.dtype == torch.float32 else 'nats_b200_evict_compact', _p(k), _p(v), _p(roles), _p(rank), _p(size_global), _p(size_local), _p(state),
               B, H, N, D, chunk_size, sliding_window, _p(cache_k), _p(cache_v), _p(valid), cache_k.shape[2],
               _stream(k.device))
 

@@ -94,7 +94,7 @@ def forward_llama_nats_chunk_one_way(self, hidden_states: torch.Tensor, position
     scale = hd ** -0.5
     if start_pos == 0:
         out = F_.prefill_attention(q, keys, values, F_.roles_from_token_states_info(info), self.chunk_size,
-                                   self.local_seq_max_length, scale)
+                                   self.local_seq_max_length, scale, token_major=True)
     elif q_len == 1:
         out = layer_cache.decode_attention(q, scale)
     else:

@@ -1,0 +1,105 @@
+"""Role metadata kernels whose blocks go over the chunks in several steps: sizes around the step and the block."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import nats_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(1, 1, 4), (1023, 1, 4), (1024, 1, 4), (1025, 1, 64), (5000, 1, 256), (3001, 2, 64), (4097, 16, 64), (9000, 48, 96), (70000, 32, 128), (9000, 5000, 5000)]
+
+
+def dev():
+    return torch.device('cuda', 0)
+
+
+def draw_roles(B, H, Nc, seed):
+    roles = orc.make_roles(B, H, Nc, 0.05, 0.3, seed=seed)
+    roles[0, 0] = orc.ROLE_LOCAL                                # a head without a global chunk
+    roles[-1, -1, Nc // 2:] = orc.ROLE_SLIDING
+    return roles
+
+
+@pytest.mark.parametrize('N,C,SW', SHAPES)
+def test_row_limits_and_visible_counts(N, C, SW):
+    from neuralattentionsearch_b200 import _lib
+    B, H, rep = 2, 2, 3
+    Nc, Nt = -(-N // C), -(-N // 128)
+    roles = draw_roles(B, H, Nc, N)
+    r = torch.from_numpy(roles).to(dev())
+    lim = torch.empty(B, H, Nc, dtype=torch.int32, device=dev())
+    tmax, tmin = (torch.empty(B, H, Nt, dtype=torch.int32, device=dev()) for _ in range(2))
+    n_vis = torch.empty(B, H * rep, N, dtype=torch.int32, device=dev())
+    _lib.call('nats_b200_role_prep', r.data_ptr(), B, H, N, C, SW, lim.data_ptr(), tmax.data_ptr(), tmin.data_ptr(), None, None)
+    _lib.call('nats_b200_visible_counts', lim.data_ptr(), B, H * rep, H, N, C, n_vis.data_ptr(), None)
+    ref = np.minimum(orc.row_limit(roles, C, SW), orc.NO_LIMIT).astype(np.int64)
+    assert np.array_equal(lim.cpu().numpy(), ref)
+    for b in range(B):
+        for h in range(H):
+            d = np.ones(N + 1, np.int64)                         # key q appears at row q, key k leaves behind row lim
+            size = np.minimum(np.arange(1, Nc + 1) * C, N) - np.arange(Nc) * C
+            np.subtract.at(d, np.minimum(ref[b, h] + 1, N), size)
+            want = np.cumsum(d[:N])
+            got = n_vis.cpu().numpy()[b, h * rep:(h + 1) * rep]
+            assert (got == want).all()
+
+
+@pytest.mark.parametrize('N,C,SW', SHAPES)
+def test_eviction_plan(N, C, SW):
+    from neuralattentionsearch_b200 import functional as F_
+    B, H = 2, 2
+    Nc, full = -(-N // C), N // C
+    roles = draw_roles(B, H, Nc, N + 1)
+    r = torch.from_numpy(roles).to(dev())
+    rank = torch.empty(B, H, Nc, dtype=torch.int32, device=dev())
+    sg, sl = (torch.empty(B, H, dtype=torch.long, device=dev()) for _ in range(2))
+    state = torch.zeros(8, dtype=torch.int32, device=dev())
+    F_.evict_plan(r, N, C, SW, rank, sg, sl, state)
+    lens = []
+    for b in range(B):
+        for h in range(H):
+            x = roles[b, h, :full]
+            g = x == orc.ROLE_GLOBAL
+            last = np.flatnonzero(g)[-1] if g.any() else -1
+            keep = np.zeros(Nc, bool)
+            keep[:full] = g | ((x == orc.ROLE_LOCAL) & (np.arange(full) > last))
+            before = np.cumsum(keep) - keep
+            assert np.array_equal(rank[b, h].cpu().numpy(), np.where(keep, before, -1 - before))
+            assert sg[b, h].item() == SW + C * g.sum() and sl[b, h].item() == C * (keep.sum() - g.sum())
+            lens.append(SW + C * keep.sum())
+    assert state.cpu().tolist() == [max(lens), 0, 0, 0, 0, 0, 0, 0]
+
+
+def test_output_in_token_order_holds_the_same_bits():
+    from neuralattentionsearch_b200 import prefill_attention
+    g = torch.Generator().manual_seed(0)
+    for B, Hq, Hkv, N, D in ((2, 6, 2, 700, 64), (1, 8, 4, 513, 128), (2, 2, 2, 200, 256), (1, 4, 2, 150, 32)):
+        q, k, v = (torch.randn(B, h, N, D, generator=g).mul_(0.5).to(dev()).bfloat16() for h in (Hq, Hkv, Hkv))
+        roles = torch.from_numpy(orc.make_roles(B, Hkv, -(-N // 32), 0.1, 0.3, seed=N)).to(dev())
+        a = prefill_attention(q, k, v, roles, 32, 128)
+        b = prefill_attention(q, k, v, roles, 32, 128, token_major=True)
+        assert b.shape == a.shape and torch.equal(a, b)
+        assert D == 32 or b.transpose(1, 2).is_contiguous()
+
+
+@pytest.mark.parametrize('B,Hq,Hkv,N,D,C,SW', [(1, 4, 4, 1000, 64, 16, 64), (2, 8, 2, 513, 128, 1, 32), (1, 2, 2, 300, 256, 64, 128), (1, 2, 1, 9, 64, 8, 8)])
+def test_fp32_prompts_are_rounded_by_the_kernels(B, Hq, Hkv, N, D, C, SW):
+    """q, k, v in fp32: the output before its rounding to bf16, the cache bytes of a prompt given in bf16; also for tensors the
+    rounding kernels do not take (not contiguous)."""
+    from neuralattentionsearch_b200 import NAtSChunkLayerCache, prefill_attention
+    g = torch.Generator().manual_seed(N)
+    q, k, v = (torch.randn(B, h, N, D, generator=g).mul_(0.5).to(dev()) for h in (Hq, Hkv, Hkv))
+    roles = torch.from_numpy(orc.make_roles(B, Hkv, -(-N // C), 0.2, 0.3, seed=N)).to(dev())
+    outs, caches = [], []
+    strided = [t.transpose(1, 2).contiguous().transpose(1, 2) for t in (q, k, v)]
+    for qq, kk, vv in ((q, k, v), strided, [t.bfloat16() for t in (q, k, v)]):
+        cache = NAtSChunkLayerCache(B, Hkv, SW, chunk_size=C, device=dev())
+        cache.update(kk, vv, roles)
+        outs.append(prefill_attention(qq, kk, vv, roles, C, SW))
+        cache.post_update(N)
+        caches.append(cache)
+    assert outs[0].dtype == outs[1].dtype == torch.float32 and outs[2].dtype == torch.bfloat16
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0].bfloat16(), outs[2])
+    for c in caches[:2]:
+        assert torch.equal(c.cache_k, caches[2].cache_k) and torch.equal(c.cache_v, caches[2].cache_v) and torch.equal(c.valid_tokens, caches[2].valid_tokens)
