@@ -18,6 +18,7 @@ SIGNATURES = {
     'nats_b200_build_info': (_c.c_char_p, []),
     'nats_b200_role_prep': (_I, [_P, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P]),
     'nats_b200_prefill_workspace_bytes': (_SZ, [_I, _I, _I, _I]),
+    'nats_b200_prefill_workspace_bytes_for': (_SZ, [_I, _I, _I, _I, _I]),
     'nats_b200_prefill_fwd': (_I, [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _P, _SZ, _P, _P, _P]),
     'nats_b200_prefill_fwd_out': (_I, [_P, _P, _P, _P, _I, _I, _P, _I, _I, _I, _I, _I, _I, _I, _F, _P, _SZ, _P, _P, _P]),
     'nats_b200_to_bf16': (_I, [_P, _P, _c.c_longlong, _P, _P, _c.c_longlong, _P, _P, _c.c_longlong, _P]),

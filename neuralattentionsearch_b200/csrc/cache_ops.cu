@@ -103,8 +103,8 @@ __device__ unsigned long long tile_limits(const int32_t* __restrict__ lim, int N
 
 // The chunks that stay visible for good, in order, and how many of them lie in front of every 128-row tile (chunks divide a
 // tile: cpt per tile).  All threads of the block call, after scan_role_limits.
-__device__ void list_far_chunks(const int32_t* __restrict__ lim, int Nc, int cpt, int32_t* __restrict__ list,
-                                int32_t* __restrict__ before_tile, int (*s)[kPrepWarps]) {
+__device__ void list_far_chunks(const int32_t* __restrict__ lim, int Nc, int cpt, int Ntk, int32_t* __restrict__ list,
+                                int32_t* __restrict__ before_tile, int32_t* __restrict__ open_max, int max_listed, int (*s)[kPrepWarps]) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int base = 0, buf = 0;
     for (int c0 = 0; c0 < Nc; c0 += kPrepThreads, buf ^= 1) {
@@ -119,6 +119,11 @@ __device__ void list_far_chunks(const int32_t* __restrict__ lim, int Nc, int cpt
         if (c < Nc && c % cpt == 0) before_tile[c / cpt] = rank;
         base += __reduce_add_sync(0xffffffffu, all);
     }
+    if (tid == 0) before_tile[Ntk] = base;
+    if (base <= max_listed) return;
+    __syncthreads();
+    for (int kt = tid; kt < Ntk; kt += kPrepThreads)
+        if (before_tile[kt + 1] > max_listed) open_max[kt] = kNoLimit;
 }
 
 __global__ void __launch_bounds__(kPrepThreads)
@@ -138,7 +143,8 @@ role_prep_kernel(const uint8_t* __restrict__ roles, int Nc, int N, int C, int SW
     scan_role_limits(roles, Nc, C, SW, 0, lim, s, &first_gf);
     const unsigned long long mine = tile_limits(lim, N, C, Nt, 0, Nt, tmax, tmin, far.list ? far.open_max + (size_t)bh * Nt : nullptr);
     if (far.list != nullptr)
-        list_far_chunks(lim, Nc, kTile / C, far.list + (size_t)bh * Nc, far.before_tile + (size_t)bh * Nt, s);
+        list_far_chunks(lim, Nc, kTile / C, Nt, far.list + (size_t)bh * Nc, far.before_tile + (size_t)bh * (Nt + 1), far.open_max + (size_t)bh * Nt,
+                        far.max_listed, s);
     if (kept != nullptr) {
         if (mine) atomicAdd(&kept_sm, mine);
         __syncthreads();
@@ -193,7 +199,8 @@ __global__ void __launch_bounds__(kPrepThreads) role_prep_past_kernel(const Past
     const unsigned long long mine = tile_limits(lim, p.Nkv, p.C, p.Ntk, p.q_off, p.Nt, p.tmax + (size_t)bh * p.Ntk, p.tmin + (size_t)bh * p.Ntk,
                                                 p.far.list ? p.far.open_max + (size_t)bh * p.Ntk : nullptr);
     if (p.far.list != nullptr)
-        list_far_chunks(lim, p.Nc, kTile / p.C, p.far.list + (size_t)bh * p.Nc, p.far.before_tile + (size_t)bh * p.Ntk, s);
+        list_far_chunks(lim, p.Nc, kTile / p.C, p.Ntk, p.far.list + (size_t)bh * p.Nc, p.far.before_tile + (size_t)bh * (p.Ntk + 1),
+                        p.far.open_max + (size_t)bh * p.Ntk, p.far.max_listed, s);
     if (p.kept != nullptr) {
         if (mine) atomicAdd(&kept_sm, mine);
         __syncthreads();

@@ -12,11 +12,12 @@
 //   warps 8-11  softmax of head slot 1  softmax in registers, P written back over S as packed bf16
 //
 // Chunks finer than a tile: far behind the queries only the global chunks are still visible, a few in every tile.  Those
-// are not computed in place but gathered: the keys of 128 / C listed chunks (FarLists) make a full tile, copied chunk by
-// chunk (boxes of C rows) or, below 8 rows, with tile::gather4.  The bitmap then only holds the tiles from the first one on
-// in which some other chunk is still visible.  The work of a query tile falls from the tiles that hold a visible key towards
-// the keys that are visible: prompt of 8192 tokens with one role per token, 10 % global, 0.91 -> 0.29 ms; forward of
-// 8 x 4096 tokens with chunks of 16, 0.51 -> 0.26 ms.
+// are not computed in place but gathered: the keys of 128 / C listed chunks (FarLists) make a full tile.  Chunks of 8 rows and
+// more are copied chunk by chunk (boxes of C rows); finer ones come from a copy of the listed rows in the workspace, made once
+// per call (far_rows_kernel), since single rows arrive at ~8 cycles each from tile::gather4, 4000 for a K / V tile pair.  The
+// bitmap then only holds the tiles from the first one on in which some other chunk is still visible.  The work of a query
+// tile falls from the tiles that hold a visible key towards the keys that are visible: prompt of 8192 tokens with one role
+// per token, 10 % global, 0.91 -> 0.21 ms (0.29 with tile::gather4); forward of 8 x 4096 tokens with chunks of 16, 0.51 -> 0.26 ms.
 // Which KV tiles are visited comes from the role bitmap: a bitmap of kept tiles is built in shared memory from the
 // per-tile max / min row limits (nats_b200_role_prep); tiles without a visible entry are never loaded.  Only tiles
 // whose min limit does not cover the whole query tile (and the diagonal) pay for per-element masking.
@@ -78,7 +79,6 @@ struct PrefillParams {
     // Nc / Ntk: chunks / 128-row tiles of the KV sequence, Nt: query tiles.
     int Hq, Hkv, N, Nkv, q_off, C, Nc, Nt, Ntk, nrep, n_groups;   // n_groups = ceil(nrep / heads per item)
     int c_shift;                      // log2(C), -1 if C is no power of two
-    int head_rows;                    // rows from one kv-head to the next
 
     float scale_log2;
 };
@@ -149,12 +149,6 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
     asm volatile(
         "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5}], [%2], %6;"
         ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "l"(policy) : "memory");
-}
-// four rows (r0 .. r3 of a 2-D map whose box is one row high), 64 columns from c0
-__device__ __forceinline__ void tma_gather4(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int r0, int r1, int r2, int r3, uint64_t policy) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5, %6, %7}], [%2], %8;"
-        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(r0), "r"(r1), "r"(r2), "r"(r3), "l"(policy) : "memory");
 }
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
@@ -576,7 +570,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 }
                 int far_keys = 0;
                 if (open != nullptr) {
-                    far_keys = p.far_before[(size_t)bh * p.Ntk + near_first] * p.C;
+                    far_keys = p.far_before[(size_t)bh * (p.Ntk + 1) + near_first] * p.C;
                     n_kept += (far_keys + kTile - 1) / kTile;
                 }
                 if (lane == 0) {
@@ -642,23 +636,16 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             for (int j = 0; j < hd.n_kept && ok; ++j) {
                 bool partial;
                 const bool far = FINE && j < n_far;
-                const int row0 = far ? 0 : walk.next(partial) * kTile;
-                // rows of a gathered tile.  Chunks of 8 rows and more: lane i copies whole chunks, i-th of the tile, 32 rows
-                // further on, ...; a slot behind the last listed chunk takes rows behind the sequence, which read as zero.
-                // Finer chunks: lane i copies the four rows 4 i .. 4 i + 3; a key behind the last one repeats the last one.
-                // Both kinds of filler are masked.
-                int4 rows = make_int4(0, 0, 0, 0);
+                const int row0 = far ? j * kTile : walk.next(partial) * kTile;
+                // Rows of a gathered tile: of the copy of the listed rows, or (chunks of 8 rows and more) lane i copies the i-th
+                // chunk of the tile; a slot behind the last listed chunk takes rows behind the sequence, which read as zero.
+                // Filler keys are masked.
                 const int cpt = far ? kTile >> p.c_shift : 1;
-                if (far && p.C < 8) {
-                    int* r = &rows.x;
-#pragma unroll
-                    for (int x = 0; x < 4; ++x) {
-                        const int key = min(j * kTile + lane * 4 + x, hd.far_keys - 1);
-                        r[x] = hd.bh * p.head_rows + far_list[key / p.C] * p.C + key % p.C;
-                    }
-                } else if (far) {
+                const bool boxes = far && p.C >= 8;
+                int box_row = 0;
+                if (boxes) {
                     const int i = j * cpt + (lane & (cpt - 1));
-                    rows.x = i * p.C < hd.far_keys ? far_list[i] * p.C : p.Nkv;
+                    box_row = i * p.C < hd.far_keys ? far_list[i] * p.C : p.Nkv;
                 }
 #pragma unroll 1
                 for (int kv = 0; kv < 2 && ok; ++kv, ++g) {
@@ -680,24 +667,19 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 #endif
                     if (lane == 0 && !withhold) {
                         mbar_expect_tx(smem_u32(&sm.bar_full[s]), TILE_BYTES);
-                        if (!far) {
-                            const CUtensorMap* map = kv == 0 ? &map_k : &map_v;
+                        if (!boxes) {
+                            const CUtensorMap* map = kv == 0 ? (far ? &map_k_far : &map_k) : (far ? &map_v_far : &map_v);
                             for (int x = 0; x < NBOX; ++x)
                                 tma_load_3d(smem_u32(&sm.ring[s][x * kBoxBytes]), map, smem_u32(&sm.bar_full[s]), x * 64, row0, hd.bh, pol_kv);
                         }
                     }
                     __syncwarp();
-                    if (far && !withhold) {
+                    if (boxes && !withhold) {
                         const CUtensorMap* map = kv == 0 ? &map_k_far : &map_v_far;
                         const uint32_t dst = smem_u32(&sm.ring[s][0]), bar = smem_u32(&sm.bar_full[s]);
-                        if (p.C < 8) {
-                            for (int x = 0; x < NBOX; ++x)
-                                tma_gather4(dst + x * kBoxBytes + lane * 512, map, bar, x * 64, rows.x, rows.y, rows.z, rows.w, pol_kv);
-                        } else {
-                            // cpt <= 16 divides 32: the lanes of a chunk share its boxes
-                            for (int x = lane / cpt; x < NBOX; x += 32 / cpt)
-                                tma_load_3d(dst + x * kBoxBytes + (lane & (cpt - 1)) * p.C * 128, map, bar, x * 64, rows.x, hd.bh, pol_kv);
-                        }
+                        // cpt <= 16 divides 32: the lanes of a chunk share its boxes
+                        for (int x = lane / cpt; x < NBOX; x += 32 / cpt)
+                            tma_load_3d(dst + x * kBoxBytes + (lane & (cpt - 1)) * p.C * 128, map, bar, x * 64, box_row, hd.bh, pol_kv);
                         __syncwarp();
                     }
                 }
@@ -1103,8 +1085,8 @@ static EncodeTiledFn get_encode_fn() {
 
 // [heads, N, D] bf16 viewed as a 3-D tensor (D innermost); box = 64 x box_rows x 1 with 128-byte swizzle; rows past N read zero
 // 3-D map over [heads, rows, D] bf16; consecutive heads are head_stride_rows rows apart (>= rows: a cache buffer is
-// longer than the part of it that is valid; rows behind `rows` read as zero).  flat: a 2-D map over `rows` rows.
-static int make_map(CUtensorMap* map, const void* base, long long heads, long long N, int D, int box_rows, long long head_stride_rows = 0, bool flat = false) {
+// longer than the part of it that is valid; rows behind `rows` read as zero).
+static int make_map(CUtensorMap* map, const void* base, long long heads, long long N, int D, int box_rows, long long head_stride_rows = 0) {
     EncodeTiledFn fn = get_encode_fn();
     if (!fn) return fail(NATS_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     if (head_stride_rows <= 0) head_stride_rows = N;
@@ -1112,39 +1094,84 @@ static int make_map(CUtensorMap* map, const void* base, long long heads, long lo
     cuuint64_t strides[2] = {(cuuint64_t)D * 2, (cuuint64_t)head_stride_rows * D * 2};
     cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
     cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, flat ? 2 : 3, const_cast<void*>(base), dims, strides, box, estr,
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(NATS_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
     return NATS_OK;
 }
 
-struct PrefillWs { size_t lim, tmax, tmin, counter, total, list, before, open, total_far; };
-// N = rows of the KV sequence.  `total` bytes are enough for any call; with `total_far` bytes the lists of the chunks that
-// stay visible have room behind them (0: this chunk size has no such lists).
-static PrefillWs prefill_ws(int B, int Hkv, int N, int C) {
+struct PrefillWs { size_t lim, tmax, tmin, counter, total, list, before, open, rows_k, rows_v, total_far; int row_cap; };
+// N = rows of the KV sequence.  `total` bytes are enough for any call; with `total_far` bytes there is room for what the
+// gathered tiles need (0: this chunk size has none): the lists of the chunks that stay visible and, for chunks below 8 rows,
+// copies of their K and V rows, up to row_cap (a quarter of the sequence) per head.  D = 0: the head_dim is not known, so that
+// there is no room for rows.
+static PrefillWs prefill_ws(int B, int Hkv, int N, int C, int D) {
     PrefillWs w = {};
-    const size_t Nc = cdiv(N, C), Nt = cdiv(N, kTile);
-    const size_t per_tile = align_up((size_t)B * Hkv * Nt * 4, 256), per_chunk = align_up((size_t)B * Hkv * Nc * 4, 256);
+    const size_t BH = (size_t)B * Hkv, Nc = cdiv(N, C), Nt = cdiv(N, kTile);
+    const size_t per_tile = align_up(BH * Nt * 4, 256), per_chunk = align_up(BH * Nc * 4, 256);
     w.lim = 0;
     w.tmax = per_chunk;
     w.tmin = w.tmax + per_tile;
     w.counter = w.tmin + per_tile;
     w.total = w.counter + 256;
-    if (C < kTile && kTile % C == 0) {
+    if (C < kTile && kTile % C == 0 && (C >= 8 || D > 0)) {
         w.list = w.total;
         w.before = w.list + per_chunk;
-        w.open = w.before + per_tile;
-        w.total_far = w.open + per_tile;
+        w.open = w.before + align_up(BH * (Nt + 1) * 4, 256);
+        w.rows_k = w.rows_v = w.total_far = w.open + per_tile;
+        if (C < 8) {
+            w.row_cap = (N / 4 + kTile - 1) / kTile * kTile;
+            w.rows_v = w.rows_k + BH * w.row_cap * D * 2;
+            w.total_far = w.rows_v + BH * w.row_cap * D * 2;
+        }
     }
     return w;
 }
 
-// Whether a call gathers the far chunks.  Below kFarMinRows positions there are at most 15 tiles in front of a query tile
-// and little to gather.  The rows of all heads must be addressable by the 32-bit row index of a gather.
+// Whether a call gathers the far chunks: where there is room, except below kFarMinRows positions, where at most 15 tiles lie
+// in front of a query tile and there is little to gather.
 constexpr int kFarMinRows = 2048;
-static bool use_far_lists(const PrefillWs& w, size_t workspace_bytes, int B, int Hkv, int N, int q_off, long long head_rows, bool pair) {
-    return w.total_far != 0 && workspace_bytes >= w.total_far && q_off + N >= kFarMinRows && !pair && (long long)B * Hkv * head_rows <= 0x7fffffffLL;
+static bool use_far(const PrefillWs& w, size_t workspace_bytes, int q_end, bool pair) {
+    return w.total_far != 0 && workspace_bytes >= w.total_far && q_end >= kFarMinRows && !pair;
+}
+static FarLists far_lists(const PrefillWs& w, uint8_t* ws, int C) {
+    FarLists far = {(int32_t*)(ws + w.list), (int32_t*)(ws + w.before), (int32_t*)(ws + w.open), 0x7fffffff};
+    if (w.row_cap) far.max_listed = w.row_cap / C;
+    return far;
+}
+
+// Copies the listed rows of K and V (see PrefillWs), 64 per block; the last tile is filled up with zeros.  Moves 4 D bytes per
+// row and tensor: 3 MB for 8192 tokens with 10 % global.
+constexpr int kFarThreads = 256, kFarRowsPerBlock = 64;
+struct FarRowsParams {
+    const uint8_t* k; const uint8_t* v;              // [BH, head_rows, D] bf16
+    uint8_t* rows_k; uint8_t* rows_v;                // [BH, cap, D]
+    const int32_t* list; const int32_t* before_tile;
+    long long head_rows;
+    int Nc, Ntk, Nkv, C, D, cap;
+};
+__global__ void __launch_bounds__(kFarThreads) far_rows_kernel(const FarRowsParams p) {
+    const int bh = blockIdx.y;
+    const int count = min((long long)p.before_tile[(size_t)bh * (p.Ntk + 1) + p.Ntk] * p.C, (long long)p.cap);
+    const int r0 = blockIdx.x * kFarRowsPerBlock, r1 = min(r0 + kFarRowsPerBlock, (count + kTile - 1) / kTile * kTile);
+    const int vpt = p.D / 8;
+    const int32_t* list = p.list + (size_t)bh * p.Nc;
+    for (int i = threadIdx.x; i < (r1 - r0) * vpt; i += kFarThreads) {
+        const int r = r0 + i / vpt, vec = i % vpt;
+        uint4 a = make_uint4(0, 0, 0, 0), b = a;
+        if (r < count) {
+            const int row = list[r / p.C] * p.C + r % p.C;
+            if (row < p.Nkv) {                       // the last chunk of the sequence may be part empty
+                const size_t src = (((size_t)bh * p.head_rows + row) * vpt + vec) * 16;
+                a = ld16(p.k + src);
+                b = ld16(p.v + src);
+            }
+        }
+        const size_t dst = (((size_t)bh * p.cap + r) * vpt + vec) * 16;
+        st16(p.rows_k + dst, a);
+        st16(p.rows_v + dst, b);
+    }
 }
 
 constexpr int kMaxDevices = 64;
@@ -1200,24 +1227,29 @@ static bool use_pair_kernel(int D, int nrep) {
 static int run_prefill(const void* d_q, const void* d_k, const void* d_v, void* d_o, int B, int Hq, int Hkv, int N, int Nkv,
                        int q_off, long long kv_head_stride, int D, int C, float sm_scale, const int32_t* lim,
                        const int32_t* tmax, const int32_t* tmin, int32_t* counter, int32_t* d_status, cudaStream_t st,
-                       const FarLists& far, float* d_lse = nullptr, bool o_tokens = false, bool o_f32 = false) {
+                       const FarLists& far, uint8_t* far_k, uint8_t* far_v, int far_cap, float* d_lse = nullptr, bool o_tokens = false, bool o_f32 = false) {
     const bool pair = use_pair_kernel(D, Hq / Hkv) && !o_f32;
     CUtensorMap mq, mk, mv, mkf, mvf;
     if (int rc = make_map(&mq, d_q, B * Hq, N, D, 128)) return rc;
     if (int rc = make_map(&mk, d_k, B * Hkv, Nkv, D, pair ? 64 : 128, kv_head_stride)) return rc;     // a pair's CTA loads half the rows of a K tile
     if (int rc = make_map(&mv, d_v, B * Hkv, Nkv, D, 128, kv_head_stride)) return rc;
-    const long long head_rows = kv_head_stride > 0 ? kv_head_stride : Nkv;
     mkf = mk;
     mvf = mv;
-    if (far.list != nullptr) {
-        // boxes of one chunk, or of single rows of all heads for the gather of four rows
-        const bool rows = C < 8;
-        const long long heads = rows ? 1 : (long long)B * Hkv, n = rows ? (long long)B * Hkv * head_rows : Nkv;
-        if (int rc = make_map(&mkf, d_k, heads, n, D, rows ? 1 : C, head_rows, rows)) return rc;
-        if (int rc = make_map(&mvf, d_v, heads, n, D, rows ? 1 : C, head_rows, rows)) return rc;
+    if (far.list != nullptr && far_cap > 0) {
+        FarRowsParams f;
+        f.k = (const uint8_t*)d_k; f.v = (const uint8_t*)d_v; f.rows_k = far_k; f.rows_v = far_v; f.list = far.list; f.before_tile = far.before_tile;
+        f.head_rows = kv_head_stride > 0 ? kv_head_stride : Nkv;
+        f.Nc = cdiv(Nkv, C); f.Ntk = cdiv(Nkv, kTile); f.Nkv = Nkv; f.C = C; f.D = D; f.cap = far_cap;
+        far_rows_kernel<<<dim3(cdiv(far_cap, kFarRowsPerBlock), B * Hkv), kFarThreads, 0, st>>>(f);
+        NATS_CHECK_CUDA(cudaGetLastError());
+        if (int rc = make_map(&mkf, far_k, B * Hkv, far_cap, D, 128)) return rc;
+        if (int rc = make_map(&mvf, far_v, B * Hkv, far_cap, D, 128)) return rc;
+    } else if (far.list != nullptr) {
+        if (int rc = make_map(&mkf, d_k, B * Hkv, Nkv, D, C, kv_head_stride)) return rc;       // boxes of one chunk
+        if (int rc = make_map(&mvf, d_v, B * Hkv, Nkv, D, C, kv_head_stride)) return rc;
     }
     PrefillParams p;
-    p.far_list = far.list; p.far_before = far.before_tile; p.far_open = far.open_max; p.head_rows = (int)head_rows;
+    p.far_list = far.list; p.far_before = far.before_tile; p.far_open = far.open_max;
     p.o_batch = (long long)N * Hq * D;
     p.o_head = o_tokens ? D : (long long)N * D;
     p.o_row = o_tokens ? (long long)Hq * D : D;
@@ -1254,7 +1286,13 @@ using namespace nats;
 
 extern "C" __attribute__((visibility("default"))) size_t nats_b200_prefill_workspace_bytes(int B, int Hkv, int N, int C) {
     if (B <= 0 || Hkv <= 0 || N <= 0 || C <= 0) return 0;
-    const PrefillWs w = prefill_ws(B, Hkv, N, C);
+    const PrefillWs w = prefill_ws(B, Hkv, N, C, 0);
+    return w.total_far ? w.total_far : w.total;
+}
+
+extern "C" __attribute__((visibility("default"))) size_t nats_b200_prefill_workspace_bytes_for(int B, int Hkv, int N, int D, int C) {
+    if (B <= 0 || Hkv <= 0 || N <= 0 || D <= 0 || C <= 0) return 0;
+    const PrefillWs w = prefill_ws(B, Hkv, N, C, D);
     return w.total_far ? w.total_far : w.total;
 }
 
@@ -1272,7 +1310,7 @@ static int prefill_first_call(const void* d_q, const void* d_k, const void* d_v,
     if (D != 64 && D != 128 && D != 256) return fail(NATS_ERR_UNSUPPORTED, "prefill supports head_dim 64, 128 and 256, got %d", D);
     NATS_CHECK_ARG(N <= kMaxTiles * kTile, "N = %d exceeds the prefill limit %d", N, kMaxTiles * kTile);
     NATS_CHECK_ARG((long long)B <= 65535 && (long long)Hkv * ((Hq / Hkv + 1) / 2) <= 65535, "grid too large");
-    const PrefillWs w = prefill_ws(B, Hkv, N, C);
+    const PrefillWs w = prefill_ws(B, Hkv, N, C, D);
     if (workspace_bytes < w.total)
         return fail(NATS_ERR_WORKSPACE, "prefill workspace: %zu bytes given, %zu needed", workspace_bytes, w.total);
     uint8_t* ws = (uint8_t*)d_workspace;
@@ -1280,13 +1318,12 @@ static int prefill_first_call(const void* d_q, const void* d_k, const void* d_v,
     int32_t* tmax = (int32_t*)(ws + w.tmax);
     int32_t* tmin = (int32_t*)(ws + w.tmin);
     FarLists far;
-    if (use_far_lists(w, workspace_bytes, B, Hkv, N, 0, N, use_pair_kernel(D, Hq / Hkv) && !o_f32))
-        far = {(int32_t*)(ws + w.list), (int32_t*)(ws + w.before), (int32_t*)(ws + w.open)};
+    if (use_far(w, workspace_bytes, N, use_pair_kernel(D, Hq / Hkv) && !o_f32)) far = far_lists(w, ws, C);
     if (int rc = role_prep(d_roles, B, Hkv, N, C, SW, lim, tmax, tmin, d_kept_tiles, far, (int32_t*)(ws + w.counter), stream)) return rc;
     if (d_n_visible != nullptr)
         if (int rc = nats_b200_visible_counts(lim, B, Hq, Hkv, N, C, d_n_visible, stream)) return rc;
     return run_prefill(d_q, d_k, d_v, d_o, B, Hq, Hkv, N, N, 0, 0, D, C, sm_scale, lim, tmax, tmin,
-                       (int32_t*)(ws + w.counter), d_status, (cudaStream_t)stream, far, d_lse, o_tokens, o_f32);
+                       (int32_t*)(ws + w.counter), d_status, (cudaStream_t)stream, far, ws + w.rows_k, ws + w.rows_v, w.row_cap, d_lse, o_tokens, o_f32);
 }
 
 extern "C" __attribute__((visibility("default"))) int nats_b200_prefill_fwd(const void* d_q, const void* d_k, const void* d_v, void* d_o, const uint8_t* d_roles,
@@ -1338,7 +1375,7 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_prefill_past_fwd
     const long long n_kv = (long long)t0 + fill + x_len;
     NATS_CHECK_ARG(n_kv <= cache_capacity, "the cache holds %d rows, %lld are needed (the new tokens must have been appended)", cache_capacity, n_kv);
     NATS_CHECK_ARG(n_kv <= (long long)kMaxTiles * kTile, "cache + new tokens = %lld rows exceed the prefill limit %d", n_kv, kMaxTiles * kTile);
-    const PrefillWs w = prefill_ws(B, Hkv, (int)n_kv, C);
+    const PrefillWs w = prefill_ws(B, Hkv, (int)n_kv, C, D);
     if (workspace_bytes < w.total)
         return fail(NATS_ERR_WORKSPACE, "prefill workspace: %zu bytes given, %zu needed", workspace_bytes, w.total);
     uint8_t* ws = (uint8_t*)d_workspace;
@@ -1346,12 +1383,12 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_prefill_past_fwd
     int32_t* tmax = (int32_t*)(ws + w.tmax);
     int32_t* tmin = (int32_t*)(ws + w.tmin);
     FarLists far;
-    if (use_far_lists(w, workspace_bytes, B, Hkv, x_len, t0 + fill, cache_capacity, use_pair_kernel(D, Hq / Hkv)))
-        far = {(int32_t*)(ws + w.list), (int32_t*)(ws + w.before), (int32_t*)(ws + w.open)};
+    if (use_far(w, workspace_bytes, (int)n_kv, use_pair_kernel(D, Hq / Hkv))) far = far_lists(w, ws, C);
     if (int rc = role_prep_past(d_roles_new, d_valid, d_size_global, d_size_local, B, Hkv, x_len, C, SW,
                                           valid_stride, t0, fill, tail, lim, tmax, tmin, d_kept_tiles, far, (int32_t*)(ws + w.counter), stream)) return rc;
     return run_prefill(d_q, d_cache_k, d_cache_v, d_o, B, Hq, Hkv, x_len, (int)n_kv, t0 + fill, cache_capacity, D, C, sm_scale,
-                       lim, tmax, tmin, (int32_t*)(ws + w.counter), d_status, (cudaStream_t)stream, far);
+                       lim, tmax, tmin, (int32_t*)(ws + w.counter), d_status, (cudaStream_t)stream, far,
+                       ws + w.rows_k, ws + w.rows_v, w.row_cap);
 }
 
 // =================================================================================================
@@ -1393,7 +1430,7 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_prefill_fwd_stat
     int B, int Hq, int Hkv, int N, int D, int C, int SW, float sm_scale,
     int64_t* d_kept_tiles, int32_t* d_status, void* stream) {
     if (B <= 0 || Hkv <= 0 || N <= 0 || C <= 0) return fail(NATS_ERR_INVALID_ARG, "bad shape B=%d Hkv=%d N=%d C=%d", B, Hkv, N, C);
-    const size_t need = nats::prefill_ws(B, Hkv, N, C).total;
+    const size_t need = nats::prefill_ws(B, Hkv, N, C, D).total;
     if (need > nats::kStaticScratchBytes)
         return fail(NATS_ERR_WORKSPACE,
                     "this shape needs %zu bytes of role metadata, the built-in scratch holds %zu: use nats_b200_prefill_fwd "

@@ -248,7 +248,7 @@ def prefill_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, roles: 
         dtype = torch.float32 if o_f32 else torch.bfloat16
         o = torch.empty(B, N, Hq, D, dtype=dtype, device=dev).transpose(1, 2) if token_major else torch.empty(B, Hq, N, D, dtype=dtype, device=dev)
     lib = _lib.lib()
-    nbytes = lib.nats_b200_prefill_workspace_bytes(B, Hkv, N, chunk_size)
+    nbytes = lib.nats_b200_prefill_workspace_bytes_for(B, Hkv, N, qb.shape[-1], chunk_size)
     ws = _workspace('prefill', dev, nbytes)
     _call(dev, 'nats_b200_prefill_fwd_out', _p(qb), _p(kb), _p(vb), _p(o), int(token_major), int(o_f32), _p(roles.contiguous()), B, Hq, Hkv, N,
               qb.shape[-1], chunk_size, sliding_window, scale, _p(ws), ws.numel(), _p(kept_tiles), _p(status_word(dev)), _stream(dev))
@@ -409,7 +409,7 @@ def nats_chunk_attention_fwd(q, k, v, seq_info, end_seqs_idx, causal, sm_scale, 
     lse = torch.empty(B, Hq, N, dtype=torch.float32, device=dev)
     n_vis = torch.empty(B, Hq, N, dtype=torch.int32, device=dev)
     lib = _lib.lib()
-    ws = _workspace('prefill', dev, lib.nats_b200_prefill_workspace_bytes(B, Hkv, N, nats_chunk_size))
+    ws = _workspace('prefill', dev, lib.nats_b200_prefill_workspace_bytes_for(B, Hkv, N, D, nats_chunk_size))
     _call(dev, 'nats_b200_prefill_fwd_stats', _p(qb), _p(kb), _p(vb), _p(o), _p(roles), B, Hq, Hkv, N, D, nats_chunk_size,
               local_seq_max_length, float(sm_scale), _p(ws), ws.numel(), None, _p(lse), _p(n_vis), _p(status_word(dev)),
               _stream(dev))
@@ -501,7 +501,7 @@ def prefill_attention_past(q: torch.Tensor, cache_k: torch.Tensor, cache_v: torc
     qb = _as_bf16(q)
     o = torch.empty_like(qb)
     lib = _lib.lib()
-    nbytes = lib.nats_b200_prefill_past_workspace_bytes(B, Hkv, t0 + fill + x_len, chunk_size)
+    nbytes = lib.nats_b200_prefill_workspace_bytes_for(B, Hkv, t0 + fill + x_len, D, chunk_size)
     ws = _workspace('prefill', dev, nbytes)
     scale = (1.0 / math.sqrt(D)) if sm_scale is None else float(sm_scale)
     _call(dev, 'nats_b200_prefill_past_fwd', _p(qb), _p(cache_k), _p(cache_v), _p(o), _p(roles_new.contiguous()), _p(valid),
