@@ -39,7 +39,7 @@ struct DecodeParams {
     const long long* size_local;
     const int32_t* state;          // [0] = T0
     int32_t* counters;             // [B*Hkv]   (workspace)
-    float* partials;               // [B*Hkv, max_splits (x strands), nrep, D+2]   (workspace)
+    float* partials;               // [B*Hkv, max_splits, nrep, D+2] or [B*Hkv, max_splits, strands, nrep, D+4]   (workspace)
     int Hq, Hkv, nrep, Lcap, SW, fill, max_splits;
     int fill_from_state;           // 1: the number of tokens in the unfinished chunk is read from state[4] (static launches)
     float scale_log2;              // sm_scale * log2(e)
@@ -373,20 +373,25 @@ __global__ void __launch_bounds__(kDecThreads) decode_kernel(const DecodeParams 
 // a quarter of the columns of O.  The arithmetic on every value is the one of decode_kernel in the same order -- the running
 // maximum, the row sum and each accumulator see the strand's tiles in sequence, strands and segments are combined in the same
 // two steps -- so that a head's output does not depend on which of the two kernels the size of the batch selects.
-// With the placement in the same launch, 192 replayed steps of 2 sequences x 8 kv-heads over ~2.9k rows and their prompt of
-// 6000 tokens take 3.95 instead of 5.43 ms.
+// One launch in a graph of 20, us, decode_kernel / strands, head_dim 128, 2900 rows per head: 24 segments 21.1 / 10.9, 48
+// 21.0 / 12.2, 96 21.6 / 13.5, 144 21.6 / 21.6; 12000 rows, 96 segments 24.0 / 17.2, 8000 rows, 128 segments 21.1 / 23.2.
+// head_dim 64: 24 segments 18.6 / 9.0, 144 18.8 / 11.8, 192 19.9 / 17.3, 288 20.0 / 20.1.  What is left of a short launch (10 us) is
+// a chain of latencies: sizes, copies, scores, partial results, ticket, combination.
 constexpr int kStrandTiles = kSeg / kTileTok / kDecWarps;
 constexpr int kStrandTilesPerWarp = kStrandTiles / kDecWarps;
 static_assert(kStrandTiles % kDecWarps == 0, "tiles of a strand are dealt to the warps in equal numbers");
 
-template <int D>
-constexpr int strand_smem() { return kStrandTiles * (2 * kTileTok * D * 2 + 32 * 16 + kMaxRep * 4); }
+template <int D, bool BOTH>
+constexpr int strand_smem() { return kStrandTiles * ((BOTH ? 2 : 1) * kTileTok * D * 2 + 32 * 16 + kMaxRep * 4); }
 
-template <int D, bool STEP>
+// BOTH: V has slots of its own and its copies start together with those of K.  Otherwise a warp puts V where it has just read
+// K, half the shared memory: three blocks instead of one on an SM at head_dim 128, for launches of more blocks than SMs.
+template <int D, bool STEP, bool BOTH>
 __global__ void __launch_bounds__(kDecThreads) decode_strand_kernel(const DecodeParams p) {
-    constexpr int ROWB = D * 2, CHUNKS = ROWB / 16, TILE_BYTES = kTileTok * ROWB, STAGE_BYTES = 2 * TILE_BYTES;
+    constexpr int ROWB = D * 2, CHUNKS = ROWB / 16, TILE_BYTES = kTileTok * ROWB;
+    constexpr int V_SLOTS = BOTH ? kStrandTiles * TILE_BYTES : 0, TILES_BYTES = kStrandTiles * TILE_BYTES + V_SLOTS;
     constexpr int CP_PER_LANE = kTileTok * CHUNKS / 32, ROWS_PER_CP = 32 / CHUNKS;
-    constexpr int TPW = kStrandTilesPerWarp, PSTRIDE = D + 2;
+    constexpr int TPW = kStrandTilesPerWarp, PSTRIDE = D + 4;      // a partial result: D columns, maximum, row sum (16-byte rows)
     constexpr int NP = D / 16 / kDecWarps;           // 16-column blocks of O per warp
     constexpr unsigned FULL = 0xffffffffu;
     const float NEG_INF = -INFINITY;
@@ -406,8 +411,8 @@ __global__ void __launch_bounds__(kDecThreads) decode_strand_kernel(const Decode
     if (seg < nsplit) {
     const int r0 = seg * kSeg, r1 = min(Ltot, r0 + kSeg);
 
-    float4* s_score = reinterpret_cast<float4*>(dsm + kStrandTiles * STAGE_BYTES);             // [tile][lane]
-    float (*s_tmax)[kMaxRep] = reinterpret_cast<float (*)[kMaxRep]>(dsm + kStrandTiles * (STAGE_BYTES + 32 * 16));
+    float4* s_score = reinterpret_cast<float4*>(dsm + TILES_BYTES);             // [tile][lane]
+    float (*s_tmax)[kMaxRep] = reinterpret_cast<float (*)[kMaxRep]>(dsm + TILES_BYTES + kStrandTiles * 32 * 16);
     __shared__ unsigned s_vmask[kStrandTiles];
 
     const __nv_bfloat16* ck = p.ck + (size_t)bh * p.Lcap * D;
@@ -424,8 +429,36 @@ __global__ void __launch_bounds__(kDecThreads) decode_strand_kernel(const Decode
         if (lane == 0) p.valid[(size_t)bh * p.Lcap + T0 + fill] = 1;
     }
 
-    // ---- which tokens of this warp's tiles exist and are valid, then all of their copies (one group per tile) ----
+    // ---- copies of this warp's tiles, one group each; which of their tokens exist and are valid is read meanwhile (ring tiles
+    // without a valid slot are copied here too: their bytes cost less than waiting for the flags) ----
     const uint32_t tiles = (uint32_t)__cvta_generic_to_shared(dsm);
+    auto issue = [&](int x, const __nv_bfloat16* cache, const __nv_bfloat16* fresh, int slots) {
+        const int t = x * kDecWarps + warp;                                   // tile of the strand
+        const int i0 = r0 + (t * kDecWarps + strand) * kTileTok;
+        if (i0 < r1) {
+            const uint32_t dst = tiles + slots + t * TILE_BYTES;
+            const int c = lane % CHUNKS, rsub = lane / CHUNKS;
+            const bool plain = i0 + kTileTok <= len;                          // whole tile inside ring + kept tokens: logical == physical
+#pragma unroll
+            for (int y = 0; y < CP_PER_LANE; ++y) {
+                const int r = y * ROWS_PER_CP + rsub;
+                const int i = i0 + r;
+                const bool ok = plain || i < r1;
+                const __nv_bfloat16* src = cache;
+                if (plain || i < len) src = cache + (size_t)i * D;
+                else if (i < len + fill) src = cache + (size_t)(T0 + (i - len)) * D;
+                else if (ok) src = fresh;
+                cp_async16(dst + r * ROWB + ((c ^ (r & 7)) << 4), src + c * 8, ok);
+            }
+        }
+        cp_async_commit();
+    };
+#pragma unroll
+    for (int x = 0; x < TPW; ++x) issue(x, ck, kn, 0);
+    if (BOTH) {
+#pragma unroll
+        for (int x = 0; x < TPW; ++x) issue(x, cv, vn, V_SLOTS);
+    }
     unsigned vmask[TPW];
     {
         bool ok[TPW];
@@ -437,31 +470,6 @@ __global__ void __launch_bounds__(kDecThreads) decode_strand_kernel(const Decode
         }
 #pragma unroll
         for (int x = 0; x < TPW; ++x) vmask[x] = __ballot_sync(FULL, ok[x]) & 0xffffu;
-    }
-#pragma unroll
-    for (int x = 0; x < TPW; ++x) {
-        const int t = x * kDecWarps + warp;                                   // tile of the strand
-        const int i0 = r0 + (t * kDecWarps + strand) * kTileTok;
-        if (vmask[x] != 0u) {
-            const uint32_t dst = tiles + t * STAGE_BYTES;
-            const int c = lane % CHUNKS, rsub = lane / CHUNKS;
-            // whole tile inside ring + kept tokens: logical == physical
-            const bool plain = i0 + kTileTok <= len;
-#pragma unroll
-            for (int y = 0; y < CP_PER_LANE; ++y) {
-                const int r = y * ROWS_PER_CP + rsub;
-                const int i = i0 + r;
-                const bool ok = plain || i < r1;
-                const __nv_bfloat16 *kp = ck, *vp = cv;
-                if (plain || i < len) { kp = ck + (size_t)i * D; vp = cv + (size_t)i * D; }
-                else if (i < len + fill) { const size_t ph = (size_t)(T0 + (i - len)); kp = ck + ph * D; vp = cv + ph * D; }
-                else if (ok) { kp = kn; vp = vn; }
-                const uint32_t off = r * ROWB + ((c ^ (r & 7)) << 4);
-                cp_async16(dst + off, kp + c * 8, ok);
-                cp_async16(dst + TILE_BYTES + off, vp + c * 8, ok);
-            }
-        }
-        cp_async_commit();
     }
     const int hrow = lane >> 2, quad = lane & 3;
     uint32_t qa[D / 16][2];
@@ -477,14 +485,19 @@ __global__ void __launch_bounds__(kDecThreads) decode_strand_kernel(const Decode
 #pragma unroll
     for (int x = 0; x < TPW; ++x) {
         const int t = x * kDecWarps + warp;
-        if (x == 0) cp_async_wait<TPW - 1>();
-        else if (x == 1) cp_async_wait<TPW - 2>();
-        else if (x == 2) cp_async_wait<(TPW > 2 ? TPW - 3 : 0)>();
-        else cp_async_wait<0>();
+        // groups in flight behind K of this tile: K of the later ones, and V of all or of the earlier ones
+        if (!BOTH) cp_async_wait<TPW - 1>();
+        else if (x == 0) cp_async_wait<2 * TPW - 1>();
+        else if (x == 1) cp_async_wait<2 * TPW - 2>();
+        else if (x == 2) cp_async_wait<2 * TPW - 3>();
+        else cp_async_wait<2 * TPW - 4>();
         __syncwarp();                                // every lane's copies of the tile are there
         if (lane == 0) s_vmask[t] = vmask[x];
-        if (vmask[x] == 0u) continue;
-        const uint32_t sk = tiles + t * STAGE_BYTES;
+        if (vmask[x] == 0u) {
+            if (!BOTH) cp_async_commit();
+            continue;
+        }
+        const uint32_t sk = tiles + t * TILE_BYTES;
         float sc[2][4];
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
@@ -499,6 +512,10 @@ __global__ void __launch_bounds__(kDecThreads) decode_strand_kernel(const Decode
                 mma_bf16(sc[nt], qa[2 * kp + 1][0], 0u, qa[2 * kp + 1][1], 0u, kb[2], kb[3]);
             }
         }
+        if (!BOTH) {
+            __syncwarp();                            // every lane is done with K: V takes its place
+            issue(x, cv, vn, 0);
+        }
         float s[4];
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt)
@@ -511,7 +528,8 @@ __global__ void __launch_bounds__(kDecThreads) decode_strand_kernel(const Decode
         s_score[t * 32 + lane] = make_float4(s[0], s[1], s[2], s[3]);
         if (quad == 0) s_tmax[t][hrow] = mt;
     }
-    static_assert(TPW >= 2 && TPW <= 4, "wait counts above");
+    static_assert(TPW == 4, "wait counts above");
+    cp_async_wait<0>();
     __syncthreads();
     // ---- online softmax over the strand's tiles; this warp's columns of O += P . V ----
     float oacc[2 * NP][4];
@@ -533,7 +551,7 @@ __global__ void __launch_bounds__(kDecThreads) decode_strand_kernel(const Decode
 #pragma unroll
         for (int n = 0; n < 2 * NP; ++n) { oacc[n][0] *= alpha; oacc[n][1] *= alpha; }
         const uint32_t pa0 = pack2_bf16(p0, p1), pa2 = pack2_bf16(p2, p3);
-        const uint32_t sv = tiles + t * STAGE_BYTES + TILE_BYTES;
+        const uint32_t sv = tiles + V_SLOTS + t * TILE_BYTES;
 #pragma unroll
         for (int np = 0; np < NP; ++np) {
             uint32_t vb[4];
@@ -585,35 +603,51 @@ __global__ void __launch_bounds__(kDecThreads) decode_strand_kernel(const Decode
         s_seg_l[idx] = l;
     }
     __syncthreads();
-    for (int idx = tid; idx < nrep * D; idx += kDecThreads) {
-        const int h = idx / D, d = idx % D;
+    // four columns per thread, 16-byte loads: with nrep * D = 512 every thread makes one pass over the strands
+    for (int idx = tid; idx < nrep * (D / 4); idx += kDecThreads) {
+        const int h = idx / (D / 4), d = (idx % (D / 4)) * 4;
         float mf = NEG_INF;
         for (int sgm = 0; sgm < nsplit; ++sgm) mf = fmaxf(mf, s_seg_m[sgm * nrep + h]);
         const float mu = (mf == NEG_INF) ? 0.f : mf;
-        float a = 0.f, l = 0.f;
-#pragma unroll 2
+        float a[4] = {0.f, 0.f, 0.f, 0.f}, l = 0.f;
+#pragma unroll 4
         for (int sgm = 0; sgm < nsplit; ++sgm) {
-            float as = 0.f;
+            float as[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int w = 0; w < kDecWarps; ++w) {
                 const int st = sgm * kDecWarps + w;
-                as = fmaf(__ldcg(parts + ((size_t)st * nrep + h) * PSTRIDE + d), s_wgt[st * nrep + h], as);
+                const float4 x = __ldcg(reinterpret_cast<const float4*>(parts + ((size_t)st * nrep + h) * PSTRIDE + d));
+                const float wgt = s_wgt[st * nrep + h];
+                as[0] = fmaf(x.x, wgt, as[0]);
+                as[1] = fmaf(x.y, wgt, as[1]);
+                as[2] = fmaf(x.z, wgt, as[2]);
+                as[3] = fmaf(x.w, wgt, as[3]);
             }
             const float wgt = fast_exp2(s_seg_m[sgm * nrep + h] - mu);
-            a = fmaf(as, wgt, a);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) a[e] = fmaf(as[e], wgt, a[e]);
             l = fmaf(s_seg_l[sgm * nrep + h], wgt, l);
         }
         const float inv = l > 0.f ? 1.f / l : 0.f;
-        p.o[((size_t)b * p.Hq + (size_t)hkv * nrep + h) * D + d] = __float2bfloat16_rn(a * inv);
+        uint2 w;
+        w.x = pack2_bf16(a[0] * inv, a[1] * inv);
+        w.y = pack2_bf16(a[2] * inv, a[3] * inv);
+        *reinterpret_cast<uint2*>(p.o + ((size_t)b * p.Hq + (size_t)hkv * nrep + h) * D + d) = w;
     }
     if (STEP) finish_step(p, bh, gridDim.y * gridDim.z, T0, fill);
 }
 
-// Segments of a launch up to which every strand gets its own block: 4 x 74 strands are two per SM.
+// Segments of a launch up to which every strand gets its own block (measured at decode_strand_kernel), and up to which V gets slots
+// of its own: as long as all strands fit on the chip at once (148 SMs, one block each at head_dim 128, three at 64), where it
+// is 1 to 5 % faster; behind that it loses (head_dim 128, 48 segments 17.9 against 12.2 us; 64, 128 segments 18.5 against 14.9).
 #ifndef NATS_STRAND_SEGMENTS
-#define NATS_STRAND_SEGMENTS 74
+#define NATS_STRAND_SEGMENTS (D == 64 ? 192 : 96)
 #endif
-constexpr int kStrandSegments = NATS_STRAND_SEGMENTS;
+#ifndef NATS_STRAND_BOTH
+#define NATS_STRAND_BOTH (D == 64 ? 111 : 37)
+#endif
+constexpr int strand_segments(int D) { return NATS_STRAND_SEGMENTS; }
+constexpr int strand_both_segments(int D) { return NATS_STRAND_BOTH; }
 
 // the opt-in to more than 48 KB of dynamic shared memory is a per-device attribute of a kernel
 template <class Kernel>
@@ -628,16 +662,22 @@ static cudaError_t allow_smem(Kernel kernel, int smem, bool (&done)[64]) {
     return e;
 }
 
+template <int D, bool STEP, bool BOTH>
+static cudaError_t launch_strands(const DecodeParams& p, dim3 grid, cudaStream_t st) {
+    static bool done[64] = {};
+    const cudaError_t e = allow_smem(decode_strand_kernel<D, STEP, BOTH>, strand_smem<D, BOTH>(), done);
+    if (e != cudaSuccess) return e;
+    grid.x *= kDecWarps;
+    decode_strand_kernel<D, STEP, BOTH><<<grid, kDecThreads, strand_smem<D, BOTH>(), st>>>(p);
+    return cudaGetLastError();
+}
+
 template <int D, bool STEP>
 static cudaError_t launch_decode(const DecodeParams& p, dim3 grid, cudaStream_t st) {
     cudaError_t e;
-    if ((long long)grid.x * grid.y * grid.z <= kStrandSegments) {
-        static bool done[64] = {};
-        if ((e = allow_smem(decode_strand_kernel<D, STEP>, strand_smem<D>(), done)) != cudaSuccess) return e;
-        grid.x *= kDecWarps;
-        decode_strand_kernel<D, STEP><<<grid, kDecThreads, strand_smem<D>(), st>>>(p);
-        return cudaGetLastError();
-    }
+    const long long segments = (long long)grid.x * grid.y * grid.z;
+    if (segments <= strand_segments(D))
+        return segments <= strand_both_segments(D) ? launch_strands<D, STEP, true>(p, grid, st) : launch_strands<D, STEP, false>(p, grid, st);
     constexpr int smem = kDecWarps * kDecStages * 2 * kTileTok * D * 2;
     static bool done[64] = {};
     if ((e = allow_smem(decode_kernel<D, STEP>, smem, done)) != cudaSuccess) return e;
@@ -647,9 +687,11 @@ static cudaError_t launch_decode(const DecodeParams& p, dim3 grid, cudaStream_t 
 
 static size_t decode_counter_bytes(int B, int Hkv) { return align_up((size_t)B * Hkv * sizeof(int32_t), 256); }
 static int decode_max_splits(int max_len) { return cdiv(max_len + 1, kSeg); }
-// partial results kept per (batch, kv-head) and split: one, or one per strand where a launch may be of that kind (a launch has
-// at least one segment per (batch, kv-head))
-static int decode_parts_per_split(int B, int Hkv) { return (long long)B * Hkv <= kStrandSegments ? kDecWarps : 1; }
+// floats of the partial results of a split of a (batch, kv-head): one per query head, or one per strand and query head where a
+// launch may be of that kind (a launch has at least one segment per (batch, kv-head))
+static size_t decode_split_floats(int B, int Hkv, int nrep, int D) {
+    return (long long)B * Hkv <= strand_segments(D) ? (size_t)kDecWarps * nrep * (D + 4) : (size_t)nrep * (D + 2);
+}
 
 }  // namespace nats
 
@@ -659,7 +701,7 @@ extern "C" __attribute__((visibility("default"))) size_t nats_b200_decode_worksp
     if (B <= 0 || Hq <= 0 || Hkv <= 0 || D <= 0 || max_len < 0 || Hq % Hkv) return 0;
     const int nrep = Hq / Hkv;
     return decode_counter_bytes(B, Hkv) +
-           (size_t)B * Hkv * decode_max_splits(max_len) * decode_parts_per_split(B, Hkv) * nrep * (D + 2) * sizeof(float);
+           (size_t)B * Hkv * decode_max_splits(max_len) * decode_split_floats(B, Hkv, nrep, D) * sizeof(float);
 }
 
 static int decode_impl(const void* d_q, const void* d_k_new, const void* d_v_new, void* d_o,
