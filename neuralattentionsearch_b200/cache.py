@@ -144,7 +144,9 @@ class NAtSChunkLayerCache:
         if x_len == 0:
             return self.cache_k[:, :, :self.n_ctx_data], self.cache_v[:, :, :self.n_ctx_data]
         self._tokens_info = token_states_info
-        self._roles = None if token_states_info is None else F_.roles_from_token_states_info(token_states_info)
+        # a single token that leaves its chunk unfinished carries a placeholder: nothing reads its role
+        unread = x_len == 1 and self._buf_k is not None and self.chunk_fill_size < self.chunk_size
+        self._roles = None if token_states_info is None or unread else F_.roles_from_token_states_info(token_states_info)
         if self._buf_k is None and self._pending is None:
             self._pending = (key_states, value_states)
             self._plan_ahead(x_len)
@@ -463,7 +465,9 @@ class NAtSCache:
     def merge_new_x_values_in_chunk(x_cache, x_new, chunk_size: int, chunk_merge_method: str = 'mean'):
         """Running pooled hidden state of an unfinished chunk: sum of x / C for 'mean', running max for 'max'."""
         if chunk_merge_method == 'mean':
-            part = (x_new / chunk_size).sum(1, keepdim=True)
+            part = x_new / chunk_size
+            if x_new.shape[1] != 1:
+                part = part.sum(1, keepdim=True)
             return part if x_cache is None else x_cache + part
         if x_cache is None:
             return x_new if x_new.shape[1] == 1 else x_new.max(1, keepdim=True)[0]
