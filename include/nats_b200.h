@@ -122,7 +122,7 @@ int nats_b200_visible_counts(const int32_t* d_lim, int B, int Hq, int Hkv, int N
  * The role metadata goes to a scratch array built into the library: nats_b200_prefill_static_scratch_bytes() bytes
  * (1 MiB) of device memory per GPU that loads the library, held until the process exits.  Shapes whose metadata
  * does not fit -- B*Hkv*(ceil(N/C) + 2*ceil(N/128)) int32 values plus padding -- are rejected with NATS_ERR_WORKSPACE.
- * The lists of the gathered tiles (chunk sizes that divide 128, 2048 tokens and more) are used where they fit as well;
+ * The lists of the gathered tiles (chunk sizes that divide 128; 1024 tokens and more, 2048 from chunks of 32 on) are used where they fit as well;
  * where they do not, the sums run over the same keys in another order than in nats_b200_prefill_fwd.
  * This call and the library allocate nothing: no cudaMalloc / cudaFree, no allocating library routine.
  * The first call on a device looks up the scratch array's device address (once per device, with that device

@@ -1129,11 +1129,12 @@ static PrefillWs prefill_ws(int B, int Hkv, int N, int C, int D) {
     return w;
 }
 
-// Whether a call gathers the far chunks: where there is room, except below kFarMinRows positions, where at most 15 tiles lie
-// in front of a query tile and there is little to gather.
-constexpr int kFarMinRows = 2048;
-static bool use_far(const PrefillWs& w, size_t workspace_bytes, int q_end, bool pair) {
-    return w.total_far != 0 && workspace_bytes >= w.total_far && q_end >= kFarMinRows && !pair;
+// Whether a call gathers the far chunks: where there is room and the sequence is long enough.  Eight sequences, 16 / 8 heads,
+// window 256, in place / gathered, us: chunks of 1 (head_dim 64) 512 tokens 40 / 42, 1024 91 / 66, 1536 162 / 89, 2000 253 / 115;
+// chunks of 16 (128) 512 38 / 38, 1024 78 / 69, 2000 181 / 133; chunks of 64 (64) 1024 53 / 53, 1536 82 / 79, 2000 112 / 108.
+static int far_min_rows(int C) { return C <= 16 ? 1024 : 2048; }
+static bool use_far(const PrefillWs& w, size_t workspace_bytes, int C, int q_end, bool pair) {
+    return w.total_far != 0 && workspace_bytes >= w.total_far && q_end >= far_min_rows(C) && !pair;
 }
 static FarLists far_lists(const PrefillWs& w, uint8_t* ws, int C) {
     FarLists far = {(int32_t*)(ws + w.list), (int32_t*)(ws + w.before), (int32_t*)(ws + w.open), 0x7fffffff};
@@ -1318,7 +1319,7 @@ static int prefill_first_call(const void* d_q, const void* d_k, const void* d_v,
     int32_t* tmax = (int32_t*)(ws + w.tmax);
     int32_t* tmin = (int32_t*)(ws + w.tmin);
     FarLists far;
-    if (use_far(w, workspace_bytes, N, use_pair_kernel(D, Hq / Hkv) && !o_f32)) far = far_lists(w, ws, C);
+    if (use_far(w, workspace_bytes, C, N, use_pair_kernel(D, Hq / Hkv) && !o_f32)) far = far_lists(w, ws, C);
     if (int rc = role_prep(d_roles, B, Hkv, N, C, SW, lim, tmax, tmin, d_kept_tiles, far, (int32_t*)(ws + w.counter), stream)) return rc;
     if (d_n_visible != nullptr)
         if (int rc = nats_b200_visible_counts(lim, B, Hq, Hkv, N, C, d_n_visible, stream)) return rc;
@@ -1383,7 +1384,7 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_prefill_past_fwd
     int32_t* tmax = (int32_t*)(ws + w.tmax);
     int32_t* tmin = (int32_t*)(ws + w.tmin);
     FarLists far;
-    if (use_far(w, workspace_bytes, (int)n_kv, use_pair_kernel(D, Hq / Hkv))) far = far_lists(w, ws, C);
+    if (use_far(w, workspace_bytes, C, (int)n_kv, use_pair_kernel(D, Hq / Hkv))) far = far_lists(w, ws, C);
     if (int rc = role_prep_past(d_roles_new, d_valid, d_size_global, d_size_local, B, Hkv, x_len, C, SW,
                                           valid_stride, t0, fill, tail, lim, tmax, tmin, d_kept_tiles, far, (int32_t*)(ws + w.counter), stream)) return rc;
     return run_prefill(d_q, d_cache_k, d_cache_v, d_o, B, Hq, Hkv, x_len, (int)n_kv, t0 + fill, cache_capacity, D, C, sm_scale,

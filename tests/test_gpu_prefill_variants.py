@@ -39,7 +39,7 @@ def test_mask_bits_of_every_chunk_granularity(C):
 @pytest.mark.parametrize('C,N,p_global,p_local', [(1, 2048, 0.1, 0.3), (2, 2500, 0.05, 0.3), (4, 2177, 0.2, 0.1), (8, 2300, 0.1, 0.3),
                                                   (16, 3001, 0.03, 0.1), (32, 2600, 0.3, 0.0), (64, 4000, 0.1, 0.6), (16, 2304, 1.0, 0.0),
                                                   (1, 2304, 0.0, 1.0), (32, 2304, 0.0, 0.0),
-                                                  (1, 2304, 1.0, 0.0), (2, 3000, 0.6, 0.2)])
+                                                  (1, 2304, 1.0, 0.0), (2, 3000, 0.6, 0.2), (1, 1024, 0.1, 0.3), (16, 1500, 0.1, 0.2)])
 @pytest.mark.parametrize('D', [64, 128, 256])
 def test_far_chunks_are_gathered(C, N, p_global, p_local, D):
     """Prompts long enough for the gathered tiles: every way of gathering (copied rows, boxes of 8 to 64 rows), a last gathered
