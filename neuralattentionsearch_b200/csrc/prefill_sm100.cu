@@ -71,6 +71,7 @@ struct PrefillParams {
     const int32_t* far_list;
     const int32_t* far_before;
     const int32_t* far_open;
+    int far_cap, far_rows;            // chunks below 8 rows: rows of the copy in front of its tails, and with them; else 0
     int32_t* status;
     int32_t* work_counter;            // next work item; zero at launch (the role metadata kernel in front clears it)
     int total_items;                  // B * Hkv * n_groups * Nt
@@ -347,9 +348,11 @@ struct ItemHeader {
     int nslots;     // 1 or 2 query heads in this item
     int n_kept;     // 128-column KV tiles: gathered ones first, then the kept tiles of the bitmap
     int far_keys;   // keys of the gathered tiles (the last one may be part empty)
+    int far_tail;   // chunks below 8 rows: row of the copy that holds the last far_keys % 8 of them, zeros behind
 };
 
 constexpr int kBitWords = kMaxTiles / 32;
+constexpr int kTailRows = 8;    // rows of the smallest box: 128 bytes each, one swizzle atom
 
 // K/V ring: slots of one 128-row tile each, filled in the order K_0 V_0 K_1 V_1 ... of the kept tiles (all items in
 // one sequence).  A K slot is free again when both heads' Q.K^T of that tile have completed, a V slot after both P.V.
@@ -457,7 +460,8 @@ template <int D, bool FINE>
 __global__ void __launch_bounds__(kPrefillThreads, 1)
 prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_k_far,
-               const __grid_constant__ CUtensorMap map_v_far, const PrefillParams p) {
+               const __grid_constant__ CUtensorMap map_v_far, const __grid_constant__ CUtensorMap map_k_copy,
+               const __grid_constant__ CUtensorMap map_v_copy, const PrefillParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     using Smem = PrefillSmem<D>;
     Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
@@ -577,6 +581,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                     ItemHeader hd;
                     hd.valid = 1; hd.t = t; hd.b = z; hd.bh = bh; hd.head0 = hkv * p.nrep + grp * Smem::kHeads;
                     hd.nslots = min(Smem::kHeads, p.nrep - grp * Smem::kHeads); hd.n_kept = n_kept; hd.far_keys = far_keys;
+                    hd.far_tail = p.far_cap + kTailRows * max(near_first, 0);
                     sm.item[slot] = hd;
                 }
             } else if (lane == 0) {
@@ -637,15 +642,18 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 bool partial;
                 const bool far = FINE && j < n_far;
                 const int row0 = far ? j * kTile : walk.next(partial) * kTile;
-                // Rows of a gathered tile: of the copy of the listed rows, or (chunks of 8 rows and more) lane i copies the i-th
-                // chunk of the tile; a slot behind the last listed chunk takes rows behind the sequence, which read as zero.
-                // Filler keys are masked.
-                const int cpt = far ? kTile >> p.c_shift : 1;
-                const bool boxes = far && p.C >= 8;
+                // Rows of a gathered tile: a box of 128 rows of the copy of the listed rows, or boxes of box_rows rows, the i-th
+                // from lane i: a listed chunk where it lies, or (chunks below 8 rows, only for the part empty tile) eight rows
+                // of the copy or its tail.  What lies behind the last listed key of the item is read as zero, from rows
+                // behind the array: P is zero there, and 0 * V is zero only for a finite V, so no later key may stand there.
+                const int far_left = hd.far_keys - j * kTile;
+                const bool boxes = far && (p.far_cap == 0 || far_left < kTile);
+                const int box_shift = far ? max(p.c_shift, 3) : 3, box_rows = 1 << box_shift, n_boxes = kTile >> box_shift;
                 int box_row = 0;
                 if (boxes) {
-                    const int i = j * cpt + (lane & (cpt - 1));
-                    box_row = i * p.C < hd.far_keys ? far_list[i] * p.C : p.Nkv;
+                    const int key = j * kTile + ((lane & (n_boxes - 1)) << box_shift);
+                    if (p.far_cap == 0) box_row = key < hd.far_keys ? far_list[key >> box_shift] * box_rows : p.Nkv;
+                    else box_row = key + box_rows <= hd.far_keys ? key : key < hd.far_keys ? hd.far_tail : p.far_rows;
                 }
 #pragma unroll 1
                 for (int kv = 0; kv < 2 && ok; ++kv, ++g) {
@@ -668,7 +676,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                     if (lane == 0 && !withhold) {
                         mbar_expect_tx(smem_u32(&sm.bar_full[s]), TILE_BYTES);
                         if (!boxes) {
-                            const CUtensorMap* map = kv == 0 ? (far ? &map_k_far : &map_k) : (far ? &map_v_far : &map_v);
+                            const CUtensorMap* map = kv == 0 ? (far ? &map_k_copy : &map_k) : (far ? &map_v_copy : &map_v);
                             for (int x = 0; x < NBOX; ++x)
                                 tma_load_3d(smem_u32(&sm.ring[s][x * kBoxBytes]), map, smem_u32(&sm.bar_full[s]), x * 64, row0, hd.bh, pol_kv);
                         }
@@ -677,9 +685,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                     if (boxes && !withhold) {
                         const CUtensorMap* map = kv == 0 ? &map_k_far : &map_v_far;
                         const uint32_t dst = smem_u32(&sm.ring[s][0]), bar = smem_u32(&sm.bar_full[s]);
-                        // cpt <= 16 divides 32: the lanes of a chunk share its boxes
-                        for (int x = lane / cpt; x < NBOX; x += 32 / cpt)
-                            tma_load_3d(dst + x * kBoxBytes + (lane & (cpt - 1)) * p.C * 128, map, bar, x * 64, box_row, hd.bh, pol_kv);
+                        // n_boxes <= 16 divides 32: the lanes of a box share its parts of 64 columns
+                        for (int x = lane / n_boxes; x < NBOX; x += 32 / n_boxes)
+                            tma_load_3d(dst + x * kBoxBytes + (lane & (n_boxes - 1)) * box_rows * 128, map, bar, x * 64, box_row, hd.bh, pol_kv);
                         __syncwarp();
                     }
                 }
@@ -1101,10 +1109,11 @@ static int make_map(CUtensorMap* map, const void* base, long long heads, long lo
     return NATS_OK;
 }
 
-struct PrefillWs { size_t lim, tmax, tmin, counter, total, list, before, open, rows_k, rows_v, total_far; int row_cap; };
+struct PrefillWs { size_t lim, tmax, tmin, counter, total, list, before, open, rows_k, rows_v, total_far; int row_cap, copy_rows; };
 // N = rows of the KV sequence.  `total` bytes are enough for any call; with `total_far` bytes there is room for what the
 // gathered tiles need (0: this chunk size has none): the lists of the chunks that stay visible and, for chunks below 8 rows,
-// copies of their K and V rows, up to row_cap (a quarter of the sequence) per head.  D = 0: the head_dim is not known, so that
+// copies of their K and V rows, up to row_cap (a quarter of the sequence) per head, and tails of kTailRows per tile (see
+// far_rows_kernel), copy_rows in all.  D = 0: the head_dim is not known, so that
 // there is no room for rows.
 static PrefillWs prefill_ws(int B, int Hkv, int N, int C, int D) {
     PrefillWs w = {};
@@ -1122,8 +1131,9 @@ static PrefillWs prefill_ws(int B, int Hkv, int N, int C, int D) {
         w.rows_k = w.rows_v = w.total_far = w.open + per_tile;
         if (C < 8) {
             w.row_cap = (N / 4 + kTile - 1) / kTile * kTile;
-            w.rows_v = w.rows_k + BH * w.row_cap * D * 2;
-            w.total_far = w.rows_v + BH * w.row_cap * D * 2;
+            w.copy_rows = w.row_cap + kTailRows * (int)Nt;
+            w.rows_v = w.rows_k + BH * w.copy_rows * D * 2;
+            w.total_far = w.rows_v + BH * w.copy_rows * D * 2;
         }
     }
     return w;
@@ -1142,34 +1152,45 @@ static FarLists far_lists(const PrefillWs& w, uint8_t* ws, int C) {
     return far;
 }
 
-// Copies the listed rows of K and V (see PrefillWs), 64 per block; the last tile is filled up with zeros.  Moves 4 D bytes per
-// row and tensor: 3 MB for 8192 tokens with 10 % global.
+// Copies the listed rows of K and V (see PrefillWs), 64 per block.  Behind them stand kTailRows rows for every 128-row tile: the
+// last of the rows listed in front of the tile that do not make a whole group of eight, then zeros (the part empty tile of an
+// item is loaded in groups of eight and must not hold rows of later keys).  Moves 4 D bytes per row and tensor: 3 MB for 8192
+// tokens with 10 % global.
 constexpr int kFarThreads = 256, kFarRowsPerBlock = 64;
 struct FarRowsParams {
     const uint8_t* k; const uint8_t* v;              // [BH, head_rows, D] bf16
-    uint8_t* rows_k; uint8_t* rows_v;                // [BH, cap, D]
+    uint8_t* rows_k; uint8_t* rows_v;                // [BH, rows, D]
     const int32_t* list; const int32_t* before_tile;
     long long head_rows;
-    int Nc, Ntk, Nkv, C, D, cap;
+    int Nc, Ntk, Nkv, C, D, cap, rows;
 };
 __global__ void __launch_bounds__(kFarThreads) far_rows_kernel(const FarRowsParams p) {
     const int bh = blockIdx.y;
-    const int count = min((long long)p.before_tile[(size_t)bh * (p.Ntk + 1) + p.Ntk] * p.C, (long long)p.cap);
-    const int r0 = blockIdx.x * kFarRowsPerBlock, r1 = min(r0 + kFarRowsPerBlock, (count + kTile - 1) / kTile * kTile);
-    const int vpt = p.D / 8;
+    const int32_t* before = p.before_tile + (size_t)bh * (p.Ntk + 1);
     const int32_t* list = p.list + (size_t)bh * p.Nc;
+    const int count = min((long long)before[p.Ntk] * p.C, (long long)p.cap);
+    const int r0 = blockIdx.x * kFarRowsPerBlock, r1 = min(r0 + kFarRowsPerBlock, p.rows);
+    const int vpt = p.D / 8;
     for (int i = threadIdx.x; i < (r1 - r0) * vpt; i += kFarThreads) {
         const int r = r0 + i / vpt, vec = i % vpt;
+        int n = count, key = r;                      // copied: the key-th of n listed rows
+        if (r >= p.cap) {
+            n = before[(r - p.cap) / kTailRows] * p.C;
+            if (n > p.cap) continue;
+            key = n / kTailRows * kTailRows + r % kTailRows;
+        } else if (r >= count) {
+            continue;
+        }
         uint4 a = make_uint4(0, 0, 0, 0), b = a;
-        if (r < count) {
-            const int row = list[r / p.C] * p.C + r % p.C;
+        if (key < n) {
+            const int row = list[key / p.C] * p.C + key % p.C;
             if (row < p.Nkv) {                       // the last chunk of the sequence may be part empty
                 const size_t src = (((size_t)bh * p.head_rows + row) * vpt + vec) * 16;
                 a = ld16(p.k + src);
                 b = ld16(p.v + src);
             }
         }
-        const size_t dst = (((size_t)bh * p.cap + r) * vpt + vec) * 16;
+        const size_t dst = (((size_t)bh * p.rows + r) * vpt + vec) * 16;
         st16(p.rows_k + dst, a);
         st16(p.rows_v + dst, b);
     }
@@ -1179,7 +1200,8 @@ constexpr int kMaxDevices = 64;
 
 template <int D, bool FINE>
 static int launch_prefill(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mkf,
-                          const CUtensorMap& mvf, const PrefillParams& p, cudaStream_t st) {
+                          const CUtensorMap& mvf, const CUtensorMap& mkc, const CUtensorMap& mvc, const PrefillParams& p,
+                          cudaStream_t st) {
     const size_t smem = sizeof(PrefillSmem<D>);
     int dev = 0, sms = 0;
     NATS_CHECK_CUDA(cudaGetDevice(&dev));
@@ -1191,7 +1213,7 @@ static int launch_prefill(const CUtensorMap& mq, const CUtensorMap& mk, const CU
     }
     NATS_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int grid = p.total_items < sms ? p.total_items : sms;      // one persistent CTA per SM
-    prefill_kernel<D, FINE><<<grid, kPrefillThreads, smem, st>>>(mq, mk, mv, mkf, mvf, p);
+    prefill_kernel<D, FINE><<<grid, kPrefillThreads, smem, st>>>(mq, mk, mv, mkf, mvf, mkc, mvc, p);
     NATS_CHECK_CUDA(cudaGetLastError());
     return NATS_OK;
 }
@@ -1228,29 +1250,33 @@ static bool use_pair_kernel(int D, int nrep) {
 static int run_prefill(const void* d_q, const void* d_k, const void* d_v, void* d_o, int B, int Hq, int Hkv, int N, int Nkv,
                        int q_off, long long kv_head_stride, int D, int C, float sm_scale, const int32_t* lim,
                        const int32_t* tmax, const int32_t* tmin, int32_t* counter, int32_t* d_status, cudaStream_t st,
-                       const FarLists& far, uint8_t* far_k, uint8_t* far_v, int far_cap, float* d_lse = nullptr, bool o_tokens = false, bool o_f32 = false) {
+                       const FarLists& far, uint8_t* far_k, uint8_t* far_v, int far_cap, int far_rows, float* d_lse = nullptr, bool o_tokens = false, bool o_f32 = false) {
     const bool pair = use_pair_kernel(D, Hq / Hkv) && !o_f32;
-    CUtensorMap mq, mk, mv, mkf, mvf;
+    CUtensorMap mq, mk, mv, mkf, mvf, mkc, mvc;
     if (int rc = make_map(&mq, d_q, B * Hq, N, D, 128)) return rc;
     if (int rc = make_map(&mk, d_k, B * Hkv, Nkv, D, pair ? 64 : 128, kv_head_stride)) return rc;     // a pair's CTA loads half the rows of a K tile
     if (int rc = make_map(&mv, d_v, B * Hkv, Nkv, D, 128, kv_head_stride)) return rc;
-    mkf = mk;
-    mvf = mv;
+    mkf = mkc = mk;
+    mvf = mvc = mv;
     if (far.list != nullptr && far_cap > 0) {
         FarRowsParams f;
         f.k = (const uint8_t*)d_k; f.v = (const uint8_t*)d_v; f.rows_k = far_k; f.rows_v = far_v; f.list = far.list; f.before_tile = far.before_tile;
         f.head_rows = kv_head_stride > 0 ? kv_head_stride : Nkv;
-        f.Nc = cdiv(Nkv, C); f.Ntk = cdiv(Nkv, kTile); f.Nkv = Nkv; f.C = C; f.D = D; f.cap = far_cap;
-        far_rows_kernel<<<dim3(cdiv(far_cap, kFarRowsPerBlock), B * Hkv), kFarThreads, 0, st>>>(f);
+        f.Nc = cdiv(Nkv, C); f.Ntk = cdiv(Nkv, kTile); f.Nkv = Nkv; f.C = C; f.D = D; f.cap = far_cap; f.rows = far_rows;
+        far_rows_kernel<<<dim3(cdiv(far_rows, kFarRowsPerBlock), B * Hkv), kFarThreads, 0, st>>>(f);
         NATS_CHECK_CUDA(cudaGetLastError());
-        if (int rc = make_map(&mkf, far_k, B * Hkv, far_cap, D, 128)) return rc;
-        if (int rc = make_map(&mvf, far_v, B * Hkv, far_cap, D, 128)) return rc;
+        if (int rc = make_map(&mkc, far_k, B * Hkv, far_rows, D, 128)) return rc;
+        if (int rc = make_map(&mvc, far_v, B * Hkv, far_rows, D, 128)) return rc;
+        if (int rc = make_map(&mkf, far_k, B * Hkv, far_rows, D, kTailRows)) return rc;
+        if (int rc = make_map(&mvf, far_v, B * Hkv, far_rows, D, kTailRows)) return rc;
     } else if (far.list != nullptr) {
         if (int rc = make_map(&mkf, d_k, B * Hkv, Nkv, D, C, kv_head_stride)) return rc;       // boxes of one chunk
         if (int rc = make_map(&mvf, d_v, B * Hkv, Nkv, D, C, kv_head_stride)) return rc;
     }
     PrefillParams p;
     p.far_list = far.list; p.far_before = far.before_tile; p.far_open = far.open_max;
+    p.far_cap = far.list != nullptr ? far_cap : 0;
+    p.far_rows = far_rows;
     p.o_batch = (long long)N * Hq * D;
     p.o_head = o_tokens ? D : (long long)N * D;
     p.o_row = o_tokens ? (long long)Hq * D : D;
@@ -1272,13 +1298,13 @@ static int run_prefill(const void* d_q, const void* d_k, const void* d_v, void* 
         return launch_prefill_pair(mq, mk, mv, p, st);
     }
     if (p.c_shift >= 5 && far.list == nullptr) {
-        if (D == 64) return launch_prefill<64, false>(mq, mk, mv, mkf, mvf, p, st);
-        if (D == 256) return launch_prefill<256, false>(mq, mk, mv, mkf, mvf, p, st);
-        return launch_prefill<128, false>(mq, mk, mv, mkf, mvf, p, st);
+        if (D == 64) return launch_prefill<64, false>(mq, mk, mv, mkf, mvf, mkc, mvc, p, st);
+        if (D == 256) return launch_prefill<256, false>(mq, mk, mv, mkf, mvf, mkc, mvc, p, st);
+        return launch_prefill<128, false>(mq, mk, mv, mkf, mvf, mkc, mvc, p, st);
     }
-    if (D == 64) return launch_prefill<64, true>(mq, mk, mv, mkf, mvf, p, st);
-    if (D == 256) return launch_prefill<256, true>(mq, mk, mv, mkf, mvf, p, st);
-    return launch_prefill<128, true>(mq, mk, mv, mkf, mvf, p, st);
+    if (D == 64) return launch_prefill<64, true>(mq, mk, mv, mkf, mvf, mkc, mvc, p, st);
+    if (D == 256) return launch_prefill<256, true>(mq, mk, mv, mkf, mvf, mkc, mvc, p, st);
+    return launch_prefill<128, true>(mq, mk, mv, mkf, mvf, mkc, mvc, p, st);
 }
 
 }  // namespace nats
@@ -1324,7 +1350,7 @@ static int prefill_first_call(const void* d_q, const void* d_k, const void* d_v,
     if (d_n_visible != nullptr)
         if (int rc = nats_b200_visible_counts(lim, B, Hq, Hkv, N, C, d_n_visible, stream)) return rc;
     return run_prefill(d_q, d_k, d_v, d_o, B, Hq, Hkv, N, N, 0, 0, D, C, sm_scale, lim, tmax, tmin,
-                       (int32_t*)(ws + w.counter), d_status, (cudaStream_t)stream, far, ws + w.rows_k, ws + w.rows_v, w.row_cap, d_lse, o_tokens, o_f32);
+                       (int32_t*)(ws + w.counter), d_status, (cudaStream_t)stream, far, ws + w.rows_k, ws + w.rows_v, w.row_cap, w.copy_rows, d_lse, o_tokens, o_f32);
 }
 
 extern "C" __attribute__((visibility("default"))) int nats_b200_prefill_fwd(const void* d_q, const void* d_k, const void* d_v, void* d_o, const uint8_t* d_roles,
@@ -1389,7 +1415,7 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_prefill_past_fwd
                                           valid_stride, t0, fill, tail, lim, tmax, tmin, d_kept_tiles, far, (int32_t*)(ws + w.counter), stream)) return rc;
     return run_prefill(d_q, d_cache_k, d_cache_v, d_o, B, Hq, Hkv, x_len, (int)n_kv, t0 + fill, cache_capacity, D, C, sm_scale,
                        lim, tmax, tmin, (int32_t*)(ws + w.counter), d_status, (cudaStream_t)stream, far,
-                       ws + w.rows_k, ws + w.rows_v, w.row_cap);
+                       ws + w.rows_k, ws + w.rows_v, w.row_cap, w.copy_rows);
 }
 
 // =================================================================================================

@@ -51,6 +51,34 @@ def test_far_chunks_are_gathered(C, N, p_global, p_local, D):
     assert_close_attn(run_prefill(q, k, v, roles, C, SW), orc.prefill_attention(q, k, v, roles, C, SW))
 
 
+@pytest.mark.parametrize('C', [1, 2, 4, 8, 16, 32, 64])
+@pytest.mark.parametrize('D', [64, 128, 256])
+def test_gathered_tiles_hold_no_key_of_the_future(C, D):
+    """K and V that are not finite from some position on (what stands behind the end of a prompt, or one bad token) leave every
+    row in front of the tile of that position as it is: a masked key is multiplied by an exact zero, which needs a finite V."""
+    from neuralattentionsearch_b200 import check_status, prefill_attention
+    B, Hq, Hkv, N = 1, 2, 1, 2700
+    SW = C * max(1, 200 // C)
+    roles = orc.make_roles(B, Hkv, -(-N // C), 0.1, 0.3, seed=C)
+    roles[..., -(-N // C) // 2:][..., ::7] = orc.ROLE_GLOBAL
+    q, k, v = (t.to(dev()).bfloat16() for t in inputs(B, Hq, Hkv, N, D, seed=C + D, sigma=0.5))
+    r = torch.from_numpy(roles).to(dev())
+    clean = prefill_attention(q, k, v, r, C, SW)
+    assert torch.isfinite(clean).all()
+    for first, last in ((2300, N), (1800, 1801), (1999, N)):
+        at = first // C * C                                      # from a chunk's first token on, and that chunk is a global one
+        rr = r.clone()
+        rr[..., first // C] = orc.ROLE_GLOBAL
+        want = prefill_attention(q, k, v, rr, C, SW)
+        for bad in (float('inf'), float('nan')):
+            kk, vv = k.clone(), v.clone()
+            kk[:, :, at:last], vv[:, :, at:last] = bad, bad
+            got = prefill_attention(q, kk, vv, rr, C, SW)
+            assert torch.equal(got[:, :, :at // 128 * 128], want[:, :, :at // 128 * 128])
+            assert not torch.isfinite(got[:, :, last - 1]).any()
+    check_status(dev())
+
+
 @pytest.mark.parametrize('C', [1, 16, 64])
 def test_far_chunks_of_a_call_over_a_cache(C):
     """Segments over the compacted cache (ragged, the second one starting inside a chunk) equal one call over the sequence."""
