@@ -144,8 +144,10 @@ class NAtSChunkLayerCache:
         if x_len == 0:
             return self.cache_k[:, :, :self.n_ctx_data], self.cache_v[:, :, :self.n_ctx_data]
         self._tokens_info = token_states_info
-        # a single token that leaves its chunk unfinished carries a placeholder: nothing reads its role
-        unread = x_len == 1 and self._buf_k is not None and self.chunk_fill_size < self.chunk_size
+        # the role of a fused single token that leaves its chunk unfinished is a placeholder nothing reads; a token that is written
+        # now may be a segment of its own, whose roles ``prefill_attention`` reads
+        unread = fused and x_len == 1 and self._buf_k is not None and self.chunk_fill_size < self.chunk_size and \
+            token_states_info is not None and (token_states_info.is_floating_point() or token_states_info.dtype == torch.uint8)
         self._roles = None if token_states_info is None or unread else F_.roles_from_token_states_info(token_states_info)
         if self._buf_k is None and self._pending is None:
             self._pending = (key_states, value_states)

@@ -112,6 +112,7 @@ SEG_SHAPES = [
     (1, 6, 2, 128, 32, 128, [96, 2000], 0.02, 0.10, 34),                      # first call shorter than the window
     (1, 4, 1, 128, 128, 512, [2048, 2048], 0.0, 0.3, 35),                     # no global chunk after the first
     (2, 2, 2, 64, 1, 16, [300, 212], 0.10, 0.30, 36),                         # token-granular roles
+    (2, 4, 2, 64, 16, 64, [300, 1, 3, 1, 14, 1, 200, 1], 0.10, 0.30, 37),     # segments of one token, one of them completes a chunk
 ]
 
 

@@ -136,3 +136,21 @@ def test_hf_patch_attaches_role_heads_and_samples_roles():
     assert torch.equal(info[:, :, 1].argmax(-1), want)
     with pytest.raises(TypeError):
         att(hidden_states=x, position_embeddings=(x, x), past_key_values=None)
+
+
+def test_roles_of_a_single_token_are_kept_unless_nothing_reads_them():
+    """A token handed over as a segment (not fused) keeps its roles for ``prefill_attention``; a fused one that leaves its chunk
+    unfinished has none to keep, and one that completes it does."""
+    from neuralattentionsearch_b200 import NAtSChunkLayerCache
+    B, H, C, D = 2, 3, 4, 8
+    info = torch.nn.functional.one_hot(torch.randint(0, 3, (B, H, 1)), 3).float()
+    want = info.argmax(-1).to(torch.uint8)
+    for fused, third in ((False, True), (True, False)):
+        cache = NAtSChunkLayerCache(B, H, 8, chunk_size=C, device=torch.device('cpu'))
+        cache.update(torch.randn(B, H, 2, D), torch.randn(B, H, 2, D), info)
+        cache.post_update(2)
+        cache.update(torch.randn(B, H, 1, D), torch.randn(B, H, 1, D), info, fused=fused)
+        assert torch.equal(cache._roles, want) if third else cache._roles is None
+        cache.post_update(1)
+        cache.update(torch.randn(B, H, 1, D), torch.randn(B, H, 1, D), info, fused=fused)
+        assert torch.equal(cache._roles, want)
