@@ -210,7 +210,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 if (lane == 0) {
                     ItemHeader hd;
                     hd.valid = 1; hd.t = t; hd.b = z; hd.bh = bh; hd.head0 = hkv * p.nrep + grp * 4 + (int)cta * 2;
-                    hd.nslots = 2; hd.n_kept = n_kept; hd.far_keys = hd.far_tail = 0;
+                    hd.nslots = 2; hd.n_kept = n_kept; hd.far_keys = 0;
                     sm.item[slot] = hd;
                 }
             } else if (lane == 0) {

@@ -348,7 +348,6 @@ struct ItemHeader {
     int nslots;     // 1 or 2 query heads in this item
     int n_kept;     // 128-column KV tiles: gathered ones first, then the kept tiles of the bitmap
     int far_keys;   // keys of the gathered tiles (the last one may be part empty)
-    int far_tail;   // chunks below 8 rows: row of the copy that holds the last far_keys % 8 of them, zeros behind
 };
 
 constexpr int kBitWords = kMaxTiles / 32;
@@ -373,6 +372,7 @@ struct PrefillSmem {
     uint32_t tmem_base;
     int abort_flag;
     int pipe_lock;                             // held by the issuer whose batch of MMAs is being queued
+    int far_tail[2];                           // per item, chunks below 8 rows: row of the copy that holds the last far_keys % 8 listed ones
 };
 static_assert(sizeof(PrefillSmem<128>) <= 232448 && sizeof(PrefillSmem<256>) <= 232448, "shared memory of the widest kernels");
 
@@ -581,8 +581,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                     ItemHeader hd;
                     hd.valid = 1; hd.t = t; hd.b = z; hd.bh = bh; hd.head0 = hkv * p.nrep + grp * Smem::kHeads;
                     hd.nslots = min(Smem::kHeads, p.nrep - grp * Smem::kHeads); hd.n_kept = n_kept; hd.far_keys = far_keys;
-                    hd.far_tail = p.far_cap + kTailRows * max(near_first, 0);
                     sm.item[slot] = hd;
+                    if (FINE) sm.far_tail[slot] = p.far_cap + kTailRows * max(near_first, 0);
                 }
             } else if (lane == 0) {
                 sm.item[slot].valid = 0;
@@ -653,7 +653,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 if (boxes) {
                     const int key = j * kTile + ((lane & (n_boxes - 1)) << box_shift);
                     if (p.far_cap == 0) box_row = key < hd.far_keys ? far_list[key >> box_shift] * box_rows : p.Nkv;
-                    else box_row = key + box_rows <= hd.far_keys ? key : key < hd.far_keys ? hd.far_tail : p.far_rows;
+                    else box_row = key + box_rows <= hd.far_keys ? key : key < hd.far_keys ? sm.far_tail[slot] : p.far_rows;
                 }
 #pragma unroll 1
                 for (int kv = 0; kv < 2 && ok; ++kv, ++g) {
