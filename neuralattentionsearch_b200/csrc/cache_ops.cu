@@ -63,10 +63,9 @@ static_assert(kPrepWarps == 32, "a warp holds one value per warp of the block");
 
 // Per 128-row KV tile: max / min of the limits of the chunks it overlaps, and how many query tiles keep it.  Query row i
 // sits at position q_off + i; there are Nt query tiles of 128 rows.  Fine chunks: a warp per tile (coalesced loads); others:
-// a thread per tile.  open_max (may be null): max over the chunks that are not visible for good.  Returns this thread's share
-// of the kept count.
+// a thread per tile.  open_max (may be null) and dense_min: see FarLists.  Returns this thread's share of the kept count.
 __device__ unsigned long long tile_limits(const int32_t* __restrict__ lim, int Nkv, int C, int Ntk, int q_off, int Nt,
-                                          int32_t* __restrict__ tmax, int32_t* __restrict__ tmin, int32_t* __restrict__ open_max) {
+                                          int32_t* __restrict__ tmax, int32_t* __restrict__ tmin, int32_t* __restrict__ open_max, int dense_min) {
     unsigned long long mine = 0;
     const bool wide = C < 16;
     const int lane = threadIdx.x & 31;
@@ -74,22 +73,24 @@ __device__ unsigned long long tile_limits(const int32_t* __restrict__ lim, int N
     for (int kt = first_tile; kt < Ntk; kt += step) {
         const int c0 = (int)(((long long)kt * kTile) / C);
         const int c1 = (int)(min((long long)kt * kTile + kTile - 1, (long long)Nkv - 1) / C);
-        int mx = -1, mn = kNoLimit, om = -1;
+        int mx = -1, mn = kNoLimit, om = -1, listed = 0;
         for (int c = wide ? c0 + lane : c0; c <= c1; c += wide ? 32 : 1) {
             const int l = lim[c];
             mx = max(mx, l);
             mn = min(mn, l);
             if (l != kNoLimit) om = max(om, l);
+            else ++listed;
         }
         if (wide) {
             mx = __reduce_max_sync(0xffffffffu, mx);
             mn = __reduce_min_sync(0xffffffffu, mn);
             om = __reduce_max_sync(0xffffffffu, om);
+            listed = __reduce_add_sync(0xffffffffu, listed);
             if (lane != 0) continue;
         }
         tmax[kt] = mx;
         tmin[kt] = mn;
-        if (open_max != nullptr) open_max[kt] = om;
+        if (open_max != nullptr) open_max[kt] = 2 * min(om, kOpenMax) + (listed >= dense_min ? 1 : 0);
         // query tiles t that keep the tile: last row position >= first tile row, first row position <= mx
         const long long first = (long long)kt * kTile - q_off - (kTile - 1);
         const int t_min = first <= 0 ? 0 : (int)((first + kTile - 1) / kTile);
@@ -102,14 +103,17 @@ __device__ unsigned long long tile_limits(const int32_t* __restrict__ lim, int N
 }
 
 // The chunks that stay visible for good, in order, and how many of them lie in front of every 128-row tile (chunks divide a
-// tile: cpt per tile).  All threads of the block call, after scan_role_limits.
+// tile: cpt per tile), without those of dense tiles.  All threads of the block call, after scan_role_limits and tile_limits.
 __device__ void list_far_chunks(const int32_t* __restrict__ lim, int Nc, int cpt, int Ntk, int32_t* __restrict__ list,
-                                int32_t* __restrict__ before_tile, int32_t* __restrict__ open_max, int max_listed, int (*s)[kPrepWarps]) {
+                                int32_t* __restrict__ before_tile, int32_t* __restrict__ open_max, int max_listed, int dense_min, int (*s)[kPrepWarps]) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int base = 0, buf = 0;
+    const bool any_dense = dense_min <= cpt;
+    if (any_dense) __syncthreads();                       // open_max of every tile is there
     for (int c0 = 0; c0 < Nc; c0 += kPrepThreads, buf ^= 1) {
         const int c = c0 + tid;
-        const bool keep = c < Nc && lim[c] == kNoLimit;
+        const bool dense = any_dense && c < Nc && (open_max[c / cpt] & 1);
+        const bool keep = c < Nc && lim[c] == kNoLimit && !dense;
         const unsigned m = __ballot_sync(0xffffffffu, keep);
         if (lane == 0) s[buf][warp] = __popc(m);
         __syncthreads();
@@ -123,7 +127,7 @@ __device__ void list_far_chunks(const int32_t* __restrict__ lim, int Nc, int cpt
     if (base <= max_listed) return;
     __syncthreads();
     for (int kt = tid; kt < Ntk; kt += kPrepThreads)
-        if (before_tile[kt + 1] > max_listed) open_max[kt] = kNoLimit;
+        if (before_tile[kt + 1] > max_listed) open_max[kt] = 2 * kOpenMax;
 }
 
 __global__ void __launch_bounds__(kPrepThreads)
@@ -141,10 +145,10 @@ role_prep_kernel(const uint8_t* __restrict__ roles, int Nc, int N, int C, int SW
     __shared__ unsigned long long kept_sm;
     if (tid == 0) kept_sm = 0;
     scan_role_limits(roles, Nc, C, SW, 0, lim, s, &first_gf);
-    const unsigned long long mine = tile_limits(lim, N, C, Nt, 0, Nt, tmax, tmin, far.list ? far.open_max + (size_t)bh * Nt : nullptr);
+    const unsigned long long mine = tile_limits(lim, N, C, Nt, 0, Nt, tmax, tmin, far.list ? far.open_max + (size_t)bh * Nt : nullptr, far.dense_min);
     if (far.list != nullptr)
         list_far_chunks(lim, Nc, kTile / C, Nt, far.list + (size_t)bh * Nc, far.before_tile + (size_t)bh * (Nt + 1), far.open_max + (size_t)bh * Nt,
-                        far.max_listed, s);
+                        far.max_listed, far.dense_min, s);
     if (kept != nullptr) {
         if (mine) atomicAdd(&kept_sm, mine);
         __syncthreads();
@@ -197,10 +201,10 @@ __global__ void __launch_bounds__(kPrepThreads) role_prep_past_kernel(const Past
     }
     __syncthreads();
     const unsigned long long mine = tile_limits(lim, p.Nkv, p.C, p.Ntk, p.q_off, p.Nt, p.tmax + (size_t)bh * p.Ntk, p.tmin + (size_t)bh * p.Ntk,
-                                                p.far.list ? p.far.open_max + (size_t)bh * p.Ntk : nullptr);
+                                                p.far.list ? p.far.open_max + (size_t)bh * p.Ntk : nullptr, p.far.dense_min);
     if (p.far.list != nullptr)
         list_far_chunks(lim, p.Nc, kTile / p.C, p.Ntk, p.far.list + (size_t)bh * p.Nc, p.far.before_tile + (size_t)bh * (p.Ntk + 1),
-                        p.far.open_max + (size_t)bh * p.Ntk, p.far.max_listed, s);
+                        p.far.open_max + (size_t)bh * p.Ntk, p.far.max_listed, p.far.dense_min, s);
     if (p.kept != nullptr) {
         if (mine) atomicAdd(&kept_sm, mine);
         __syncthreads();

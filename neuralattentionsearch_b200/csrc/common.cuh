@@ -30,15 +30,18 @@ int fail(int code, const char* fmt, ...);
             return ::nats::fail(NATS_ERR_CUDA, "%s failed: %s", #expr, cudaGetErrorString(e_));   \
     } while (0)
 
-// Chunks that stay visible for good, per (batch, kv-head): list [Nc] = their indices in order, before_tile [Ntk + 1] = how many
-// of them lie in front of a 128-row KV tile (at the end: all), open_max [Ntk] = largest row limit of the tile's other chunks
-// (-1: it has none; kNoLimit: more than max_listed lie in front of the next tile).  list == nullptr: not wanted.  Only for chunk
-// sizes that divide a tile.
+// Chunks that stay visible for good, per (batch, kv-head), without those of dense tiles (dense_min of them or more in a 128-row KV
+// tile): list [Nc] = their indices in order, before_tile [Ntk + 1] = how many of them lie in front of a tile (at the end: all),
+// open_max [Ntk] = twice the largest row limit of the tile's other chunks (-1: it has none; kOpenMax: as large or larger, or more
+// than max_listed lie in front of the next tile), plus one if the tile is dense.  list == nullptr: not wanted.  Only for
+// chunk sizes that divide a tile.
+constexpr int kOpenMax = 0x3fffffff;
 struct FarLists {
     int32_t* list = nullptr;
     int32_t* before_tile = nullptr;
     int32_t* open_max = nullptr;
     int max_listed = 0x7fffffff;
+    int dense_min = 0x7fffffff;
 };
 
 // the C entry points nats_b200_role_prep / _past with the lists beside the limits; *d_counter (may be null) is set to zero

@@ -15,7 +15,8 @@
 // are not computed in place but gathered: the keys of 128 / C listed chunks (FarLists) make a full tile.  Chunks of 8 rows and
 // more are copied chunk by chunk (boxes of C rows); finer ones come from a copy of the listed rows in the workspace, made once
 // per call (far_rows_kernel), since single rows arrive at ~8 cycles each from tile::gather4, 4000 for a K / V tile pair.  The
-// bitmap then only holds the tiles from the first one on in which some other chunk is still visible.  The work of a query
+// bitmap then only holds the tiles from the first one on in which some other chunk is still visible, and dense ones in front of
+// it: a tile nearly all of whose chunks are listed is cheaper in place (see far_dense_min).  The work of a query
 // tile falls from the tiles that hold a visible key towards the keys that are visible: prompt of 8192 tokens with one role
 // per token, 10 % global, 0.91 -> 0.21 ms (0.29 with tile::gather4); forward of 8 x 4096 tokens with chunks of 16, 0.51 -> 0.26 ms.
 // Which KV tiles are visited comes from the role bitmap: a bitmap of kept tiles is built in shared memory from the
@@ -67,7 +68,7 @@ struct PrefillParams {
     const int32_t* tile_max;          // [B,Hkv,Ntk]: max / min of lim over the chunks of a 128-row KV tile
     const int32_t* tile_min;
     // chunks visible for good (see FarLists), or all nullptr: the tiles in front of the first tile with another visible chunk
-    // are not walked, their listed chunks are gathered into full tiles instead
+    // are not walked (but for the dense ones), their listed chunks are gathered into full tiles instead
     const int32_t* far_list;
     const int32_t* far_before;
     const int32_t* far_open;
@@ -547,8 +548,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 const int kt_last = q_hi / kTile;
                 const int32_t* tmax = p.tile_max + (size_t)bh * p.Ntk;
                 const int32_t* tmin = p.tile_min + (size_t)bh * p.Ntk;
-                // The tiles in front of near_first hold no visible chunk but listed ones: they are left out of the bitmap.
-                // near_first <= the tile of the first query row, so every listed key in front of it is in that row's past.
+                // The tiles in front of near_first hold no visible chunk but listed ones: only the dense ones among them, whose chunks
+                // are not gathered, stay in the bitmap.  near_first <= the tile of the first query row, so every listed key in
+                // front of it is in that row's past.
                 const int32_t* open = FINE && p.far_open != nullptr ? p.far_open + (size_t)bh * p.Ntk : nullptr;
                 const int near_cap = q_lo / kTile;
                 int near_first = open != nullptr ? -1 : 0;
@@ -560,11 +562,12 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                     unsigned m = __ballot_sync(0xffffffffu, keep);
                     unsigned pm = __ballot_sync(0xffffffffu, partial);
                     if (near_first < 0) {
-                        const unsigned om = __ballot_sync(0xffffffffu, kt <= near_cap && (kt == near_cap || open[kt] >= q_lo));
+                        const int o = kt <= near_cap ? open[kt] : 0;
+                        const unsigned om = __ballot_sync(0xffffffffu, kt <= near_cap && (kt == near_cap || (o >> 1) >= q_lo));
                         if (om != 0u) near_first = s0 + __ffs(om) - 1;
-                        const unsigned from = om != 0u ? 0xffffffffu << (near_first - s0) : 0u;
-                        m &= from;
-                        pm &= from;
+                        const unsigned in_place = __ballot_sync(0xffffffffu, o & 1) | (om != 0u ? 0xffffffffu << (near_first - s0) : 0u);
+                        m &= in_place;
+                        pm &= in_place;
                     }
                     if (lane == 0) {
                         sm.keep[slot][s0 >> 5] = m;
@@ -1146,9 +1149,22 @@ static int far_min_rows(int C) { return C <= 16 ? 1024 : 2048; }
 static bool use_far(const PrefillWs& w, size_t workspace_bytes, int C, int q_end, bool pair) {
     return w.total_far != 0 && workspace_bytes >= w.total_far && q_end >= far_min_rows(C) && !pair;
 }
-static FarLists far_lists(const PrefillWs& w, uint8_t* ws, int C) {
-    FarLists far = {(int32_t*)(ws + w.list), (int32_t*)(ws + w.before), (int32_t*)(ws + w.open), 0x7fffffff};
+// How many listed chunks make a tile dense, so that it stays in place.  A gathered tile costs more than one in place where its
+// boxes are many (all chunks global, 24576 tokens, time over the same in place: 64 boxes a tile (chunks of 8, head_dim 256) 2.4, 32
+// (16 / 256, 8 / 128) 1.6 and 1.5, 16 (32 / 256, 16 / 128, 8 / 64) 1.16, 1.09 and 1.11, fewer 1.00 to 1.02), the masks of a tile
+// in place make it about 1/8 dearer; a full tile needs neither masks nor gathering.  Chunks below 8 have no dense tiles: their
+// copies are loaded in boxes of 128 rows, and the test would cost them 3 of 178 us (8192 tokens, one role per token).
+static int far_dense_min(int C, int D) {
+    if (C < 8) return 0x7fffffff;
+    const int cpt = kTile / C, boxes = cpt * (D / 64);
+    const int cost = boxes >= 64 ? 39 : boxes >= 32 ? 25 : 16;             // of a gathered tile, in 16ths of a full one
+    return min(cpt, cdiv(cpt * 18, cost));
+}
+static FarLists far_lists(const PrefillWs& w, uint8_t* ws, int C, int D) {
+    FarLists far;
+    far.list = (int32_t*)(ws + w.list); far.before_tile = (int32_t*)(ws + w.before); far.open_max = (int32_t*)(ws + w.open);
     if (w.row_cap) far.max_listed = w.row_cap / C;
+    far.dense_min = far_dense_min(C, D);
     return far;
 }
 
@@ -1345,7 +1361,7 @@ static int prefill_first_call(const void* d_q, const void* d_k, const void* d_v,
     int32_t* tmax = (int32_t*)(ws + w.tmax);
     int32_t* tmin = (int32_t*)(ws + w.tmin);
     FarLists far;
-    if (use_far(w, workspace_bytes, C, N, use_pair_kernel(D, Hq / Hkv) && !o_f32)) far = far_lists(w, ws, C);
+    if (use_far(w, workspace_bytes, C, N, use_pair_kernel(D, Hq / Hkv) && !o_f32)) far = far_lists(w, ws, C, D);
     if (int rc = role_prep(d_roles, B, Hkv, N, C, SW, lim, tmax, tmin, d_kept_tiles, far, (int32_t*)(ws + w.counter), stream)) return rc;
     if (d_n_visible != nullptr)
         if (int rc = nats_b200_visible_counts(lim, B, Hq, Hkv, N, C, d_n_visible, stream)) return rc;
@@ -1410,7 +1426,7 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_prefill_past_fwd
     int32_t* tmax = (int32_t*)(ws + w.tmax);
     int32_t* tmin = (int32_t*)(ws + w.tmin);
     FarLists far;
-    if (use_far(w, workspace_bytes, C, (int)n_kv, use_pair_kernel(D, Hq / Hkv))) far = far_lists(w, ws, C);
+    if (use_far(w, workspace_bytes, C, (int)n_kv, use_pair_kernel(D, Hq / Hkv))) far = far_lists(w, ws, C, D);
     if (int rc = role_prep_past(d_roles_new, d_valid, d_size_global, d_size_local, B, Hkv, x_len, C, SW,
                                           valid_stride, t0, fill, tail, lim, tmax, tmin, d_kept_tiles, far, (int32_t*)(ws + w.counter), stream)) return rc;
     return run_prefill(d_q, d_cache_k, d_cache_v, d_o, B, Hq, Hkv, x_len, (int)n_kv, t0 + fill, cache_capacity, D, C, sm_scale,

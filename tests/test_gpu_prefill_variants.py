@@ -39,11 +39,13 @@ def test_mask_bits_of_every_chunk_granularity(C):
 @pytest.mark.parametrize('C,N,p_global,p_local', [(1, 2048, 0.1, 0.3), (2, 2500, 0.05, 0.3), (4, 2177, 0.2, 0.1), (8, 2300, 0.1, 0.3),
                                                   (16, 3001, 0.03, 0.1), (32, 2600, 0.3, 0.0), (64, 4000, 0.1, 0.6), (16, 2304, 1.0, 0.0),
                                                   (1, 2304, 0.0, 1.0), (32, 2304, 0.0, 0.0),
-                                                  (1, 2304, 1.0, 0.0), (2, 3000, 0.6, 0.2), (1, 1024, 0.1, 0.3), (16, 1500, 0.1, 0.2)])
+                                                  (1, 2304, 1.0, 0.0), (2, 3000, 0.6, 0.2), (1, 1024, 0.1, 0.3), (16, 1500, 0.1, 0.2),
+                                                  (8, 2500, 0.5, 0.2), (16, 2500, 0.85, 0.1), (64, 4000, 0.9, 0.1)])
 @pytest.mark.parametrize('D', [64, 128, 256])
 def test_far_chunks_are_gathered(C, N, p_global, p_local, D):
     """Prompts long enough for the gathered tiles: every way of gathering (copied rows, boxes of 8 to 64 rows), a last gathered
-    tile that is full, part empty or missing (no global chunk but the first), all chunks global (more rows than are copied), all local."""
+    tile that is full, part empty or missing (no global chunk but the first), all chunks global (more rows than are copied), all local, and so many global ones
+    that some or all items leave their tiles in place."""
     B, Hq, Hkv = (2, 4, 2) if D == 64 else (1, 3, 1)
     SW = C * max(1, 200 // C)
     roles = orc.make_roles(B, Hkv, -(-N // C), p_global, p_local, seed=N + C)
