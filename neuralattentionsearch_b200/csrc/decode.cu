@@ -373,10 +373,9 @@ __global__ void __launch_bounds__(kDecThreads) decode_kernel(const DecodeParams 
 // a quarter of the columns of O.  The arithmetic on every value is the one of decode_kernel in the same order -- the running
 // maximum, the row sum and each accumulator see the strand's tiles in sequence, strands and segments are combined in the same
 // two steps -- so that a head's output does not depend on which of the two kernels the size of the batch selects.
-// One launch in a graph of 20, us, decode_kernel / strands, head_dim 128, 2900 rows per head: 24 segments 21.1 / 10.9, 48
-// 21.0 / 12.2, 96 21.6 / 13.5, 144 21.6 / 21.6; 12000 rows, 96 segments 24.0 / 17.2, 8000 rows, 128 segments 21.1 / 23.2.
-// head_dim 64: 24 segments 18.6 / 9.0, 144 18.8 / 11.8, 192 19.9 / 17.3, 288 20.0 / 20.1.  What is left of a short launch (10 us) is
-// a chain of latencies: sizes, copies, scores, partial results, ticket, combination.
+// One launch in a graph of 20, us, decode_kernel / strands, four query heads per kv-head, 2900 rows per head, head_dim 128: 24
+// segments 21.8 / 10.9, 96 21.9 / 13.4; head_dim 64: 24 segments 18.2 / 8.9, 144 18.8 / 11.8 (lines: use_strands).  What is left of a
+// short launch (10 us) is a chain of latencies: sizes, copies, scores, partial results, ticket, combination.
 constexpr int kStrandTiles = kSeg / kTileTok / kDecWarps;
 constexpr int kStrandTilesPerWarp = kStrandTiles / kDecWarps;
 static_assert(kStrandTiles % kDecWarps == 0, "tiles of a strand are dealt to the warps in equal numbers");
@@ -637,17 +636,24 @@ __global__ void __launch_bounds__(kDecThreads) decode_strand_kernel(const Decode
     if (STEP) finish_step(p, bh, gridDim.y * gridDim.z, T0, fill);
 }
 
-// Segments of a launch up to which every strand gets its own block (measured at decode_strand_kernel), and up to which V gets slots
-// of its own: as long as all strands fit on the chip at once (148 SMs, one block each at head_dim 128, three at 64), where it
-// is 1 to 5 % faster; behind that it loses (head_dim 128, 48 segments 17.9 against 12.2 us; 64, 128 segments 18.5 against 14.9).
-#ifndef NATS_STRAND_SEGMENTS
-#define NATS_STRAND_SEGMENTS (D == 64 ? 192 : 96)
-#endif
-#ifndef NATS_STRAND_BOTH
-#define NATS_STRAND_BOTH (D == 64 ? 111 : 37)
-#endif
-constexpr int strand_segments(int D) { return NATS_STRAND_SEGMENTS; }
-constexpr int strand_both_segments(int D) { return NATS_STRAND_BOTH; }
+// Launches (segments in all, `splits` of them per (batch, kv-head)) in which every strand gets its own block.  Time of decode_kernel
+// over that of strands, 1 / 2 / 4 / 8 query heads per kv-head, on both sides of the lines:
+//   head_dim 64    1 split: 160 segments 1.02 / 1.02 / 1.03 / 1.02, 192 0.72 / 0.73 / 0.73 / 0.73;  8 splits: 160 1.12 / 1.14 / 1.21 / 1.26,
+//                  192 0.95 / 0.91 / 0.97 / 1.07;  16 splits: 96 1.11 / 1.09 / 1.12 / 1.26, 112 0.95 / 0.93 / 1.02 / 1.14;
+//                  24 splits, 72 segments: 1.01 / 0.94 / 1.04 / 1.24;  48 splits, 96: 0.72 / 0.67 / 0.79 / 1.10
+//   head_dim 128   1 split: 72 segments 1.00 / 1.02 / 1.02 / 0.99, 80 0.94 / 0.94 / 0.96 / 0.92;  2 to 8 splits: 96 segments 1.11 to 1.79, 112
+//                  0.73 to 1.17;  16 splits: 96 1.05 / 1.09 / 1.27 / 1.24;  24 splits: 96 0.95 / 1.04 / 1.29 / 1.21;  32 splits: 96
+//                  0.85 / 0.98 / 1.24 / 1.16;  96 splits: 96 0.60 / 0.80 / 1.21 / 1.11
+// One split needs no combination in decode_kernel; with many splits the last block of a head combines four times as many
+// partial results, which more query heads make up for (decode_kernel goes over them head by head).
+constexpr int max_strand_segments(int D) { return D == 64 ? 160 : 96; }
+static bool use_strands(int D, long long segments, int splits, int nrep) {
+    if (D == 64) return segments <= (splits <= 12 ? max_strand_segments(64) : 96) && splits <= (nrep < 8 ? 16 : 48);
+    return segments <= (splits == 1 ? 72 : max_strand_segments(128)) && splits <= (nrep == 1 ? 16 : nrep < 4 ? 24 : 96);
+}
+// V gets slots of its own while all strands fit on the chip at once (148 SMs, one block each at head_dim 128, three at 64): 3 to 12 %
+// faster at 64; at 128 2 % up to 3 splits, but 4 to 14 % slower at 4 and 16 to 32 % at 16 (8 to 32 segments).
+static bool use_both(int D, long long segments, int splits) { return D == 64 ? segments <= 111 : segments <= 37 && splits <= 3; }
 
 // the opt-in to more than 48 KB of dynamic shared memory is a per-device attribute of a kernel
 template <class Kernel>
@@ -676,8 +682,8 @@ template <int D, bool STEP>
 static cudaError_t launch_decode(const DecodeParams& p, dim3 grid, cudaStream_t st) {
     cudaError_t e;
     const long long segments = (long long)grid.x * grid.y * grid.z;
-    if (segments <= strand_segments(D))
-        return segments <= strand_both_segments(D) ? launch_strands<D, STEP, true>(p, grid, st) : launch_strands<D, STEP, false>(p, grid, st);
+    if (use_strands(D, segments, grid.x, p.nrep))
+        return use_both(D, segments, grid.x) ? launch_strands<D, STEP, true>(p, grid, st) : launch_strands<D, STEP, false>(p, grid, st);
     constexpr int smem = kDecWarps * kDecStages * 2 * kTileTok * D * 2;
     static bool done[64] = {};
     if ((e = allow_smem(decode_kernel<D, STEP>, smem, done)) != cudaSuccess) return e;
@@ -690,7 +696,7 @@ static int decode_max_splits(int max_len) { return cdiv(max_len + 1, kSeg); }
 // floats of the partial results of a split of a (batch, kv-head): one per query head, or one per strand and query head where a
 // launch may be of that kind (a launch has at least one segment per (batch, kv-head))
 static size_t decode_split_floats(int B, int Hkv, int nrep, int D) {
-    return (long long)B * Hkv <= strand_segments(D) ? (size_t)kDecWarps * nrep * (D + 4) : (size_t)nrep * (D + 2);
+    return (long long)B * Hkv <= max_strand_segments(D) ? (size_t)kDecWarps * nrep * (D + 4) : (size_t)nrep * (D + 2);
 }
 
 }  // namespace nats

@@ -2,6 +2,8 @@
 import pytest
 import torch
 
+from test_gpu_parity import assert_close_attn
+
 pytestmark = pytest.mark.gpu
 
 GLOBAL, LOCAL, SLIDING = 0, 1, 2
@@ -31,34 +33,80 @@ def data(B, Hq, Hkv, N, D, C, seed):
     return k, v, roles.to(dev()), toks
 
 
-# cache lengths (window + tokens + the new one) around one and two segments of 1024 tokens, around tiles of 16, and short ones
+def kernel_of(cache, Hq, D, bound=None, fill=None):
+    """Which kernel a step of this cache runs: the lines of use_strands and use_both in csrc/decode.cu."""
+    splits = -(-((cache._t0_bound if bound is None else bound) + (cache.chunk_fill_size if fill is None else fill) + 1) // 1024)
+    B, H = cache._buf_k.shape[:2]
+    segments, nrep = B * H * splits, Hq // H
+    if D == 64:
+        if segments > (160 if splits <= 12 else 96) or splits > (16 if nrep < 8 else 48):
+            return 'segments'
+        return 'strands, V beside K' if segments <= 111 else 'strands, V in place of K'
+    if segments > (72 if splits == 1 else 96) or splits > (16 if nrep == 1 else 24 if nrep < 4 else 96):
+        return 'segments'
+    return 'strands, V beside K' if segments <= 37 and splits <= 3 else 'strands, V in place of K'
+
+
+def attend(cache, q, i, k, v, roles):
+    """One step of sequences i of the inputs; returns the output and the kernel that ran."""
+    full = cache.chunk_fill_size + 1 == cache.chunk_size
+    cache.update(k[i].contiguous(), v[i].contiguous(), roles[i].contiguous() if full else None, fused=True)
+    ran = kernel_of(cache, q.shape[1], q.shape[-1], fill=cache.chunk_fill_size - 1)
+    o = cache.decode_attention(q[i].contiguous())
+    cache.post_update(1)
+    return o, ran
+
+
+# cache lengths (window + tokens + the new one) around one, two and three segments of 1024 tokens, around tiles of 16, and short ones
 @pytest.mark.parametrize('N,C,SW', [(1, 16, 64), (40, 16, 64), (959, 32, 64), (960, 32, 64), (991, 1, 32), (992, 1, 32), (1983, 64, 64), (2000, 8, 64),
                                     (3000, 128, 512)])
-@pytest.mark.parametrize('D,Hq', [(64, 8), (128, 32), (128, 64)])
+@pytest.mark.parametrize('D,Hq', [(64, 8), (64, 64), (128, 32), (128, 64)])
 def test_a_head_decodes_the_same_whatever_the_batch(N, C, SW, D, Hq):
-    """Ten sequences of 8 kv-heads run in blocks of a whole segment, one sequence in a block per strand: same bits."""
-    B, Hkv = 10, 8
+    """The same sequences in a large batch (a block per segment), in one of middle size (strands, V in the place of K) and alone
+    (strands, with room for both where there are few segments per head): same bits, and those of a head are right."""
+    Hkv = 8
+    B = 26 if D == 64 else 13
     k, v, roles, toks = data(B, Hq, Hkv, N, D, C, seed=N + D)
-    every = make_cache(k, v, roles, C, SW)
-    single = [make_cache(k[i:i + 1].contiguous(), v[i:i + 1].contiguous(), roles[i:i + 1].contiguous(), C, SW) for i in (0, 7)]
+    splits = -(-(SW + (N + len(toks)) // C * C + C) // 1024)     # of the longest sequence, at the last steps
+    mid = -(-(112 if D == 64 else 38) // (Hkv * splits))
+    batches = [slice(0, B), slice(0, mid), slice(0, 1), slice(mid - 1, mid)]
+    caches = [make_cache(k[i].contiguous(), v[i].contiguous(), roles[i].contiguous(), C, SW) for i in batches]
     chunk_roles = torch.arange(B * Hkv, device=dev()).remainder(3).to(torch.uint8).view(B, Hkv, 1)
-    for q, kn, vn in toks:
-        full = every.chunk_fill_size + 1 == C
-        every.update(kn, vn, chunk_roles if full else None, fused=True)
-        o = every.decode_attention(q)
-        every.post_update(1)
+    ran = set()
+    for step, (q, kn, vn) in enumerate(toks):
+        (o, r0), (om, r1), (oa, r2), (ob, r3) = [attend(c, q, i, kn, vn, chunk_roles) for c, i in zip(caches, batches)]
+        ran.update((('large', r0), ('middle', r1)))
+        assert r2.startswith('strands') and r3.startswith('strands')
         assert torch.isfinite(o).all()
-        for i, c in zip((0, 7), single):
-            s = slice(i, i + 1)
-            c.update(kn[s].contiguous(), vn[s].contiguous(), chunk_roles[s].contiguous() if full else None, fused=True)
-            oi = c.decode_attention(q[s].contiguous())
-            c.post_update(1)
-            assert torch.equal(oi, o[s])
+        assert torch.equal(om, o[:mid]) and torch.equal(oa, o[:1]) and torch.equal(ob, o[mid - 1:mid])
+        if step == 0:                                            # the first sequence sees everything it has kept, which is everything
+            keys, vals = (torch.cat([x[:1], y[:1]], 2).float() for x, y in ((k, kn), (v, vn)))
+            s = torch.einsum('hrd,hnd->hrn', q[0].float().view(Hkv, Hq // Hkv, D), keys[0]) * D ** -0.5
+            assert_close_attn(o[:1], torch.einsum('hrn,hnd->hrd', s.softmax(-1), vals[0]).reshape(1, Hq, 1, D))
+    assert ran >= {('large', 'segments'), ('middle', 'strands, V in place of K')} and ('middle', 'segments') not in ran
 
 
-@pytest.mark.parametrize('B,C,SW,N,D', [(1, 1, 32, 700, 64), (2, 16, 64, 1010, 128), (12, 4, 64, 900, 128), (12, 1, 16, 300, 64), (1, 128, 256, 1100, 128)])
-def test_one_launch_per_step_equals_the_two_it_replaces(B, C, SW, N, D):
-    """Outputs, cache bytes, flags, sizes and step counters over steps that complete chunks of every role."""
+@pytest.mark.parametrize('N,D,nrep,B', [(15500, 64, 2, 7), (15500, 128, 1, 7), (23900, 128, 2, 5), (47500, 64, 8, 3), (64000, 128, 4, 2), (97000, 128, 8, 2)])
+def test_heads_of_many_segments(N, D, nrep, B):
+    """The longest heads that run as strands: one head alone, and in a batch that runs in blocks of a segment."""
+    C, SW = 128, 512
+    k, v, roles, toks = data(B, nrep, 1, N, D, C, seed=N)
+    both = [make_cache(k[:b].contiguous(), v[:b].contiguous(), roles[:b].contiguous(), C, SW) for b in (B, 1)]
+    for q, kn, vn in toks:
+        (o, r0), (oa, r1) = [attend(c, q, slice(0, b), kn, vn, roles[:, :, :1]) for c, b in zip(both, (B, 1))]
+        assert r0 == 'segments' and r1.startswith('strands')
+        assert torch.isfinite(o).all() and torch.equal(oa, o[:1])
+
+
+STEP_SHAPES = [(1, 1, 32, 700, 64, 'strands'), (2, 16, 64, 1010, 128, 'strands'), (12, 4, 64, 900, 128, 'segments'), (9, 1, 16, 300, 64, 'strands'),
+               (1, 128, 256, 1100, 128, 'strands'), (12, 1, 16, 300, 64, 'segments'), (26, 1, 32, 1500, 64, 'segments'), (26, 16, 64, 2100, 64, 'segments'),
+               (14, 4, 64, 2100, 128, 'segments')]
+
+
+@pytest.mark.parametrize('B,C,SW,N,D,kernel', STEP_SHAPES)
+def test_one_launch_per_step_equals_the_two_it_replaces(B, C, SW, N, D, kernel):
+    """Outputs, cache bytes, flags, sizes and step counters over steps that complete chunks of every role; the shapes for blocks of a
+    segment have heads of one, two and three segments in launches of room for more."""
     from neuralattentionsearch_b200 import functional as F_
     Hkv, Hq, steps = 8, 16, max(10, C + 3)
     k, v, roles, _ = data(B, Hq, Hkv, N, D, C, seed=N)
@@ -66,6 +114,7 @@ def test_one_launch_per_step_equals_the_two_it_replaces(B, C, SW, N, D):
     g = torch.Generator().manual_seed(1)
     for c in (a, b):
         c.prepare_static_decode(steps, Hq, D)
+    assert kernel_of(a, Hq, D, bound=a._static_bound, fill=C - 1).startswith(kernel)
     for _ in range(steps):
         q, kn, vn = (torch.randn(B, h, 1, D, generator=g).mul_(0.5).to(dev()).bfloat16() for h in (Hq, Hkv, Hkv))
         r = torch.randint(0, 3, (B, Hkv), generator=g).to(torch.uint8).to(dev())
@@ -78,3 +127,40 @@ def test_one_launch_per_step_equals_the_two_it_replaces(B, C, SW, N, D):
         for x, y in ((oa, ob), (a._buf_k, b._buf_k), (a._buf_v, b._buf_v), (a._buf_valid, b._buf_valid), (a.size_global_kv, b.size_global_kv),
                      (a.size_local_kv, b.size_local_kv), (a._state, b._state)):
             assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize('B,C,SW,N,D', [(26, 2, 32, 1500, 64), (14, 4, 64, 2100, 128)])
+def test_large_recorded_steps_replay(B, C, SW, N, D):
+    """A step in blocks of a segment, recorded once and replayed: outputs, cache bytes and counters of the steps called one by one."""
+    Hkv, Hq, steps = 8, 16, 9
+    k, v, roles, _ = data(B, Hq, Hkv, N, D, C, seed=N + 1)
+    a, b = (make_cache(k, v, roles, C, SW) for _ in range(2))
+    g = torch.Generator().manual_seed(2)
+    ins = [tuple(torch.randn(B, h, 1, D, generator=g).mul_(0.5).to(dev()).bfloat16() for h in (Hq, Hkv, Hkv)) for _ in range(steps)]
+    rs = [torch.randint(0, 3, (B, Hkv), generator=g).to(torch.uint8).to(dev()) for _ in range(steps)]
+    for c in (a, b):
+        c.prepare_static_decode(steps, Hq, D)
+        assert kernel_of(c, Hq, D, bound=c._static_bound, fill=C - 1) == 'segments'
+    outs = [torch.empty_like(q) for q, _, _ in ins]
+    for (q, kn, vn), r, o in zip(ins, rs, outs):
+        a.decode_step_static(q, kn, vn, r, o)
+    held, hr, out = [t.clone() for t in ins[0]], rs[0].clone(), torch.empty_like(outs[0])
+    b.decode_step_static(*held, hr, out)                         # one step outside of the graph first
+    assert torch.equal(out, outs[0])
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        graph.capture_begin()
+        b.decode_step_static(*held, hr, out, recording=True)
+        graph.capture_end()
+    torch.cuda.current_stream().wait_stream(side)
+    for i in range(1, steps):
+        for t, x in zip(held, ins[i]):
+            t.copy_(x)
+        hr.copy_(rs[i])
+        graph.replay()
+        assert torch.equal(out, outs[i]), i
+    b.note_static_steps(steps - 1)
+    for x, y in ((a._buf_k, b._buf_k), (a._buf_v, b._buf_v), (a._buf_valid, b._buf_valid), (a.size_global_kv, b.size_global_kv),
+                 (a.size_local_kv, b.size_local_kv), (a._state, b._state)):
+        assert torch.equal(x, y)
