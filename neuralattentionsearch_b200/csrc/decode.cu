@@ -39,7 +39,7 @@ struct DecodeParams {
     const long long* size_local;
     const int32_t* state;          // [0] = T0
     int32_t* counters;             // [B*Hkv]   (workspace)
-    float* partials;               // [B*Hkv, max_splits, nrep, D+2] or [B*Hkv, max_splits, strands, nrep, D+4]   (workspace)
+    float* partials;               // [B*Hkv, max_splits, nrep, D+2] or [B*Hkv, splits of the launch, strands, nrep, D+4]   (workspace)
     int Hq, Hkv, nrep, Lcap, SW, fill, max_splits;
     int fill_from_state;           // 1: the number of tokens in the unfinished chunk is read from state[4] (static launches)
     float scale_log2;              // sm_scale * log2(e)
@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(kDecThreads) decode_strand_kernel(const Decode
     const int nsplit = (Ltot + kSeg - 1) / kSeg;
     if (!STEP && seg >= nsplit) return;
     extern __shared__ __align__(128) uint8_t dsm[];
-    float* parts = p.partials + (size_t)bh * p.max_splits * kDecWarps * nrep * PSTRIDE;
+    float* parts = p.partials + (size_t)bh * gridDim.x * nrep * PSTRIDE;      // gridDim.x: strands of the launch's splits
     if (seg < nsplit) {
     const int r0 = seg * kSeg, r1 = min(Ltot, r0 + kSeg);
 
@@ -693,10 +693,13 @@ static cudaError_t launch_decode(const DecodeParams& p, dim3 grid, cudaStream_t 
 
 static size_t decode_counter_bytes(int B, int Hkv) { return align_up((size_t)B * Hkv * sizeof(int32_t), 256); }
 static int decode_max_splits(int max_len) { return cdiv(max_len + 1, kSeg); }
-// floats of the partial results of a split of a (batch, kv-head): one per query head, or one per strand and query head where a
-// launch may be of that kind (a launch has at least one segment per (batch, kv-head))
-static size_t decode_split_floats(int B, int Hkv, int nrep, int D) {
-    return (long long)B * Hkv <= max_strand_segments(D) ? (size_t)kDecWarps * nrep * (D + 4) : (size_t)nrep * (D + 2);
+// floats of the partial results: one set per split of a (batch, kv-head) and query head, or, in launches of strands, four per segment
+// of the launch and query head (such a launch has at most max_strand_segments of them, and at least one per (batch, kv-head))
+static size_t decode_partial_floats(int B, int Hkv, int nrep, int D, int max_splits) {
+    const long long heads = (long long)B * Hkv, limit = max_strand_segments(D);
+    const size_t whole = (size_t)heads * max_splits * nrep * (D + 2);
+    const size_t strands = heads > limit ? 0 : (size_t)min(heads * max_splits, limit) * kDecWarps * nrep * (D + 4);
+    return whole > strands ? whole : strands;
 }
 
 }  // namespace nats
@@ -706,8 +709,7 @@ using namespace nats;
 extern "C" __attribute__((visibility("default"))) size_t nats_b200_decode_workspace_bytes(int B, int Hq, int Hkv, int D, int max_len) {
     if (B <= 0 || Hq <= 0 || Hkv <= 0 || D <= 0 || max_len < 0 || Hq % Hkv) return 0;
     const int nrep = Hq / Hkv;
-    return decode_counter_bytes(B, Hkv) +
-           (size_t)B * Hkv * decode_max_splits(max_len) * decode_split_floats(B, Hkv, nrep, D) * sizeof(float);
+    return decode_counter_bytes(B, Hkv) + decode_partial_floats(B, Hkv, nrep, D, decode_max_splits(max_len)) * sizeof(float);
 }
 
 static int decode_impl(const void* d_q, const void* d_k_new, const void* d_v_new, void* d_o,

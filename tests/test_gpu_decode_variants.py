@@ -98,6 +98,29 @@ def test_heads_of_many_segments(N, D, nrep, B):
         assert torch.isfinite(o).all() and torch.equal(oa, o[:1])
 
 
+@pytest.mark.parametrize('B,nrep,D,L', [(2, 8, 64, 10000), (1, 8, 128, 12000), (1, 1, 64, 900), (9, 4, 128, 900), (12, 8, 128, 900), (20, 2, 64, 5000)])
+def test_a_launch_stays_inside_its_workspace(B, nrep, D, L):
+    """A workspace of the size asked for, bytes behind it: the largest launches of strands and ones of whole segments."""
+    from neuralattentionsearch_b200 import functional as F_
+    H, C, SW = 8, 128, 512
+    g = torch.Generator(device=dev()).manual_seed(L)
+    k, v = (torch.randn(B, H, L + C, D, generator=g, device=dev()).bfloat16() for _ in range(2))
+    valid = torch.ones(B, H, L + C, dtype=torch.uint8, device=dev())
+    sg, sl = torch.full((B, H), L, dtype=torch.long, device=dev()), torch.zeros(B, H, dtype=torch.long, device=dev())
+    state = torch.zeros(8, dtype=torch.int32, device=dev())
+    state[0] = L
+    q, kn = (torch.randn(B, h, 1, D, generator=g, device=dev()).bfloat16() for h in (H * nrep, H))
+    need = F_.decode_workspace_bytes(B, H * nrep, H, D, L + C)
+    ws = torch.full((need + 65536,), 0x5a, dtype=torch.uint8, device=dev())
+    ws[:need] = 0
+    o = torch.empty_like(q)
+    F_.decode_fwd(q, kn, kn, o, k, v, valid, sg, sl, state, 3, L, C, SW, D ** -0.5, ws[:need])
+    assert (ws[need:] == 0x5a).all()
+    keys, vals = (torch.cat([x[:1, :, :L + 3], kn[:1]], 2)[0].float() for x in (k, v))
+    s = torch.einsum('hrd,hnd->hrn', q[0].float().view(H, nrep, D), keys) * D ** -0.5
+    assert_close_attn(o[:1], torch.einsum('hrn,hnd->hrd', s.softmax(-1), vals).reshape(1, H * nrep, 1, D))
+
+
 STEP_SHAPES = [(1, 1, 32, 700, 64, 'strands'), (2, 16, 64, 1010, 128, 'strands'), (12, 4, 64, 900, 128, 'segments'), (9, 1, 16, 300, 64, 'strands'),
                (1, 128, 256, 1100, 128, 'strands'), (12, 1, 16, 300, 64, 'segments'), (26, 1, 32, 1500, 64, 'segments'), (26, 16, 64, 2100, 64, 'segments'),
                (14, 4, 64, 2100, 128, 'segments')]

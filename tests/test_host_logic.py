@@ -154,3 +154,17 @@ def test_roles_of_a_single_token_are_kept_unless_nothing_reads_them():
         cache.post_update(1)
         cache.update(torch.randn(B, H, 1, D), torch.randn(B, H, 1, D), info, fused=fused)
         assert torch.equal(cache._roles, want)
+
+
+@pytest.mark.parametrize('B,H,nrep,D', [(12, 8, 4, 128), (12, 8, 8, 128), (1, 8, 4, 128), (20, 8, 8, 64), (1, 1, 1, 64), (64, 8, 4, 128)])
+def test_decode_workspace_holds_the_partial_results_and_no_more(B, H, nrep, D):
+    """One partial result per split of 1024 tokens and query head, or four per segment of the largest launch that runs as strands."""
+    from neuralattentionsearch_b200 import functional as F_
+    limit, last = {64: 160, 128: 96}[D], 0
+    for max_len in (127, 1023, 1024, 5000, 16384, 131072):
+        splits = max_len // 1024 + 1
+        strands = 0 if B * H > limit else 4 * (D + 4) * min(limit, B * H * splits)
+        need = F_.decode_workspace_bytes(B, H * nrep, H, D, max_len)
+        assert need == -(-B * H * 4 // 256) * 256 + 4 * nrep * max(B * H * splits * (D + 2), strands)
+        assert need >= last
+        last = need
