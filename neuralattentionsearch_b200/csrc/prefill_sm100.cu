@@ -342,7 +342,7 @@ __device__ unsigned long long g_trace[64];
 
 // ---- shared memory --------------------------------------------------------------------------------
 struct ItemHeader {
-    int valid;      // 0: no more work
+    int valid;      // 0: no more work; else 1 + the KV tile in front of which the keys are gathered
     int t;          // query tile
     int b, bh;      // batch index, b * Hkv + kv-head
     int head0;      // query head of slot 0
@@ -373,8 +373,8 @@ struct PrefillSmem {
     uint32_t tmem_base;
     int abort_flag;
     int pipe_lock;                             // held by the issuer whose batch of MMAs is being queued
-    int far_tail[2];                           // per item, chunks below 8 rows: row of the copy that holds the last far_keys % 8 listed ones
 };
+static_assert(sizeof(ItemHeader) == 32, "a ninth word, loaded by every warp per item, made the kernel 1 to 1.5 % slower");
 static_assert(sizeof(PrefillSmem<128>) <= 232448 && sizeof(PrefillSmem<256>) <= 232448, "shared memory of the widest kernels");
 
 constexpr int kListConsumers = 1 + 2 + 8;     // producer, two issuers, one lane of each of the eight softmax warps
@@ -582,10 +582,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 }
                 if (lane == 0) {
                     ItemHeader hd;
-                    hd.valid = 1; hd.t = t; hd.b = z; hd.bh = bh; hd.head0 = hkv * p.nrep + grp * Smem::kHeads;
+                    hd.valid = 1 + max(near_first, 0); hd.t = t; hd.b = z; hd.bh = bh; hd.head0 = hkv * p.nrep + grp * Smem::kHeads;
                     hd.nslots = min(Smem::kHeads, p.nrep - grp * Smem::kHeads); hd.n_kept = n_kept; hd.far_keys = far_keys;
                     sm.item[slot] = hd;
-                    if (FINE) sm.far_tail[slot] = p.far_cap + kTailRows * max(near_first, 0);
                 }
             } else if (lane == 0) {
                 sm.item[slot].valid = 0;
@@ -656,7 +655,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 if (boxes) {
                     const int key = j * kTile + ((lane & (n_boxes - 1)) << box_shift);
                     if (p.far_cap == 0) box_row = key < hd.far_keys ? far_list[key >> box_shift] * box_rows : p.Nkv;
-                    else box_row = key + box_rows <= hd.far_keys ? key : key < hd.far_keys ? sm.far_tail[slot] : p.far_rows;
+                    else box_row = key + box_rows <= hd.far_keys ? key : key < hd.far_keys ? p.far_cap + kTailRows * (hd.valid - 1) : p.far_rows;
                 }
 #pragma unroll 1
                 for (int kv = 0; kv < 2 && ok; ++kv, ++g) {
