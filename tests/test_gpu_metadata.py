@@ -74,16 +74,18 @@ def test_eviction_plan(N, C, SW):
 def test_output_in_token_order_holds_the_same_bits():
     from neuralattentionsearch_b200 import prefill_attention
     g = torch.Generator().manual_seed(0)
-    for B, Hq, Hkv, N, D in ((2, 6, 2, 700, 64), (1, 8, 4, 513, 128), (2, 2, 2, 200, 256), (1, 4, 2, 150, 32)):
+    for B, Hq, Hkv, N, D, C in ((2, 6, 2, 700, 64, 32), (1, 8, 4, 513, 128, 32), (2, 2, 2, 200, 256, 32), (1, 4, 2, 150, 32, 32), (1, 4, 2, 1700, 64, 16),
+                                (1, 4, 2, 1500, 128, 1)):        # the last two with gathered tiles
         q, k, v = (torch.randn(B, h, N, D, generator=g).mul_(0.5).to(dev()).bfloat16() for h in (Hq, Hkv, Hkv))
-        roles = torch.from_numpy(orc.make_roles(B, Hkv, -(-N // 32), 0.1, 0.3, seed=N)).to(dev())
-        a = prefill_attention(q, k, v, roles, 32, 128)
-        b = prefill_attention(q, k, v, roles, 32, 128, token_major=True)
+        roles = torch.from_numpy(orc.make_roles(B, Hkv, -(-N // C), 0.1, 0.3, seed=N)).to(dev())
+        a = prefill_attention(q, k, v, roles, C, 128)
+        b = prefill_attention(q, k, v, roles, C, 128, token_major=True)
         assert b.shape == a.shape and torch.equal(a, b)
         assert D == 32 or b.transpose(1, 2).is_contiguous()
 
 
-@pytest.mark.parametrize('B,Hq,Hkv,N,D,C,SW', [(1, 4, 4, 1000, 64, 16, 64), (2, 8, 2, 513, 128, 1, 32), (1, 2, 2, 300, 256, 64, 128), (1, 2, 1, 9, 64, 8, 8)])
+@pytest.mark.parametrize('B,Hq,Hkv,N,D,C,SW', [(1, 4, 4, 1000, 64, 16, 64), (2, 8, 2, 513, 128, 1, 32), (1, 2, 2, 300, 256, 64, 128), (1, 2, 1, 9, 64, 8, 8),
+                                               (1, 4, 2, 1700, 64, 16, 64), (1, 4, 2, 1500, 128, 1, 64)])
 def test_fp32_prompts_are_rounded_by_the_kernels(B, Hq, Hkv, N, D, C, SW):
     """q, k, v in fp32: the output before its rounding to bf16, the cache bytes of a prompt given in bf16; also for tensors the
     rounding kernels do not take (not contiguous)."""

@@ -166,7 +166,8 @@ def test_reference_named_entry_points():
     assert_close_attn(o3, orc.prefill_attention(q, k, v, roles1, 1, 16), 'nats_attention')
 
 
-@pytest.mark.parametrize('B,Hq,Hkv,N,D,C,SW', [(2, 4, 2, 1000, 64, 16, 64), (1, 8, 2, 2048, 128, 128, 512), (1, 2, 2, 333, 128, 1, 16)])
+@pytest.mark.parametrize('B,Hq,Hkv,N,D,C,SW', [(2, 4, 2, 1000, 64, 16, 64), (1, 8, 2, 2048, 128, 128, 512), (1, 2, 2, 333, 128, 1, 16),
+                                              (2, 4, 2, 2500, 64, 16, 64), (1, 2, 2, 2200, 128, 1, 64)])      # with gathered tiles
 def test_forward_statistics_for_the_backward(B, Hq, Hkv, N, D, C, SW):
     """o, M (log2-sum-exp per row) and the visible-key counts of the training forward's contract."""
     from neuralattentionsearch_b200 import check_status

@@ -53,6 +53,31 @@ def test_far_chunks_are_gathered(C, N, p_global, p_local, D):
     assert_close_attn(run_prefill(q, k, v, roles, C, SW), orc.prefill_attention(q, k, v, roles, C, SW))
 
 
+@pytest.mark.parametrize('C', [1, 4])
+def test_workspace_without_room_for_copied_rows(C):
+    """A C caller who asks for the workspace without the head_dim (no room for copies of rows) gets the tiles computed in place; one byte
+    less than the full size does the same."""
+    from neuralattentionsearch_b200 import _lib, check_status
+    from neuralattentionsearch_b200.functional import status_word
+    B, Hq, Hkv, N, D, SW = 1, 4, 2, 2000, 64, 64
+    roles = orc.make_roles(B, Hkv, -(-N // C), 0.1, 0.3, seed=C)
+    q, k, v = inputs(B, Hq, Hkv, N, D, seed=C, sigma=0.5)
+    ref = orc.prefill_attention(q, k, v, roles, C, SW)
+    qd, kd, vd, r = *(t.to(dev()).bfloat16() for t in (q, k, v)), torch.from_numpy(roles).to(dev())
+    lib, outs = _lib.lib(), []
+    small, full = lib.nats_b200_prefill_workspace_bytes(B, Hkv, N, C), lib.nats_b200_prefill_workspace_bytes_for(B, Hkv, N, D, C)
+    assert small < full
+    for nbytes in (small, full - 1, full):
+        ws, o = torch.full((nbytes + 4096,), 0x5a, dtype=torch.uint8, device=dev()), torch.empty_like(qd)
+        _lib.call('nats_b200_prefill_fwd', qd.data_ptr(), kd.data_ptr(), vd.data_ptr(), o.data_ptr(), r.data_ptr(), B, Hq, Hkv, N, D, C, SW, D ** -0.5,
+                  ws.data_ptr(), nbytes, None, status_word(dev()).data_ptr(), torch.cuda.current_stream().cuda_stream)
+        check_status(dev())
+        assert (ws[nbytes:] == 0x5a).all()
+        assert_close_attn(o, ref)
+        outs.append(o)
+    assert torch.equal(outs[0], outs[1]) and not torch.equal(outs[1], outs[2])
+
+
 @pytest.mark.parametrize('C', [1, 2, 4, 8, 16, 32, 64])
 @pytest.mark.parametrize('D', [64, 128, 256])
 def test_gathered_tiles_hold_no_key_of_the_future(C, D):

@@ -61,6 +61,29 @@ def test_static_scratch_prefill_equals_regular_prefill_twice():
         assert torch.equal(kept, kept_ref)
 
 
+@pytest.mark.parametrize('B,Hq,Hkv,N,C,fits', [(2, 8, 2, 1500, 8, True), (32, 8, 8, 4096, 8, False)])
+def test_static_scratch_with_and_without_room_for_the_lists(B, Hq, Hkv, N, C, fits):
+    """Prompts long enough for gathered tiles: the same bits where the lists fit into the scratch as well, the same values from sums
+    in another order where they do not."""
+    from neuralattentionsearch_b200 import _lib, check_status, prefill_attention
+    from neuralattentionsearch_b200.functional import status_word
+    from test_gpu_parity import assert_close_attn
+    dev, D, SW = torch.device('cuda', 0), 64, 128
+    size, with_lists = 1 << 20, _lib.lib().nats_b200_prefill_workspace_bytes(B, Hkv, N, C)
+    assert (with_lists <= size) == fits
+    g = torch.Generator(device=dev).manual_seed(0)
+    q, k, v = (torch.randn(B, h, N, D, generator=g, device=dev).mul_(0.5).bfloat16() for h in (Hq, Hkv, Hkv))
+    roles = _roles(B, Hkv, -(-N // C), 5).to(dev)
+    ref, o = prefill_attention(q, k, v, roles, C, SW), torch.full_like(q, float('nan'))
+    _lib.call('nats_b200_prefill_fwd_static', q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), roles.data_ptr(), B, Hq, Hkv, N, D, C, SW,
+              D ** -0.5, None, status_word(dev).data_ptr(), torch.cuda.current_stream(dev).cuda_stream)
+    check_status(dev)
+    if fits:
+        assert torch.equal(o, ref)
+    else:
+        assert_close_attn(o, ref)
+
+
 def test_static_scratch_rejects_shapes_beyond_its_size():
     from neuralattentionsearch_b200 import _lib
     dev = torch.device('cuda', 0)
