@@ -69,7 +69,7 @@ int nats_b200_role_prep(const uint8_t* d_roles, int B, int Hkv, int N, int C, in
  * divide 128 also the lists of the chunks that stay visible, without which the call works but visits more tiles). */
 size_t nats_b200_prefill_workspace_bytes(int B, int Hkv, int N, int C);
 /* The same with the head_dim: for chunks below 8 tokens it has room for copies of the K / V rows that stay visible (a quarter
- * of the sequence), without which the call works but visits more tiles.  Also for calls over a cache (N = rows of cache and
+ * of the sequence and 8 rows per 128), without which the call works but visits more tiles.  Also for calls over a cache (N = rows of cache and
  * new tokens, as nats_b200_prefill_past_workspace_bytes takes them). */
 size_t nats_b200_prefill_workspace_bytes_for(int B, int Hkv, int N, int D, int C);
 

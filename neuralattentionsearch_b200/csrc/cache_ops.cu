@@ -216,8 +216,9 @@ __global__ void __launch_bounds__(kPrepThreads) role_prep_past_kernel(const Past
 // are one short of a chunk boundary.  A row of chunk x sees the rows up to its own, less C for every chunk that has ended by
 // x.  A block takes span chunks of a kv-head: one pass over the limits counts the chunks that have ended in front of its first
 // chunk and, in a histogram, at each of its chunks; a scan turns it into the number per chunk, and the rows are written for
-// each query head of the group.  (A loop over the chunks in front of every row is quadratic in the length.)
-constexpr int kCountRows = 4096;                 // rows per block, about
+// each query head of the group.  A block reads all limits up to its last chunk, so that the reads still grow with the square of the
+// length, by span rows at a time (a loop over the chunks in front of every row reads one chunk per row and chunk).
+constexpr int kCountRows = 4096;                 // rows per block; 256 chunks (the histogram) where those are fewer
 
 __global__ void __launch_bounds__(kScanThreads)
 visible_count_kernel(const int32_t* __restrict__ lim, int Hq, int Hkv, int N, int C, int Nc, int span, int32_t* __restrict__ out) {

@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(kDecThreads) decode_strand_kernel(const Decode
     const int my_tiles = (n_tiles - strand + kDecWarps - 1) / kDecWarps;
 #pragma unroll 4
     for (int t = 0; t < my_tiles; ++t) {
-        if (s_vmask[t] == 0u) continue;              // nothing visible in this tile (nothing was copied either)
+        if (s_vmask[t] == 0u) continue;              // nothing visible in this tile (what was copied of it is not looked at)
         const float4 s = s_score[t * 32 + lane];
         const float m_new = fmaxf(m_run, s_tmax[t][hrow]);
         const float mu = (m_new == NEG_INF) ? 0.f : m_new;
