@@ -18,6 +18,88 @@
 
 namespace nats {
 
+// Visibility bits of 32 consecutive key columns for the query rows of a warp (lane r: the row at position q0 + r).  Lane i
+// passes column col = first column + i; bit i of lane r's result = column i is visible to row r.  A column is visible to the
+// rows at positions col .. lim[col / C], so a lane has its column's bits for all 32 rows from one coalesced load, and five
+// exchange steps transpose the 32 x 32 bit matrix.  That is ~60 instructions for any chunk size; a loop over the chunks of a
+// tile pays a dependent load and the mask words for each of them: prompt of 8192 tokens, 32 / 8 heads, one role per token
+// 6.63 -> 0.91 ms, forward of 8 x 4096 tokens with chunks of 16 0.57 -> 0.51 ms.  Where 32 columns always lie in one chunk
+// the compare of visible_bits_coarse is cheaper (32k tokens, chunks of 128: 3 % slower with the transposition).
+__device__ __forceinline__ uint32_t visible_bits(const int32_t* __restrict__ lim, int col, int q0, int Nkv, int C, int c_shift, int lane) {
+    const int l = col < Nkv ? lim[c_shift >= 0 ? col >> c_shift : col / C] : -1;
+    const int lo = max(col - q0, 0), hi = min(l - q0, 31);
+    uint32_t x = (hi < lo) ? 0u : (0xffffffffu >> (31 - hi)) & (0xffffffffu << lo);
+    uint32_t m = 0x0000ffffu;
+#pragma unroll
+    for (int j = 16; j > 0; j >>= 1) {
+        const uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
+        x = (lane & j) ? (x & ~m) | ((y >> j) & m) : (x & m) | ((y & m) << j);
+        m ^= m << (j >> 1);
+    }
+    return x;
+}
+
+// The same for one row at position q when the 32 columns from col0 on lie in one chunk.
+__device__ __forceinline__ uint32_t visible_bits_coarse(const int32_t* __restrict__ lim, int col0, int q, int Nkv, int c_shift) {
+    const int n = min(q + 1, Nkv) - col0;                    // columns in the past of the row
+    if (n <= 0 || q > lim[col0 >> c_shift]) return 0u;
+    return n >= 32 ? 0xffffffffu : (1u << n) - 1u;
+}
+
+// Walks the set bits of an item's kept-tile bitmap in ascending order.
+struct PairTileWalk {
+    const uint32_t* keep;
+    const uint32_t* part;
+    int w;
+    uint32_t cur, pcur;
+    __device__ __forceinline__ void init(const uint32_t* k, const uint32_t* p) {
+        keep = k; part = p; w = 0; cur = k[0]; pcur = p[0];
+    }
+    // next kept tile; the caller asks for no more tiles than the item has
+    __device__ __forceinline__ int next(bool& partial) {
+        while (cur == 0u) { ++w; cur = keep[w]; pcur = part[w]; }
+        const int b = __ffs(cur) - 1;
+        cur &= cur - 1u;
+        partial = (pcur >> b) & 1u;
+        return w * 32 + b;
+    }
+};
+
+// The two issuers queue their MMAs in whole batches (the P.V of a tile and the Q.K^T of the next): the tensor pipe runs
+// MMAs in the order they were queued, so batches that interleaved would finish together and keep the two heads in step --
+// both in their softmax, then both waiting for the tensor pipe.  With whole batches one head's scores are ready a batch
+// earlier than the other's, and from then on one head's softmax overlaps the other head's MMAs.
+#ifndef NATS_LOCK_SLEEP_NS
+#define NATS_LOCK_SLEEP_NS 0       // pause between attempts to take the lock (0: none; 40 ns and 100 ns were measured slower)
+#endif
+__device__ __forceinline__ bool pipe_acquire(int* lock, int lane, volatile int* abort_flag, int32_t* status) {
+    int got = 1;
+    if (lane == 0) {
+        if (atomicCAS(lock, 0, 1) != 0) {
+            const unsigned long long t0 = global_ns();
+            got = 0;
+#pragma unroll 1
+            for (uint32_t it = 0;; ++it) {
+                if (NATS_LOCK_SLEEP_NS > 0) __nanosleep(NATS_LOCK_SLEEP_NS);
+                if (atomicCAS(lock, 0, 1) == 0) { got = 1; break; }
+                if ((it & 63u) == 63u) {
+                    if (*abort_flag) break;
+                    if (global_ns() - t0 > kWaitLimitNs) {
+                        *abort_flag = 1;
+                        atomicCAS(status, 0, kErrPipeLock);
+                        break;
+                    }
+                }
+            }
+        }
+    }
+    return __shfl_sync(0xffffffffu, got, 0) != 0;
+}
+__device__ __forceinline__ void pipe_release(int* lock, int lane) {
+    __syncwarp();
+    if (lane == 0) atomicExch(lock, 0);
+}
+
 __device__ __forceinline__ uint32_t cluster_ctarank() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -247,7 +329,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             if (!ok) break;
             const ItemHeader hd = sm.item[slot];
             if (!hd.valid) break;
-            TileWalk walk;
+            PairTileWalk walk;
             walk.init(sm.keep[slot], sm.part[slot]);
             for (int j = 0; j < hd.n_kept && ok; ++j) {
                 bool partial;
@@ -406,7 +488,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             const int qpos = p.q_off + hd.t * kTile + row;
             const int32_t* lim = p.lim + (size_t)hd.bh * p.Nc;
             float m_ref = -INFINITY, l_sum = 0.f;
-            TileWalk walk;
+            PairTileWalk walk;
             walk.init(sm.keep[slot], sm.part[slot]);
             for (int j = 0; j < n; ++j, ++gt) {
                 bool partial;

@@ -1,15 +1,16 @@
 // Role-masked chunked flash-attention prefill for sm_100a: TMA-fed tcgen05.mma with TMEM accumulators.
 //
 // A work item = one 128-row query tile x one kv-head x up to two query heads of that kv-head's group.  The two heads
-// share every K/V tile that is loaded and keep the tensor pipe busy in turns: while the softmax warps of one head
-// work on its 128 x 128 score tile S = Q.K^T in TMEM, the tensor core runs the other head's O += P.V and next Q.K^T.
+// share every K/V tile that is loaded.  S = Q.K^T of a step (tile, head) is read into registers at once, P has TMEM columns of its
+// own: the tensor core computes the next scores and O += P.V of earlier steps while the softmax warps of both heads work.
 // The kernel is persistent: one CTA per SM takes items from a global counter (heaviest query tiles first).
 //
-//   warp 0      TMA producer: K and V of every kept KV tile, item after item, through one ring of tile-sized slots
+//   warp 0      TMA producer: K and V of every kept KV tile, item after item, through one ring of tile-sized slots, and what the
+//               softmax warps need to know about a tile (which one it is, which masks it needs, the row limits of its columns)
 //   warp 3      scheduler: fetches the next item, builds its kept-tile bitmap while the current item runs, loads its Q tiles
-//   warps 1,2   MMA issuers of head slot 0 / 1 (one elected lane each): S_h = Q_h.K^T (SS, N = 128), O_h += P_h.V (TS, P from TMEM)
+//   warp 1      MMA issuer (one lane) of S = Q_h.K^T (SS, N = 128), warp 2 of O_h += P_h.V (TS, P from TMEM)
 //   warps 4-7   softmax of head slot 0: one thread per query row, the 128-entry score row read with tcgen05.ld, online
-//   warps 8-11  softmax of head slot 1  softmax in registers, P written back over S as packed bf16
+//   warps 8-11  softmax of head slot 1  softmax in registers, P written to TMEM as packed bf16
 //
 // Chunks finer than a tile: far behind the queries only the global chunks are still visible, a few in every tile.  Those
 // are not computed in place but gathered: the keys of 128 / C listed chunks (FarLists) make a full tile.  Chunks of 8 rows and
@@ -23,8 +24,7 @@
 // per-tile max / min row limits (nats_b200_role_prep); tiles without a visible entry are never loaded.  Only tiles
 // whose min limit does not cover the whole query tile (and the diagonal) pay for per-element masking.
 //
-// TMEM (512 columns), head slot h: S_h [256 h, 256 h + 128), O_h [256 h + 128, 256 h + 128 + D); P_h (bf16) aliases
-// the first 64 columns of S_h.  Every mbarrier wait is bounded: on a time-out the CTA raises the caller's status
+// TMEM (512 columns): see PrefillTmem.  Every mbarrier wait is bounded: on a time-out the CTA raises the caller's status
 // word, drains and exits.
 #include <cuda.h>
 
@@ -57,7 +57,7 @@ constexpr float kRescaleThreshold = 8.0f;               // log2 units: O is resc
 #endif
 constexpr unsigned long long kWaitLimitNs = NATS_WAIT_LIMIT_NS;
 
-enum : int { kErrQ = 1, kErrKvFull, kErrKvEmpty, kErrSFull, kErrPFull, kErrOFull, kErrList, kErrOEmpty, kErrSmemAlign, kErrPipeLock };
+enum : int { kErrQ = 1, kErrKvFull, kErrKvEmpty, kErrSFull, kErrPFull, kErrOFull, kErrList, kErrOEmpty, kErrSmemAlign, kErrPipeLock, kErrSEmpty };
 
 struct PrefillParams {
     void* o;                          // [B,Hq,N,D], or with the heads inside the tokens [B,N,Hq,D]: strides in elements
@@ -243,34 +243,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
         : "memory");
 }
 
-// Visibility bits of 32 consecutive key columns for the query rows of a warp (lane r: the row at position q0 + r).  Lane i
-// passes column col = first column + i; bit i of lane r's result = column i is visible to row r.  A column is visible to the
-// rows at positions col .. lim[col / C], so a lane has its column's bits for all 32 rows from one coalesced load, and five
-// exchange steps transpose the 32 x 32 bit matrix.  That is ~60 instructions for any chunk size; a loop over the chunks of a
-// tile pays a dependent load and the mask words for each of them: prompt of 8192 tokens, 32 / 8 heads, one role per token
-// 6.63 -> 0.91 ms, forward of 8 x 4096 tokens with chunks of 16 0.57 -> 0.51 ms.  Where 32 columns always lie in one chunk
-// the compare of visible_bits_coarse is cheaper (32k tokens, chunks of 128: 3 % slower with the transposition).
-__device__ __forceinline__ uint32_t visible_bits(const int32_t* __restrict__ lim, int col, int q0, int Nkv, int C, int c_shift, int lane) {
-    const int l = col < Nkv ? lim[c_shift >= 0 ? col >> c_shift : col / C] : -1;
-    const int lo = max(col - q0, 0), hi = min(l - q0, 31);
-    uint32_t x = (hi < lo) ? 0u : (0xffffffffu >> (31 - hi)) & (0xffffffffu << lo);
-    uint32_t m = 0x0000ffffu;
-#pragma unroll
-    for (int j = 16; j > 0; j >>= 1) {
-        const uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
-        x = (lane & j) ? (x & ~m) | ((y >> j) & m) : (x & m) | ((y & m) << j);
-        m ^= m << (j >> 1);
-    }
-    return x;
-}
-
-// The same for one row at position q when the 32 columns from col0 on lie in one chunk.
-__device__ __forceinline__ uint32_t visible_bits_coarse(const int32_t* __restrict__ lim, int col0, int q, int Nkv, int c_shift) {
-    const int n = min(q + 1, Nkv) - col0;                    // columns in the past of the row
-    if (n <= 0 || q > lim[col0 >> c_shift]) return 0u;
-    return n >= 32 ? 0xffffffffu : (1u << n) - 1u;
-}
-
 // 32-byte store (one sector) to a 32-byte aligned global address
 __device__ __forceinline__ void st32(void* p, const uint32_t (&w)[8]) {
     asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
@@ -364,36 +336,49 @@ struct PrefillSmem {
     uint8_t q[kHeads][kTileBytes];             // one Q tile per head slot; D/64 boxes of 16 KB each
     uint8_t ring[kSlots][kTileBytes];          // K or V tile; D/64 boxes of 16 KB each
     uint32_t keep[2][kBitWords];               // bit kt: KV tile kt of the item has a visible entry (double buffered)
-    uint32_t part[2][kBitWords];               // bit kt: the tile needs element masking
+    // what the softmax warps need to know about a tile, from the producer: (tile << 2) | kLimits | kCausal (a gathered tile: tile -1),
+    // and with kLimits the row limit of each of its columns
+    static constexpr int kMetas = D == 128 ? 3 : 8;
+    alignas(16) int32_t limits[kMetas][kTile];
+    int32_t tile[kMetas];
     ItemHeader item[2];
     unsigned long long bar_q_full[2], bar_q_empty[2];          // per head slot: its Q tile has landed / its last Q.K^T of the item is done
     unsigned long long bar_full[kSlots], bar_empty[kSlots];
-    unsigned long long bar_s_full[2], bar_p_full[2][2], bar_o_full[2], bar_o_empty[2];
+    unsigned long long bar_s_full[2], bar_s_empty[2];          // per head slot / per score buffer
+    unsigned long long bar_p_full[2], bar_o_full[2], bar_o_empty[2];
     unsigned long long bar_list_full[2], bar_list_empty[2];
     uint32_t tmem_base;
     int abort_flag;
-    int pipe_lock;                             // held by the issuer whose batch of MMAs is being queued
 };
 static_assert(sizeof(ItemHeader) == 32, "a ninth word, loaded by every warp per item, made the kernel 1 to 1.5 % slower");
 static_assert(sizeof(PrefillSmem<128>) <= 232448 && sizeof(PrefillSmem<256>) <= 232448, "shared memory of the widest kernels");
 
+// TMEM columns: O of each head slot, one score buffer for all steps (what 512 columns hold at head_dim 128; at 256 there is one head)
+// or one per head slot, P (bf16) of each head slot
+template <int D>
+struct PrefillTmem {
+    static constexpr uint32_t kScoreBufs = D == 64 ? 2 : 1;
+    static constexpr uint32_t kHeads = D <= 128 ? 2 : 1;
+    static __device__ __forceinline__ uint32_t o(uint32_t h) { return h * D; }
+    static __device__ __forceinline__ uint32_t s(uint32_t b) { return kHeads * D + b * 128; }
+    static __device__ __forceinline__ uint32_t p(uint32_t h) { return kHeads * D + kScoreBufs * 128 + h * 64; }
+};
+
 constexpr int kListConsumers = 1 + 2 + 8;     // producer, two issuers, one lane of each of the eight softmax warps
+
+enum : int { kCausal = 1, kLimits = 2 };      // some column of the tile lies behind some row / a chunk's row limit cuts through the tile
 
 // Walks the set bits of an item's kept-tile bitmap in ascending order.
 struct TileWalk {
     const uint32_t* keep;
-    const uint32_t* part;
     int w;
-    uint32_t cur, pcur;
-    __device__ __forceinline__ void init(const uint32_t* k, const uint32_t* p) {
-        keep = k; part = p; w = 0; cur = k[0]; pcur = p[0];
-    }
+    uint32_t cur;
+    __device__ __forceinline__ void init(const uint32_t* k) { keep = k; w = 0; cur = k[0]; }
     // next kept tile; the caller asks for no more tiles than the item has
-    __device__ __forceinline__ int next(bool& partial) {
-        while (cur == 0u) { ++w; cur = keep[w]; pcur = part[w]; }
+    __device__ __forceinline__ int next() {
+        while (cur == 0u) cur = keep[++w];
         const int b = __ffs(cur) - 1;
         cur &= cur - 1u;
-        partial = (pcur >> b) & 1u;
         return w * 32 + b;
     }
 };
@@ -406,40 +391,28 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatil
     const bool ok = mbar_wait<RELAX>(bar, parity, abort_flag, status, code);
     return __all_sync(0xffffffffu, ok);
 }
-
-// The two issuers queue their MMAs in whole batches (the P.V of a tile and the Q.K^T of the next): the tensor pipe runs
-// MMAs in the order they were queued, so batches that interleaved would finish together and keep the two heads in step --
-// both in their softmax, then both waiting for the tensor pipe.  With whole batches one head's scores are ready a batch
-// earlier than the other's, and from then on one head's softmax overlaps the other head's MMAs.
-#ifndef NATS_LOCK_SLEEP_NS
-#define NATS_LOCK_SLEEP_NS 0       // pause between attempts to take the lock (0: none; 40 ns and 100 ns were measured slower)
-#endif
-__device__ __forceinline__ bool pipe_acquire(int* lock, int lane, volatile int* abort_flag, int32_t* status) {
-    int got = 1;
-    if (lane == 0) {
-        if (atomicCAS(lock, 0, 1) != 0) {
-            const unsigned long long t0 = global_ns();
-            got = 0;
+// The same for the softmax warps, whose code has to stay short: bounded by a number of looks (the time limit of an issuer's or the
+// producer's wait runs out first and sets the abort flag).
+__device__ __forceinline__ bool warp_wait_short(uint32_t bar, uint32_t parity, volatile int* abort_flag, int32_t* status, int code) {
+    if (__builtin_expect(__all_sync(0xffffffffu, mbar_try_wait(bar, parity)), 1)) return true;
 #pragma unroll 1
-            for (uint32_t it = 0;; ++it) {
-                if (NATS_LOCK_SLEEP_NS > 0) __nanosleep(NATS_LOCK_SLEEP_NS);
-                if (atomicCAS(lock, 0, 1) == 0) { got = 1; break; }
-                if ((it & 63u) == 63u) {
-                    if (*abort_flag) break;
-                    if (global_ns() - t0 > kWaitLimitNs) {
-                        *abort_flag = 1;
-                        atomicCAS(status, 0, kErrPipeLock);
-                        break;
-                    }
-                }
-            }
-        }
+    for (uint32_t it = 0; it < (1u << 26); ++it) {
+        if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+        if (__any_sync(0xffffffffu, *abort_flag)) return false;
     }
-    return __shfl_sync(0xffffffffu, got, 0) != 0;
+    *abort_flag = 1;
+    atomicCAS(status, 0, code);
+    return false;
 }
-__device__ __forceinline__ void pipe_release(int* lock, int lane) {
-    __syncwarp();
-    if (lane == 0) atomicExch(lock, 0);
+
+// Waits of the producer, the issuers and the scheduler: a look and a branch in their code, the loop is a function of its own.
+__device__ __noinline__ bool util_wait_loop(uint32_t bar, uint32_t parity, volatile int* abort_flag, int32_t* status, int code, bool relax) {
+    return __all_sync(0xffffffffu, relax ? mbar_wait<kRelaxNs>(bar, parity, abort_flag, status, code) : mbar_wait(bar, parity, abort_flag, status, code));
+}
+template <int RELAX = 0>
+__device__ __forceinline__ bool util_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int32_t* status, int code) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    return util_wait_loop(bar, parity, abort_flag, status, code, RELAX > 0);
 }
 
 // Persistent kernel: every CTA takes work items (query tile x kv-head x head pair) from a global counter until none is
@@ -448,15 +421,21 @@ __device__ __forceinline__ void pipe_release(int* lock, int lane) {
 // next item's K/V through the same ring without a bubble, Q of the next item is loaded as soon as the last Q.K^T of the
 // current one has completed, and a head's epilogue only delays that head's own chain.
 //
-// Per head and kept tile j the chain is  S = Q.K_j^T (8 or 4 MMAs of N = 128)  ->  softmax over the 128-entry row held in
-// registers  ->  P (bf16) over the first 64 columns of S, handed over once per tile (a hand-over per half of 64 keys costs
-// the softmax warps a second wait + fence + arrive and buys nothing, because a batch is queued whole: 1.16 against 1.13 ms)
-// ->  O += P.V_j  ->  S = Q.K_{j+1}^T.  The two heads
-// run this chain half a period apart, so that one head's softmax (MUFU and issue slots of the four SM sub-partitions)
-// overlaps the other head's MMAs on the tensor pipe.
+// Per step (kept tile j, head):  S = Q.K_j^T (D / 16 MMAs of N = 128)  ->  the 128-entry score row in registers, S free for the next
+// step's scores  ->  softmax  ->  P (bf16) in columns of its own, free since P.V_{j-1}  ->  O += P.V_j.  Q.K^T needs only free scores,
+// P.V only P: two issuers, each in step order, nothing else orders the MMAs.  (With P over S and a head's P.V_j and Q.K_{j+1}^T queued
+// as one batch a head's chain was softmax, then batch, ~4300 cycles a tile for 2048 of MMAs; now ~3000.)
 //
-// FINE: chunks that are not a multiple of 32 keys, or gathered tiles.  Without it the loops carry neither the transposed masks
-// nor the gathered tiles: 32k tokens with chunks of 128 take 1.7 % longer with both in the code.
+// What binds it is instruction fetch before the pipes (of the cycles between two issues of a scheduler its warps spend 1.5 to 2.3 in
+// stalls for instructions, MUFU busy 55 %, tensor pipe 55 %): the warps of both heads stream through a tile's straight-line code
+// at different places, next to the issuer of their scheduler.  So the code is kept short: the heads of an issuer in a rolled loop
+// and waits as a look and a branch (text of <128, false> 74.8 -> 57.7 KB), rows masked by one compare per column with limits that the
+// producer leaves in shared memory, the epilogue in pieces of 32 columns.  us per launch, P over S / the above without the short
+// code / all: 32k tokens 1258 / 1259 / 1075, 2 x 131k 23394 / 22086 / 19370, 8 x 15001 3804 / 3954 / 3257, 8192 tokens with one role
+// per token 179 / 179 / 144, 8 x 4096 with chunks of 16 237 / 262 / 195.
+//
+// FINE: chunks that are not a multiple of 32 keys, or gathered tiles.  Without it the loops carry neither the masks column by column
+// nor the gathered tiles.
 template <int D, bool FINE>
 __global__ void __launch_bounds__(kPrefillThreads, 1)
 prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -468,6 +447,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
     constexpr int NBOX = D / 64;                       // TMA boxes per tile
     constexpr int NS = Smem::kSlots;
+    using TM = PrefillTmem<D>;
+    constexpr uint32_t SB = TM::kScoreBufs;
     constexpr uint32_t TILE_BYTES = Smem::kTileBytes;  // one Q, K or V tile (128 rows)
     constexpr uint32_t IDESC_QK = instr_desc(kTile, false);
     constexpr uint32_t IDESC_PV = instr_desc(D, true);
@@ -482,7 +463,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             bad = 1;
         }
         sm.abort_flag = bad;
-        sm.pipe_lock = 0;
     }
     __syncthreads();
     if (sm.abort_flag) return;                         // an earlier CTA gave up: do not start (uniform for the CTA)
@@ -491,14 +471,14 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     if (tid == 0) {
         for (int s = 0; s < NS; ++s) {
             mbar_init(smem_u32(&sm.bar_full[s]), 1);
-            mbar_init(smem_u32(&sm.bar_empty[s]), 2);
+            mbar_init(smem_u32(&sm.bar_empty[s]), 1);
         }
         for (int h = 0; h < 2; ++h) {
             mbar_init(smem_u32(&sm.bar_q_full[h]), 1);
             mbar_init(smem_u32(&sm.bar_q_empty[h]), 1);              // one arrival per item that uses the head slot
             mbar_init(smem_u32(&sm.bar_s_full[h]), 1);
-            mbar_init(smem_u32(&sm.bar_p_full[h][0]), 4);          // one arrival per softmax warp
-            mbar_init(smem_u32(&sm.bar_p_full[h][1]), 4);
+            mbar_init(smem_u32(&sm.bar_s_empty[h]), 4);            // one arrival per softmax warp
+            mbar_init(smem_u32(&sm.bar_p_full[h]), 4);
             mbar_init(smem_u32(&sm.bar_o_full[h]), 1);
             mbar_init(smem_u32(&sm.bar_o_empty[h]), 4);
             mbar_init(smem_u32(&sm.bar_list_full[h]), 1);
@@ -530,7 +510,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         const uint64_t pol_q = l2_policy_evict_first();
         for (int ic = 0; ok; ++ic) {
             const int slot = ic & 1, use = ic >> 1;
-            if (use > 0) ok = warp_wait<kRelaxNs>(smem_u32(&sm.bar_list_empty[slot]), (use - 1) & 1, abort_flag, p.status, kErrList);
+            if (use > 0) ok = util_wait<kRelaxNs>(smem_u32(&sm.bar_list_empty[slot]), (use - 1) & 1, abort_flag, p.status, kErrList);
             if (!ok) break;
             int w = 0;
             if (lane == 0) w = atomicAdd(p.work_counter, 1);
@@ -547,7 +527,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 const int q_lo = p.q_off + t * kTile, q_hi = p.q_off + min(t * kTile + kTile, p.N) - 1;
                 const int kt_last = q_hi / kTile;
                 const int32_t* tmax = p.tile_max + (size_t)bh * p.Ntk;
-                const int32_t* tmin = p.tile_min + (size_t)bh * p.Ntk;
                 // The tiles in front of near_first hold no visible chunk but listed ones: only the dense ones among them, whose chunks
                 // are not gathered, stay in the bitmap.  near_first <= the tile of the first query row, so every listed key in
                 // front of it is in that row's past.
@@ -557,22 +536,15 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 for (int s0 = 0; s0 <= kt_last; s0 += 32) {        // tiles 0..kt_last with a visible entry
                     const int kt = s0 + lane;
                     const bool keep = kt <= kt_last && tmax[kt] >= q_lo;
-                    // element masking is needed where the causal edge or a chunk's row limit cuts through the tile
-                    const bool partial = keep && (kt * kTile + kTile - 1 > q_lo || tmin[kt] < q_hi);
                     unsigned m = __ballot_sync(0xffffffffu, keep);
-                    unsigned pm = __ballot_sync(0xffffffffu, partial);
                     if (near_first < 0) {
                         const int o = kt <= near_cap ? open[kt] : 0;
                         const unsigned om = __ballot_sync(0xffffffffu, kt <= near_cap && (kt == near_cap || (o >> 1) >= q_lo));
                         if (om != 0u) near_first = s0 + __ffs(om) - 1;
                         const unsigned in_place = __ballot_sync(0xffffffffu, o & 1) | (om != 0u ? 0xffffffffu << (near_first - s0) : 0u);
                         m &= in_place;
-                        pm &= in_place;
                     }
-                    if (lane == 0) {
-                        sm.keep[slot][s0 >> 5] = m;
-                        sm.part[slot][s0 >> 5] = pm;
-                    }
+                    if (lane == 0) sm.keep[slot][s0 >> 5] = m;
                     n_kept += __popc(m);
                 }
                 int far_keys = 0;
@@ -602,7 +574,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 // empty slot may run a whole item ahead of the other one, so that an arrival per item would complete the
                 // barrier twice before this warp looks at it, and the wait for the older phase would not end
                 if (h < hd.nslots) {
-                    if (q_loads[h] > 0) ok = warp_wait<kRelaxNs>(smem_u32(&sm.bar_q_empty[h]), (q_loads[h] - 1) & 1, abort_flag, p.status, kErrQ);
+                    if (q_loads[h] > 0) ok = util_wait<kRelaxNs>(smem_u32(&sm.bar_q_empty[h]), (q_loads[h] - 1) & 1, abort_flag, p.status, kErrQ);
                     if (!ok) break;
                     if (lane == 0) {
                         mbar_expect_tx(smem_u32(&sm.bar_q_full[h]), TILE_BYTES);
@@ -624,6 +596,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     } else if (warp == 0) {
         // =============================== TMA producer ===============================
         uint32_t g = 0;                                 // ring slots filled so far (all items): two per kept tile
+        int meta = 0;                                   // entry of the next tile
         const uint64_t pol_kv = l2_policy_evict_last();
 #ifdef NATS_TRACE
         unsigned long long tr_prod_wait = 0, tr_prod_n = 0;
@@ -632,18 +605,35 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         bool ok = true;
         for (int ic = 0; ok; ++ic) {
             const int slot = ic & 1;
-            ok = warp_wait(smem_u32(&sm.bar_list_full[slot]), (ic >> 1) & 1, abort_flag, p.status, kErrList);
+            ok = util_wait(smem_u32(&sm.bar_list_full[slot]), (ic >> 1) & 1, abort_flag, p.status, kErrList);
             if (!ok) break;
             const ItemHeader hd = sm.item[slot];
             if (!hd.valid) break;
             TileWalk walk;
-            walk.init(sm.keep[slot], sm.part[slot]);
+            walk.init(sm.keep[slot]);
             const int n_far = (hd.far_keys + kTile - 1) / kTile;
+            // Looked up a tile ahead, while the producer waits for a ring slot: which tile comes next, whether its rows need masks,
+            // and the row limits of its columns lane, 32 + lane, ...
+            const int q_lo = p.q_off + hd.t * kTile, q_hi = p.q_off + min(hd.t * kTile + kTile, p.N) - 1;
+            const int32_t* lim = p.lim + (size_t)hd.bh * p.Nc;
+            const int32_t* tmin = p.tile_min + (size_t)hd.bh * p.Ntk;
+            int next_tile = 0, next_min = 0;
+            int32_t next_lim[4];
+            auto look_up = [&](int j) {
+                if (FINE && j < n_far) return;
+                next_tile = walk.next();
+                next_min = tmin[next_tile];
+#pragma unroll
+                for (int w = 0; w < 4; ++w) {
+                    const int col = next_tile * kTile + 32 * w + lane;
+                    next_lim[w] = col < p.Nkv ? lim[!FINE || p.c_shift >= 0 ? col >> p.c_shift : col / p.C] : -1;
+                }
+            };
+            look_up(0);
             const int32_t* far_list = p.far_list + (size_t)hd.bh * p.Nc;       // read only while n_far > 0
             for (int j = 0; j < hd.n_kept && ok; ++j) {
-                bool partial;
                 const bool far = FINE && j < n_far;
-                const int row0 = far ? j * kTile : walk.next(partial) * kTile;
+                const int row0 = far ? j * kTile : next_tile * kTile;
                 // Rows of a gathered tile: a box of 128 rows of the copy of the listed rows, or boxes of box_rows rows, the i-th
                 // from lane i: a listed chunk where it lies, or (chunks below 8 rows, only for the part empty tile) eight rows
                 // of the copy or its tail.  What lies behind the last listed key of the item is read as zero, from rows
@@ -663,12 +653,24 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 #ifdef NATS_TRACE
                     const unsigned long long tp0 = clock64();
 #endif
-                    if (g >= (uint32_t)NS) ok = warp_wait<kRelaxProdNs>(smem_u32(&sm.bar_empty[s]), ((g / NS) & 1) ^ 1, abort_flag, p.status, kErrKvEmpty);
+                    if (g >= (uint32_t)NS) ok = util_wait<kRelaxProdNs>(smem_u32(&sm.bar_empty[s]), ((g / NS) & 1) ^ 1, abort_flag, p.status, kErrKvEmpty);
 #ifdef NATS_TRACE
                     tr_prod_wait += clock64() - tp0;
                     ++tr_prod_n;
 #endif
                     if (!ok) break;
+                    if (kv == 0) {
+                        // the ring slot of K is free: so is this entry (kMetas tiles ago: its scores have been masked)
+                        const int flags = far ? (far_left < kTile ? kCausal : 0)
+                                              : (row0 + kTile - 1 > q_lo ? kCausal : 0) | (next_min < q_hi ? kLimits : 0);
+                        if (flags & kLimits) {
+#pragma unroll
+                            for (int w = 0; w < 4; ++w) sm.limits[meta][32 * w + lane] = next_lim[w];
+                        }
+                        if (lane == 0) sm.tile[meta] = far ? -4 | flags : next_tile << 2 | flags;
+                        meta = meta + 1 == Smem::kMetas ? 0 : meta + 1;
+                        __syncwarp();
+                    }
 #ifdef NATS_TEST_WITHHOLD_FIRST_V
                     // test builds only: the V tile of a CTA's first kept tile is never loaded, so that a bounded wait runs out
                     const bool withhold = g == 1;
@@ -693,6 +695,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                         __syncwarp();
                     }
                 }
+                if (j + 1 < hd.n_kept) look_up(j + 1);
             }
             if (ok && lane == 0) mbar_arrive(smem_u32(&sm.bar_list_empty[slot]));
         }
@@ -705,160 +708,126 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 mbar_wait(smem_u32(&sm.bar_full[x % NS]), (x / NS) & 1, nullptr, p.status, kErrKvFull);
         }
     } else if (warp == 1 || warp == 2) {
-        // =============================== MMA issuers: warp 1 for head slot 0, warp 2 for head slot 1 ===============================
-        // Per head and kept tile j:  O_h += P_j.V_j, then S_h = Q_h.K_{j+1}^T,
-        // which overwrites P_j: the tensor pipe runs one thread's MMAs in issue order.  A ring slot is released when both
-        // issuers have committed the MMAs that read it; an issuer whose head slot is empty in an item (odd group size)
-        // only keeps the barrier counts going.
-        const int h = warp - 1;
-        constexpr uint32_t T16 = TILE_BYTES >> 4;
+        // =============================== MMA issuers: warp 1 for S = Q.K^T, warp 2 for O += P.V ===============================
+        // Each walks the steps (item, KV tile, head slot) in the same order and waits only for what its own MMAs read or
+        // overwrite, so that Q.K^T of later steps runs beside the softmax and the P.V of earlier ones.
         // descriptors as (low word, high word): the high word (stride byte offset 1024, version, 128-byte swizzle) is the
         // same for Q, K and V; the low word holds the start address >> 4 and the leading byte offset >> 4
-        const uint64_t q_desc = smem_desc(smem_u32(&sm.q[0][0]), 16, 1024) + (uint64_t)(h < Smem::kHeads ? h * T16 : 0);
-        const uint64_t k_desc0 = smem_desc(smem_u32(&sm.ring[0][0]), 16, 1024);
-        const uint64_t v_desc0 = smem_desc(smem_u32(&sm.ring[0][0]), kBoxBytes, 1024);
+        constexpr uint32_t T16 = TILE_BYTES >> 4;
+        const bool qk = warp == 1;
+        const uint64_t q_desc = smem_desc(smem_u32(&sm.q[0][0]), 16, 1024);
+        const uint64_t r_desc = smem_desc(smem_u32(&sm.ring[0][0]), qk ? 16 : kBoxBytes, 1024);
         const uint32_t desc_hi = (uint32_t)(q_desc >> 32);
-        const uint32_t q_lo = (uint32_t)q_desc, k_lo0 = (uint32_t)k_desc0, v_lo0 = (uint32_t)v_desc0;
-        const uint32_t tS = tmem + h * 256, tO = tmem + h * 256 + 128;
-        auto issue_qk = [&](int s) {
-            // S[128 x 128] = Q_h[128 x D] . K_j[128 x D]^T : D/16 MMAs of K = 16
-            const uint32_t kl = k_lo0 + (uint32_t)s * T16;
-            mma_ss_lo<0>(tS, q_lo, kl, desc_hi, IDESC_QK);
-#pragma unroll
-            for (int ks = 1; ks < D / 16; ++ks) {
-                const uint32_t off = ((ks / 4) * kBoxBytes + (ks % 4) * 32) >> 4;
-                mma_ss_lo<1>(tS, q_lo + off, kl + off, desc_hi, IDESC_QK);
-            }
-        };
-        auto issue_pv_half = [&](int s, int half, bool first) {
-            // O_h[128 x D] (+)= P_j[128 x 64 keys of this half] . V_j[64 x D] : 4 MMAs of K = 16; V is MN-major (D contiguous)
-            const uint32_t vl = v_lo0 + (uint32_t)s * T16 + (uint32_t)(half * 4 * (2048 >> 4));
-            const uint32_t aP = tS + half * 32;
-            if (first) mma_ts_lo<0>(tO, aP, vl, desc_hi, IDESC_PV);
-            else mma_ts_lo<1>(tO, aP, vl, desc_hi, IDESC_PV);
-#pragma unroll
-            for (int k4 = 1; k4 < 4; ++k4) mma_ts_lo<1>(tO, aP + k4 * 8, vl + (uint32_t)(k4 * (2048 >> 4)), desc_hi, IDESC_PV);
-        };
+        const uint32_t q_lo0 = (uint32_t)q_desc, r_lo0 = (uint32_t)r_desc;
+        uint32_t g = 0;               // ring slots of the items so far
+        uint32_t k = 0;               // steps so far (one score buffer)
+        // tiles and items of head slot 0 / 1 so far: slot 1 has been empty in `gap` tiles and `skip` items
+        uint32_t gt = 0, na = 0, gap = 0, skip = 0;
         TR_DECL(8);
-#ifdef NATS_TRACE
-        unsigned long long tr_lock = 0, tr_pv = 0;
-#endif
-        uint32_t g = 0;          // ring slots consumed so far (all items, both issuers count alike)
-        uint32_t gt = 0;         // tiles of this head (items in which its slot is used)
-        uint32_t na = 0;         // items in which this head's slot was used
         bool ok = true;
         for (int ic = 0; ok; ++ic) {
             const int slot = ic & 1;
-            ok = warp_wait(smem_u32(&sm.bar_list_full[slot]), (ic >> 1) & 1, abort_flag, p.status, kErrList);
+            ok = util_wait(smem_u32(&sm.bar_list_full[slot]), (ic >> 1) & 1, abort_flag, p.status, kErrList);
             if (!ok) break;
             const ItemHeader hd = sm.item[slot];
             if (!hd.valid) break;
-            const int n = hd.n_kept;
-            const bool active = h < hd.nslots;
-            if (active) ok = warp_wait(smem_u32(&sm.bar_q_full[h]), na & 1, abort_flag, p.status, kErrQ);
-            // ---- S of the first tile ----
-            if (ok) ok = warp_wait(smem_u32(&sm.bar_full[g % NS]), (g / NS) & 1, abort_flag, p.status, kErrKvFull);
-            if (ok && active) ok = pipe_acquire(&sm.pipe_lock, lane, abort_flag, p.status);
-            if (!ok) break;
-            tc_fence_after();
-            if (lane == 0) {
-                if (active) {
-                    issue_qk(g % NS);
-                    tc_commit(smem_u32(&sm.bar_s_full[h]));
-                } else {
-                    // an empty head slot only keeps the counts going; for a used one the head's softmax warps release the
-                    // ring slots and the Q tile when they see the scores (a commit costs the issuer ~50 cycles each)
-                    mbar_arrive(smem_u32(&sm.bar_empty[g % NS]));
-                }
-            }
-            if (active) pipe_release(&sm.pipe_lock, lane);
-            __syncwarp();
-            // ---- tiles ----
-            for (int j = 0; j < n && ok; ++j) {
-                const uint32_t gv = g + 2 * j + 1;             // ring index of V_j; K_{j+1} follows it
-                const int sv = gv % NS;
-                TR(0);
-                ok = warp_wait(smem_u32(&sm.bar_full[sv]), (gv / NS) & 1, abort_flag, p.status, kErrKvFull);
-                TR(1);
-                const bool more = j + 1 < n;
-                const uint32_t gk = gv + 1;
-                if (ok && active) {
-                    TR(2);
-                    // the first P.V of an item overwrites O_h: the previous item's epilogue must have read it
-                    if (ok && j == 0 && na > 0) ok = warp_wait(smem_u32(&sm.bar_o_empty[h]), (na - 1) & 1, abort_flag, p.status, kErrOEmpty);
-                    TR(3);
-                    if (ok) ok = warp_wait(smem_u32(&sm.bar_p_full[h][1]), (gt + j) & 1, abort_flag, p.status, kErrPFull);
-                    TR(4);
-                }
-                if (ok && more) ok = warp_wait(smem_u32(&sm.bar_full[gk % NS]), (gk / NS) & 1, abort_flag, p.status, kErrKvFull);
-                TR(5);
-                // everything the batch needs is there: queue it as a whole.  (The lock is never held across a wait for a
-                // ring slot: the slot may be one the other head still has to release, which it can only do by queueing its
-                // own batch.)
-                if (ok && active) ok = pipe_acquire(&sm.pipe_lock, lane, abort_flag, p.status);
-                if (!ok) break;
-#ifdef NATS_TRACE
-                { const unsigned long long t_ = clock64(); tr_lock += t_ - tr_t; tr_t = t_; }
-#endif
-                tc_fence_after();
-                if (lane == 0) {
-                    if (active) {
-                        issue_pv_half(sv, 0, j == 0);
-                        issue_pv_half(sv, 1, false);
-                        if (!more) tc_commit(smem_u32(&sm.bar_o_full[h]));
-                        tc_commit(smem_u32(&sm.bar_empty[sv]));        // V_j is free as soon as P.V has run: the ring is short
-                    } else {
-                        mbar_arrive(smem_u32(&sm.bar_empty[sv]));
-                    }
-#ifdef NATS_TRACE
-                    { const unsigned long long t_ = clock64(); tr_pv += t_ - tr_t; tr_t = t_; }
-#endif
-                }
-                if (lane == 0) {
-                    if (more) {
-                        if (active) {
-                            issue_qk(gk % NS);
+            const int n = hd.n_kept, nslots = hd.nslots;
+            if (qk) {
+                for (int j = 0; j < n && ok; ++j) {
+                    const uint32_t gk = g + 2 * j;                 // ring index of K_j
+                    TR(0);
+                    ok = util_wait(smem_u32(&sm.bar_full[gk % NS]), (gk / NS) & 1, abort_flag, p.status, kErrKvFull);
+                    TR(1);
+                    const uint32_t kl = r_lo0 + (gk % NS) * T16;
+#pragma unroll 1
+                    for (int h = 0; h < nslots && ok; ++h) {
+                        const uint32_t items = na - (h ? skip : 0), tiles = gt + j - (h ? gap : 0);
+                        if (j == 0) ok = util_wait(smem_u32(&sm.bar_q_full[h]), items & 1, abort_flag, p.status, kErrQ);
+                        TR(2);
+                        // the scores this step overwrites are in the registers of their softmax warps
+                        const uint32_t sb = SB == 2 ? h : 0, use = SB == 2 ? tiles : k++;
+                        if (ok && use > 0) ok = util_wait(smem_u32(&sm.bar_s_empty[sb]), (use - 1) & 1, abort_flag, p.status, kErrSEmpty);
+                        if (!ok) break;
+                        TR(3);
+                        tc_fence_after();
+                        if (lane == 0) {
+                            // S[128 x 128] = Q_h[128 x D] . K_j[128 x D]^T : D/16 MMAs of K = 16
+                            const uint32_t tS = tmem + TM::s(sb), ql = q_lo0 + (uint32_t)h * T16;
+                            mma_ss_lo<0>(tS, ql, kl, desc_hi, IDESC_QK);
+#pragma unroll
+                            for (int ks = 1; ks < D / 16; ++ks) {
+                                const uint32_t off = ((ks / 4) * kBoxBytes + (ks % 4) * 32) >> 4;
+                                mma_ss_lo<1>(tS, ql + off, kl + off, desc_hi, IDESC_QK);
+                            }
                             tc_commit(smem_u32(&sm.bar_s_full[h]));
-                        } else {
-                            mbar_arrive(smem_u32(&sm.bar_empty[gk % NS]));
+                            if (h == nslots - 1) tc_commit(smem_u32(&sm.bar_empty[gk % NS]));
+                            if (j == n - 1) tc_commit(smem_u32(&sm.bar_q_empty[h]));
                         }
+                        __syncwarp();
+                        TR(4);
                     }
                 }
-                if (active) pipe_release(&sm.pipe_lock, lane);
-                __syncwarp();
-                TR(6);
-#ifdef NATS_TRACE
-                tr_acc[7] += 1;
-#endif
+            } else {
+                for (int j = 0; j < n && ok; ++j) {
+                    const uint32_t gv = g + 2 * j + 1;             // ring index of V_j
+                    TR(0);
+                    ok = util_wait(smem_u32(&sm.bar_full[gv % NS]), (gv / NS) & 1, abort_flag, p.status, kErrKvFull);
+                    TR(1);
+                    const uint32_t vl = r_lo0 + (gv % NS) * T16;
+#pragma unroll 1
+                    for (int h = 0; h < nslots && ok; ++h) {
+                        const uint32_t items = na - (h ? skip : 0), tiles = gt + j - (h ? gap : 0);
+                        // the first P.V of an item overwrites O_h: the previous item's epilogue must have read it
+                        if (j == 0 && items > 0) ok = util_wait(smem_u32(&sm.bar_o_empty[h]), (items - 1) & 1, abort_flag, p.status, kErrOEmpty);
+                        TR(2);
+                        if (ok) ok = util_wait(smem_u32(&sm.bar_p_full[h]), tiles & 1, abort_flag, p.status, kErrPFull);
+                        if (!ok) break;
+                        TR(3);
+                        tc_fence_after();
+                        if (lane == 0) {
+                            // O_h[128 x D] (+)= P_j[128 x 128 keys] . V_j[128 x D] : 8 MMAs of K = 16; V is MN-major (D contiguous)
+                            const uint32_t tO = tmem + TM::o(h), tP = tmem + TM::p(h);
+                            if (j == 0) mma_ts_lo<0>(tO, tP, vl, desc_hi, IDESC_PV);
+                            else mma_ts_lo<1>(tO, tP, vl, desc_hi, IDESC_PV);
+#pragma unroll
+                            for (int ks = 1; ks < 8; ++ks) mma_ts_lo<1>(tO, tP + ks * 8, vl + (uint32_t)(ks * (2048 >> 4)), desc_hi, IDESC_PV);
+                            tc_commit(smem_u32(&sm.bar_o_full[h]));
+                            if (h == nslots - 1) tc_commit(smem_u32(&sm.bar_empty[gv % NS]));
+                        }
+                        __syncwarp();
+                        TR(4);
+                    }
+                }
             }
             g += 2 * n;
-            if (active) { gt += n; ++na; }
+            gt += n;
+            ++na;
+            if (nslots == 1) { gap += n; ++skip; }
             if (ok && lane == 0) mbar_arrive(smem_u32(&sm.bar_list_empty[slot]));
         }
-#ifdef NATS_TRACE
-        if (h == 0) { TR_DUMP(16, 8); if (tr_on) { g_trace[24] = tr_lock; g_trace[25] = tr_pv; } }
-#endif
+        if (qk) { TR_DUMP(16, 8); } else { TR_DUMP(40, 8); }
     } else if (warp >= 4) {
         // =============================== softmax + epilogue ===============================
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsHigh));
         const int h = (warp - 4) / 4;                    // head slot
         const int row = (warp & 3) * 32 + lane;          // query row inside the tile == TMEM lane
         const uint32_t lane_addr = ((uint32_t)((warp & 3) * 32)) << 16;
-        const uint32_t tS = tmem + lane_addr + h * 256;
-        const uint32_t tO = tmem + lane_addr + h * 256 + 128;
+        const uint32_t sb = SB == 2 ? h : 0;             // score buffer
+        const uint32_t tS = tmem + lane_addr + TM::s(sb);
+        const uint32_t tP = tmem + lane_addr + TM::p(h);
+        const uint32_t tO = tmem + lane_addr + TM::o(h);
         const float scale = p.scale_log2;
         const bool o_wide = (reinterpret_cast<uintptr_t>(p.o) & 31u) == 0;     // 32-byte stores need a 32-byte aligned output
-        uint32_t gt = 0, na = 0;                         // tiles / items of this head so far
-        uint32_t g = 0;                                  // ring slots of all items so far (two per kept tile), as the issuers count
-        const bool releaser = (warp & 3) == 0 && lane == 0;   // one thread per head frees ring slots and the Q tile
+        uint32_t gt = 0;                                 // tiles of this head so far
+        int metas = 0;                                   // tiles of all items so far, modulo kMetas
         bool ok = true;
-        TR_DECL(10);
+        TR_DECL(12);
 #ifdef NATS_TRACE
         unsigned long long tr_epi_ld = 0;
 #endif
         for (int ic = 0; ok; ++ic) {
             const int slot = ic & 1;
-            ok = warp_wait(smem_u32(&sm.bar_list_full[slot]), (ic >> 1) & 1, abort_flag, p.status, kErrList);
+            ok = warp_wait_short(smem_u32(&sm.bar_list_full[slot]), (ic >> 1) & 1, abort_flag, p.status, kErrList);
             if (!ok) break;
             const ItemHeader hd = sm.item[slot];
             if (!hd.valid) break;
@@ -866,50 +835,53 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             if (h < hd.nslots) {
                 const int n = hd.n_kept;
                 const int qpos = p.q_off + hd.t * kTile + row;   // position of this thread's query row in the KV sequence
-                const int32_t* lim = p.lim + (size_t)hd.bh * p.Nc;
                 float m_ref = -INFINITY, l_sum = 0.f;
-                TileWalk walk;
-                walk.init(sm.keep[slot], sm.part[slot]);
+                int meta = metas;
                 for (int j = 0; j < n; ++j, ++gt) {
-                    bool partial;
-                    // visibility bits of this row for the 128 columns of a tile that is not fully visible
-                    uint32_t bits[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
-                    const int far_left = FINE ? hd.far_keys - j * kTile : 0;             // keys of the gathered tiles from this tile on
-                    if (far_left > 0) {
-                        // a gathered tile: all its keys are visible to every row; the last one may be part empty
-                        partial = far_left < kTile;
-                        if (partial) {
-#pragma unroll
-                            for (int w = 0; w < 4; ++w) bits[w] = far_left >= 32 * w + 32 ? 0xffffffffu : far_left <= 32 * w ? 0u : (1u << (far_left - 32 * w)) - 1u;
-                        }
-                    } else if (const int k0 = walk.next(partial) * kTile; partial) {    // k0: first key column of the tile
-#pragma unroll
-                        for (int w = 0; w < 4; ++w)
-                            bits[w] = !FINE || p.c_shift >= 5 ? visible_bits_coarse(lim, k0 + 32 * w, qpos, p.Nkv, p.c_shift)
-                                                     : visible_bits(lim, k0 + 32 * w + lane, qpos - lane, p.Nkv, p.C, p.c_shift, lane);
-                    }
-                    // S of tile j is complete; so is O += P.V of tile j - 1, which the same thread issued in front of it
                     TR(0);
-                    ok = warp_wait(smem_u32(&sm.bar_s_full[h]), gt & 1, abort_flag, p.status, kErrSFull);
+                    ok = warp_wait_short(smem_u32(&sm.bar_s_full[h]), gt & 1, abort_flag, p.status, kErrSFull);
                     if (!ok) break;
                     tc_fence_after();
-                    if (releaser) {
-                        // Q.K^T of tile j is complete: this head is done with K_j and, on the item's last tile, with its Q tile
-                        mbar_arrive(smem_u32(&sm.bar_empty[(g + 2 * j) % NS]));
-                        if (j == n - 1) mbar_arrive(smem_u32(&sm.bar_q_empty[h]));
-                    }
                     TR(1);
-                    // the score row of this thread in registers: four loads in flight, one wait
+                    // the score row of this thread in registers: four loads in flight, one wait; the buffer is then free
                     uint32_t sreg[kTile];
 #pragma unroll
                     for (int c = 0; c < 4; ++c) tmem_ld32(tS + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&sreg[c * 32]));
                     tc_wait_ld();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&sm.bar_s_empty[sb]));
                     TR(2);
-                    if (partial) {
+                    // masks: -inf, of which exp2 makes an exact 0
+                    const int tile = sm.tile[meta];
+                    if (tile & kLimits) {
+                        const int32_t* limits = sm.limits[meta];
+                        if (FINE) {
 #pragma unroll
-                        for (int i = 0; i < kTile; ++i)
-                            if (!((bits[i >> 5] >> (i & 31)) & 1u)) sreg[i] = 0xff800000u;      // -inf: exp2 gives exactly 0
+                            for (int i = 0; i < kTile; i += 4) {
+                                const int4 l = *reinterpret_cast<const int4*>(limits + i);
+                                if (qpos > l.x) sreg[i] = 0xff800000u;
+                                if (qpos > l.y) sreg[i + 1] = 0xff800000u;
+                                if (qpos > l.z) sreg[i + 2] = 0xff800000u;
+                                if (qpos > l.w) sreg[i + 3] = 0xff800000u;
+                            }
+                        } else {
+                            // 32 columns lie in one chunk
+#pragma unroll
+                            for (int w = 0; w < 4; ++w) {
+                                const bool hidden = qpos > limits[32 * w];
+#pragma unroll
+                                for (int i = 0; i < 32; ++i) sreg[32 * w + i] = hidden ? 0xff800000u : sreg[32 * w + i];
+                            }
+                        }
                     }
+                    if (tile & kCausal) {
+                        // the last column this row may see; the last gathered tile ends with the listed keys
+                        const int last = FINE && tile < 0 ? hd.far_keys - j * kTile - 1 : qpos - (tile >> 2) * kTile;
+#pragma unroll
+                        for (int i = 0; i < kTile; ++i) sreg[i] = i > last ? 0xff800000u : sreg[i];
+                    }
+                    meta = meta + 1 == Smem::kMetas ? 0 : meta + 1;
                     float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
 #pragma unroll
                     for (int i = 0; i < kTile; i += 8) {
@@ -931,7 +903,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                         m_ref = mx;
                     }
                     if (j > 0 && __any_sync(0xffffffffu, need)) {
-                        // O_h is rescaled in place (the P.V of the previous tile is complete, see above)
+                        // O_h is rescaled in place, behind the P.V of the previous tile
+                        ok = warp_wait_short(smem_u32(&sm.bar_o_full[h]), (gt - 1) & 1, abort_flag, p.status, kErrOFull);
+                        if (!ok) break;
+                        tc_fence_after();
 #pragma unroll 1
                         for (int c = 0; c < D / 32; ++c) {
                             uint32_t r[32];
@@ -944,37 +919,35 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                     }
                     const float m_neg = (m_ref == -INFINITY) ? 0.f : -m_ref;
                     TR(3);
-                    // P = exp2(S * scale - m), row sum in fp32, P packed to bf16 over the first 64 columns of S
+                    // P = exp2(S * scale - m), row sum in fp32, P packed to bf16
                     const uint64_t scale2 = pack2(scale, scale), mneg2 = pack2(m_neg, m_neg);
                     uint64_t ls2 = pack2(0.f, 0.f);
+                    // the P.V of this head's previous tile must have read what is overwritten below: asked now, it has long ended
+                    const bool pv_done = mbar_try_wait(smem_u32(&sm.bar_o_full[h]), (gt - 1) & 1);
+                    uint32_t pk[kTile / 2];
 #pragma unroll
-                    for (int half = 0; half < 2; ++half) {
-#pragma unroll
-                        for (int c = 0; c < 2; ++c) {
-                            uint32_t pk[16];
-                            const int base = half * 64 + c * 32;
-#pragma unroll
-                            for (int i = 0; i < 32; i += 2) {
-                                const uint64_t x2 = fma2(pack2(__uint_as_float(sreg[base + i]), __uint_as_float(sreg[base + i + 1])), scale2, mneg2);
-                                float x0, x1;
-                                unpack2(x2, x0, x1);
-                                const float p0 = ex2(x0), p1 = ex2(x1);
-                                ls2 = add2(ls2, pack2(p0, p1));
-                                pk[i / 2] = pack_bf16(p0, p1);
-                            }
-                            tmem_st16(tS + half * 32 + c * 16, pk);
-                        }
-                        // a batch is queued when all of P is there: one hand-over per tile (wait, fence, arrive), not one per half
-                        if (half == 1) {
-                            tc_wait_st();
-                            tc_fence_before();
-                            __syncwarp();                         // every lane's row of P is in TMEM and fenced
-                            if (lane == 0) mbar_arrive(smem_u32(&sm.bar_p_full[h][1]));
-                        }
-#ifdef NATS_TRACE
-                        if (half == 0) TR(4); else TR(5);
-#endif
+                    for (int i = 0; i < kTile; i += 2) {
+                        const uint64_t x2 = fma2(pack2(__uint_as_float(sreg[i]), __uint_as_float(sreg[i + 1])), scale2, mneg2);
+                        float x0, x1;
+                        unpack2(x2, x0, x1);
+                        const float p0 = ex2(x0), p1 = ex2(x1);
+                        ls2 = add2(ls2, pack2(p0, p1));
+                        pk[i / 2] = pack_bf16(p0, p1);
                     }
+                    TR(4);
+                    if (__builtin_expect(!__all_sync(0xffffffffu, pv_done), 0)) {
+                        ok = warp_wait_short(smem_u32(&sm.bar_o_full[h]), (gt - 1) & 1, abort_flag, p.status, kErrOFull);
+                        if (!ok) break;
+                    }
+                    tc_fence_after();
+                    TR(9);
+                    tmem_st32(tP, *reinterpret_cast<const uint32_t(*)[32]>(&pk[0]));
+                    tmem_st32(tP + 32, *reinterpret_cast<const uint32_t(*)[32]>(&pk[32]));
+                    tc_wait_st();
+                    tc_fence_before();
+                    __syncwarp();                         // every lane's row of P is in TMEM and fenced
+                    if (lane == 0) mbar_arrive(smem_u32(&sm.bar_p_full[h]));
+                    TR(10);
                     {
                         float a, b;
                         unpack2(ls2, a, b);
@@ -983,7 +956,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 }
                 // epilogue: O / l -> bf16 -> global; O_h is handed back to the issuer as soon as it sits in registers
                 TR(0);
-                if (ok) ok = warp_wait(smem_u32(&sm.bar_o_full[h]), na & 1, abort_flag, p.status, kErrOFull);
+                if (ok) ok = warp_wait_short(smem_u32(&sm.bar_o_full[h]), (gt - 1) & 1, abort_flag, p.status, kErrOFull);
                 TR(6);
                 if (ok) {
                     tc_fence_after();
@@ -991,7 +964,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                     const int qi = hd.t * kTile + row;           // query row
                     const long long o_at = hd.b * p.o_batch + (hd.head0 + h) * p.o_head + qi * p.o_row;
                     __nv_bfloat16* orow = (__nv_bfloat16*)p.o + o_at;
-                    constexpr int OW = D < 128 ? D : 128;          // columns of O held in registers at a time
+                    constexpr int OW = 32;                         // columns of O held in registers at a time
                     if (p.lse != nullptr && qi < p.N)
                         p.lse[((size_t)hd.b * p.Hq + hd.head0 + h) * p.N + qi] = l_sum > 0.f ? m_ref + log2f(l_sum) : -INFINITY;
 #pragma unroll 1
@@ -1042,18 +1015,17 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                         }
                     }
                 }
-                ++na;
                 TR(7);
 #ifdef NATS_TRACE
-                tr_acc[9] += n;
+                tr_acc[11] += n;
 #endif
             }
-            g += 2 * hd.n_kept;
+            metas = (metas + hd.n_kept) % Smem::kMetas;
             __syncwarp();
             if (ok && lane == 0) mbar_arrive(smem_u32(&sm.bar_list_empty[slot]));
         }
 #ifdef NATS_TRACE
-        if (warp == 4) { TR_DUMP(0, 10); if (tr_on) g_trace[10] = tr_epi_ld; }
+        if (warp == 4) TR_DUMP(0, 12);
 #endif
     }
     // ---- teardown ----
