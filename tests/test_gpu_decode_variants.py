@@ -187,3 +187,38 @@ def test_large_recorded_steps_replay(B, C, SW, N, D):
     for x, y in ((a._buf_k, b._buf_k), (a._buf_v, b._buf_v), (a._buf_valid, b._buf_valid), (a.size_global_kv, b.size_global_kv),
                  (a.size_local_kv, b.size_local_kv), (a._state, b._state)):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize('B,C,SW,N,D,kernel', [(1, 1, 32, 700, 64, 'strands'), (2, 4, 64, 1010, 128, 'strands'), (2, 64, 128, 1100, 128, 'strands'),
+                                               (12, 4, 64, 900, 128, 'segments'), (26, 1, 32, 1500, 64, 'segments')])
+def test_steps_recorded_back_to_back(B, C, SW, N, D, kernel):
+    """Steps whose launches overlap (nothing between them in the graph): outputs, cache bytes and counters of steps that are waited for
+    one by one, over steps that complete chunks and steps that do not."""
+    Hkv, Hq, steps = 8, 16, 11
+    k, v, roles, _ = data(B, Hq, Hkv, N, D, C, seed=N + 2)
+    a, b = (make_cache(k, v, roles, C, SW) for _ in range(2))
+    g = torch.Generator().manual_seed(3)
+    ins = [tuple(torch.randn(B, h, 1, D, generator=g).mul_(0.5).to(dev()).bfloat16() for h in (Hq, Hkv, Hkv)) for _ in range(steps)]
+    rs = [torch.randint(0, 3, (B, Hkv), generator=g).to(torch.uint8).to(dev()) for _ in range(steps)]
+    for c in (a, b):
+        c.prepare_static_decode(2 * steps, Hq, D)
+        assert kernel_of(c, Hq, D, bound=c._static_bound, fill=C - 1).startswith(kernel)
+    want, got = ([torch.empty_like(q) for q, _, _ in ins] for _ in range(2))
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    for again in range(2):
+        for (q, kn, vn), r, o in zip(ins, rs, want):
+            a.decode_step_static(q, kn, vn, r, o)
+            torch.cuda.synchronize()
+        if not again:
+            side.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(side):
+                graph.capture_begin()
+                for (q, kn, vn), r, o in zip(ins, rs, got):
+                    b.decode_step_static(q, kn, vn, r, o, recording=True)
+                graph.capture_end()
+            torch.cuda.current_stream().wait_stream(side)
+        graph.replay()
+        b.note_static_steps(steps)
+        for x, y in zip(want + [a._buf_k, a._buf_v, a._buf_valid, a.size_global_kv, a.size_local_kv, a._state],
+                        got + [b._buf_k, b._buf_v, b._buf_valid, b.size_global_kv, b.size_local_kv, b._state]):
+            assert torch.equal(x, y)
