@@ -432,7 +432,8 @@ __device__ __forceinline__ bool util_wait(uint32_t bar, uint32_t parity, volatil
 // and waits as a look and a branch (text of <128, false> 74.8 -> 57.7 KB), rows masked by one compare per column with limits that the
 // producer leaves in shared memory, the epilogue in pieces of 32 columns.  us per launch, P over S / the above without the short
 // code / all: 32k tokens 1258 / 1259 / 1075, 2 x 131k 23394 / 22086 / 19370, 8 x 15001 3804 / 3954 / 3257, 8192 tokens with one role
-// per token 179 / 179 / 144, 8 x 4096 with chunks of 16 237 / 262 / 195.
+// per token 179 / 179 / 144, 8 x 4096 with chunks of 16 237 / 262 / 195.  Then one compare per column for limits and diagonal together
+// where 32 columns lie in one chunk (1065 -> 1053, 19600 -> 19130, 3260 -> 3215), MMAs in a loop with FINE (144 -> 142, 195 -> 187).
 //
 // FINE: chunks that are not a multiple of 32 keys, or gathered tiles.  Without it the loops carry neither the masks column by column
 // nor the gathered tiles.
@@ -755,9 +756,12 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                             const uint32_t tS = tmem + TM::s(sb), ql = q_lo0 + (uint32_t)h * T16;
                             mma_ss_lo<0>(tS, ql, kl, desc_hi, IDESC_QK);
 #pragma unroll
-                            for (int ks = 1; ks < D / 16; ++ks) {
-                                const uint32_t off = ((ks / 4) * kBoxBytes + (ks % 4) * 32) >> 4;
-                                mma_ss_lo<1>(tS, ql + off, kl + off, desc_hi, IDESC_QK);
+                            for (int ks = 1; ks < 4; ++ks) mma_ss_lo<1>(tS, ql + 2 * ks, kl + 2 * ks, desc_hi, IDESC_QK);
+#pragma unroll(FINE ? 1 : 3)
+                            for (int x = 1; x < NBOX; ++x) {
+                                const uint32_t off = (uint32_t)x * (kBoxBytes >> 4);
+#pragma unroll
+                                for (int ks = 0; ks < 4; ++ks) mma_ss_lo<1>(tS, ql + off + 2 * ks, kl + off + 2 * ks, desc_hi, IDESC_QK);
                             }
                             tc_commit(smem_u32(&sm.bar_s_full[h]));
                             if (h == nslots - 1) tc_commit(smem_u32(&sm.bar_empty[gk % NS]));
@@ -787,10 +791,18 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                         if (lane == 0) {
                             // O_h[128 x D] (+)= P_j[128 x 128 keys] . V_j[128 x D] : 8 MMAs of K = 16; V is MN-major (D contiguous)
                             const uint32_t tO = tmem + TM::o(h), tP = tmem + TM::p(h);
-                            if (j == 0) mma_ts_lo<0>(tO, tP, vl, desc_hi, IDESC_PV);
-                            else mma_ts_lo<1>(tO, tP, vl, desc_hi, IDESC_PV);
+                            if (FINE) {
+                                // two at a time: 8 x 4096 tokens, head_dim 64, chunks of 16 195 -> 187 us; with the larger tiles in place
+                                // that are the rule without FINE all eight in a row are faster (32k tokens 1075 against 1107)
+#pragma unroll 2
+                                for (int ks = 0; ks < 8; ++ks)
+                                    mma_ts(tO, tP + ks * 8, ((uint64_t)desc_hi << 32) | (vl + (uint32_t)(ks * (2048 >> 4))), IDESC_PV, j > 0 || ks > 0);
+                            } else {
+                                if (j == 0) mma_ts_lo<0>(tO, tP, vl, desc_hi, IDESC_PV);
+                                else mma_ts_lo<1>(tO, tP, vl, desc_hi, IDESC_PV);
 #pragma unroll
-                            for (int ks = 1; ks < 8; ++ks) mma_ts_lo<1>(tO, tP + ks * 8, vl + (uint32_t)(ks * (2048 >> 4)), desc_hi, IDESC_PV);
+                                for (int ks = 1; ks < 8; ++ks) mma_ts_lo<1>(tO, tP + ks * 8, vl + (uint32_t)(ks * (2048 >> 4)), desc_hi, IDESC_PV);
+                            }
                             tc_commit(smem_u32(&sm.bar_o_full[h]));
                             if (h == nslots - 1) tc_commit(smem_u32(&sm.bar_empty[gv % NS]));
                         }
@@ -854,32 +866,27 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                     TR(2);
                     // masks: -inf, of which exp2 makes an exact 0
                     const int tile = sm.tile[meta];
-                    if (tile & kLimits) {
+                    if (FINE && (tile & kLimits)) {
                         const int32_t* limits = sm.limits[meta];
-                        if (FINE) {
 #pragma unroll
-                            for (int i = 0; i < kTile; i += 4) {
-                                const int4 l = *reinterpret_cast<const int4*>(limits + i);
-                                if (qpos > l.x) sreg[i] = 0xff800000u;
-                                if (qpos > l.y) sreg[i + 1] = 0xff800000u;
-                                if (qpos > l.z) sreg[i + 2] = 0xff800000u;
-                                if (qpos > l.w) sreg[i + 3] = 0xff800000u;
-                            }
-                        } else {
-                            // 32 columns lie in one chunk
-#pragma unroll
-                            for (int w = 0; w < 4; ++w) {
-                                const bool hidden = qpos > limits[32 * w];
-#pragma unroll
-                                for (int i = 0; i < 32; ++i) sreg[32 * w + i] = hidden ? 0xff800000u : sreg[32 * w + i];
-                            }
+                        for (int i = 0; i < kTile; i += 4) {
+                            const int4 l = *reinterpret_cast<const int4*>(limits + i);
+                            if (qpos > l.x) sreg[i] = 0xff800000u;
+                            if (qpos > l.y) sreg[i + 1] = 0xff800000u;
+                            if (qpos > l.z) sreg[i + 2] = 0xff800000u;
+                            if (qpos > l.w) sreg[i + 3] = 0xff800000u;
                         }
                     }
-                    if (tile & kCausal) {
+                    if (FINE ? tile & kCausal : tile & (kCausal | kLimits)) {
                         // the last column this row may see; the last gathered tile ends with the listed keys
                         const int last = FINE && tile < 0 ? hd.far_keys - j * kTile - 1 : qpos - (tile >> 2) * kTile;
 #pragma unroll
-                        for (int i = 0; i < kTile; ++i) sreg[i] = i > last ? 0xff800000u : sreg[i];
+                        for (int w = 0; w < 4; ++w) {
+                            // without FINE 32 columns lie in one chunk
+                            const int last_w = !FINE && (tile & kLimits) && qpos > sm.limits[meta][32 * w] ? -1 : last;
+#pragma unroll
+                            for (int i = 32 * w; i < 32 * w + 32; ++i) sreg[i] = i > last_w ? 0xff800000u : sreg[i];
+                        }
                     }
                     meta = meta + 1 == Smem::kMetas ? 0 : meta + 1;
                     float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
