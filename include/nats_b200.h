@@ -191,6 +191,12 @@ int nats_b200_evict_compact_f32(const float* d_k, const float* d_v, const uint8_
 int nats_b200_cache_append(const void* d_k_new, const void* d_v_new, void* d_cache_k, void* d_cache_v, uint8_t* d_valid,
                            int B, int Hkv, int x_len, int D, int Lcap, int pos, void* stream);
 
+/* The same into larger buffers (other memory than the old ones, capacity Lcap): rows [0, pos) and their flags come from the old ones
+ * (old_rows rows per head), everything behind the new tokens is zero and invalid. */
+int nats_b200_cache_grow_append(const void* d_old_k, const void* d_old_v, const uint8_t* d_old_valid, int old_rows,
+                                const void* d_k_new, const void* d_v_new, void* d_cache_k, void* d_cache_v, uint8_t* d_valid,
+                                int B, int Hkv, int x_len, int D, int Lcap, int pos, void* stream);
+
 /* Role metadata of such a call (what nats_b200_role_prep is to a first call), over the physical layout as KV sequence of
  * n_kv = t0 + fill + x_len rows; query row i sits at position t0 + fill + i.
  *   d_roles_new  uint8 [B,Hkv,ceil((fill+x_len)/C)]: roles of the chunks from the unfinished one on (what the reference

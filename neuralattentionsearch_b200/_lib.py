@@ -30,6 +30,7 @@ SIGNATURES = {
     'nats_b200_evict_compact': (_I, [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P, _P, _I, _P]),
     'nats_b200_evict_compact_f32': (_I, [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P, _P, _I, _P]),
     'nats_b200_cache_append': (_I, [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P]),
+    'nats_b200_cache_grow_append': (_I, [_P, _P, _P, _I, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P]),
     'nats_b200_role_prep_past': (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P]),
     'nats_b200_prefill_past_workspace_bytes': (_SZ, [_I, _I, _I, _I]),
     'nats_b200_prefill_past_fwd': (_I, [_P, _P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _F,

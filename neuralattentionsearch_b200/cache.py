@@ -107,18 +107,23 @@ class NAtSChunkLayerCache:
         tail = self.chunk_fill_size * self.bsz * self.n_msks
         return int(ring + main + tail) * self._buf_k.shape[-1] * 2 * 2
 
-    def _alloc(self, cap: int, D: int, dtype=torch.bfloat16):
+    def _buffers(self, cap: int, D: int):
         dev = self.device
-        self._buf_k = torch.empty(self.bsz, self.n_msks, cap, D, dtype=dtype, device=dev)
-        self._buf_v = torch.empty(self.bsz, self.n_msks, cap, D, dtype=dtype, device=dev)
-        self._buf_valid = torch.empty(self.bsz, self.n_msks, cap, dtype=torch.uint8, device=dev)
+        k, v = (torch.empty(self.bsz, self.n_msks, cap, D, dtype=torch.bfloat16, device=dev) for _ in range(2))
+        return k, v, torch.empty(self.bsz, self.n_msks, cap, dtype=torch.uint8, device=dev)
+
+    def _alloc(self, cap: int, D: int):
+        self._buf_k, self._buf_v, self._buf_valid = self._buffers(cap, D)
+
+    def _grown_capacity(self, need: int) -> int:
+        cap = self._buf_k.shape[2]
+        return math.ceil(max(need + self.headroom, cap + cap // 2) / self.chunk_size) * self.chunk_size
 
     def _grow(self, need: int):
         cap = self._buf_k.shape[2]
         if need <= cap:
             return
-        new_cap = max(need + self.headroom, cap + cap // 2)
-        new_cap = math.ceil(new_cap / self.chunk_size) * self.chunk_size
+        new_cap = self._grown_capacity(need)
         old_k, old_v, old_valid = self._buf_k, self._buf_v, self._buf_valid
         dev, D = self.device, old_k.shape[-1]
         self._buf_k = torch.zeros(self.bsz, self.n_msks, new_cap, D, dtype=old_k.dtype, device=dev)
@@ -159,8 +164,12 @@ class NAtSChunkLayerCache:
             # several tokens over an existing cache: they are appended behind the unfinished chunk, as the reference does
             # (:239-256); ``prefill_attention`` then attends over the buffer and ``post_update`` compacts it
             pos = self.n_ctx_data
-            self._grow(pos + x_len)
-            F_.cache_append(kb, vb, self._buf_k, self._buf_v, self._buf_valid, pos)
+            if pos + x_len > self._buf_k.shape[2]:
+                larger = self._buffers(self._grown_capacity(pos + x_len), self._buf_k.shape[-1])
+                F_.cache_grow_append(self._buf_k, self._buf_v, self._buf_valid, kb, vb, *larger, pos)
+                self._buf_k, self._buf_v, self._buf_valid = larger
+            else:
+                F_.cache_append(kb, vb, self._buf_k, self._buf_v, self._buf_valid, pos)
             self._pending = None
             self._plan_ahead_past()
             return self._buf_k[:, :, :pos + x_len], self._buf_v[:, :, :pos + x_len]

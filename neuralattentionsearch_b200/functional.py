@@ -476,6 +476,14 @@ def cache_append(k_new: torch.Tensor, v_new: torch.Tensor, cache_k: torch.Tensor
               cache_k.shape[2], pos, _stream(k_new.device))
 
 
+def cache_grow_append(old_k: torch.Tensor, old_v: torch.Tensor, old_valid: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor,
+                      cache_k: torch.Tensor, cache_v: torch.Tensor, valid: torch.Tensor, pos: int) -> None:
+    """``cache_append`` into larger, uninitialised buffers, which get the rows in front of ``pos`` from the old ones."""
+    B, H, x_len, D = k_new.shape
+    _call(k_new.device, 'nats_b200_cache_grow_append', _p(old_k), _p(old_v), _p(old_valid), old_k.shape[2], _p(k_new), _p(v_new),
+          _p(cache_k), _p(cache_v), _p(valid), B, H, x_len, D, cache_k.shape[2], pos, _stream(k_new.device))
+
+
 def prefill_attention_past(q: torch.Tensor, cache_k: torch.Tensor, cache_v: torch.Tensor, valid: torch.Tensor,
                            roles_new: torch.Tensor, size_global: torch.Tensor, size_local: torch.Tensor,
                            t0: int, fill: int, tail: int, chunk_size: int, sliding_window: int,

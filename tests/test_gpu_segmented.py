@@ -249,3 +249,25 @@ def test_attention_layer_segmented_forward_equals_one_call():
     a, b = cache.cache_model[0], one_cache.cache_model[0]
     assert torch.equal(a.size_global_kv, b.size_global_kv) and torch.equal(a.size_local_kv, b.size_local_kv)
     assert (a.n_ctx_data, a.chunk_fill_size, a.get_seq_length()) == (b.n_ctx_data, b.chunk_fill_size, N)
+
+
+@pytest.mark.parametrize('pos,x_len,old_rows,rows', [(0, 2, 64, 70), (37, 100, 64, 137), (64, 64, 64, 1000), (63, 2, 64, 65), (1500, 701, 1600, 2400)])
+@pytest.mark.parametrize('B,H,D', [(1, 1, 64), (2, 3, 128), (1, 2, 256)])
+def test_append_into_larger_buffers(pos, x_len, old_rows, rows, B, H, D):
+    """Old rows, new tokens and zeros of the larger buffers, whatever stood there; nothing behind them."""
+    from neuralattentionsearch_b200 import functional as F_
+    dev = torch.device('cuda', 0)
+    g = torch.Generator(device=dev).manual_seed(pos + D)
+    ok, ov = (torch.randn(B, H, old_rows, D, generator=g, device=dev).bfloat16() for _ in range(2))
+    kn, vn = (torch.randn(B, H, x_len, D, generator=g, device=dev).bfloat16() for _ in range(2))
+    oval = torch.randint(0, 2, (B, H, old_rows), generator=g, device=dev, dtype=torch.uint8)
+    n = B * H * rows
+    space = [torch.full((n * w + 4096,), 7, dtype=t, device=dev) for w, t in ((D, torch.bfloat16), (D, torch.bfloat16), (1, torch.uint8))]
+    k, v, valid = space[0][:n * D].view(B, H, rows, D), space[1][:n * D].view(B, H, rows, D), space[2][:n].view(B, H, rows)
+    F_.cache_grow_append(ok, ov, oval, kn, vn, k, v, valid, pos)
+    for got, old, new in ((k, ok, kn), (v, ov, vn), (valid[..., None], oval[..., None], torch.ones(B, H, x_len, 1, dtype=torch.uint8, device=dev))):
+        want = torch.zeros_like(got)
+        want[:, :, :pos], want[:, :, pos:pos + x_len] = old[:, :, :pos], new
+        assert torch.equal(got, want)
+    for t, w in zip(space, (D, D, 1)):
+        assert (t[n * w:] == 7).all()
