@@ -235,6 +235,12 @@ int nats_b200_evict_plan_past(const uint8_t* d_roles_new, int B, int Hkv, int n_
                               int32_t* d_rank, int32_t* d_base, int64_t* d_size_global, int64_t* d_size_local,
                               int32_t* d_state, void* stream);
 
+/* Either of the two plans (d_base == NULL: a first call) with the new d_state[0] and *d_status written to the two words of pinned host
+ * memory at h_report as well; they are there when the kernel has ended. */
+int nats_b200_evict_plan_report(const uint8_t* d_roles, int B, int Hkv, int n_tokens, int C, int SW, int32_t* d_rank, int32_t* d_base,
+                                int64_t* d_size_global, int64_t* d_size_local, int32_t* d_state, const int32_t* d_status,
+                                int32_t* h_report, void* stream);
+
 /* Step 3 -- data movement, out of place: old cache (with the appended tokens) -> new cache buffer.  Ring slots behind
  * tail_old receive the last min(#completed chunks, SW/C) chunks (move_sliding_window_tokens_to_head :391-437), the
  * others are copied; [SW, base*C) is copied; kept chunks go to [base*C, len); the new unfinished chunk to

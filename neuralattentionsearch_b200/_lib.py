@@ -36,6 +36,7 @@ SIGNATURES = {
     'nats_b200_prefill_past_fwd': (_I, [_P, _P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _F,
                                         _P, _SZ, _P, _P, _P]),
     'nats_b200_evict_plan_past': (_I, [_P, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P, _P]),
+    'nats_b200_evict_plan_report': (_I, [_P, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P]),
     'nats_b200_evict_compact_past': (_I, [_P, _P, _P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I,
                                           _P, _P, _P, _I, _P]),
     'nats_b200_rope_split_heads': (_I, [_P, _P, _P, _c.c_longlong, _c.c_longlong, _c.c_longlong, _P, _P, _c.c_longlong, _P, _P, _P,

@@ -356,8 +356,7 @@ class NAtSChunkLayerCache:
         base = torch.empty(self.bsz, self.n_msks, dtype=torch.int32, device=dev)
         sg, sl = self.size_global_kv.clone(), self.size_local_kv.clone()
         state = torch.zeros(8, dtype=torch.int32, device=dev)
-        F_.evict_plan_past(roles, n_tokens, C, SW, rank, base, sg, sl, state)
-        self._plan = (('past', n_tokens), rank, base, sg, sl, state, F_.read_word_async(state))
+        self._plan = (('past', n_tokens), rank, base, sg, sl, state, F_.evict_plan_report(roles, n_tokens, C, SW, rank, base, sg, sl, state))
 
     def _plan_ahead(self, N: int):
         """The keep-set of a first call depends on the roles only, so it is planned as soon as ``update`` knows them: the
@@ -375,8 +374,7 @@ class NAtSChunkLayerCache:
         sg = torch.empty(self.bsz, self.n_msks, dtype=torch.long, device=dev)
         sl = torch.empty_like(sg)
         state = torch.zeros(8, dtype=torch.int32, device=dev)
-        F_.evict_plan(roles, N, C, SW, rank, sg, sl, state)
-        self._plan = (N, rank, sg, sl, state, F_.read_word_async(state))
+        self._plan = (N, rank, sg, sl, state, F_.evict_plan_report(roles, N, C, SW, rank, None, sg, sl, state))
 
     def _evict_after_prefill(self, x_len: int):
         C, SW = self.chunk_size, self.sliding_window_size

@@ -260,9 +260,10 @@ visible_count_kernel(const int32_t* __restrict__ lim, int Hq, int Hkv, int N, in
 // =================================================================================================
 // evict_plan: keep flags -> destination ranks (ballot + prefix sum), sizes, max length
 // =================================================================================================
-__device__ __forceinline__ void publish_max_len(int32_t* state, int len, int nblocks) {
+__device__ __forceinline__ void publish_max_len(int32_t* state, int len, int nblocks, const int32_t* status = nullptr, int32_t* report = nullptr) {
     // state[1] accumulates the maximum over blocks; the last block to arrive publishes it in state[0]
     // and leaves the scratch words zero for the next call.  No block ever waits for another.
+    // report (host memory, may be null) gets the maximum and *status as well.
     __shared__ int last;
     if (threadIdx.x == 0) {
         atomicMax(&state[1], len);
@@ -274,6 +275,10 @@ __device__ __forceinline__ void publish_max_len(int32_t* state, int len, int nbl
             const int m = atomicExch(&state[1], 0);
             state[0] = m;
             state[2] = 0;
+            if (report != nullptr) {
+                report[0] = m;
+                report[1] = *reinterpret_cast<const volatile int32_t*>(status);
+            }
         }
     }
 }
@@ -284,7 +289,8 @@ __device__ __forceinline__ void publish_max_len(int32_t* state, int len, int nbl
 __global__ void __launch_bounds__(kPrepThreads)
 evict_plan_kernel(const uint8_t* __restrict__ roles, int Nc, int n_full, int C, int SW,
                   int32_t* __restrict__ rank, long long* __restrict__ size_global,
-                  long long* __restrict__ size_local, int32_t* __restrict__ state, int32_t* __restrict__ base) {
+                  long long* __restrict__ size_local, int32_t* __restrict__ state, int32_t* __restrict__ base,
+                  const int32_t* status, int32_t* report) {
     const int bh = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     roles += (size_t)bh * Nc;
     rank += (size_t)bh * Nc;
@@ -329,7 +335,7 @@ evict_plan_kernel(const uint8_t* __restrict__ roles, int Nc, int n_full, int C, 
         size_local[bh] = sl;
         if (base != nullptr) base[bh] = (int)((last_g >= 0 ? sg0 : sg0 + sl0) / C);
     }
-    publish_max_len(state, (int)(sg + sl), gridDim.x);
+    publish_max_len(state, (int)(sg + sl), gridDim.x, status, report);
 }
 
 // =================================================================================================
@@ -638,7 +644,7 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_evict_plan(const
     NATS_CHECK_ARG(d_roles && d_rank && d_size_global && d_size_local && d_state, "null pointer");
     const int Nc = cdiv(N, C);
     evict_plan_kernel<<<B * Hkv, kPrepThreads, 0, (cudaStream_t)stream>>>(
-        d_roles, Nc, N / C, C, SW, d_rank, (long long*)d_size_global, (long long*)d_size_local, d_state, nullptr);
+        d_roles, Nc, N / C, C, SW, d_rank, (long long*)d_size_global, (long long*)d_size_local, d_state, nullptr, nullptr, nullptr);
     NATS_CHECK_CUDA(cudaGetLastError());
     return NATS_OK;
 }
@@ -682,7 +688,21 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_evict_plan_past(
     NATS_CHECK_ARG(d_roles_new && d_rank && d_base && d_size_global && d_size_local && d_state, "null pointer");
     evict_plan_kernel<<<B * Hkv, kPrepThreads, 0, (cudaStream_t)stream>>>(
         d_roles_new, cdiv(n_tokens, C), n_tokens / C, C, SW, d_rank, (long long*)d_size_global, (long long*)d_size_local,
-        d_state, d_base);
+        d_state, d_base, nullptr, nullptr);
+    NATS_CHECK_CUDA(cudaGetLastError());
+    return NATS_OK;
+}
+
+extern "C" __attribute__((visibility("default"))) int nats_b200_evict_plan_report(
+    const uint8_t* d_roles, int B, int Hkv, int n_tokens, int C, int SW, int32_t* d_rank, int32_t* d_base,
+    int64_t* d_size_global, int64_t* d_size_local, int32_t* d_state, const int32_t* d_status, int32_t* h_report, void* stream) {
+    if (int rc = check_common(B, Hkv, n_tokens, C, SW)) return rc;
+    NATS_CHECK_ARG(d_roles && d_rank && d_size_global && d_size_local && d_state && d_status && h_report, "null pointer");
+    void* report = nullptr;
+    NATS_CHECK_CUDA(cudaHostGetDevicePointer(&report, h_report, 0));
+    evict_plan_kernel<<<B * Hkv, kPrepThreads, 0, (cudaStream_t)stream>>>(
+        d_roles, cdiv(n_tokens, C), n_tokens / C, C, SW, d_rank, (long long*)d_size_global, (long long*)d_size_local,
+        d_state, d_base, d_status, (int32_t*)report);
     NATS_CHECK_CUDA(cudaGetLastError());
     return NATS_OK;
 }

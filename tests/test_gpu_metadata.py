@@ -105,3 +105,37 @@ def test_fp32_prompts_are_rounded_by_the_kernels(B, Hq, Hkv, N, D, C, SW):
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0].bfloat16(), outs[2])
     for c in caches[:2]:
         assert torch.equal(c.cache_k, caches[2].cache_k) and torch.equal(c.cache_v, caches[2].cache_v) and torch.equal(c.valid_tokens, caches[2].valid_tokens)
+
+
+@pytest.mark.parametrize('B,H,N,C,SW', [(1, 1, 64, 64, 64), (2, 3, 700, 16, 64), (3, 5, 5001, 1, 32)])
+@pytest.mark.parametrize('past', [False, True])
+def test_planned_size_reaches_the_host(B, H, N, C, SW, past):
+    """The plan that reports the new extent to pinned host memory: sizes, ranks and state of the plain one, the same number on the host, for
+    several reports under way at once; a raised status word comes along."""
+    from neuralattentionsearch_b200 import _lib, functional as F_
+    dev = torch.device('cuda', 0)
+    g = torch.Generator(device=dev).manual_seed(N)
+    outs, reports = [], []
+    roles = [torch.randint(0, 3, (B, H, -(-N // C)), generator=g, device=dev).to(torch.uint8) for _ in range(3)]
+
+    def buffers():
+        sizes = [torch.full((B, H), x, dtype=torch.long, device=dev) for x in (SW + 3 * C, 2 * C)]
+        return [torch.empty(B, H, roles[0].shape[-1], dtype=torch.int32, device=dev), torch.empty(B, H, dtype=torch.int32, device=dev) if past else None,
+                *sizes, torch.zeros(8, dtype=torch.int32, device=dev)]
+
+    for r in roles:
+        outs.append(buffers())
+        reports.append(F_.evict_plan_report(r, N, C, SW, *outs[-1]))
+    for r, out, report in zip(roles, outs, reports):
+        want = buffers()
+        if past:
+            F_.evict_plan_past(r, N, C, SW, *want)
+        else:
+            F_.evict_plan(r, N, C, SW, want[0], *want[2:])
+        for x, y in zip(want, out):
+            assert x is None or torch.equal(x, y)
+        assert report() == int(want[-1][0]) == int((want[2] + want[3]).max())
+    F_.status_word(dev).fill_(5)
+    with pytest.raises(_lib.NatsB200Error, match='code 5'):
+        F_.evict_plan_report(roles[0], N, C, SW, *buffers())()
+    F_.check_status(dev)
