@@ -59,20 +59,25 @@ def build(force: bool = False, verbose: bool = False) -> str:
 
 
 WAIT_TEST_LIB = os.path.join(HERE, '..', 'tests', '_build', 'libnats_b200_waittest.so')
+WAIT_TEST_LIB_LAST_O = os.path.join(HERE, '..', 'tests', '_build', 'libnats_b200_waittest_last_o.so')
 
 
 def build_wait_test(force: bool = False) -> str:
-    """A TEST-ONLY build of the prefill entry points (never loaded by the package): every bounded wait gives up after 3 ms
-    instead of 400 ms and the K/V producer withholds one V tile per CTA, so that a test can watch a wait run out, the kernel
-    return with a status code and the context stay usable."""
-    lib = os.path.abspath(WAIT_TEST_LIB)
+    """Two TEST-ONLY builds of the prefill entry points (never loaded by the package): every bounded wait gives up after 3 ms
+    (about 6 ms in the softmax warps) instead of 400 ms, and the K/V producer withholds one V tile per CTA, or the issuer does not tell that
+    an item's last P.V has ended, so that a test can watch a wait run out, the kernel return with a status code and the context stay
+    usable.  Returns the path of the first one."""
     srcs = [os.path.join(CSRC, f) for f in ('prefill_sm100.cu', 'cache_ops.cu')]
-    if not force and os.path.exists(lib) and all(os.path.getmtime(x) <= os.path.getmtime(lib) for x in srcs + [__file__]):
-        return lib
-    os.makedirs(os.path.dirname(lib), exist_ok=True)
-    cmd = [_nvcc(), *NVCC_FLAGS, '-DNATS_WAIT_LIMIT_NS=3000000ull', '-DNATS_TEST_WITHHOLD_FIRST_V=1', '-shared', '-o', lib, *srcs]
-    subprocess.run(cmd, check=True)
-    return lib
+    procs = []
+    for lib, define in ((WAIT_TEST_LIB, 'NATS_TEST_WITHHOLD_FIRST_V'), (WAIT_TEST_LIB_LAST_O, 'NATS_TEST_WITHHOLD_LAST_O')):
+        lib = os.path.abspath(lib)
+        if not force and os.path.exists(lib) and all(os.path.getmtime(x) <= os.path.getmtime(lib) for x in srcs + [__file__]):
+            continue
+        os.makedirs(os.path.dirname(lib), exist_ok=True)
+        procs.append(subprocess.Popen([_nvcc(), *NVCC_FLAGS, '-DNATS_WAIT_LIMIT_NS=3000000ull', f'-D{define}=1', '-shared', '-o', lib, *srcs]))
+    if any([pr.wait() for pr in procs]):
+        raise RuntimeError('nvcc failed on the test-only library')
+    return os.path.abspath(WAIT_TEST_LIB)
 
 
 if __name__ == '__main__':

@@ -111,6 +111,11 @@ __device__ __forceinline__ unsigned long long global_ns() {
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
     return t;
 }
+__device__ __forceinline__ uint32_t sm_cycles() {         // wraps every 2.2 s at 1965 MHz
+    uint32_t t;
+    asm volatile("mov.u32 %0, %clock;" : "=r"(t));
+    return t;
+}
 // Bounded wait.  Returns false when the wait was given up (by this thread or, earlier, by another one of the CTA).
 // With abort_flag == nullptr only the time limit ends the wait (used to drain copies after the CTA has given up).
 // RELAX > 0: sleep that many nanoseconds between polls (roles that run ahead of the critical path and should not take
@@ -391,18 +396,31 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatil
     const bool ok = mbar_wait<RELAX>(bar, parity, abort_flag, status, code);
     return __all_sync(0xffffffffu, ok);
 }
-// The same for the softmax warps, whose code has to stay short: bounded by a number of looks (the time limit of an issuer's or the
-// producer's wait runs out first and sets the abort flag).
-__device__ __forceinline__ bool warp_wait_short(uint32_t bar, uint32_t parity, volatile int* abort_flag, int32_t* status, int code) {
-    if (__builtin_expect(__all_sync(0xffffffffu, mbar_try_wait(bar, parity)), 1)) return true;
-#pragma unroll 1
-    for (uint32_t it = 0; it < (1u << 26); ++it) {
-        if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-        if (__any_sync(0xffffffffu, *abort_flag)) return false;
+// The same for the softmax warps, whose code has to stay short: a loop around the look, the SM's cycle counter as the clock, and what
+// follows a time-out in a function of its own.  They wait about twice as long as the other warps (0.8 s at 1965 MHz): where a softmax
+// warp waits for an issuer that waits in turn, the status names the issuer's wait.  Behind the last item of a CTA nobody else is left to
+// give up: the epilogue's wait for the last P.V ends by this limit only.  A look in front of the loop saves the others reading the clock;
+// with FINE the shorter code is worth more: us per call, a limit on the number of looks (none in time) / this with / this without the look in
+// front, forward of 8 x 4096 tokens with chunks of 16 187.8 / 189.9 / 182.4, 32k tokens with chunks of 128 1053 / 1048 / 1061, 8 x 15001
+// 3211 / 3200 / 3240, 2 x 131k 19270 / 19260 / 19290.
+constexpr uint32_t kSoftmaxWaitCycles = (uint32_t)(4 * kWaitLimitNs);
+static_assert(4 * kWaitLimitNs < (1ull << 32), "the cycle counter is read with 32 bits");
+__device__ __noinline__ bool give_up(volatile int* abort_flag, int32_t* status, int code) {
+    if (*abort_flag == 0) {
+        *abort_flag = 1;
+        atomicCAS(status, 0, code);
     }
-    *abort_flag = 1;
-    atomicCAS(status, 0, code);
     return false;
+}
+template <bool FINE>
+__device__ __forceinline__ bool warp_wait_short(uint32_t bar, uint32_t parity, volatile int* abort_flag, int32_t* status, int code) {
+    if (!FINE && __builtin_expect(__all_sync(0xffffffffu, mbar_try_wait(bar, parity)), 1)) return true;
+    const uint32_t t0 = sm_cycles();
+#pragma unroll 1
+    do {
+        if (__builtin_expect(__all_sync(0xffffffffu, mbar_try_wait(bar, parity)), 1)) return true;
+    } while (__all_sync(0xffffffffu, sm_cycles() - t0 < kSoftmaxWaitCycles && *abort_flag == 0));
+    return give_up(abort_flag, status, code);
 }
 
 // Waits of the producer, the issuers and the scheduler: a look and a branch in their code, the loop is a function of its own.
@@ -803,6 +821,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 #pragma unroll
                                 for (int ks = 1; ks < 8; ++ks) mma_ts_lo<1>(tO, tP + ks * 8, vl + (uint32_t)(ks * (2048 >> 4)), desc_hi, IDESC_PV);
                             }
+#ifdef NATS_TEST_WITHHOLD_LAST_O
+                            // test builds only: the end of an item's last P.V is never told, so that the epilogue's wait runs out
+                            if (j < n - 1)
+#endif
                             tc_commit(smem_u32(&sm.bar_o_full[h]));
                             if (h == nslots - 1) tc_commit(smem_u32(&sm.bar_empty[gv % NS]));
                         }
@@ -839,7 +861,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 #endif
         for (int ic = 0; ok; ++ic) {
             const int slot = ic & 1;
-            ok = warp_wait_short(smem_u32(&sm.bar_list_full[slot]), (ic >> 1) & 1, abort_flag, p.status, kErrList);
+            ok = warp_wait_short<FINE>(smem_u32(&sm.bar_list_full[slot]), (ic >> 1) & 1, abort_flag, p.status, kErrList);
             if (!ok) break;
             const ItemHeader hd = sm.item[slot];
             if (!hd.valid) break;
@@ -851,7 +873,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 int meta = metas;
                 for (int j = 0; j < n; ++j, ++gt) {
                     TR(0);
-                    ok = warp_wait_short(smem_u32(&sm.bar_s_full[h]), gt & 1, abort_flag, p.status, kErrSFull);
+                    ok = warp_wait_short<FINE>(smem_u32(&sm.bar_s_full[h]), gt & 1, abort_flag, p.status, kErrSFull);
                     if (!ok) break;
                     tc_fence_after();
                     TR(1);
@@ -911,7 +933,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                     }
                     if (j > 0 && __any_sync(0xffffffffu, need)) {
                         // O_h is rescaled in place, behind the P.V of the previous tile
-                        ok = warp_wait_short(smem_u32(&sm.bar_o_full[h]), (gt - 1) & 1, abort_flag, p.status, kErrOFull);
+                        ok = warp_wait_short<FINE>(smem_u32(&sm.bar_o_full[h]), (gt - 1) & 1, abort_flag, p.status, kErrOFull);
                         if (!ok) break;
                         tc_fence_after();
 #pragma unroll 1
@@ -943,7 +965,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                     }
                     TR(4);
                     if (__builtin_expect(!__all_sync(0xffffffffu, pv_done), 0)) {
-                        ok = warp_wait_short(smem_u32(&sm.bar_o_full[h]), (gt - 1) & 1, abort_flag, p.status, kErrOFull);
+                        ok = warp_wait_short<FINE>(smem_u32(&sm.bar_o_full[h]), (gt - 1) & 1, abort_flag, p.status, kErrOFull);
                         if (!ok) break;
                     }
                     tc_fence_after();
@@ -963,7 +985,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 }
                 // epilogue: O / l -> bf16 -> global; O_h is handed back to the issuer as soon as it sits in registers
                 TR(0);
-                if (ok) ok = warp_wait_short(smem_u32(&sm.bar_o_full[h]), (gt - 1) & 1, abort_flag, p.status, kErrOFull);
+                if (ok) ok = warp_wait_short<FINE>(smem_u32(&sm.bar_o_full[h]), (gt - 1) & 1, abort_flag, p.status, kErrOFull);
                 TR(6);
                 if (ok) {
                     tc_fence_after();

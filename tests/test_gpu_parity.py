@@ -962,6 +962,44 @@ def test_a_wait_that_runs_out_returns_a_status_and_leaves_the_context_usable():
     assert_close_attn(good, orc.prefill_attention(q, k, v, roles_np, C, SW), 'after the timed-out launch')
 
 
+@pytest.mark.parametrize('D,C,N,Hq', [(64, 16, 100, 2), (128, 128, 128, 2), (128, 32, 77, 1), (256, 64, 128, 1)])
+def test_the_last_wait_of_a_block_runs_out_by_the_clock(D, C, N, Hq):
+    """A test-only build (a wait limit of about 6 ms in the softmax warps) whose issuer does not tell that an item's last P.V has ended.  The
+    launch has one item, behind which the other warps leave: only the epilogue's own limit can end its wait.  The status names that
+    wait (6), and the product library computes a correct prefill in the same context afterwards."""
+    import ctypes
+    import os
+    import time
+    from neuralattentionsearch_b200 import build as nbuild, check_status, prefill_attention
+    path = os.path.abspath(nbuild.WAIT_TEST_LIB_LAST_O)
+    if not os.path.exists(path):
+        pytest.skip('the test-only library has not been built (python -c "from neuralattentionsearch_b200 import build; build.build_wait_test()")')
+    h = ctypes.CDLL(path)
+    P, I = ctypes.c_void_p, ctypes.c_int
+    h.nats_b200_prefill_workspace_bytes.restype = ctypes.c_size_t
+    h.nats_b200_prefill_workspace_bytes.argtypes = [I, I, I, I]
+    h.nats_b200_prefill_fwd.restype = I
+    h.nats_b200_prefill_fwd.argtypes = [P] * 5 + [I] * 7 + [ctypes.c_float, P, ctypes.c_size_t, P, P, P]
+    B, Hkv, SW = 1, 1, 2 * C
+    roles_np = orc.make_roles(B, Hkv, -(-N // C), 0.1, 0.3, seed=3)
+    roles = torch.from_numpy(roles_np).to(dev())
+    q, k, v = inputs(B, Hq, Hkv, N, D, seed=8)
+    qd, kd, vd = (t.to(dev()).bfloat16() for t in (q, k, v))
+    o = torch.full_like(qd, 123.0)
+    ws = torch.empty(h.nats_b200_prefill_workspace_bytes(B, Hkv, N, C), dtype=torch.uint8, device=dev())
+    status = torch.zeros(1, dtype=torch.int32, device=dev())
+    torch.cuda.synchronize()
+    t0 = time.perf_counter()
+    assert h.nats_b200_prefill_fwd(qd.data_ptr(), kd.data_ptr(), vd.data_ptr(), o.data_ptr(), roles.data_ptr(), B, Hq, Hkv, N, D, C, SW,
+                                   D ** -0.5, ws.data_ptr(), ws.numel(), None, status.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert time.perf_counter() - t0 < 0.5
+    assert int(status.item()) == 6
+    good = prefill_attention(qd, kd, vd, roles, C, SW)
+    check_status(dev())
+    assert_close_attn(good, orc.prefill_attention(q, k, v, roles_np, C, SW), 'after the timed-out launch')
+
+
 PAIR_CHILD = r'''
 import sys, numpy as np, torch
 sys.path.insert(0, sys.argv[1])
