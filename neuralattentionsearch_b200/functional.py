@@ -117,22 +117,23 @@ class _PinnedWords:
             cls._free.setdefault(dev, []).append(word)
 
 
-class _PlannedSize:
-    """The size of the compacted cache, which a plan kernel writes to pinned host memory with the device's prefill status word beside
-    it.  Calling the object waits for that kernel and returns the size (and raises if a kernel in front of it had given up a bounded
-    wait); the pinned words go back to the pool when the value has been read or the object is dropped.  The kernel writes them
-    itself: two copies on a side stream, and the events that order them, took 40 us of the host's time per prompt."""
+_side_streams: dict = {}
 
-    def __init__(self, roles: torch.Tensor, n_tokens: int, chunk_size: int, sliding_window: int, rank: torch.Tensor, base: torch.Tensor | None,
-                 size_global: torch.Tensor, size_local: torch.Tensor, state: torch.Tensor):
-        self.dev, self.word = roles.device, None
-        B, H, _ = roles.shape
-        word = _PinnedWords.take(self.dev)
-        _call(self.dev, 'nats_b200_evict_plan_report', _p(roles), B, H, n_tokens, chunk_size, sliding_window, _p(rank), _p(base), _p(size_global),
-              _p(size_local), _p(state), _p(status_word(self.dev)), _p(word), _stream(self.dev))
-        self.done = torch.cuda.Event()
-        self.done.record(torch.cuda.current_stream(self.dev))
-        self.word = word
+
+def _side_stream(device: torch.device) -> torch.cuda.Stream:
+    """One extra stream per device for small read-backs that must not sit between two kernels of the caller's stream."""
+    st = _side_streams.get(device.index)
+    if st is None:
+        st = _side_streams[device.index] = torch.cuda.Stream(device)
+    return st
+
+
+class _PinnedValue:
+    """An int32 value on its way to a pinned word, with the device's prefill status word beside it; ``done`` is the event behind what
+    writes them.  Calling the object waits for it and returns the value (and raises if a kernel that ran before had given up a
+    bounded wait); the pinned words go back to the pool when the value has been read or the object is dropped."""
+
+    word = None
 
     def __call__(self) -> int:
         self.done.synchronize()
@@ -144,7 +145,7 @@ class _PlannedSize:
 
     def _release(self):
         if self.word is not None:
-            self.done.synchronize()          # the kernel must not write a word that somebody else already holds
+            self.done.synchronize()          # nothing must be written to a word that somebody else already holds
             _PinnedWords.give_back(self.dev, self.word)
             self.word = None
 
@@ -153,6 +154,49 @@ class _PlannedSize:
             self._release()
         except Exception:
             pass
+
+
+class _AsyncWord(_PinnedValue):
+    """An int32 scalar of the device on its way to the host."""
+
+    def __init__(self, src: torch.Tensor):
+        self.dev = src.device
+        word = _PinnedWords.take(self.dev)
+        # The two small copies run on a side stream behind what the current stream holds so far: on the current stream they
+        # would stand between the kernel that wrote ``src`` and the (long) kernel the caller launches next, ~10 us per step.
+        main = torch.cuda.current_stream(self.dev)
+        side = _side_stream(self.dev)
+        ready = torch.cuda.Event()
+        ready.record(main)
+        side.wait_event(ready)
+        with torch.cuda.stream(side):
+            word[:1].copy_(src[:1], non_blocking=True)
+            word[1:].copy_(status_word(self.dev), non_blocking=True)
+            self.done = torch.cuda.Event()
+            self.done.record(side)
+        src.record_stream(side)
+        self.word = word
+
+
+def read_word_async(src: torch.Tensor) -> _AsyncWord:
+    """Starts copying the int32 scalar ``src[0]`` to the host behind the current stream's work; call the result to get the value."""
+    return _AsyncWord(src)
+
+
+class _PlannedSize(_PinnedValue):
+    """The size of the compacted cache, which a plan kernel writes to pinned host memory itself: two copies on a side stream, and the
+    events that order them, took 40 us of the host's time per prompt."""
+
+    def __init__(self, roles: torch.Tensor, n_tokens: int, chunk_size: int, sliding_window: int, rank: torch.Tensor, base: torch.Tensor | None,
+                 size_global: torch.Tensor, size_local: torch.Tensor, state: torch.Tensor):
+        self.dev = roles.device
+        B, H, _ = roles.shape
+        word = _PinnedWords.take(self.dev)
+        _call(self.dev, 'nats_b200_evict_plan_report', _p(roles), B, H, n_tokens, chunk_size, sliding_window, _p(rank), _p(base), _p(size_global),
+              _p(size_local), _p(state), _p(status_word(self.dev)), _p(word), _stream(self.dev))
+        self.done = torch.cuda.Event()
+        self.done.record(torch.cuda.current_stream(self.dev))
+        self.word = word
 
 
 def evict_plan_report(roles: torch.Tensor, n_tokens: int, chunk_size: int, sliding_window: int, rank: torch.Tensor, base: torch.Tensor | None,

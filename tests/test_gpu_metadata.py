@@ -139,3 +139,26 @@ def test_planned_size_reaches_the_host(B, H, N, C, SW, past):
     with pytest.raises(_lib.NatsB200Error, match='code 5'):
         F_.evict_plan_report(roles[0], N, C, SW, *buffers())()
     F_.check_status(dev)
+
+
+def test_scalars_are_read_back_behind_the_callers_stream():
+    """``read_word_async``: the value that the caller's stream has written when the call is made, several at once and dropped unread ones among
+    them; a raised status word comes along."""
+    from neuralattentionsearch_b200 import _lib, functional as F_
+    dev = torch.device('cuda', 0)
+    x = torch.randn(2048, 2048, device=dev)
+    for stream in (torch.cuda.current_stream(), torch.cuda.Stream()):
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            words, reads = torch.zeros(6, 4, dtype=torch.int32, device=dev), []
+            for i, w in enumerate(words):
+                x = (x @ x).clamp_(-1, 1)                         # the copy has something to wait for
+                w.fill_(100 + i)
+                reads.append(F_.read_word_async(w))
+                words[i, 1:].fill_(-1)
+            del reads[2]
+            assert [r() for r in reads] == [100, 101, 103, 104, 105]
+    F_.status_word(dev).fill_(5)
+    with pytest.raises(_lib.NatsB200Error, match='code 5'):
+        F_.read_word_async(words[0])()
+    F_.check_status(dev)
