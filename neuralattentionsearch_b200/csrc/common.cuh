@@ -23,11 +23,15 @@ int fail(int code, const char* fmt, ...);
         if (!(cond)) return ::nats::fail(NATS_ERR_INVALID_ARG, __VA_ARGS__); \
     } while (0)
 
+// A call that has failed leaves its error behind in the runtime, too, where the check behind the next launch would find it and report a
+// launch that was right: the error is taken from there as well.
 #define NATS_CHECK_CUDA(expr)                                                                     \
     do {                                                                                          \
         cudaError_t e_ = (expr);                                                                  \
-        if (e_ != cudaSuccess)                                                                    \
+        if (e_ != cudaSuccess) {                                                                  \
+            (void)cudaGetLastError();                                                             \
             return ::nats::fail(NATS_ERR_CUDA, "%s failed: %s", #expr, cudaGetErrorString(e_));   \
+        }                                                                                         \
     } while (0)
 
 // Chunks that stay visible for good, per (batch, kv-head), without those of dense tiles (dense_min of them or more in a 128-row KV

@@ -1088,8 +1088,10 @@ static EncodeTiledFn get_encode_fn() {
     void* ptr = nullptr;
     cudaDriverEntryPointQueryResult qres;
     if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) != cudaSuccess ||
-        qres != cudaDriverEntryPointSuccess)
+        qres != cudaDriverEntryPointSuccess) {
+        (void)cudaGetLastError();
         return nullptr;
+    }
     fn = (EncodeTiledFn)ptr;
     return fn;
 }
@@ -1456,9 +1458,8 @@ static int static_scratch(void** out) {
     if (dev < 0 || dev >= kMaxDevices) return fail(NATS_ERR_UNSUPPORTED, "device index %d is outside [0, %d)", dev, kMaxDevices);
     if (g_prefill_scratch_addr[dev] == nullptr) {
         void* ptr = nullptr;
-        cudaError_t e = cudaGetSymbolAddress(&ptr, g_prefill_scratch);
-        if (e != cudaSuccess || ptr == nullptr)
-            return fail(NATS_ERR_CUDA, "cudaGetSymbolAddress(g_prefill_scratch) failed on device %d: %s", dev, cudaGetErrorString(e));
+        NATS_CHECK_CUDA(cudaGetSymbolAddress(&ptr, g_prefill_scratch));
+        if (ptr == nullptr) return fail(NATS_ERR_CUDA, "no address of g_prefill_scratch on device %d", dev);
         g_prefill_scratch_addr[dev] = ptr;
     }
     *out = g_prefill_scratch_addr[dev];

@@ -162,3 +162,31 @@ def test_scalars_are_read_back_behind_the_callers_stream():
     with pytest.raises(_lib.NatsB200Error, match='code 5'):
         F_.read_word_async(words[0])()
     F_.check_status(dev)
+
+
+def test_a_refused_cuda_call_does_not_fail_the_next_one():
+    """A report that is to go to memory the device cannot be given an address of is refused (by the runtime, before any launch), and the
+    same call with pinned memory right behind it succeeds."""
+    import numpy as np
+    from neuralattentionsearch_b200 import _lib, functional as F_
+    rt = pytest.importorskip('cuda.bindings.runtime')
+    dev = torch.device('cuda', 0)
+    B, H, N, C, SW = 1, 2, 300, 16, 64
+    roles = torch.zeros(B, H, -(-N // C), dtype=torch.uint8, device=dev)
+    rank = torch.empty(B, H, roles.shape[-1], dtype=torch.int32, device=dev)
+    sg, sl, state = torch.empty(B, H, dtype=torch.long, device=dev), torch.empty(B, H, dtype=torch.long, device=dev), torch.zeros(8, dtype=torch.int32, device=dev)
+    pageable, pinned = np.zeros(1 << 12, dtype=np.int32), torch.zeros(2, dtype=torch.int32, pin_memory=True)
+    err, _ = rt.cudaHostGetDevicePointer(pageable.ctypes.data, 0)
+    rt.cudaGetLastError()
+    if err == rt.cudaError_t.cudaSuccess:
+        pytest.skip('this system gives out device addresses of pageable memory')
+
+    def report(host):
+        _lib.call('nats_b200_evict_plan_report', roles.data_ptr(), B, H, N, C, SW, rank.data_ptr(), None, sg.data_ptr(), sl.data_ptr(), state.data_ptr(),
+                  F_.status_word(dev).data_ptr(), host, torch.cuda.current_stream().cuda_stream)
+    for _ in range(2):
+        with pytest.raises(_lib.NatsB200Error, match='cudaHostGetDevicePointer'):
+            report(pageable.ctypes.data)
+        report(pinned.data_ptr())
+        torch.cuda.synchronize()
+        assert int(pinned[0]) == int((sg + sl).max())
