@@ -343,7 +343,11 @@ struct PrefillSmem {
     uint32_t keep[2][kBitWords];               // bit kt: KV tile kt of the item has a visible entry (double buffered)
     // what the softmax warps need to know about a tile, from the producer: (tile << 2) | kLimits | kCausal (a gathered tile: tile -1),
     // and with kLimits the row limit of each of its columns
+    // A softmax warp reads an entry behind its arrival at bar_s_empty, so that a finished Q.K^T does not show that the entry has been read; a
+    // finished P.V does, since it needed the P of both heads.  When the producer writes the entry of tile T it has waited for the slots of
+    // K_T and of V_(T-1), one of which held V_(T - kSlots/2 - 1): entries of tiles up to that one are free.
     static constexpr int kMetas = D == 128 ? 3 : 8;
+    static_assert(kMetas >= kSlots / 2 + 1, "an entry could be overwritten before the softmax warps have read it");
     alignas(16) int32_t limits[kMetas][kTile];
     int32_t tile[kMetas];
     ItemHeader item[2];
@@ -679,7 +683,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 #endif
                     if (!ok) break;
                     if (kv == 0) {
-                        // the ring slot of K is free: so is this entry (kMetas tiles ago: its scores have been masked)
+                        // the ring slots of this K and of the V in front are free: so is the entry (see kMetas)
                         const int flags = far ? (far_left < kTile ? kCausal : 0)
                                               : (row0 + kTile - 1 > q_lo ? kCausal : 0) | (next_min < q_hi ? kLimits : 0);
                         if (flags & kLimits) {
