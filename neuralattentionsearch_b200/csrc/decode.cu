@@ -46,10 +46,9 @@ struct DecodeParams {
     PlaceParams place;             // STEP kernels only
 };
 
-// Decode kernels that follow one another in a stream overlap their launches (programmatic dependent launch): a kernel may be
-// scheduled once every block of the one in front has started, and looks at memory only behind this wait, that is when that
-// kernel has ended.  Bound by the latency of one step, not by bytes: 193 recorded steps of two sequences (32 / 8 heads of 128, 2200
-// rows per head) behind a prompt of 6000 tokens 3353 -> 3133 us together with the counters beside the ticket (last_arrival).
+// Decode kernels that follow one another in a stream may overlap (programmatic dependent launch; where they do: overlaps): a kernel is
+// then scheduled once every block of the one in front has started, and looks at memory only behind this wait, that is when that
+// kernel has ended.
 __device__ __forceinline__ void wait_for_previous_launch() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -57,7 +56,9 @@ __device__ __forceinline__ void wait_for_previous_launch() {
 
 // Ticket of a block that has left its results: true for the last of n blocks of the (batch, kv-head).
 // STEP, no chunk completed: every block of the launch has read the step counters by now, the last one to come here advances
-// them.  Another warp does that beside the ticket, so that no step waits for it.
+// them.  Another warp does that beside the ticket, so that no step waits for it: a recorded step of 16 heads of 128 (four query heads each,
+// 2400 rows) 13.0 -> 12.0 us against counters advanced behind the output; 512 heads of 4400 rows 174.4 -> 173.4.  (One arrival per
+// block or per head makes no difference: 64 sequences of 8 heads, 7000 rows, 208.7 us either way.)
 template <bool STEP>
 __device__ __forceinline__ bool last_arrival(const DecodeParams& p, int bh, int n, int fill) {
     __shared__ int s_last;
@@ -669,20 +670,39 @@ static bool use_strands(int D, long long segments, int splits, int nrep) {
 // faster at 64; at 128 2 % up to 3 splits, but 4 to 14 % slower at 4 and 16 to 32 % at 16 (8 to 32 segments).
 static bool use_both(int D, long long segments, int splits) { return D == 64 ? segments <= 111 : segments <= 37 && splits <= 3; }
 
-// the opt-in to more than 48 KB of dynamic shared memory is a per-device attribute of a kernel
-template <class Kernel>
-static cudaError_t allow_smem(Kernel kernel, int smem, bool (&done)[64]) {
+// Whether a launch of n blocks overlaps the end of one like it in front of it (see wait_for_previous_launch).  Blocks that find no place
+// beside that launch's go where its blocks end first, so that some SMs hold more of them than others.  That costs more than it gives unless
+// all find a place beside it, or the launch fills every SM's places as it is.  us per recorded step, behind one another / overlapped (rows
+// per head without the window of 512, chunks of 128):
+//   head_dim 64    strands: 8 heads x 1100 rows (96 of 444 places) 8.43 / 8.23, 16 x 1900 (256 of 444) 9.60 / 9.90, 16 x 3900 (384 of 444)
+//                  11.68 / 11.21, 32 x 1900 (512 of 740) 10.74 / 11.52, 16 x 7800 (640 of 740) 16.64 / 15.94; segments: 64 x 1900 (256 of 592)
+//                  16.27 / 15.90, 64 x 3900 (384 of 592) 17.72 / 19.11, 128 x 1900 (512 of 592) 17.97 / 17.45, 128 x 3900 (768) 31.97 / 31.48
+//   head_dim 128   strands: 16 heads x 1100 rows (192 of 444) 11.29 / 10.91, 16 x 1900 (256 of 444) 11.97 / 12.58, 16 x 3900 (384 of 444) 14.74 /
+//                  14.32; segments: 32 x 1900 (128 of 296) 16.72 / 16.53, 64 x 1100 (192 of 296) 22.24 / 21.74, 128 x 3900 (768) 52.28 / 51.71
+struct Places { int sms, per_sm; };
+static bool overlaps(long long n, const Places& at) {
+    return 2 * n <= (long long)at.sms * at.per_sm || n > (long long)at.sms * (at.per_sm - 1);
+}
+
+// The opt-in to more than 48 KB of dynamic shared memory is a per-device attribute of a kernel; the blocks that fit beside one another are
+// counted with it.
+static cudaError_t prepare_kernel(void (*kernel)(const DecodeParams), int smem, Places (&known)[64], Places& at) {
     int dev = -1;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64 || !done[dev]) {
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
-    }
-    return e;
+    const bool kept = dev >= 0 && dev < 64;
+    at = kept ? known[dev] : Places{};
+    if (at.sms > 0 && at.per_sm > 0) return cudaSuccess;
+    if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&at.sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&at.per_sm, kernel, kDecThreads, (size_t)smem)) != cudaSuccess) return e;
+    if (kept) known[dev] = at;
+    return cudaSuccess;
 }
 
-static cudaError_t launch_overlapped(void (*kernel)(const DecodeParams), const DecodeParams& p, dim3 grid, int smem, cudaStream_t st) {
+static cudaError_t launch(void (*kernel)(const DecodeParams), const DecodeParams& p, dim3 grid, int smem, Places (&known)[64], cudaStream_t st) {
+    Places at;
+    if (const cudaError_t e = prepare_kernel(kernel, smem, known, at)) return e;
     cudaLaunchAttribute attr = {};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
@@ -692,29 +712,25 @@ static cudaError_t launch_overlapped(void (*kernel)(const DecodeParams), const D
     cfg.dynamicSmemBytes = (size_t)smem;
     cfg.stream = st;
     cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = overlaps((long long)grid.x * grid.y * grid.z, at) ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, p);
 }
 
 template <int D, bool STEP, bool BOTH>
 static cudaError_t launch_strands(const DecodeParams& p, dim3 grid, cudaStream_t st) {
-    static bool done[64] = {};
-    const cudaError_t e = allow_smem(decode_strand_kernel<D, STEP, BOTH>, strand_smem<D, BOTH>(), done);
-    if (e != cudaSuccess) return e;
+    static Places known[64] = {};
     grid.x *= kDecWarps;
-    return launch_overlapped(decode_strand_kernel<D, STEP, BOTH>, p, grid, strand_smem<D, BOTH>(), st);
+    return launch(decode_strand_kernel<D, STEP, BOTH>, p, grid, strand_smem<D, BOTH>(), known, st);
 }
 
 template <int D, bool STEP>
 static cudaError_t launch_decode(const DecodeParams& p, dim3 grid, cudaStream_t st) {
-    cudaError_t e;
     const long long segments = (long long)grid.x * grid.y * grid.z;
     if (use_strands(D, segments, grid.x, p.nrep))
         return use_both(D, segments, grid.x) ? launch_strands<D, STEP, true>(p, grid, st) : launch_strands<D, STEP, false>(p, grid, st);
     constexpr int smem = kDecWarps * kDecStages * 2 * kTileTok * D * 2;
-    static bool done[64] = {};
-    if ((e = allow_smem(decode_kernel<D, STEP>, smem, done)) != cudaSuccess) return e;
-    return launch_overlapped(decode_kernel<D, STEP>, p, grid, smem, st);
+    static Places known[64] = {};
+    return launch(decode_kernel<D, STEP>, p, grid, smem, known, st);
 }
 
 static size_t decode_counter_bytes(int B, int Hkv) { return align_up((size_t)B * Hkv * sizeof(int32_t), 256); }

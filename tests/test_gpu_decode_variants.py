@@ -222,3 +222,48 @@ def test_steps_recorded_back_to_back(B, C, SW, N, D, kernel):
         for x, y in zip(want + [a._buf_k, a._buf_v, a._buf_valid, a.size_global_kv, a.size_local_kv, a._state],
                         got + [b._buf_k, b._buf_v, b._buf_valid, b.size_global_kv, b.size_local_kv, b._state]):
             assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize('B,rows,D,blocks,overlap', [(2, 1900, 64, 256, False), (2, 3900, 64, 384, True), (1, 3900, 64, 192, True), (4, 1900, 64, 512, False),
+                                                     (8, 1900, 64, 256, True), (8, 3900, 64, 384, False), (16, 1900, 64, 512, True),
+                                                     (2, 1100, 128, 192, True), (2, 1900, 128, 256, False), (2, 3900, 128, 384, True), (4, 1900, 128, 128, True),
+                                                     (8, 1100, 128, 192, True), (16, 1900, 128, 512, True)])
+def test_which_recorded_steps_overlap(B, rows, D, blocks, overlap):
+    """The edge between two recorded steps: programmatic where the launches overlap, full where the second starts behind the first (the
+    rule of csrc/decode.cu, for 148 SMs).  Outputs, cache and counters equal those of steps that are waited for either way."""
+    import ctypes
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip('the numbers of blocks are for 148 SMs')
+    Hkv, C, SW, steps = 8, 128, 512, 6
+    Hq = 4 * Hkv
+    g = torch.Generator(device=dev()).manual_seed(rows)
+    k, v = (torch.randn(B, Hkv, rows, D, generator=g, device=dev()).bfloat16() for _ in range(2))
+    roles = torch.full((B, Hkv, -(-rows // C)), GLOBAL, dtype=torch.uint8, device=dev())
+    a, b = (make_cache(k, v, roles, C, SW) for _ in range(2))
+    ins = [tuple(torch.randn(B, h, 1, D, generator=g, device=dev()).bfloat16() for h in (Hq, Hkv, Hkv)) for _ in range(steps)]
+    r = torch.randint(0, 3, (B, Hkv), generator=g, device=dev()).to(torch.uint8)
+    want, got = ([torch.empty_like(q) for q, _, _ in ins] for _ in range(2))
+    for c in (a, b):
+        c.prepare_static_decode(22, Hq, D)
+    splits = -(-(a._static_bound + C) // 1024)
+    assert B * Hkv * splits * (1 if kernel_of(a, Hq, D, bound=a._static_bound, fill=C - 1) == 'segments' else 4) == blocks
+    for (q, kn, vn), o in zip(ins, want):
+        a.decode_step_static(q, kn, vn, r, o)
+        torch.cuda.synchronize()
+    graph, side = torch.cuda.CUDAGraph(keep_graph=True), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        graph.capture_begin()
+        for (q, kn, vn), o in zip(ins, got):
+            b.decode_step_static(q, kn, vn, r, o, recording=True)
+        graph.capture_end()
+    # an edge's data: from_port, to_port, type (1: programmatic), five reserved bytes
+    n, nodes, data8 = ctypes.c_size_t(steps), [(ctypes.c_void_p * steps)() for _ in range(2)], (ctypes.c_uint8 * (8 * steps))()
+    assert ctypes.CDLL('libcuda.so.1').cuGraphGetEdges_v2(ctypes.c_void_p(graph.raw_cuda_graph()), *nodes, data8, ctypes.byref(n)) == 0
+    assert [data8[8 * i + 2] for i in range(n.value)] == [int(overlap)] * (steps - 1)
+    graph.instantiate()
+    graph.replay()
+    torch.cuda.synchronize()
+    for x, y in zip(want + [a._buf_k, a._buf_v, a._buf_valid, a.size_global_kv, a.size_local_kv, a._state],
+                    got + [b._buf_k, b._buf_v, b._buf_valid, b.size_global_kv, b.size_local_kv, b._state]):
+        assert torch.equal(x, y)
