@@ -131,3 +131,31 @@ def test_far_chunks_of_a_call_over_a_cache(C):
         check_status(dev())
         assert_close_attn(o, whole[:, :, s])
         pos += n
+
+
+@pytest.mark.parametrize('D', [64, 128, 256])
+@pytest.mark.parametrize('Hq,Hkv', [(4, 2), (3, 1)])
+@pytest.mark.parametrize('C,N,p_global', [(128, 1100, 1.0), (32, 900, 1.0), (24, 900, 1.0), (16, 1500, 0.4), (1, 2048, 0.2)])
+def test_rows_whose_maximum_grows_in_every_tile(D, Hq, Hkv, C, N, p_global):
+    """Keys that grow along the sequence: the reference maximum of a row moves in every tile for one query head of a pair, in every second
+    one for the other, so that O is rescaled again and again behind the P.V of the tile in front (chunks of a multiple of 32 tokens and
+    others, gathered tiles, items of one and of two heads)."""
+    SW = C * max(1, 200 // C)
+    q, k, v = inputs(1, Hq, Hkv, N, D, seed=N + D, sigma=0.5)
+    per_tile = 12.0                                               # growth of the scores, in powers of two
+    slope = torch.where(torch.arange(Hq) % 2 == 0, 1.0, 0.45).view(1, -1, 1, 1)
+    q = (q + slope).bfloat16().float()
+    k = (k + (torch.arange(N) * (per_tile / 128 * 0.6931 / D ** 0.5)).view(1, 1, -1, 1)).bfloat16().float()
+    roles = orc.make_roles(1, Hkv, -(-N // C), p_global, 0.0, seed=C)
+    if p_global == 1.0:
+        # how often the kernel's rule (a growth of more than 8) moves the reference of a row that sees all keys up to its own
+        s = torch.einsum('hqd,hkd->hqk', q[0], k[0].repeat_interleave(Hq // Hkv, 0)) * (D ** -0.5 * 1.4427)
+        s.masked_fill_(torch.ones(N, N, dtype=torch.bool).triu(1), float('-inf'))
+        tops = torch.stack([t.amax(-1) for t in s.split(128, -1)], -1)
+        ref, moves = tops[..., 0], torch.zeros(Hq, N)
+        for j in range(1, tops.shape[-1]):
+            move = tops[..., j] > ref + 8
+            ref, moves = torch.where(move, tops[..., j], ref), moves + move
+        tiles = torch.arange(N) // 128
+        assert (moves[0] >= tiles - 1).float().mean() > 0.9 and (moves[1] >= tiles // 2 - 1).float().mean() > 0.9 and (moves[1] < tiles).float().mean() > 0.5
+    assert_close_attn(run_prefill(q, k, v, roles, C, SW), orc.prefill_attention(q, k, v, roles, C, SW))
