@@ -189,7 +189,7 @@ def test_large_recorded_steps_replay(B, C, SW, N, D):
         assert torch.equal(x, y)
 
 
-@pytest.mark.parametrize('B,C,SW,N,D,kernel', [(1, 1, 32, 700, 64, 'strands'), (2, 4, 64, 1010, 128, 'strands'), (2, 64, 128, 1100, 128, 'strands'),
+@pytest.mark.parametrize('B,C,SW,N,D,kernel', [(1, 1, 32, 700, 64, 'strands'), (2, 4, 64, 1010, 128, 'strands'), (2, 64, 128, 1142, 128, 'strands'),
                                                (12, 4, 64, 900, 128, 'segments'), (26, 1, 32, 1500, 64, 'segments')])
 def test_steps_recorded_back_to_back(B, C, SW, N, D, kernel):
     """Steps whose launches overlap (nothing between them in the graph): outputs, cache bytes and counters of steps that are waited for
@@ -205,6 +205,7 @@ def test_steps_recorded_back_to_back(B, C, SW, N, D, kernel):
         assert kernel_of(c, Hq, D, bound=c._static_bound, fill=C - 1).startswith(kernel)
     want, got = ([torch.empty_like(q) for q, _, _ in ins] for _ in range(2))
     graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    assert N % C + steps >= C                                     # the first replay completes a chunk
     for again in range(2):
         for (q, kn, vn), r, o in zip(ins, rs, want):
             a.decode_step_static(q, kn, vn, r, o)
@@ -222,6 +223,7 @@ def test_steps_recorded_back_to_back(B, C, SW, N, D, kernel):
         for x, y in zip(want + [a._buf_k, a._buf_v, a._buf_valid, a.size_global_kv, a.size_local_kv, a._state],
                         got + [b._buf_k, b._buf_v, b._buf_valid, b.size_global_kv, b.size_local_kv, b._state]):
             assert torch.equal(x, y)
+        assert a.chunk_fill_size == b.chunk_fill_size == (N + (again + 1) * steps) % C == int(b._state[4])
 
 
 @pytest.mark.parametrize('B,rows,D,blocks,overlap', [(2, 1900, 64, 256, False), (2, 3900, 64, 384, True), (1, 3900, 64, 192, True), (4, 1900, 64, 512, False),
