@@ -387,8 +387,8 @@ __global__ void __launch_bounds__(kDecThreads) decode_kernel(const DecodeParams 
 // a quarter of the columns of O.  The arithmetic on every value is the one of decode_kernel in the same order -- the running
 // maximum, the row sum and each accumulator see the strand's tiles in sequence, strands and segments are combined in the same
 // two steps -- so that a head's output does not depend on which of the two kernels the size of the batch selects.
-// One launch in a graph of 20, us, decode_kernel / strands, four query heads per kv-head, 2900 rows per head, head_dim 128: 24
-// segments 21.8 / 10.9, 96 21.9 / 13.4; head_dim 64: 24 segments 18.2 / 8.9, 144 18.8 / 11.8 (lines: use_strands).  What is left of a
+// One launch in a graph of 20, us, decode_kernel / strands, four query heads per kv-head, 2800 rows per head, head_dim 128: 24
+// segments 18.9 / 10.8, 96 19.3 / 13.1; head_dim 64: 24 segments 16.1 / 8.6, 144 16.5 / 11.7 (lines: use_strands).  What is left of a
 // short launch (10 us) is a chain of latencies: sizes, copies, scores, partial results, ticket, combination.
 constexpr int kStrandTiles = kSeg / kTileTok / kDecWarps;
 constexpr int kStrandTilesPerWarp = kStrandTiles / kDecWarps;
@@ -652,13 +652,15 @@ __global__ void __launch_bounds__(kDecThreads) decode_strand_kernel(const Decode
 }
 
 // Launches (segments in all, `splits` of them per (batch, kv-head)) in which every strand gets its own block.  Time of decode_kernel
-// over that of strands, 1 / 2 / 4 / 8 query heads per kv-head, on both sides of the lines:
-//   head_dim 64    1 split: 160 segments 1.02 / 1.02 / 1.03 / 1.02, 192 0.72 / 0.73 / 0.73 / 0.73;  8 splits: 160 1.12 / 1.14 / 1.21 / 1.26,
-//                  192 0.95 / 0.91 / 0.97 / 1.07;  16 splits: 96 1.11 / 1.09 / 1.12 / 1.26, 112 0.95 / 0.93 / 1.02 / 1.14;
-//                  24 splits, 72 segments: 1.01 / 0.94 / 1.04 / 1.24;  48 splits, 96: 0.72 / 0.67 / 0.79 / 1.10
-//   head_dim 128   1 split: 72 segments 1.00 / 1.02 / 1.02 / 0.99, 80 0.94 / 0.94 / 0.96 / 0.92;  2 to 8 splits: 96 segments 1.11 to 1.79, 112
-//                  0.73 to 1.17;  16 splits: 96 1.05 / 1.09 / 1.27 / 1.24;  24 splits: 96 0.95 / 1.04 / 1.29 / 1.21;  32 splits: 96
-//                  0.85 / 0.98 / 1.24 / 1.16;  96 splits: 96 0.60 / 0.80 / 1.21 / 1.11
+// over that of strands in a graph of 20 (each of them overlapping where overlaps() says so), 1 / 2 / 4 / 8 query heads per kv-head, on both
+// sides of the lines:
+//   head_dim 64    1 split: 160 segments 1.19 / 1.18 / 1.19 / 1.19, 192 0.85 / 0.84 / 0.87 / 0.87;  8 splits: 160 1.10 / 1.14 / 1.23 / 1.31,
+//                  192 0.92 / 0.92 / 0.98 / 1.10;  16 splits: 96 0.99 / 0.97 / 1.04 / 1.23, 112 1.01 / 0.96 / 1.00 / 1.09;
+//                  24 splits, 72 segments: 0.89 / 0.83 / 0.98 / 1.21;  48 splits, 96: 0.65 / 0.63 / 0.76 / 1.07
+//   head_dim 128   1 split: 72 segments 1.06 / 1.06 / 1.08 / 1.06, 96 1.03 / 1.04 / 1.05 / 1.02;  4 and 8 splits: 96 segments 1.08 to 1.39, 112
+//                  0.83 to 1.14;  16 splits: 96 0.98 / 1.07 / 1.28 / 1.31;  24 splits: 96 0.93 / 1.04 / 1.36 / 1.38;  48 splits: 96 0.77 /
+//                  0.94 / 1.32 / 1.31
+// Recorded steps (4 query heads): the same lines but for head_dim 64 with 8 splits, where 112 and 144 segments are at 0.96 and 0.95.
 // One split needs no combination in decode_kernel; with many splits the last block of a head combines four times as many
 // partial results, which more query heads make up for (decode_kernel goes over them head by head).
 constexpr int max_strand_segments(int D) { return D == 64 ? 160 : 96; }
@@ -666,8 +668,9 @@ static bool use_strands(int D, long long segments, int splits, int nrep) {
     if (D == 64) return segments <= (splits <= 12 ? max_strand_segments(64) : 96) && splits <= (nrep < 8 ? 16 : 48);
     return segments <= (splits == 1 ? 72 : max_strand_segments(128)) && splits <= (nrep == 1 ? 16 : nrep < 4 ? 24 : 96);
 }
-// V gets slots of its own while all strands fit on the chip at once (148 SMs, one block each at head_dim 128, three at 64): 3 to 12 %
-// faster at 64; at 128 2 % up to 3 splits, but 4 to 14 % slower at 4 and 16 to 32 % at 16 (8 to 32 segments).
+// V gets slots of its own while all strands fit on the chip at once (148 SMs, one block each at head_dim 128, three at 64).  Time of
+// strands with V in the place of K over this, 8 to 36 segments: head_dim 64 1.02 to 1.04 with 2 and 3 splits, 0.99 to 1.00 with 1 and 4, 0.95 to
+// 0.99 with 8, 48 to 96 segments 0.92 to 1.05; head_dim 128 up to 3 splits 0.98 to 1.00, recorded steps 1.00 to 1.03, with 4 splits 0.82 to 0.93.
 static bool use_both(int D, long long segments, int splits) { return D == 64 ? segments <= 111 : segments <= 37 && splits <= 3; }
 
 // Whether a launch of n blocks overlaps the end of one like it in front of it (see wait_for_previous_launch).  Blocks that find no place

@@ -2,7 +2,7 @@
 // multiple of four.  Included by prefill_sm100.cu after its helpers.
 //
 // A work item = one 128-row query tile x one kv-head x FOUR query heads of its group: CTA c of the pair owns heads
-// 2c and 2c + 1 (head slots 0 and 1, as in the single-CTA kernel) with their Q tiles, score / P / O columns and softmax
+// 2c and 2c + 1 (head slots 0 and 1) with their Q tiles, score / P / O columns and softmax
 // warps.  What the pair shares is every K / V tile: each CTA loads only HALF of it -- K rows [64 c, 64 c + 64) (half of the
 // N dimension of S = Q.K^T) and V columns [64 c, 64 c + 64) (half of the N dimension of O += P.V) -- and the MMAs are
 // issued by the leader CTA with cta_group::2: one instruction runs both SMs' tensor cores, each on its own A operand (its
@@ -22,9 +22,8 @@ namespace nats {
 // passes column col = first column + i; bit i of lane r's result = column i is visible to row r.  A column is visible to the
 // rows at positions col .. lim[col / C], so a lane has its column's bits for all 32 rows from one coalesced load, and five
 // exchange steps transpose the 32 x 32 bit matrix.  That is ~60 instructions for any chunk size; a loop over the chunks of a
-// tile pays a dependent load and the mask words for each of them: prompt of 8192 tokens, 32 / 8 heads, one role per token
-// 6.63 -> 0.91 ms, forward of 8 x 4096 tokens with chunks of 16 0.57 -> 0.51 ms.  Where 32 columns always lie in one chunk
-// the compare of visible_bits_coarse is cheaper (32k tokens, chunks of 128: 3 % slower with the transposition).
+// tile pays a dependent load and the mask words for each of them.  Where 32 columns always lie in one chunk the compare of
+// visible_bits_coarse is cheaper.
 __device__ __forceinline__ uint32_t visible_bits(const int32_t* __restrict__ lim, int col, int q0, int Nkv, int C, int c_shift, int lane) {
     const int l = col < Nkv ? lim[c_shift >= 0 ? col >> c_shift : col / C] : -1;
     const int lo = max(col - q0, 0), hi = min(l - q0, 31);

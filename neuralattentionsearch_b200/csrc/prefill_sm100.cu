@@ -446,16 +446,17 @@ __device__ __forceinline__ bool util_wait(uint32_t bar, uint32_t parity, volatil
 // Per step (kept tile j, head):  S = Q.K_j^T (D / 16 MMAs of N = 128)  ->  the 128-entry score row in registers, S free for the next
 // step's scores  ->  softmax  ->  P (bf16) in columns of its own, free since P.V_{j-1}  ->  O += P.V_j.  Q.K^T needs only free scores,
 // P.V only P: two issuers, each in step order, nothing else orders the MMAs.  (With P over S and a head's P.V_j and Q.K_{j+1}^T queued
-// as one batch a head's chain was softmax, then batch, ~4300 cycles a tile for 2048 of MMAs; now ~3000.)
+// as one batch a head's chain was softmax, then batch, 4317 cycles a tile for 2048 of MMAs; now 2873.)
 //
-// What binds it is instruction fetch before the pipes (of the cycles between two issues of a scheduler its warps spend 1.5 to 2.3 in
-// stalls for instructions, MUFU busy 55 %, tensor pipe 55 %): the warps of both heads stream through a tile's straight-line code
-// at different places, next to the issuer of their scheduler.  So the code is kept short: the heads of an issuer in a rolled loop
-// and waits as a look and a branch (text of <128, false> 74.8 -> 57.7 KB), rows masked by one compare per column with limits that the
-// producer leaves in shared memory, the epilogue in pieces of 32 columns.  us per launch, P over S / the above without the short
-// code / all: 32k tokens 1258 / 1259 / 1075, 2 x 131k 23394 / 22086 / 19370, 8 x 15001 3804 / 3954 / 3257, 8192 tokens with one role
-// per token 179 / 179 / 144, 8 x 4096 with chunks of 16 237 / 262 / 195.  Then one compare per column for limits and diagonal together
-// where 32 columns lie in one chunk (1065 -> 1053, 19600 -> 19130, 3260 -> 3215), MMAs in a loop with FINE (144 -> 142, 195 -> 187).
+// What binds it now is the pipes and what stands between them: MUFU 70 % and tensor pipe 69 % busy on a small case with chunks of 128, 50 % and 25 %
+// with chunks of 16, where masks take as long as a third of the softmax.  Instruction fetch bound it before: the warps of both heads stream
+// through a tile's straight-line code at different places, next to the issuer of their scheduler, and spent 1.5 to 2.4 warps per issue in
+// stalls for instructions (now 0.3).  So the code is kept short: the heads of an issuer in a rolled loop and waits as a look and a branch,
+// rows masked by one compare per column with limits that the producer leaves in shared memory, the epilogue in pieces of 32 columns.
+// us per launch, P over S / the above without the short code / with it: 32k tokens 1258 / 1185 / 1075, 2 x 131k 23394 / 21175 / 19370,
+// 8 x 15001 3804 / 3684 / 3257, 8192 tokens with one role per token 179 / 195 / 144, 8 x 4096 with chunks of 16 237 / 288 / 195.  Then
+// one compare per column for limits and diagonal together where 32 columns lie in one chunk (1065 -> 1053, 19600 -> 19130, 3260 -> 3215),
+// MMAs in a loop with FINE (144 -> 142, 195 -> 187), waits without a look in front of their loop with FINE (142 -> 141, 188 -> 182).
 //
 // FINE: chunks that are not a multiple of 32 keys, or gathered tiles.  Without it the loops carry neither the masks column by column
 // nor the gathered tiles.
@@ -1123,10 +1124,10 @@ struct PrefillWs { size_t lim, tmax, tmin, counter, total, list, before, open, r
 // gathered tiles need (0: this chunk size has none): the lists of the chunks that stay visible and, for chunks below 8 rows,
 // copies of their K and V rows, up to row_cap (a quarter of the sequence) per head, and tails of kTailRows per tile (see
 // far_rows_kernel), copy_rows in all.  The line of a quarter is one of memory: a prompt of 8192 tokens with one role per token, 32 / 8
-// heads of 128, takes with room for an eighth / a quarter / a half 177 / 177 / 178 us at 10 % global, 346 / 229 / 228 at 20 %, 618 / 442 /
-// 336 at 40 %.  From 8 rows on boxes of K and V themselves need no copy: chunks of 8, boxes / copies, 10, 20 and 40 % global, us:
-// head_dim 64 82 / 85, 111 / 111, 174 / 240; 128 172 / 166, 251 / 213, 417 / 405; 256 160 / 122, 256 / 160, 422 / 302.  D = 0: the head_dim is not known, so that
-// there is no room for rows.
+// heads of 128, takes with room for an eighth / a quarter / a half 138 / 138 / 138 us at 10 % global, 251 / 180 / 181 at 20 %, 430 / 324 /
+// 267 at 40 %.  From 8 rows on boxes of K and V themselves need no copy and no room; at head_dim 128 and 256 they are the slower
+// way: 8192 tokens, chunks of 8, 32 / 8 heads, boxes / copies, 10, 20 and 40 % global, us: head_dim 64 116 / 119, 167 / 162, 278 / 317; 128
+// 154 / 129, 234 / 170, 392 / 321; 256 401 / 307, 630 / 405, 1034 / 795.  D = 0: the head_dim is not known, so that there is no room for rows.
 static PrefillWs prefill_ws(int B, int Hkv, int N, int C, int D) {
     PrefillWs w = {};
     const size_t BH = (size_t)B * Hkv, Nc = cdiv(N, C), Nt = cdiv(N, kTile);
@@ -1152,17 +1153,20 @@ static PrefillWs prefill_ws(int B, int Hkv, int N, int C, int D) {
 }
 
 // Whether a call gathers the far chunks: where there is room and the sequence is long enough.  Eight sequences, 16 / 8 heads,
-// window 256, in place / gathered, us: chunks of 1 (head_dim 64) 512 tokens 40 / 42, 1024 91 / 66, 1536 162 / 89, 2000 253 / 115;
-// chunks of 16 (128) 512 38 / 38, 1024 78 / 69, 2000 181 / 133; chunks of 64 (64) 1024 53 / 53, 1536 82 / 79, 2000 112 / 108.
+// window 256, 10 % global, in place / gathered, us: chunks of 1 (head_dim 64) 512 tokens 29 / 34, 1024 62 / 52, 1536 106 / 71, 2000 159 / 92;
+// chunks of 16 (128) 512 29 / 31, 1024 58 / 52, 1536 92 / 70, 2000 134 / 92; chunks of 32 (128) 512 28 / 30, 1024 55 / 52, 1536 86 / 77, 2000
+// 122 / 101, 3000 201 / 144; chunks of 64 (64) 512 29 / 30, 1024 53 / 49, 1536 80 / 72, 2000 106 / 93, 3000 173 / 141.  (For chunks above
+// 16 the line was drawn where an earlier form of the kernel broke even; the present one would gather from 1024 on.)
 static int far_min_rows(int C) { return C <= 16 ? 1024 : 2048; }
 static bool use_far(const PrefillWs& w, size_t workspace_bytes, int C, int q_end, bool pair) {
     return w.total_far != 0 && workspace_bytes >= w.total_far && q_end >= far_min_rows(C) && !pair;
 }
 // How many listed chunks make a tile dense, so that it stays in place.  A gathered tile costs more than one in place where its
-// boxes are many (all chunks global, 24576 tokens, time over the same in place: 64 boxes a tile (chunks of 8, head_dim 256) 2.4, 32
-// (16 / 256, 8 / 128) 1.6 and 1.5, 16 (32 / 256, 16 / 128, 8 / 64) 1.16, 1.09 and 1.11, fewer 1.00 to 1.02), the masks of a tile
-// in place make it about 1/8 dearer; a full tile needs neither masks nor gathering.  Chunks below 8 have no dense tiles: their
-// copies are loaded in boxes of 128 rows, and the test would cost them 3 of 178 us (8192 tokens, one role per token).
+// boxes are many (all chunks global, 12288 tokens, time over the same in place: 64 boxes a tile (chunks of 8, head_dim 256) 2.20, 32
+// (16 / 256, 8 / 128) 1.25 and 1.59, 16 (32 / 256, 16 / 128, 8 / 64) 1.04, 1.16 and 1.25, fewer 1.00 to 1.04), the masks of a tile
+// in place make it up to 1/12 dearer; a full tile needs neither masks nor gathering.  With 100, 90 and 70 % of the chunks global the rule
+// takes at most 4 % longer than the better of gathering all and nothing (eleven pairs of chunk size and head_dim), and is up to 7 %
+// faster than both.  Chunks below 8 have no dense tiles: their copies are loaded in boxes of 128 rows, and the test would cost them time.
 static int far_dense_min(int C, int D) {
     if (C < 8) return 0x7fffffff;
     const int cpt = kTile / C, boxes = cpt * (D / 64);
