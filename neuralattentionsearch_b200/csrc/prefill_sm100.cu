@@ -303,19 +303,6 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     return d;
 }
 
-#ifdef NATS_TRACE
-// development builds only: cycle stamps of one softmax warp and one issuer of CTA 0, summed per phase
-__device__ unsigned long long g_trace[64];
-#define TR_DECL(n) unsigned long long tr_acc[n] = {}; unsigned long long tr_t = clock64(); const bool tr_on = blockIdx.x == 0 && lane == 0
-#define TR_RESET() do { tr_t = clock64(); } while (0)
-#define TR(i) do { const unsigned long long t_ = clock64(); tr_acc[i] += t_ - tr_t; tr_t = t_; } while (0)
-#define TR_DUMP(base, n) do { if (tr_on) for (int i_ = 0; i_ < n; ++i_) g_trace[base + i_] = tr_acc[i_]; } while (0)
-#else
-#define TR_DECL(n)
-#define TR_RESET()
-#define TR(i)
-#define TR_DUMP(base, n)
-#endif
 
 // ---- shared memory --------------------------------------------------------------------------------
 struct ItemHeader {
@@ -622,10 +609,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         uint32_t g = 0;                                 // ring slots filled so far (all items): two per kept tile
         int meta = 0;                                   // entry of the next tile
         const uint64_t pol_kv = l2_policy_evict_last();
-#ifdef NATS_TRACE
-        unsigned long long tr_prod_wait = 0, tr_prod_n = 0;
-        const unsigned long long tr_prod_t0 = clock64();
-#endif
         bool ok = true;
         for (int ic = 0; ok; ++ic) {
             const int slot = ic & 1;
@@ -674,14 +657,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
 #pragma unroll 1
                 for (int kv = 0; kv < 2 && ok; ++kv, ++g) {
                     const int s = g % NS;
-#ifdef NATS_TRACE
-                    const unsigned long long tp0 = clock64();
-#endif
                     if (g >= (uint32_t)NS) ok = util_wait<kRelaxProdNs>(smem_u32(&sm.bar_empty[s]), ((g / NS) & 1) ^ 1, abort_flag, p.status, kErrKvEmpty);
-#ifdef NATS_TRACE
-                    tr_prod_wait += clock64() - tp0;
-                    ++tr_prod_n;
-#endif
                     if (!ok) break;
                     if (kv == 0) {
                         // the ring slots of this K and of the V in front are free: so is the entry (see kMetas)
@@ -723,9 +699,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             }
             if (ok && lane == 0) mbar_arrive(smem_u32(&sm.bar_list_empty[slot]));
         }
-#ifdef NATS_TRACE
-        if (blockIdx.x == 0 && lane == 0) { g_trace[32] = tr_prod_wait; g_trace[33] = tr_prod_n; g_trace[34] = clock64() - tr_prod_t0; }
-#endif
         if (!ok) {
             // given up: let copies that are still in flight land before the shared memory is released
             for (uint32_t x = g > (uint32_t)NS ? g - NS : 0; x < g; ++x)
@@ -747,7 +720,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         uint32_t k = 0;               // steps so far (one score buffer)
         // tiles and items of head slot 0 / 1 so far: slot 1 has been empty in `gap` tiles and `skip` items
         uint32_t gt = 0, na = 0, gap = 0, skip = 0;
-        TR_DECL(8);
         bool ok = true;
         for (int ic = 0; ok; ++ic) {
             const int slot = ic & 1;
@@ -759,20 +731,16 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             if (qk) {
                 for (int j = 0; j < n && ok; ++j) {
                     const uint32_t gk = g + 2 * j;                 // ring index of K_j
-                    TR(0);
                     ok = util_wait(smem_u32(&sm.bar_full[gk % NS]), (gk / NS) & 1, abort_flag, p.status, kErrKvFull);
-                    TR(1);
                     const uint32_t kl = r_lo0 + (gk % NS) * T16;
 #pragma unroll 1
                     for (int h = 0; h < nslots && ok; ++h) {
                         const uint32_t items = na - (h ? skip : 0), tiles = gt + j - (h ? gap : 0);
                         if (j == 0) ok = util_wait(smem_u32(&sm.bar_q_full[h]), items & 1, abort_flag, p.status, kErrQ);
-                        TR(2);
                         // the scores this step overwrites are in the registers of their softmax warps
                         const uint32_t sb = SB == 2 ? h : 0, use = SB == 2 ? tiles : k++;
                         if (ok && use > 0) ok = util_wait(smem_u32(&sm.bar_s_empty[sb]), (use - 1) & 1, abort_flag, p.status, kErrSEmpty);
                         if (!ok) break;
-                        TR(3);
                         tc_fence_after();
                         if (lane == 0) {
                             // S[128 x 128] = Q_h[128 x D] . K_j[128 x D]^T : D/16 MMAs of K = 16
@@ -791,25 +759,20 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                             if (j == n - 1) tc_commit(smem_u32(&sm.bar_q_empty[h]));
                         }
                         __syncwarp();
-                        TR(4);
                     }
                 }
             } else {
                 for (int j = 0; j < n && ok; ++j) {
                     const uint32_t gv = g + 2 * j + 1;             // ring index of V_j
-                    TR(0);
                     ok = util_wait(smem_u32(&sm.bar_full[gv % NS]), (gv / NS) & 1, abort_flag, p.status, kErrKvFull);
-                    TR(1);
                     const uint32_t vl = r_lo0 + (gv % NS) * T16;
 #pragma unroll 1
                     for (int h = 0; h < nslots && ok; ++h) {
                         const uint32_t items = na - (h ? skip : 0), tiles = gt + j - (h ? gap : 0);
                         // the first P.V of an item overwrites O_h: the previous item's epilogue must have read it
                         if (j == 0 && items > 0) ok = util_wait(smem_u32(&sm.bar_o_empty[h]), (items - 1) & 1, abort_flag, p.status, kErrOEmpty);
-                        TR(2);
                         if (ok) ok = util_wait(smem_u32(&sm.bar_p_full[h]), tiles & 1, abort_flag, p.status, kErrPFull);
                         if (!ok) break;
-                        TR(3);
                         tc_fence_after();
                         if (lane == 0) {
                             // O_h[128 x D] (+)= P_j[128 x 128 keys] . V_j[128 x D] : 8 MMAs of K = 16; V is MN-major (D contiguous)
@@ -834,7 +797,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                             if (h == nslots - 1) tc_commit(smem_u32(&sm.bar_empty[gv % NS]));
                         }
                         __syncwarp();
-                        TR(4);
                     }
                 }
             }
@@ -844,7 +806,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             if (nslots == 1) { gap += n; ++skip; }
             if (ok && lane == 0) mbar_arrive(smem_u32(&sm.bar_list_empty[slot]));
         }
-        if (qk) { TR_DUMP(16, 8); } else { TR_DUMP(40, 8); }
     } else if (warp >= 4) {
         // =============================== softmax + epilogue ===============================
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsHigh));
@@ -860,28 +821,21 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         uint32_t gt = 0;                                 // tiles of this head so far
         int metas = 0;                                   // tiles of all items so far, modulo kMetas
         bool ok = true;
-        TR_DECL(12);
-#ifdef NATS_TRACE
-        unsigned long long tr_epi_ld = 0;
-#endif
         for (int ic = 0; ok; ++ic) {
             const int slot = ic & 1;
             ok = warp_wait_short<FINE>(smem_u32(&sm.bar_list_full[slot]), (ic >> 1) & 1, abort_flag, p.status, kErrList);
             if (!ok) break;
             const ItemHeader hd = sm.item[slot];
             if (!hd.valid) break;
-            TR(8);
             if (h < hd.nslots) {
                 const int n = hd.n_kept;
                 const int qpos = p.q_off + hd.t * kTile + row;   // position of this thread's query row in the KV sequence
                 float m_ref = -INFINITY, l_sum = 0.f;
                 int meta = metas;
                 for (int j = 0; j < n; ++j, ++gt) {
-                    TR(0);
                     ok = warp_wait_short<FINE>(smem_u32(&sm.bar_s_full[h]), gt & 1, abort_flag, p.status, kErrSFull);
                     if (!ok) break;
                     tc_fence_after();
-                    TR(1);
                     // the score row of this thread in registers: four loads in flight, one wait; the buffer is then free
                     uint32_t sreg[kTile];
 #pragma unroll
@@ -890,7 +844,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(smem_u32(&sm.bar_s_empty[sb]));
-                    TR(2);
                     // masks: -inf, of which exp2 makes an exact 0
                     const int tile = sm.tile[meta];
                     if (FINE && (tile & kLimits)) {
@@ -952,7 +905,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                         }
                     }
                     const float m_neg = (m_ref == -INFINITY) ? 0.f : -m_ref;
-                    TR(3);
                     // P = exp2(S * scale - m), row sum in fp32, P packed to bf16
                     const uint64_t scale2 = pack2(scale, scale), mneg2 = pack2(m_neg, m_neg);
                     uint64_t ls2 = pack2(0.f, 0.f);
@@ -968,20 +920,17 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                         ls2 = add2(ls2, pack2(p0, p1));
                         pk[i / 2] = pack_bf16(p0, p1);
                     }
-                    TR(4);
                     if (__builtin_expect(!__all_sync(0xffffffffu, pv_done), 0)) {
                         ok = warp_wait_short<FINE>(smem_u32(&sm.bar_o_full[h]), (gt - 1) & 1, abort_flag, p.status, kErrOFull);
                         if (!ok) break;
                     }
                     tc_fence_after();
-                    TR(9);
                     tmem_st32(tP, *reinterpret_cast<const uint32_t(*)[32]>(&pk[0]));
                     tmem_st32(tP + 32, *reinterpret_cast<const uint32_t(*)[32]>(&pk[32]));
                     tc_wait_st();
                     tc_fence_before();
                     __syncwarp();                         // every lane's row of P is in TMEM and fenced
                     if (lane == 0) mbar_arrive(smem_u32(&sm.bar_p_full[h]));
-                    TR(10);
                     {
                         float a, b;
                         unpack2(ls2, a, b);
@@ -989,9 +938,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                     }
                 }
                 // epilogue: O / l -> bf16 -> global; O_h is handed back to the issuer as soon as it sits in registers
-                TR(0);
                 if (ok) ok = warp_wait_short<FINE>(smem_u32(&sm.bar_o_full[h]), (gt - 1) & 1, abort_flag, p.status, kErrOFull);
-                TR(6);
                 if (ok) {
                     tc_fence_after();
                     const float inv = l_sum > 0.f ? 1.f / l_sum : 0.f;
@@ -1012,9 +959,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                             __syncwarp();
                             if (lane == 0) mbar_arrive(smem_u32(&sm.bar_o_empty[h]));
                         }
-#ifdef NATS_TRACE
-                        { const unsigned long long t_ = clock64(); tr_epi_ld += t_ - tr_t; tr_t = t_; }
-#endif
                         if (p.o_f32) {
                             if (qi < p.N) {
                                 float* frow = (float*)p.o + o_at + c0;
@@ -1049,18 +993,11 @@ prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                         }
                     }
                 }
-                TR(7);
-#ifdef NATS_TRACE
-                tr_acc[11] += n;
-#endif
             }
             metas = (metas + hd.n_kept) % Smem::kMetas;
             __syncwarp();
             if (ok && lane == 0) mbar_arrive(smem_u32(&sm.bar_list_empty[slot]));
         }
-#ifdef NATS_TRACE
-        if (warp == 4) TR_DUMP(0, 12);
-#endif
     }
     // ---- teardown ----
     tc_fence_before();
@@ -1498,8 +1435,3 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_prefill_fwd_stat
 
 
 
-#ifdef NATS_TRACE
-extern "C" __attribute__((visibility("default"))) int nats_b200_debug_trace(unsigned long long* host_out) {
-    return cudaMemcpyFromSymbol(host_out, nats::g_trace, sizeof(unsigned long long) * 64) == cudaSuccess ? 0 : 1;
-}
-#endif
