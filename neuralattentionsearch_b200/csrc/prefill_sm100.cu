@@ -178,14 +178,6 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// D[tmem] (+)= A[smem desc] * B[smem desc]; ACC is a compile-time flag so that no predicate has to be computed per MMA
-template <int ACC>
-__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "n"(ACC) : "memory");
-}
 // D[tmem] (+)= A[tmem] * B[smem desc]
 __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
@@ -194,9 +186,9 @@ __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_
         ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
-// The same with the descriptors given as (low word, shared high word): within one kernel only the start address and
-// the leading byte offset (low word) differ between operands, so the issuing thread adds small constants to 32-bit
-// registers instead of carrying 64-bit descriptors around.
+// D[tmem] (+)= A[smem desc] * B[smem desc], and the above, with the descriptors given as (low word, shared high word): within one kernel only
+// the start address and the leading byte offset (low word) differ between operands, so the issuing thread adds small constants to 32-bit
+// registers instead of carrying 64-bit descriptors around.  ACC is a compile-time flag so that no predicate has to be computed per MMA.
 template <int ACC>
 __device__ __forceinline__ void mma_ss_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc) {
     asm volatile(
