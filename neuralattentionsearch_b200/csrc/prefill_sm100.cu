@@ -295,7 +295,6 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     return d;
 }
 
-
 // ---- shared memory --------------------------------------------------------------------------------
 struct ItemHeader {
     int valid;      // 0: no more work; else 1 + the KV tile in front of which the keys are gathered
@@ -1336,7 +1335,6 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_prefill_fwd_stat
                               d_kept_tiles, d_status, stream, d_lse, d_n_visible);
 }
 
-
 extern "C" __attribute__((visibility("default"))) size_t nats_b200_prefill_past_workspace_bytes(int B, int Hkv, int n_kv, int C) {
     if (B <= 0 || Hkv <= 0 || n_kv <= 0 || C <= 0) return 0;
     return nats_b200_prefill_workspace_bytes(B, Hkv, n_kv, C);
@@ -1424,6 +1422,4 @@ extern "C" __attribute__((visibility("default"))) int nats_b200_prefill_fwd_stat
     return nats_b200_prefill_fwd(d_q, d_k, d_v, d_o, d_roles, B, Hq, Hkv, N, D, C, SW, sm_scale, scratch,
                                  nats::kStaticScratchBytes, d_kept_tiles, d_status, stream);
 }
-
-
 
